@@ -1,0 +1,66 @@
+"""The balanced gather of operators without row reuse (csrc/gather.cu, gather_plan.cpp) against an fp64 product.
+
+An fp32 sum of k products in order has a relative error below k * 2^-24 of the sum of the magnitudes; the rows here have
+at most 5 000 nonzeros and random signs, for which the tolerance of tests/common.py leaves an order of magnitude."""
+import numpy as np
+import pytest
+
+from tests import common
+from tile_fusion_b200 import api, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _graph(n, seed, empty=(), hubs=()):
+    """Random rows of 0 .. 9 nonzeros, some rows emptied, some with most columns."""
+    rng = np.random.default_rng(seed)
+    rows = []
+    for r in range(n):
+        k = 0 if r in empty else int(rng.integers(0, 10))
+        rows.append(np.sort(rng.choice(n, size=min(n, k), replace=False)))
+    for r, k in hubs:
+        rows[r] = np.sort(rng.choice(n, size=k, replace=False))
+    ap = np.zeros(n + 1, np.int32)
+    ap[1:] = np.cumsum([len(r) for r in rows])
+    ai = np.concatenate(rows).astype(np.int32)
+    return ap, ai, rng.uniform(-1, 1, len(ai)).astype(np.float32)
+
+
+def _scipy(t, n):
+    import scipy.sparse as sp
+    return sp.csr_matrix((t[2].astype(np.float64), t[1], t[0]), shape=(n, n))
+
+
+# widths: each group size (8, 16, 32 lanes), a second panel, widths that are no multiple of four, one column
+@pytest.mark.parametrize("n_cols", [1, 4, 31, 32, 33, 64, 68, 128, 132, 300])
+def test_gather_chain(built_lib, n_cols):
+    import torch
+    n = 5000
+    # hubs around the lengths at which a row is cut (a multiple of the unit size) and far above
+    t = _graph(n, 3, empty={0, 1, 2, n - 1}, hubs=((5, 5000), (17, 63), (18, 64), (19, 65), (4000, 256), (4001, 513)))
+    f = _graph(n, 4, hubs=((n - 1, 700),))
+    A, F = api.CSRMatrix(n, n, *t), api.CSRMatrix(n, n, *f)
+    c = synth.uniform(3, (n, n_cols))
+    cd = torch.from_numpy(c).cuda()
+    for first, B in ((t, None), (f, F)):
+        want = _scipy(t, n) @ (_scipy(first, n) @ c.astype(np.float64))
+        plan = api.Plan("spmm_spmm", A, B=B, n_cols=n_cols)
+        assert plan.info()["launches"] == 0 and plan.info()["items"] == 0  # no ticket list: the gather was chosen
+        d = torch.full((n, n_cols), float("nan"), device="cuda")
+        plan.spmm_spmm(cd, d)
+        first_bits = d.clone()
+        d.fill_(float("nan"))
+        plan.spmm_spmm(cd, d)  # the counters of cut rows must be back at zero
+        plan.status()
+        assert torch.equal(d, first_bits)  # pieces of a row are added in order: same bits every time
+        common.assert_close(d.cpu().numpy(), want, f"gather N={n_cols}")
+        # operands off the 16-byte grid
+        cu = torch.empty(n * n_cols + 1, device="cuda")[1:].view(n, n_cols).copy_(cd)
+        du = torch.full((n * n_cols + 1,), float("nan"), device="cuda")[1:].view(n, n_cols)
+        plan.spmm_spmm(cu, du)
+        plan.status()
+        assert torch.equal(du, first_bits)
+        dh = np.full((n, n_cols), np.nan, np.float32)
+        plan.spmm_spmm_host(c, dh)
+        assert np.array_equal(dh, d.cpu().numpy())
+        plan.close()

@@ -12,6 +12,7 @@
 #include <string>
 #include <vector>
 
+#include "gather.h"
 #include "gemm_tc_host.h"
 #include "host_stage.h"
 #include "kernels.cuh"
@@ -28,6 +29,12 @@ using tf::fail;
     cudaError_t e__ = (call);                                                                 \
     if (e__ != cudaSuccess)                                                                   \
       return fail(TF_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e__));          \
+  } while (0)
+
+#define TF_TRY(call)              \
+  do {                            \
+    const int rc__ = (call);      \
+    if (rc__ != TF_OK) return rc__; \
   } while (0)
 
 template <class T>
@@ -62,6 +69,41 @@ struct DevCsr {
     if (rc == TF_OK) rc = ai.upload(h.ai, (size_t)h.ap[h.m]);
     if (rc == TF_OK) rc = ax.upload(h.ax, (size_t)h.ap[h.m]);
     return rc;
+  }
+};
+
+// Operator of the balanced gather (gather.cu).
+struct DevGather {
+  bool on = false;
+  int n_units = 0, n_empty = 0, group = 32, panel_w = 128, partial_ld = 0;
+  DevBuf<int> cols;
+  DevBuf<float> vals;
+  DevBuf<int4> units, heavy;
+  DevBuf<int> rows, empty, cnt;
+  DevBuf<float> partial;
+  // n_cols: widest dense operand the operator will meet
+  int build(const tf_csr &A, int n_cols, int sm_count) {
+    group = tfk::gather_group(n_cols);
+    panel_w = 4 * group;
+    tf::GatherPlan g;
+    tf::build_gather_plan(A.m, A.ap, A.ai, A.ax, sm_count * (tfk::kGatherResident / group), g);
+    n_units = (int)g.units.size();
+    n_empty = (int)g.empty_rows.size();
+    partial_ld = (n_cols + 3) / 4 * 4;
+    const int panels = (partial_ld + panel_w - 1) / panel_w;
+    if (!g.rows.empty()) g.rows.push_back(0);  // a group looks one row ahead
+    int rc = cols.upload(reinterpret_cast<const int *>(g.cols.get()), g.n_entries);
+    if (rc == TF_OK) rc = vals.upload(g.vals.get(), g.n_entries);
+    if (rc == TF_OK) rc = units.upload(reinterpret_cast<const int4 *>(g.units.data()), g.units.size());
+    if (rc == TF_OK) rc = heavy.upload(reinterpret_cast<const int4 *>(g.heavy.data()), g.heavy.size());
+    if (rc == TF_OK) rc = rows.upload(g.rows);
+    if (rc == TF_OK) rc = empty.upload(g.empty_rows);
+    if (rc == TF_OK) rc = cnt.alloc(g.heavy.size() * (size_t)panels);
+    if (rc == TF_OK) rc = partial.alloc((size_t)g.n_slots * partial_ld);
+    if (rc != TF_OK) return rc;
+    if (cnt.n) TF_CUDA(cudaMemset(cnt.p, 0, cnt.n * sizeof(int)));
+    on = true;
+    return TF_OK;
   }
 };
 
@@ -131,6 +173,10 @@ struct tf_plan {
       return a;
     }
   } ptile, ctile;
+  // balanced gather: operators without row reuse (graphs); `second` serves both products when B == A
+  DevGather g_first, g_second;
+  int ld_t = 0;              // floats per row of the intermediate: n_cols rounded up to whole float4
+  DevBuf<float> g_pad;       // rows of C of a width that is no multiple of four, padded to ld_t
   size_t dyn_smem = 0;
   int tile_slots = 0;
   bool pipe = false;  // every item of phases 1 and 2 is a gather tile: run them on the tile pipeline
@@ -449,6 +495,28 @@ int run_march(tf_plan &p, const float *C, float *D, int item_begin, int item_end
   return TF_OK;
 }
 
+// The rest of a SpMM-SpMM plan that runs on the balanced gather.
+int make_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &F, const tf_csr &A, const tf_plan_opts &o, int sm_count,
+                     tf_plan **out) {
+  p->ld_t = (p->n_cols + 3) / 4 * 4;
+  int rc = p->g_second.build(A, p->n_cols, sm_count);
+  if (rc == TF_OK && !p->first_is_second) rc = p->g_first.build(F, p->n_cols, sm_count);
+  if (rc == TF_OK) rc = p->inter.alloc((size_t)p->m * p->ld_t);
+  if (rc == TF_OK && p->ld_t != p->n_cols) rc = p->g_pad.alloc((size_t)p->first_cols * p->ld_t);
+  if (rc == TF_OK) rc = zero_state(*p);
+  if (rc != TF_OK) return rc;
+  p->hp.inter_rows = p->m;
+  p->hp.n_prod = (p->first_is_second ? p->g_second : p->g_first).n_units;
+  p->hp.n_cons = p->g_second.n_units;
+  if (o.lattice_march >= 0 && p->n_cols % 4 == 0) {
+    rc = build_march(*p, &F, A, 0, sm_count, {});
+    if (rc != TF_OK) return rc;
+  }
+  p->sm_count = sm_count;
+  *out = p.release();
+  return TF_OK;
+}
+
 // Common plan construction for the two-operator chains.
 int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int n_cols, const tf_plan_opts *opts,
                     const tf_schedule *sched, tf_plan **out) {
@@ -483,12 +551,9 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
   cudaGetDevice(&p->device);
   p->chain = chain; p->mode = o.mode;
   p->m = A->m; p->n_cols = n_cols; p->k_dim = k_dim; p->halo_rows = o.halo_rows;
-  rc = p->second.upload(*A);
-  if (rc != TF_OK) return rc;
   if (F) {
     p->first_cols = F->n;
-    if (F == A) p->first_is_second = true;
-    else { rc = p->first.upload(*F); if (rc != TF_OK) return rc; }
+    p->first_is_second = F == A;
   }
 
   tf::PlanParams pp;
@@ -525,7 +590,8 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
         o.tile_double_buffer <= 0 && n_cols % 4 == 0 && need > 0 && need <= 226 * 1024) {
       const int max_bz = o.tile_max_bz > 0 ? o.tile_max_bz : tf::kDefaultTileMaxBz;
       tf::build_tiling(F->m, F->ap, F->ai, ps, max_bz, tf::kPipeTileRows, pt);
-      tf::build_tiling(A->m, A->ap, A->ai, ps, max_bz, tf::kPipeTileRows, ct);
+      if (pt.tiled && F != A) tf::build_tiling(A->m, A->ap, A->ai, ps, max_bz, tf::kPipeTileRows, ct);
+      else if (pt.tiled) ct = pt;
       if (pt.tiled && ct.tiled) {
         want_pipe = true;
         p->tile_slots = ps;
@@ -546,7 +612,8 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
     const bool dbl = o.tile_double_buffer > 0 || (o.tile_double_buffer == 0 && tf::kDefaultTileDoubleBuffer);
     const int cap = dbl ? slots / 2 : slots;  // half-size tiles leave room for the next chunk's copies
     if (F) tf::build_tiling(F->m, F->ap, F->ai, cap, max_bz, tile_rows, pt);
-    tf::build_tiling(A->m, A->ap, A->ai, cap, max_bz, tile_rows, ct);
+    if (F == A) ct = pt;
+    else tf::build_tiling(A->m, A->ap, A->ai, cap, max_bz, tile_rows, ct);
     if (pt.tiled || ct.tiled) {
       p->dyn_smem = (size_t)slots * 132;  // 128 B of staging + one source row id per slot
       p->tile_slots = slots;
@@ -570,6 +637,13 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
     if (rc != TF_OK) return rc;
     pp.max_ctas = p->grid;
   }
+  // No operator is tiled and nothing asks for the ticket executor's own knobs: the balanced gather runs the chain.
+  if (chain == 0 && F && o.mode == TF_MODE_STREAM && !pt.tiled && !ct.tiled && o.ring_bytes <= 0 && o.halo_rows == 0 &&
+      o.n_boundary == 0 && o.rows_per_block == 0 && o.slack_blocks < 0 && o.ctas_per_sm == 0)
+    return make_gather_plan(p, *F, *A, o, sm_count, out);
+  rc = p->second.upload(*A);
+  if (rc == TF_OK && F && F != A) rc = p->first.upload(*F);
+  if (rc != TF_OK) return rc;
   p->tile_info[0] = pt.bx; p->tile_info[1] = pt.by; p->tile_info[2] = pt.bz; p->tile_info[3] = pt.tiles();
   p->tile_info[4] = ct.bx; p->tile_info[5] = ct.by; p->tile_info[6] = ct.bz; p->tile_info[7] = ct.tiles();
   rc = tf::build_stream_plan(pp, F ? F->ap : nullptr, F ? F->ai : nullptr, A->ap, A->ai, &pt, &ct, p->hp);
@@ -760,16 +834,21 @@ int begin_host_pipe(tf_plan &p, const void *h_in, const void *h_out) {
   return TF_OK;
 }
 
-// Host pipeline: the dense input is copied in row chunks on one stream, the item list runs in segments
-// on a second as soon as the rows a segment reads have arrived, and finished output rows leave on a
-// third.  in_rows x in_cols floats come from h_in; D is m x n_cols.
-int run_host_pipeline(tf_plan &p, tfk::Params &P, const float *h_in, long long in_rows, int in_cols, float *d_in,
-                      float *h_out, float *d_out) {
+int ensure_streams(tf_plan &p) {
   if (!p.s_h2d) {
     TF_CUDA(cudaStreamCreateWithFlags(&p.s_h2d, cudaStreamNonBlocking));
     TF_CUDA(cudaStreamCreateWithFlags(&p.s_run, cudaStreamNonBlocking));
     TF_CUDA(cudaStreamCreateWithFlags(&p.s_d2h, cudaStreamNonBlocking));
   }
+  return TF_OK;
+}
+
+// Host pipeline: the dense input is copied in row chunks on one stream, the item list runs in segments
+// on a second as soon as the rows a segment reads have arrived, and finished output rows leave on a
+// third.  in_rows x in_cols floats come from h_in; D is m x n_cols.
+int run_host_pipeline(tf_plan &p, tfk::Params &P, const float *h_in, long long in_rows, int in_cols, float *d_in,
+                      float *h_out, float *d_out) {
+  TF_TRY(ensure_streams(p));
   const int ns = (int)p.segs.size();
   while ((int)p.ev_in.size() < ns) {
     cudaEvent_t a, b;
@@ -829,11 +908,7 @@ int run_host_pipeline(tf_plan &p, tfk::Params &P, const float *h_in, long long i
 // (host_stage.h).
 int run_host_march(tf_plan &p, const float *h_in, float *d_in, float *h_out, float *d_out) {
   tf_plan::March &M = p.march;
-  if (!p.s_h2d) {
-    TF_CUDA(cudaStreamCreateWithFlags(&p.s_h2d, cudaStreamNonBlocking));
-    TF_CUDA(cudaStreamCreateWithFlags(&p.s_run, cudaStreamNonBlocking));
-    TF_CUDA(cudaStreamCreateWithFlags(&p.s_d2h, cudaStreamNonBlocking));
-  }
+  TF_TRY(ensure_streams(p));
   const int ns = (int)M.slabs.size();
   while ((int)p.ev_in.size() < ns) {
     cudaEvent_t a, b;
@@ -911,6 +986,39 @@ int run_chain(tf_plan &p, tfk::Params &P, cudaStream_t s) {
   if (p.mode == TF_MODE_SCHEDULE) return run_schedule(p, P, s);
   if (p.mode == TF_MODE_UNFUSED) return run_unfused(p, P, s);
   return run_phases(p, P, 1, 2, s);
+}
+
+// out = op * X, both row-major with their own row lengths; vec_in / vec_out: rows start on 16-byte boundaries.
+int run_gather(const DevGather &g, const float *X, int ld_in, bool vec_in, float *Y, int ld_out, bool vec_out, int n_cols,
+               bool relu, cudaStream_t s) {
+  tfk::GatherParams P;
+  std::memset(&P, 0, sizeof(P));
+  P.cols = g.cols.p; P.vals = g.vals.p; P.units = g.units.p; P.rows = g.rows.p; P.heavy = g.heavy.p;
+  P.heavy_cnt = g.cnt.p; P.partial = g.partial.p; P.partial_ld = g.partial_ld;
+  P.dense = X; P.ld_in = ld_in;
+  P.out = Y; P.ld_out = ld_out;
+  P.n_cols = n_cols;
+  P.panel_w = vec_in ? g.panel_w : 128;
+  P.n_units = g.n_units;
+  P.relu = relu ? 1 : 0;
+  TF_CUDA(tfk::launch_rows_fix(g.empty.p, g.n_empty, ld_out, Y, false, s));
+  TF_CUDA(tfk::launch_gather(g.group, vec_in, vec_out, P, s));
+  return TF_OK;
+}
+
+int run_gather_spmm_spmm(tf_plan &p, const float *C, float *D, cudaStream_t s) {
+  const DevGather &f = p.first_is_second ? p.g_second : p.g_first;
+  const float *src = C;
+  int ld = p.n_cols;
+  bool vec = ld % 4 == 0 && aligned(C, 16);
+  if (p.g_pad.n) {
+    TF_CUDA(tfk::launch_pad_rows(C, p.first_cols, p.n_cols, p.ld_t, p.g_pad.p, s));
+    src = p.g_pad.p; ld = p.ld_t; vec = true;
+  }
+  int rc = run_gather(f, src, ld, vec, p.inter.p, p.ld_t, true, vec ? p.ld_t : p.n_cols, false, s);
+  if (rc != TF_OK) return rc;
+  p.launches = p.g_pad.n ? 3 : 2;
+  return run_gather(p.g_second, p.inter.p, p.ld_t, true, D, p.n_cols, p.n_cols % 4 == 0 && aligned(D, 16), p.n_cols, false, s);
 }
 
 int set_device(const tf_plan &p) {
@@ -1023,6 +1131,7 @@ int tf_exec_spmm_spmm(tf_plan *p, const float *C, float *D, void *stream) {
   int rc = set_device(*p);
   if (rc != TF_OK) return rc;
   if (march_usable(*p, C, D)) return run_march(*p, C, D, 0, p->march.n_items, false, (cudaStream_t)stream);
+  if (p->g_second.on) return run_gather_spmm_spmm(*p, C, D, (cudaStream_t)stream);
   tfk::Params P = base_params(*p);
   P.in0 = C; P.out = D;
   return run_chain(*p, P, (cudaStream_t)stream);
@@ -1104,6 +1213,10 @@ int tf_exec_phase(tf_plan *p, int phase, const float *in0, const float *in1, int
   if (phase > 0 && p->chain == 0 && march_usable(*p, in0, D))
     return phase == 1 ? run_march(*p, in0, D, 0, p->march.n_phase1, false, (cudaStream_t)stream)
                       : run_march(*p, in0, D, p->march.n_phase1, p->march.n_items, true, (cudaStream_t)stream);
+  if (p->g_second.on) {  // no exchange: phase 1 is the whole chain
+    p->launches = 0;
+    return phase == 1 ? run_gather_spmm_spmm(*p, in0, D, (cudaStream_t)stream) : TF_OK;
+  }
   tfk::Params P = base_params(*p);
   P.in0 = in0; P.in1 = in1; P.out = D; P.w_transposed = w_transposed; P.relu = relu;
   return run_phases(*p, P, phase, phase, (cudaStream_t)stream);
@@ -1139,6 +1252,21 @@ static int finish_host(tf_plan *p, float *D, size_t count) {
   return tf_plan_status(p, nullptr);
 }
 
+// Graph operators: any row of D may need any row of C, so the call is upload, both products, download; pageable arrays
+// still go through the pinned rings.
+static int run_host_whole(tf_plan &p, const float *C, size_t nin, float *D, size_t nout) {
+  int rc = ensure_streams(p);
+  if (rc == TF_OK) rc = begin_host_pipe(p, C, D);
+  if (rc != TF_OK) return rc;
+  TF_CUDA(p.host_pipe->upload(p.h_in0.p, C, nin * sizeof(float), p.s_run));
+  rc = run_gather_spmm_spmm(p, p.h_in0.p, p.h_out.p, p.s_run);
+  if (rc != TF_OK) return rc;
+  TF_CUDA(p.host_pipe->download(D, p.h_out.p, nout * sizeof(float), p.s_run));
+  TF_CUDA(p.host_pipe->finish());
+  TF_CUDA(cudaStreamSynchronize(p.s_run));
+  return TF_OK;
+}
+
 int tf_spmm_spmm_host(tf_plan *p, const float *C, float *D) {
   if (!p || !C || !D) return fail(TF_ERR_ARG, "tf_spmm_spmm_host: null argument");
   if (p->chain != 0) return fail(TF_ERR_ARG, "tf_spmm_spmm_host: plan was built for another chain");
@@ -1167,6 +1295,14 @@ int tf_spmm_spmm_host(tf_plan *p, const float *C, float *D) {
     if (rc != TF_OK) return rc;
     return tf_plan_status(p, nullptr);
   }
+  if (p->g_second.on && nd * sizeof(float) >= ((size_t)1 << 20)) {
+    const size_t nin = (size_t)p->first_cols * p->n_cols;
+    if (p->h_in0.n < nin) rc = p->h_in0.alloc(nin);
+    if (rc == TF_OK && p->h_out.n < nd) rc = p->h_out.alloc(nd);
+    if (rc == TF_OK) rc = run_host_whole(*p, C, nin, D, nd);
+    if (rc != TF_OK) return rc;
+    return tf_plan_status(p, nullptr);
+  }
   rc = stage_in(p->h_in0, C, (size_t)p->first_cols * p->n_cols, 0);
   if (rc == TF_OK && p->h_out.n < nd) rc = p->h_out.alloc(nd);
   if (rc == TF_OK) rc = tf_exec_spmm_spmm(p, p->h_in0.p, p->h_out.p, nullptr);
@@ -1185,11 +1321,7 @@ int tf_gemm_spmm_host(tf_plan *p, const float *B, const float *W, int w_transpos
     if (p->h_in0.n < nin) rc = p->h_in0.alloc(nin);
     if (rc == TF_OK && p->h_out.n < nd) rc = p->h_out.alloc(nd);
     if (rc != TF_OK) return rc;
-    if (!p->s_run) {
-      TF_CUDA(cudaStreamCreateWithFlags(&p->s_h2d, cudaStreamNonBlocking));
-      TF_CUDA(cudaStreamCreateWithFlags(&p->s_run, cudaStreamNonBlocking));
-      TF_CUDA(cudaStreamCreateWithFlags(&p->s_d2h, cudaStreamNonBlocking));
-    }
+    TF_TRY(ensure_streams(*p));
     rc = stage_in(p->h_in1, W, (size_t)p->k_dim * p->n_cols, p->s_run);  // the weight first, on the stream that uses it
     if (rc != TF_OK) return rc;
     tfk::Params P = base_params(*p);

@@ -1,0 +1,186 @@
+// Balanced gather: out = A * X on CSR operators without row reuse that a tile could hold (power-law graphs).
+//
+// The rows of X that the nonzeros name come from L2 (from HBM where X exceeds it), one row per nonzero, and nothing
+// can be reused but by luck.  What bounds such a product is how many of those row reads are in flight and how evenly
+// they are spread, so the work is cut by nonzeros and not by rows:
+//   * The host cuts the nonzeros into units of about equal work (gather_plan.cpp): whole rows up to `target` nonzeros,
+//     and pieces of the rows that are longer than that.
+//   * A unit is worked on by a group of 8, 16 or 32 lanes, four columns per lane (one float4), so that a narrow X
+//     still moves 512 bytes per warp instruction.  The group walks its nonzeros as one stream: eight row reads are
+//     issued together whatever rows of A they belong to, and a bit in the column id says where a row of A ends.
+//     Nothing waits at the head of a row, no two warps ever wait for each other, and because units are filled up to
+//     whole batches and lanes without a column read the last one again, the loop has no bounds to check (ten
+//     instructions per nonzero; a version that broadcast the entries by shuffles and checked bounds needed 37 and
+//     filled two thirds of the issue slots).
+//   * A piece of a long row leaves its sum in a slot of `partial`; the group that delivers the last piece of the row
+//     adds the slots up in order, so a result does not depend on the order in which groups run.
+// Products of a row are added in CSR order with fused multiply-adds from zero, as in the reference's row loop
+// (SpMM_SpMM.cpp:211-248); only rows that were cut are added in pieces.
+//
+// Measured (R-MAT, n = 200 000, degree 20, both products of a chain): 64 columns 183 us (11.7 TB/s of row reads), where
+// the ticket executor took 784 (58 % of its warps' time at barriers behind long rows); 128 columns 306 us, 14 TB/s, which
+// is what L2 gives.  Eight reads in flight and three CTAs per SM: four CTAs spill (229 us), four reads and five CTAs 193.
+#include <algorithm>
+
+#include "gather.h"
+#include "kernels.cuh"
+
+namespace tfk {
+
+namespace {
+
+constexpr int kGatherThreads = 256;
+constexpr int kBatch = tf::kGatherBatch;
+
+// Four columns of one lane: contiguous (VEC) or 32 apart, the last of them clamped to the last column that exists.
+template <bool VEC>
+__device__ __forceinline__ float4 load_quad(const float *p, int e1, int e2, int e3) {
+  if (VEC) return __ldg(reinterpret_cast<const float4 *>(p));
+  return make_float4(__ldg(p), __ldg(p + e1), __ldg(p + e2), __ldg(p + e3));
+}
+__device__ __forceinline__ void fma_quad(float4 &a, float v, const float4 &x) {
+  a.x = fmaf(v, x.x, a.x); a.y = fmaf(v, x.y, a.y); a.z = fmaf(v, x.z, a.z); a.w = fmaf(v, x.w, a.w);
+}
+
+// G: lanes per group.  VIN: rows of X are read as float4.  VOUT: rows of the result are written as float4.
+template <int G, bool VIN, bool VOUT>
+__global__ void __launch_bounds__(kGatherThreads, 3) gather_kernel(const GatherParams P) {
+  static_assert(!VOUT || VIN, "strided columns are stored one by one");
+  const int lane = threadIdx.x & (G - 1);
+  const int panel = blockIdx.x / P.unit_blocks;
+  const int unit = (blockIdx.x - panel * P.unit_blocks) * (kGatherThreads / G) + threadIdx.x / G;
+  if (unit >= P.n_units) return;
+  const int c0 = panel * P.panel_w, c1 = min(P.n_cols, c0 + P.panel_w);
+  // A lane without a column of its own reads the last one again instead of branching around every load.
+  const int own = c0 + (VIN ? lane * 4 : lane);
+  const int left = c1 - own;  // columns of this lane that exist (VIN: from `own` on; else element e while 32 * e < left)
+  const int col = left > 0 ? own : (VIN ? (c1 - 1) & ~3 : c1 - 1);
+  const int e1 = 32 < left ? 32 : 0, e2 = 64 < left ? 64 : 0, e3 = 96 < left ? 96 : 0;
+  const int4 u = __ldg(P.units + unit);
+  const bool piece = u.w >= 0;
+  const float *src = P.dense + col;
+  const int ld_in = P.ld_in;
+  float *dst = (piece ? P.partial : P.out) + own;
+  const int ld_dst = piece ? P.partial_ld : P.ld_out;
+  const bool relu = P.relu != 0 && !piece;
+  const bool listed = P.rows != nullptr && !piece;
+  int pos = u.x;
+  int row = listed ? __ldg(P.rows + pos) : pos;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+
+  auto put = [&](float *o, bool clamp) {
+    if (clamp) { acc.x = fmaxf(acc.x, 0.f); acc.y = fmaxf(acc.y, 0.f); acc.z = fmaxf(acc.z, 0.f); acc.w = fmaxf(acc.w, 0.f); }
+    constexpr int d = VIN ? 1 : 32;
+    if (VOUT) {
+      if (left > 0) *reinterpret_cast<float4 *>(o) = acc;
+    } else {
+      if (0 < left) o[0] = acc.x;
+      if (d < left) o[d] = acc.y;
+      if (2 * d < left) o[2 * d] = acc.z;
+      if (3 * d < left) o[3 * d] = acc.w;
+    }
+  };
+
+  // columns are read one batch ahead, values with the rows they multiply; all lanes of the group read the same ones
+  const int4 *pc = reinterpret_cast<const int4 *>(P.cols + u.y);
+  const float4 *pv = reinterpret_cast<const float4 *>(P.vals + u.y);
+  int4 nxt[kBatch / 4];
+#pragma unroll
+  for (int q = 0; q < kBatch / 4; ++q) nxt[q] = __ldg(pc + q);
+  for (int b = 0; b < u.z; ++b) {
+    int c[kBatch];
+    float v[kBatch];
+#pragma unroll
+    for (int q = 0; q < kBatch / 4; ++q) {
+      c[4 * q] = nxt[q].x; c[4 * q + 1] = nxt[q].y; c[4 * q + 2] = nxt[q].z; c[4 * q + 3] = nxt[q].w;
+    }
+    float4 x[kBatch];
+#pragma unroll
+    for (int q = 0; q < kBatch; ++q) x[q] = load_quad<VIN>(src + (size_t)(unsigned)(c[q] & 0x7fffffff) * ld_in, e1, e2, e3);
+    pc += kBatch / 4;
+#pragma unroll
+    for (int q = 0; q < kBatch / 4; ++q) {
+      const float4 w = __ldg(pv + q);
+      v[4 * q] = w.x; v[4 * q + 1] = w.y; v[4 * q + 2] = w.z; v[4 * q + 3] = w.w;
+      nxt[q] = __ldg(pc + q);
+    }
+    pv += kBatch / 4;
+#pragma unroll
+    for (int q = 0; q < kBatch; ++q) {
+      fma_quad(acc, v[q], x[q]);
+      if (c[q] < 0) {  // the row (or piece) is complete
+        put(dst + (size_t)row * ld_dst, relu);
+        acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        ++pos;
+        row = listed ? __ldg(P.rows + pos) : pos;  // (one entry more than there are rows, see the host plan)
+      }
+    }
+  }
+  if (!piece) return;
+  // a piece of a long row has been delivered; the group that delivers the last one adds them up
+  const unsigned gmask = G == 32 ? kFull : (((1u << (G & 31)) - 1u) << (threadIdx.x & 31 & ~(G - 1)));
+  const int4 h = __ldg(P.heavy + u.w);
+  __threadfence();
+  __syncwarp(gmask);
+  int last = 0;
+  int *cnt = P.heavy_cnt + (size_t)u.w * P.panels + panel;
+  if (lane == 0) last = atomicAdd(cnt, 1) == h.z - 1;
+  last = __shfl_sync(gmask, last, 0, G);
+  if (!last) return;
+  __threadfence();
+  if (lane == 0) *cnt = 0;  // ready for the next launch
+  const float *ps = P.partial + (size_t)h.y * P.partial_ld + col;
+  for (int s = 0; s < h.z; s += kBatch) {
+    float4 x[kBatch];
+#pragma unroll
+    for (int q = 0; q < kBatch; ++q) {
+      const float *o = ps + (size_t)min(s + q, h.z - 1) * P.partial_ld;
+      x[q] = VIN ? __ldcg(reinterpret_cast<const float4 *>(o)) : make_float4(__ldcg(o), __ldcg(o + e1), __ldcg(o + e2), __ldcg(o + e3));
+    }
+#pragma unroll
+    for (int q = 0; q < kBatch; ++q)
+      if (s + q < h.z) { acc.x += x[q].x; acc.y += x[q].y; acc.z += x[q].z; acc.w += x[q].w; }
+  }
+  put(P.out + own + (size_t)h.x * P.ld_out, P.relu != 0);
+}
+
+__global__ void pad_rows_kernel(const float *__restrict__ src, long long rows, int n_cols, int ld, float *__restrict__ dst) {
+  const long long total = rows * ld;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i / ld;
+    const int c = (int)(i - r * ld);
+    dst[i] = c < n_cols ? __ldg(src + r * n_cols + c) : 0.f;
+  }
+}
+
+typedef void (*GatherFn)(const GatherParams);
+template <int G>
+GatherFn pick(bool vec_out) { return vec_out ? gather_kernel<G, true, true> : gather_kernel<G, true, false>; }
+
+}  // namespace
+
+// (R-MAT n = 500 000, degree 25, 32 columns: 377 us with 8 lanes, 703 with 16, 1 018 with 32.)
+int gather_group(int n_cols) { return n_cols <= 32 ? 8 : (n_cols <= 64 ? 16 : 32); }
+
+cudaError_t launch_gather(int group, bool vec_in, bool vec_out, const GatherParams &p, cudaStream_t s) {
+  if (p.n_units <= 0) return cudaSuccess;
+  GatherFn f;
+  if (!vec_in) { f = gather_kernel<32, false, false>; group = 32; }
+  else if (group == 8) f = pick<8>(vec_out);
+  else if (group == 16) f = pick<16>(vec_out);
+  else f = pick<32>(vec_out);
+  GatherParams q = p;
+  q.panels = (p.n_cols + p.panel_w - 1) / p.panel_w;
+  q.unit_blocks = (p.n_units + kGatherThreads / group - 1) / (kGatherThreads / group);
+  f<<<q.unit_blocks * q.panels, kGatherThreads, 0, s>>>(q);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pad_rows(const float *src, long long rows, int n_cols, int ld, float *dst, cudaStream_t s) {
+  const long long total = rows * ld;
+  if (total <= 0) return cudaSuccess;
+  pad_rows_kernel<<<(int)std::min<long long>((total + 255) / 256, 148LL * 16), 256, 0, s>>>(src, rows, n_cols, ld, dst);
+  return cudaGetLastError();
+}
+
+}  // namespace tfk

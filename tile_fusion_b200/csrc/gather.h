@@ -1,0 +1,70 @@
+// Balanced gather: out = A * X for a CSR operator whose rows share too few columns for gather tiles (graphs).
+// Host plan and launcher; the kernel is in gather.cu.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <memory>
+#include <vector>
+
+namespace tf {
+
+// A unit is what one group of lanes works through: whole consecutive non-empty rows, or one piece of a row that is
+// too long for a group.  {first row (its position in `rows`) or slot of the partial sum, first entry, batches, index
+// into `heavy` or -1}.
+struct GatherUnit {
+  int pos, p0, batches, heavy;
+};
+struct GatherHeavy {
+  int row, first_slot, n_slots, pad;
+};
+constexpr int kGatherBatch = 8;             // entries a group works on together
+constexpr uint32_t kGatherEnd = 0x80000000u;  // on the column id: last entry of a row or of a piece
+
+struct GatherPlan {
+  std::vector<GatherUnit> units;      // pieces of long rows first: they take longest
+  std::vector<GatherHeavy> heavy;
+  std::vector<int> rows;              // non-empty rows in order; left empty when every row has a nonzero
+  std::vector<int> empty_rows;
+  // column | kGatherEnd and value of every nonzero, unit after unit, each unit filled up to whole batches with entries
+  // of value 0 that name its last column again (they follow the unit's last row end, so their sums go nowhere);
+  // one batch more at the end, because a group reads one batch ahead
+  std::unique_ptr<uint32_t[]> cols;
+  std::unique_ptr<float[]> vals;
+  size_t n_entries = 0;
+  int n_slots = 0;
+};
+// `groups`: lane groups resident on the device, which sets how finely the work is cut.
+void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int groups, GatherPlan &out);
+
+}  // namespace tf
+
+namespace tfk {
+
+constexpr int kGatherResident = 768;  // threads of the gather kernel resident per SM
+
+struct GatherParams {
+  const int *cols;      // column | end bit
+  const float *vals;
+  const int4 *units;
+  const int *rows;      // null: row = position
+  const int4 *heavy;
+  int *heavy_cnt;       // per (long row, panel): pieces that have delivered; zero between launches
+  float *partial;       // n_slots x partial_ld
+  const float *dense;
+  float *out;
+  int ld_in, ld_out, partial_ld;
+  int n_cols;           // columns computed
+  int panel_w, panels;  // columns per pass over the units (four per lane of a group)
+  int n_units, unit_blocks;
+  int relu;
+};
+
+// Lanes per group for a dense width: each lane owns four columns.
+int gather_group(int n_cols);
+// vec_in / vec_out: rows of X / of the result start on 16-byte boundaries.
+cudaError_t launch_gather(int group, bool vec_in, bool vec_out, const GatherParams &p, cudaStream_t s);
+// dst[r][0:ld] = src[r][0:n_cols], the rest zero: rows of a width that is no multiple of four made readable as float4.
+cudaError_t launch_pad_rows(const float *src, long long rows, int n_cols, int ld, float *dst, cudaStream_t s);
+
+}  // namespace tfk

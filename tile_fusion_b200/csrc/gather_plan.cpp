@@ -1,0 +1,89 @@
+// Host side of the balanced gather (gather.cu): cutting the nonzeros of an operator into units of about equal work.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "gather.h"
+
+namespace tf {
+
+void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int groups, GatherPlan &out) {
+  out = GatherPlan();
+  const long long nnz = ap[m];
+  const long long cost = nnz + 2LL * m;
+  // One unit per resident group where that gives units of 32 to 256 nonzeros.  Shorter ones spend their time on the three
+  // dependent reads in front of the first product, longer ones leave the device idle at the end (R-MAT n = 200 000,
+  // degree 20, 64 columns, both products: 192 us with at most 128, 183 with 256, 253 with 512).
+  const int target = (int)std::min<long long>(256, std::max<long long>(32, cost / std::max(1, groups)));
+  // A row at least this long is cut.  (Cutting only from twice that on: the same on large graphs, 25.4 instead of 22.7 us
+  // at n = 20 000, where one long row is what the launch waits for.)
+  const int long_row = target;
+  // rows and pieces first (nonzero ranges), entries afterwards
+  struct Range { int pos, j0, j1, heavy; };
+  std::vector<Range> plain, pieces;
+  int pos = 0, open_cost = 0;
+  Range open{0, 0, 0, -1};
+  auto close = [&] {
+    if (open_cost > 0) plain.push_back(open);
+    open_cost = 0;
+  };
+  for (int r = 0; r < m; ++r)
+    if (ap[r + 1] == ap[r]) out.empty_rows.push_back(r);
+  const bool listed = !out.empty_rows.empty();
+  for (int r = 0; r < m; ++r) {
+    const int len = ap[r + 1] - ap[r];
+    if (len == 0) continue;
+    if (listed) out.rows.push_back(r);
+    if (len >= long_row) {
+      close();
+      // pieces of about sqrt(len): the group that adds them up last reads as many partial rows as a piece has gathers
+      const int piece = std::max(target, std::min(512, (int)std::sqrt((double)len)));
+      const int n = (len + piece - 1) / piece;
+      out.heavy.push_back(GatherHeavy{r, out.n_slots, n, 0});
+      for (int k = 0; k < n; ++k)
+        pieces.push_back(Range{out.n_slots++, ap[r] + (int)((long long)len * k / n),
+                               ap[r] + (int)((long long)len * (k + 1) / n), (int)out.heavy.size() - 1});
+    } else {
+      if (open_cost > 0 && open_cost + len + 2 > target) close();
+      if (open_cost == 0) open = Range{pos, ap[r], ap[r], -1};
+      open.j1 = ap[r + 1];
+      open_cost += len + 2;
+    }
+    ++pos;
+  }
+  close();
+  // long rows in order of length, longest first, so that their additions at the end are not what the launch waits for
+  std::stable_sort(pieces.begin(), pieces.end(),
+                   [&](const Range &a, const Range &b) { return out.heavy[a.heavy].n_slots > out.heavy[b.heavy].n_slots; });
+  pieces.insert(pieces.end(), plain.begin(), plain.end());
+
+  out.units.resize(pieces.size());
+  size_t n = 0;
+  for (size_t i = 0; i < pieces.size(); ++i) {
+    const int batches = (pieces[i].j1 - pieces[i].j0 + kGatherBatch - 1) / kGatherBatch;
+    out.units[i] = GatherUnit{pieces[i].pos, (int)n, batches, pieces[i].heavy};
+    n += (size_t)batches * kGatherBatch;
+  }
+  out.n_entries = n + kGatherBatch;
+  out.cols.reset(new uint32_t[out.n_entries]);  // (left uninitialised: every entry is written below)
+  out.vals.reset(new float[out.n_entries]);
+  size_t w = 0;
+  int row = 0;  // plain units come in row order: the row ends inside them are found by walking ap
+  for (const Range &u : pieces) {
+    const int len = u.j1 - u.j0;
+    std::memcpy(&out.cols[w], ai + u.j0, sizeof(int) * (size_t)len);
+    std::memcpy(&out.vals[w], ax + u.j0, sizeof(float) * (size_t)len);
+    if (u.heavy < 0) {
+      while (ap[row + 1] <= u.j0) ++row;
+      for (; row < m && ap[row + 1] <= u.j1; ++row)
+        if (ap[row + 1] > ap[row]) out.cols[w + (ap[row + 1] - 1 - u.j0)] |= kGatherEnd;
+    } else {
+      out.cols[w + len - 1] |= kGatherEnd;
+    }
+    w += len;
+    for (; w % kGatherBatch != 0; ++w) { out.cols[w] = (uint32_t)ai[u.j1 - 1]; out.vals[w] = 0.f; }
+  }
+  for (int k = 0; k < kGatherBatch; ++k, ++w) { out.cols[w] = 0; out.vals[w] = 0.f; }
+}
+
+}  // namespace tf

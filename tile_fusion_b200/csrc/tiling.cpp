@@ -91,6 +91,7 @@ void build_generic_tiling(int m, const int *ap, const int *ai, int slot_cap, int
       for (int j = ap[i]; j < ap[i + 1]; ++j) out.slot[j] = (uint16_t)where[ai[j]];
     }
     staged += (long long)(out.halo.size() - h0);
+    if (2 * staged > ap[m]) { out = Tiling(); return; }  // the reuse can no longer reach 2: on graphs known half-way
     out.tile_row_ptr.push_back((int)out.rows.size());
     out.tile_halo_ptr.push_back((int)out.halo.size());
     ++tile_id;
