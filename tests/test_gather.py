@@ -64,3 +64,25 @@ def test_gather_chain(built_lib, n_cols):
         plan.spmm_spmm_host(c, dh)
         assert np.array_equal(dh, d.cpu().numpy())
         plan.close()
+
+
+def test_infinities_stay_where_they_are(built_lib):
+    """The entries that fill up a unit have value 0 and name the unit's last column again: where that column holds an
+    infinity, their product is no number and must not reach a row, long ones (cut into pieces) included."""
+    import torch
+    n, w = 5000, 32
+    t = _graph(n, 8, hubs=((5, 5000), (40, 333), (41, 65)))
+    ap, ai, ax = t
+    ax = np.abs(ax) + 0.5
+    c = np.abs(synth.uniform(3, (n, w)))
+    c[ai[ap[1:] - 1][::7]] = np.inf  # the last column of every seventh row
+    plan = api.Plan("spmm_spmm", api.CSRMatrix(n, n, ap, ai, ax), n_cols=w)
+    d = torch.empty((n, w), device="cuda")
+    plan.spmm_spmm(torch.from_numpy(c).cuda(), d)
+    plan.status()
+    A = _scipy((ap, ai, ax), n)
+    want = A @ (A @ c.astype(np.float64))
+    got = d.cpu().numpy()
+    np.testing.assert_array_equal(np.isinf(got), np.isinf(want))
+    assert not np.isnan(got).any()
+    plan.close()

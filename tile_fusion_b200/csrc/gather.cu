@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(kGatherThreads, 3) gather_kernel(const GatherP
   if (!last) return;
   __threadfence();
   if (lane == 0) *cnt = 0;  // ready for the next launch
+  acc = make_float4(0.f, 0.f, 0.f, 0.f);  // (the entries that fill up the unit went into it: 0 * infinity)
   const float *ps = P.partial + (size_t)h.y * P.partial_ld + col;
   for (int s = 0; s < h.z; s += kBatch) {
     float4 x[kBatch];
