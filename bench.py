@@ -339,7 +339,7 @@ def run_graph_workload(args):
             "clocks": clk.summary(),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": None, "peak_source": f"of {peak_kind}", "algorithmic_bytes_per_launch": nbytes,
-                         "kernel": "stream_kernel (persistent executor)", "kernel_ms": ms,
+                         "kernel": "gather kernels (and row_gemm_kernel)", "kernel_ms": ms,
                          "gather_bytes_per_step": gather, "gather_gbs": gather / (ms * 1e-3) / 1e9,
                          "gather_note": "one dense row per nonzero through L2 -> SM; random rows, so the HBM figure does not bound "
                                         "this workload: read gather_gbs against the ~13 TB/s L2 -> SM row-gather rate of this GPU"},
@@ -535,7 +535,9 @@ def run_lattice_workload(name, args, ctx, headline):
     threads = plan.info()["threads"]
     kernel = {128: "lattice_march_kernel", 672: "tile_pipeline_kernel"}.get(threads, "stream_kernel")
     if chain == "gemm_spmm" and threads == 128:
-        kernel = "tc_gemm_kernel (dense producer) + lattice_march_kernel"
+        kernel = "row_gemm_kernel (dense product) + lattice_march_kernel"
+    elif chain == "gemm_spmm" and args.mode == "stream" and world == 1:
+        kernel = "row_gemm_kernel (dense product) + gather_kernel"
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": None, "peak_source": f"of {peak_kind}", "algorithmic_bytes_per_launch": bytes_local,
                 "kernel": kernel + (" (persistent fused executor)" if "+" not in kernel else " (two launches per step)"),

@@ -124,8 +124,10 @@ typedef struct {
   int tile_max_bz;        /* gather tiles: most grid planes a tile may span, 0 = default           */
   int tile_double_buffer; /* gather tiles: >0 = tiles sized to half the staging buffer so that the copies of
                              the next column chunk overlap the current one, <0 = full-size tiles, 0 = default */
-  int tensor_cores;       /* GeMM-SpMM dense producer: 0 = tcgen05 3xTF32 when the shape allows
-                             (K % 4 == 0, N % 16 == 0, N <= 256), <0 = always the fp32 CUDA-core tile */
+  int tensor_cores;       /* GeMM-SpMM dense product: 0 = tcgen05 3xTF32, in a launch of its own in front of (or, on
+                             graphs with k < n_cols, behind) the sparse product up to N = 256, inside the ticket executor
+                             where one of its options is given, K % 4 == 0 and N % 16 == 0;
+                             <0 = always the fp32 CUDA-core tile */
   int tile_pipeline;      /* SpMM-SpMM with both operators tiled and no ring requested: 0 = run the tiles on
                              the role-split pipeline (one CTA per SM: staging warps copy the next column
                              chunk while compute warps work on the current one), <0 = never              */
@@ -133,7 +135,7 @@ typedef struct {
                              (every nonzero names the row's own grid point or one of its six neighbours):
                              0 = run the plane-marching kernel, which keeps the intermediate in shared memory,
                              <0 = never (general CSR path).  GeMM-SpMM plans on such an operator use the same
-                             kernel as the consumer of the tensor-core producer's rows (0) or the ticket executor (<0) */
+                             kernel as the consumer of the dense product's rows (0) or the balanced gather (<0) */
   int exchange;           /* tf_multi_plan only: 0 = halo rows are written by the copy engines straight into the
                              neighbours' memory (CUDA IPC) where every rank is a process of its own on one host,
                              else ncclSend / ncclRecv; <0 = always ncclSend / ncclRecv (every rank must say the same) */

@@ -1,0 +1,68 @@
+"""GeMM-SpMM on the dense product of its own launch (csrc/row_gemm.cu) and the balanced gather, in either order.
+
+Bounds on the relative error, beside the tolerance of tests/common.py: shapes of the tensor-core tile (K a multiple of 4, N
+of 16) add K / 8 * 3 sums that are cut off at 2^-23: 2e-6 up to K = 256, as in test_gpu_tc.py.  All others are as exact as
+fp32 FMAs: per eight terms one sum cut off at 2^-23, then K / 8 rounded sums, each of random sign against the rest, and the
+dropped lo * lo terms at 2^-22 of a product: below 2^-22 + 2^-24 * sqrt(K / 8) < 6e-7 up to K = 300."""
+import numpy as np
+import pytest
+
+from tests import common
+from tests.test_gather import _graph, _scipy
+from tile_fusion_b200 import api, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(t, n, k, n_cols, seed, off=0, wt=False, relu=False, plan=None):
+    import torch
+    b, w = synth.uniform(seed, (n, k)), synth.uniform(seed + 1, (k, n_cols))
+    want = _scipy(t, n) @ (b.astype(np.float64) @ w.astype(np.float64))
+    if relu:
+        want = np.maximum(want, 0)
+    plan = plan or api.Plan("gemm_spmm", api.CSRMatrix(n, n, *t), k=k, n_cols=n_cols)
+    bd = torch.empty(n * k + off, device="cuda")[off:].view(n, k).copy_(torch.from_numpy(b))
+    wd = torch.from_numpy(np.ascontiguousarray(w.T) if wt else w).cuda()
+    d = torch.full((n * n_cols + off,), float("nan"), device="cuda")[off:].view(n, n_cols)
+    plan.gemm_spmm(bd, wd, d, w_transposed=wt, relu=relu)
+    plan.status()
+    rel, _ = common.assert_close(d.cpu().numpy(), want, f"{n}x{k}x{n_cols} off={off}")
+    assert rel < (2e-6 if k % 4 == 0 and n_cols % 16 == 0 else 6e-7), rel
+    return plan, b, w, d
+
+
+# rows around a CTA's half tile, a pair's tile and a whole wave of pairs; K and N around the 32-column slices
+@pytest.mark.parametrize("m", [1, 127, 129, 255, 257, 74 * 256 + 1])
+@pytest.mark.parametrize("k,n_cols", [(4, 1), (32, 256), (36, 33), (256, 47), (17, 64), (300, 225)])
+def test_dense_product_sizes(built_lib, m, k, n_cols):
+    """The operator is a scaled permutation, so that D is the dense product."""
+    rng = np.random.default_rng(m + k)
+    t = (np.arange(m + 1, dtype=np.int32), rng.permutation(m).astype(np.int32), rng.uniform(1, 2, m).astype(np.float32))
+    _check(t, m, k, n_cols, 3, wt=(m + k) % 2 == 1, relu=m % 2 == 0)[0].close()
+
+
+@pytest.mark.parametrize("k,n_cols", [(64, 40), (40, 64), (100, 256), (256, 47), (33, 128), (8, 7)])
+def test_graph_in_either_order(built_lib, k, n_cols):
+    n = 3000
+    t = _graph(n, 5, empty={0, 7, n - 1}, hubs=((9, 3000), (11, 257)))
+    plan, b, w, d = _check(t, n, k, n_cols, 3)
+    dh = np.full((n, n_cols), np.nan, np.float32)
+    plan.gemm_spmm_host(b, w, dh)
+    np.testing.assert_array_equal(dh, d.cpu().numpy())
+    if k % 4 or n_cols % 16:  # operands off the 16-byte grid: taken where the shape does not ask for vectors
+        _check(t, n, k, n_cols, 3, off=1, plan=plan)
+    plan.close()
+
+
+@pytest.mark.parametrize("dims,k,n_cols", [((90, 70), 64, 64), ((90, 70), 20, 47), ((31, 30, 12), 100, 32), ((32, 30, 12), 36, 48)])
+def test_grid_host_call_in_pieces(built_lib, dims, k, n_cols):
+    """Host pointers on operators that name rows near their own: the call runs in pieces and gives the same bits."""
+    t = synth.laplacian(dims)
+    n = len(t[0]) - 1
+    plan, b, w, d = _check(t, n, k, n_cols, 3)
+    dh = np.full((n, n_cols), np.nan, np.float32)
+    for _ in range(2):
+        plan.gemm_spmm_host(b, w, dh)
+        np.testing.assert_array_equal(dh, d.cpu().numpy())
+    plan.close()
+    _check(t, n, k, n_cols, 3, relu=True)[0].close()

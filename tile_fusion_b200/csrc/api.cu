@@ -6,6 +6,7 @@
 #include <climits>
 #include <cstring>
 #include <condition_variable>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <thread>
@@ -18,6 +19,7 @@
 #include "kernels.cuh"
 #include "lattice_march.h"
 #include "launch.h"
+#include "row_gemm.h"
 #include "tf_internal.h"
 
 namespace {
@@ -75,22 +77,37 @@ struct DevCsr {
 // Operator of the balanced gather (gather.cu).
 struct DevGather {
   bool on = false;
-  int n_units = 0, n_empty = 0, group = 32, panel_w = 128, partial_ld = 0;
+  int n_units = 0, n_empty = 0, partial_ld = 0;
   DevBuf<int> cols;
   DevBuf<float> vals;
   DevBuf<int4> units, heavy;
   DevBuf<int> rows, empty, cnt;
   DevBuf<float> partial;
-  // n_cols: widest dense operand the operator will meet
-  int build(const tf_csr &A, int n_cols, int sm_count) {
-    group = tfk::gather_group(n_cols);
-    panel_w = 4 * group;
+  // Runs of units in row order for the host-pointer calls, where no row is cut: units [unit_begin, unit_end) read rows
+  // < in_rows of the operand, and with them every row < out_rows of the result is final.
+  struct Seg { int unit_begin, unit_end; long long in_rows, out_rows; };
+  std::vector<Seg> segs;
+  void make_segments(const tf::GatherPlan &g, int m, int n_seg) {
+    const int n = (int)g.units.size();
+    if (!g.heavy.empty() || n < 2 * n_seg) return;
+    long long need = 0;
+    for (int s = 0; s < n_seg; ++s) {
+      const int b = (int)((long long)n * s / n_seg), e = (int)((long long)n * (s + 1) / n_seg);
+      const size_t p1 = e < n ? (size_t)g.units[e].p0 : g.n_entries - tf::kGatherBatch;
+      for (size_t i = g.units[b].p0; i < p1; ++i) need = std::max<long long>(need, (g.cols[i] & ~tf::kGatherEnd) + 1LL);
+      const int pos = e < n ? g.units[e].pos : 0;
+      segs.push_back(Seg{b, e, need, e == n ? m : (g.rows.empty() ? pos : g.rows[pos])});
+    }
+  }
+  // n_cols: width of the dense operand the units are cut for; max_cols: widest one the operator will meet
+  int build(const tf_csr &A, int n_cols, int max_cols, int sm_count, int n_seg = 0) {
     tf::GatherPlan g;
-    tf::build_gather_plan(A.m, A.ap, A.ai, A.ax, sm_count * (tfk::kGatherResident / group), g);
+    tf::build_gather_plan(A.m, A.ap, A.ai, A.ax, sm_count * (tfk::kGatherResident / tfk::gather_group(n_cols)), g);
     n_units = (int)g.units.size();
     n_empty = (int)g.empty_rows.size();
-    partial_ld = (n_cols + 3) / 4 * 4;
-    const int panels = (partial_ld + panel_w - 1) / panel_w;
+    partial_ld = (std::max(n_cols, max_cols) + 3) / 4 * 4;
+    const int panels = (partial_ld + 127) / 128;  // the most any width up to that is read in
+    if (n_seg > 1) make_segments(g, A.m, n_seg);
     if (!g.rows.empty()) g.rows.push_back(0);  // a group looks one row ahead
     int rc = cols.upload(reinterpret_cast<const int *>(g.cols.get()), g.n_entries);
     if (rc == TF_OK) rc = vals.upload(g.vals.get(), g.n_entries);
@@ -177,6 +194,7 @@ struct tf_plan {
   DevGather g_first, g_second;
   int ld_t = 0;              // floats per row of the intermediate: n_cols rounded up to whole float4
   DevBuf<float> g_pad;       // rows of C of a width that is no multiple of four, padded to ld_t
+  bool spmm_first = false;   // GeMM-SpMM on the balanced gather: D = (A B) C instead of A (B C)
   size_t dyn_smem = 0;
   int tile_slots = 0;
   bool pipe = false;  // every item of phases 1 and 2 is a gather tile: run them on the tile pipeline
@@ -184,7 +202,7 @@ struct tf_plan {
   // tensor-core dense producer
   bool use_tc = false;
   int sm_count = 0;
-  DevBuf<float> w_hi, w_lo;  // split, transposed weight [n_cols][k]
+  DevBuf<float> w_hi, w_lo;  // split, transposed weight [n_cols][k] (ticket executor), [row_gemm_pad_n][row_gemm_pad_k] otherwise
   CUtensorMap tm_whi, tm_wlo;
   int tile_info[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // producer bx,by,bz,tiles ; consumer bx,by,bz,tiles
   // plane-marching executor (both operators are star stencils on one grid)
@@ -499,8 +517,8 @@ int run_march(tf_plan &p, const float *C, float *D, int item_begin, int item_end
 int make_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &F, const tf_csr &A, const tf_plan_opts &o, int sm_count,
                      tf_plan **out) {
   p->ld_t = (p->n_cols + 3) / 4 * 4;
-  int rc = p->g_second.build(A, p->n_cols, sm_count);
-  if (rc == TF_OK && !p->first_is_second) rc = p->g_first.build(F, p->n_cols, sm_count);
+  int rc = p->g_second.build(A, p->n_cols, p->n_cols, sm_count);
+  if (rc == TF_OK && !p->first_is_second) rc = p->g_first.build(F, p->n_cols, p->n_cols, sm_count);
   if (rc == TF_OK) rc = p->inter.alloc((size_t)p->m * p->ld_t);
   if (rc == TF_OK && p->ld_t != p->n_cols) rc = p->g_pad.alloc((size_t)p->first_cols * p->ld_t);
   if (rc == TF_OK) rc = zero_state(*p);
@@ -510,6 +528,32 @@ int make_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &F, const tf_csr 
   p->hp.n_cons = p->g_second.n_units;
   if (o.lattice_march >= 0 && p->n_cols % 4 == 0) {
     rc = build_march(*p, &F, A, 0, sm_count, {});
+    if (rc != TF_OK) return rc;
+  }
+  p->sm_count = sm_count;
+  *out = p.release();
+  return TF_OK;
+}
+
+// GeMM-SpMM on the balanced gather.  The two products may be taken in either order, D = A (B C) = (A B) C: the sparse
+// product reads one row of its operand per nonzero, so it is given the narrower one -- B where k < n_cols, else B C.
+// (Rows of B that do not start on 16-byte boundaries would be gathered value by value; then B C comes first.  So it does
+// on grids and bands: with a handful of nonzeros a row there is little to choose, and every consumer gives the same bits.)
+int make_gemm_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &A, const tf_plan_opts &o, bool tiled, int sm_count, tf_plan **out) {
+  p->spmm_first = !tiled && p->k_dim % 4 == 0 && p->k_dim < p->n_cols;
+  const int width = p->spmm_first ? p->k_dim : p->n_cols;
+  p->ld_t = (width + 3) / 4 * 4;
+  const size_t wn = (size_t)tfk::row_gemm_pad_n(p->n_cols) * tfk::row_gemm_pad_k(p->k_dim);
+  int rc = p->g_second.build(A, width, std::max(p->k_dim, p->n_cols), sm_count, tiled ? 16 : 0);
+  if (rc == TF_OK) rc = p->inter.alloc((size_t)p->m * p->ld_t);
+  if (rc == TF_OK) rc = p->w_hi.alloc(wn);
+  if (rc == TF_OK) rc = p->w_lo.alloc(wn);
+  if (rc == TF_OK) rc = zero_state(*p);
+  if (rc != TF_OK) return rc;
+  p->hp.inter_rows = p->m;
+  p->hp.n_cons = p->g_second.n_units;
+  if (tiled && o.lattice_march >= 0 && p->n_cols % 4 == 0) {
+    rc = build_march(*p, nullptr, A, 0, sm_count, {});
     if (rc != TF_OK) return rc;
   }
   p->sm_count = sm_count;
@@ -629,8 +673,8 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
     p->dyn_smem = std::max(p->dyn_smem, (size_t)tfk::tc_smem_bytes_host(n_cols));
     if (o.rows_per_block == 0) pp.rows_per_block = tfk::kTcRowsHost;
     pp.max_block_nnz = pp.rows_per_block * 32;
-    rc = p->w_hi.alloc((size_t)k_dim * n_cols);
-    if (rc == TF_OK) rc = p->w_lo.alloc((size_t)k_dim * n_cols);
+    rc = p->w_hi.alloc((size_t)k_dim * tfk::row_gemm_pad_n(n_cols));  // either producer's form (k_dim is a multiple of four)
+    if (rc == TF_OK) rc = p->w_lo.alloc((size_t)k_dim * tfk::row_gemm_pad_n(n_cols));
     if (rc == TF_OK) rc = tfk::tc_make_map(&p->tm_whi, p->w_hi.p, n_cols, k_dim, n_cols);
     if (rc == TF_OK) rc = tfk::tc_make_map(&p->tm_wlo, p->w_lo.p, n_cols, k_dim, n_cols);
     if (rc == TF_OK) rc = finish_plan(*p, o, sm_count, false);
@@ -641,11 +685,14 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
   if (chain == 0 && F && o.mode == TF_MODE_STREAM && !pt.tiled && !ct.tiled && o.ring_bytes <= 0 && o.halo_rows == 0 &&
       o.n_boundary == 0 && o.rows_per_block == 0 && o.slack_blocks < 0 && o.ctas_per_sm == 0)
     return make_gather_plan(p, *F, *A, o, sm_count, out);
+  p->tile_info[0] = pt.bx; p->tile_info[1] = pt.by; p->tile_info[2] = pt.bz; p->tile_info[3] = pt.tiles();
+  p->tile_info[4] = ct.bx; p->tile_info[5] = ct.by; p->tile_info[6] = ct.bz; p->tile_info[7] = ct.tiles();
+  if (chain == 1 && o.mode == TF_MODE_STREAM && o.tensor_cores >= 0 && tfk::row_gemm_supported(n_cols) &&
+      o.ring_bytes <= 0 && o.halo_rows == 0 && o.n_boundary == 0 && o.rows_per_block == 0 && o.slack_blocks < 0 && o.ctas_per_sm == 0)
+    return make_gemm_gather_plan(p, *A, o, ct.tiled, sm_count, out);
   rc = p->second.upload(*A);
   if (rc == TF_OK && F && F != A) rc = p->first.upload(*F);
   if (rc != TF_OK) return rc;
-  p->tile_info[0] = pt.bx; p->tile_info[1] = pt.by; p->tile_info[2] = pt.bz; p->tile_info[3] = pt.tiles();
-  p->tile_info[4] = ct.bx; p->tile_info[5] = ct.by; p->tile_info[6] = ct.bz; p->tile_info[7] = ct.tiles();
   rc = tf::build_stream_plan(pp, F ? F->ap : nullptr, F ? F->ai : nullptr, A->ap, A->ai, &pt, &ct, p->hp);
   if (rc != TF_OK) return rc;
   rc = p->ptile.upload(pt, F ? F->ap : nullptr, F ? F->ax : nullptr, want_pipe);
@@ -908,7 +955,11 @@ int run_host_pipeline(tf_plan &p, tfk::Params &P, const float *h_in, long long i
 // (host_stage.h).
 int run_host_march(tf_plan &p, const float *h_in, float *d_in, float *h_out, float *d_out) {
   tf_plan::March &M = p.march;
-  TF_TRY(ensure_streams(p));
+  if (!p.s_h2d) {
+    TF_CUDA(cudaStreamCreateWithFlags(&p.s_h2d, cudaStreamNonBlocking));
+    TF_CUDA(cudaStreamCreateWithFlags(&p.s_run, cudaStreamNonBlocking));
+    TF_CUDA(cudaStreamCreateWithFlags(&p.s_d2h, cudaStreamNonBlocking));
+  }
   const int ns = (int)M.slabs.size();
   while ((int)p.ev_in.size() < ns) {
     cudaEvent_t a, b;
@@ -988,9 +1039,8 @@ int run_chain(tf_plan &p, tfk::Params &P, cudaStream_t s) {
   return run_phases(p, P, 1, 2, s);
 }
 
-// out = op * X, both row-major with their own row lengths; vec_in / vec_out: rows start on 16-byte boundaries.
-int run_gather(const DevGather &g, const float *X, int ld_in, bool vec_in, float *Y, int ld_out, bool vec_out, int n_cols,
-               bool relu, cudaStream_t s) {
+// Y = op * X, both row-major with their own row lengths; vec_in / vec_out: rows start on 16-byte boundaries.
+tfk::GatherParams gather_params(const DevGather &g, const float *X, int ld_in, float *Y, int ld_out, int n_cols) {
   tfk::GatherParams P;
   std::memset(&P, 0, sizeof(P));
   P.cols = g.cols.p; P.vals = g.vals.p; P.units = g.units.p; P.rows = g.rows.p; P.heavy = g.heavy.p;
@@ -998,11 +1048,19 @@ int run_gather(const DevGather &g, const float *X, int ld_in, bool vec_in, float
   P.dense = X; P.ld_in = ld_in;
   P.out = Y; P.ld_out = ld_out;
   P.n_cols = n_cols;
-  P.panel_w = vec_in ? g.panel_w : 128;
   P.n_units = g.n_units;
+  return P;
+}
+// (a run of units: the caller has seen to the empty rows)
+int run_gather(const DevGather &g, const float *X, int ld_in, bool vec_in, float *Y, int ld_out, bool vec_out, int n_cols,
+               bool relu, cudaStream_t s, int unit_begin = 0, int unit_end = -1) {
+  tfk::GatherParams P = gather_params(g, X, ld_in, Y, ld_out, n_cols);
+  const int group = tfk::gather_group(n_cols);
+  P.panel_w = vec_in ? 4 * group : 128;
   P.relu = relu ? 1 : 0;
-  TF_CUDA(tfk::launch_rows_fix(g.empty.p, g.n_empty, ld_out, Y, false, s));
-  TF_CUDA(tfk::launch_gather(g.group, vec_in, vec_out, P, s));
+  if (unit_end >= 0) { P.units += unit_begin; P.n_units = unit_end - unit_begin; }
+  else TF_CUDA(tfk::launch_rows_fix(g.empty.p, g.n_empty, ld_out, Y, false, s));
+  TF_CUDA(tfk::launch_gather(group, vec_in, vec_out, P, s));
   return TF_OK;
 }
 
@@ -1019,6 +1077,22 @@ int run_gather_spmm_spmm(tf_plan &p, const float *C, float *D, cudaStream_t s) {
   if (rc != TF_OK) return rc;
   p.launches = p.g_pad.n ? 3 : 2;
   return run_gather(p.g_second, p.inter.p, p.ld_t, true, D, p.n_cols, p.n_cols % 4 == 0 && aligned(D, 16), p.n_cols, false, s);
+}
+
+int run_gather_gemm_spmm(tf_plan &p, const float *B, const float *W, int w_transposed, bool relu, float *D, cudaStream_t s) {
+  const int n = p.n_cols, k = p.k_dim;
+  const bool out16 = n % 4 == 0 && aligned(D, 16);
+  if (p.dyn_smem > 0 && !(aligned(B, 16) && aligned(D, 16)))
+    return fail(TF_ERR_ARG, "this plan (gather tiles or tensor-core producer) needs 16-byte aligned dense operands "
+                            "(build the plan with tile_slots < 0 and tensor_cores < 0 otherwise)");
+  TF_CUDA(tfk::row_gemm_split(W, w_transposed, k, n, p.w_hi.p, p.w_lo.p, s));
+  p.launches = 3;
+  if (p.spmm_first) {
+    TF_TRY(run_gather(p.g_second, B, k, aligned(B, 16), p.inter.p, p.ld_t, true, k, false, s));
+    return tfk::row_gemm(p.inter.p, p.m, k, p.ld_t, p.w_hi.p, p.w_lo.p, n, D, n, relu, &p.state.p->error, p.spin_limit, p.sm_count, s);
+  }
+  TF_TRY(tfk::row_gemm(B, p.m, k, k, p.w_hi.p, p.w_lo.p, n, p.inter.p, p.ld_t, false, &p.state.p->error, p.spin_limit, p.sm_count, s));
+  return run_gather(p.g_second, p.inter.p, p.ld_t, true, D, n, out16, n, relu, s);
 }
 
 int set_device(const tf_plan &p) {
@@ -1143,12 +1217,10 @@ int run_gemm_march(tf_plan &p, const float *B, const float *W, int w_transposed,
                    int item_end, bool with_halo, cudaStream_t s) {
   long long launches = 0;
   if (produce) {
-    tfk::Params P = base_params(p);
-    P.in0 = B; P.in1 = W; P.w_transposed = w_transposed;
-    int rc = prepare_tc(p, P, s);
+    TF_CUDA(tfk::row_gemm_split(W, w_transposed, p.k_dim, p.n_cols, p.w_hi.p, p.w_lo.p, s));
+    int rc = tfk::row_gemm(B, p.m, p.k_dim, p.k_dim, p.w_hi.p, p.w_lo.p, p.n_cols, p.inter.p, p.n_cols, false, &p.march.st.p[0].error,
+                           p.spin_limit, p.sm_count, s);
     if (rc != TF_OK) return rc;
-    TF_CUDA(tfk::tc_launch_gemm(P.tm_a, P.tm_whi, P.tm_wlo, p.m, p.k_dim, p.n_cols, p.inter.p, &p.march.st.p[0].error, p.spin_limit,
-                                p.sm_count, s));
     launches = 2;   // weight split + producer
   }
   int rc = run_march(p, p.inter.p, D, item_begin, item_end, with_halo, s);
@@ -1169,6 +1241,7 @@ int tf_exec_gemm_spmm(tf_plan *p, const float *B, const float *W, int w_transpos
   if (rc != TF_OK) return rc;
   if (gemm_march_usable(*p, B, D, relu))
     return run_gemm_march(*p, B, W, w_transposed, D, true, 0, p->march.n_items, false, (cudaStream_t)stream);
+  if (p->g_second.on) return run_gather_gemm_spmm(*p, B, W, w_transposed, relu != 0, D, (cudaStream_t)stream);
   tfk::Params P = base_params(*p);
   P.in0 = B; P.in1 = W; P.out = D; P.w_transposed = w_transposed; P.relu = relu;
   return run_chain(*p, P, (cudaStream_t)stream);
@@ -1215,7 +1288,9 @@ int tf_exec_phase(tf_plan *p, int phase, const float *in0, const float *in1, int
                       : run_march(*p, in0, D, p->march.n_phase1, p->march.n_items, true, (cudaStream_t)stream);
   if (p->g_second.on) {  // no exchange: phase 1 is the whole chain
     p->launches = 0;
-    return phase == 1 ? run_gather_spmm_spmm(*p, in0, D, (cudaStream_t)stream) : TF_OK;
+    if (phase != 1) return TF_OK;
+    return p->chain == 0 ? run_gather_spmm_spmm(*p, in0, D, (cudaStream_t)stream)
+                         : run_gather_gemm_spmm(*p, in0, in1, w_transposed, relu != 0, D, (cudaStream_t)stream);
   }
   tfk::Params P = base_params(*p);
   P.in0 = in0; P.in1 = in1; P.out = D; P.w_transposed = w_transposed; P.relu = relu;
@@ -1226,7 +1301,7 @@ int tf_plan_intermediate(tf_plan *p, float **dev_ptr, long long *rows, int *cols
   if (!p) return fail(TF_ERR_ARG, "tf_plan_intermediate: null plan");
   if (dev_ptr) *dev_ptr = p->inter.p;
   if (rows) *rows = p->hp.inter_rows;
-  if (cols) *cols = p->n_cols;
+  if (cols) *cols = p->ld_t ? p->ld_t : p->n_cols;
   return TF_OK;
 }
 
@@ -1254,15 +1329,59 @@ static int finish_host(tf_plan *p, float *D, size_t count) {
 
 // Graph operators: any row of D may need any row of C, so the call is upload, both products, download; pageable arrays
 // still go through the pinned rings.
-static int run_host_whole(tf_plan &p, const float *C, size_t nin, float *D, size_t nout) {
+static int run_host_whole(tf_plan &p, const float *C, size_t nin, float *D, size_t nout, const std::function<int()> &run) {
   int rc = ensure_streams(p);
   if (rc == TF_OK) rc = begin_host_pipe(p, C, D);
   if (rc != TF_OK) return rc;
   TF_CUDA(p.host_pipe->upload(p.h_in0.p, C, nin * sizeof(float), p.s_run));
-  rc = run_gather_spmm_spmm(p, p.h_in0.p, p.h_out.p, p.s_run);
+  rc = run();
   if (rc != TF_OK) return rc;
   TF_CUDA(p.host_pipe->download(D, p.h_out.p, nout * sizeof(float), p.s_run));
   TF_CUDA(p.host_pipe->finish());
+  TF_CUDA(cudaStreamSynchronize(p.s_run));
+  return TF_OK;
+}
+
+// GeMM-SpMM whose operator names rows near its own (grids, bands): rows of B arrive in pieces, each piece's rows of the
+// dense product follow, then the rows of D that have all they need, which leave while the next piece arrives.
+static int run_host_gemm_gather(tf_plan &p, const float *B, int w_transposed, bool relu, float *D) {
+  const DevGather &g = p.g_second;
+  const int ns = (int)g.segs.size(), n = p.n_cols, k = p.k_dim;
+  while ((int)p.ev_in.size() < ns) {
+    cudaEvent_t a, b;
+    TF_CUDA(cudaEventCreateWithFlags(&a, cudaEventDisableTiming));
+    TF_CUDA(cudaEventCreateWithFlags(&b, cudaEventDisableTiming));
+    p.ev_in.push_back(a); p.ev_run.push_back(b);
+  }
+  TF_TRY(begin_host_pipe(p, B, D));
+  TF_CUDA(tfk::row_gemm_split(p.h_in1.p, w_transposed, k, n, p.w_hi.p, p.w_lo.p, p.s_run));
+  TF_CUDA(tfk::launch_rows_fix(g.empty.p, g.n_empty, n, p.h_out.p, false, p.s_run));
+  long long in_done = 0, out_done = 0;
+  p.launches = 1;
+  for (int s = 0; s < ns; ++s) {
+    const DevGather::Seg &sg = g.segs[s];
+    const long long in_to = s == ns - 1 ? p.m : std::max(in_done, sg.in_rows);
+    if (in_to > in_done) {
+      float *src = p.h_in0.p + in_done * k;
+      TF_CUDA(p.host_pipe->upload(src, B + in_done * k, (size_t)(in_to - in_done) * k * 4, p.s_h2d));
+      TF_CUDA(cudaEventRecord(p.ev_in[s], p.s_h2d));
+      TF_CUDA(cudaStreamWaitEvent(p.s_run, p.ev_in[s], 0));
+      TF_TRY(tfk::row_gemm(src, (int)(in_to - in_done), k, k, p.w_hi.p, p.w_lo.p, n, p.inter.p + in_done * p.ld_t, p.ld_t, false,
+                           &p.state.p->error, p.spin_limit, p.sm_count, p.s_run));
+      in_done = in_to;
+      ++p.launches;
+    }
+    TF_TRY(run_gather(g, p.inter.p, p.ld_t, true, p.h_out.p, n, n % 4 == 0, n, relu, p.s_run, sg.unit_begin, sg.unit_end));
+    ++p.launches;
+    if (sg.out_rows > out_done) {
+      TF_CUDA(cudaEventRecord(p.ev_run[s], p.s_run));
+      TF_CUDA(cudaStreamWaitEvent(p.s_d2h, p.ev_run[s], 0));
+      TF_CUDA(p.host_pipe->download(D + out_done * n, p.h_out.p + out_done * n, (size_t)(sg.out_rows - out_done) * n * 4, p.s_d2h));
+      out_done = sg.out_rows;
+    }
+  }
+  TF_CUDA(p.host_pipe->finish());
+  TF_CUDA(cudaStreamSynchronize(p.s_d2h));
   TF_CUDA(cudaStreamSynchronize(p.s_run));
   return TF_OK;
 }
@@ -1299,7 +1418,8 @@ int tf_spmm_spmm_host(tf_plan *p, const float *C, float *D) {
     const size_t nin = (size_t)p->first_cols * p->n_cols;
     if (p->h_in0.n < nin) rc = p->h_in0.alloc(nin);
     if (rc == TF_OK && p->h_out.n < nd) rc = p->h_out.alloc(nd);
-    if (rc == TF_OK) rc = run_host_whole(*p, C, nin, D, nd);
+    if (rc == TF_OK)
+      rc = run_host_whole(*p, C, nin, D, nd, [&] { return run_gather_spmm_spmm(*p, p->h_in0.p, p->h_out.p, p->s_run); });
     if (rc != TF_OK) return rc;
     return tf_plan_status(p, nullptr);
   }
@@ -1327,6 +1447,21 @@ int tf_gemm_spmm_host(tf_plan *p, const float *B, const float *W, int w_transpos
     tfk::Params P = base_params(*p);
     P.in0 = p->h_in0.p; P.in1 = p->h_in1.p; P.out = p->h_out.p; P.w_transposed = w_transposed; P.relu = relu;
     rc = run_host_pipeline(*p, P, B, p->m, p->k_dim, p->h_in0.p, D, p->h_out.p);
+    if (rc != TF_OK) return rc;
+    return tf_plan_status(p, nullptr);
+  }
+  if (p->g_second.on && nd * sizeof(float) >= ((size_t)1 << 20)) {
+    const size_t nin = (size_t)p->m * p->k_dim;
+    if (p->h_in0.n < nin) rc = p->h_in0.alloc(nin);
+    if (rc == TF_OK && p->h_out.n < nd) rc = p->h_out.alloc(nd);
+    if (rc != TF_OK) return rc;
+    TF_TRY(ensure_streams(*p));
+    TF_TRY(stage_in(p->h_in1, W, (size_t)p->k_dim * p->n_cols, p->s_run));  // the weight first, on the stream that uses it
+    if (!p->g_second.segs.empty()) rc = run_host_gemm_gather(*p, B, w_transposed, relu != 0, D);
+    else
+      rc = run_host_whole(*p, B, nin, D, nd, [&] {
+        return run_gather_gemm_spmm(*p, p->h_in0.p, p->h_in1.p, w_transposed, relu != 0, p->h_out.p, p->s_run);
+      });
     if (rc != TF_OK) return rc;
     return tf_plan_status(p, nullptr);
   }

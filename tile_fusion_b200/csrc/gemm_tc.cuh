@@ -152,7 +152,7 @@ __device__ __forceinline__ bool tc_gemm_rows(const CUtensorMap *tmA, const CUten
     for (int i = tid; i < kTcRows * kTcKSlice; i += NT) {
       const float a = a_hi[i], h = tf32_round(a);
       a_hi[i] = h;
-      a_lo[i] = a - h;
+      a_lo[i] = tf32_round(a - h);  // (the tensor core would cut the last bits off instead)
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> async proxy (MMA) reads
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

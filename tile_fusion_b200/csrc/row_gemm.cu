@@ -1,0 +1,460 @@
+// T = B * W (optionally max(0, .)) for a tall fp32 B on the 5th-generation tensor cores, 3xTF32 inside.
+//
+// The arithmetic is that of gemm_tc.cuh, product by product: every operand is split as x = hi + lo, both rounded to TF32,
+// and hi*hi + hi*lo + lo*hi is accumulated in fp32 in tensor memory.  What differs is that nothing waits for anything it
+// does not need:
+//   * Two CTAs on neighbouring SMs work on one tile of 256 rows with tcgen05.mma.cta_group::2.  Each holds 128 rows of B
+//     and half of the columns of W, so W crosses from L2 once per 256 rows, and the tensor core reads half of it from
+//     each SM's shared memory.  (One CTA with 128 rows and all of W would need 180 bytes per clock of shared memory at
+//     N = 256, 40 % more than there are.)
+//   * A warp keeps the TMA loads of K slices of 32 columns running ahead through a ring of stages, eight warps split
+//     the raw rows, one thread of the even CTA issues the products, four warps drain the accumulator of the tile before
+//     (two accumulators of up to 256 columns in tensor memory) and write it with TMA stores.
+//   * The grid is one pair per two SMs and walks the tiles.
+// The tensor core cuts off what it adds to an accumulator instead of rounding it, so a chain of K / 8 sums drifts (rel.
+// error 2e-6 at K = 256, ten times that of fp32 FMAs).  Widths and depths that the ticket executor's tensor-core tile does
+// not take have always been multiplied with fp32 FMAs; for them the kernel has a second form that is as exact as those:
+// panels of up to 64 columns, an accumulator of its own for each K step of 8 (the small products first), and the four of a
+// slice are read back and added in registers.
+// All waits are bounded: the one that runs out sets the error flag, and every role leaves.
+#include "row_gemm.h"
+
+#include <algorithm>
+#include <string>
+
+#include "gemm_tc.cuh"
+#include "gemm_tc_host.h"
+#include "tf_internal.h"
+
+namespace tfk {
+
+namespace {
+
+constexpr int kRgEpiWarps = 4, kRgSplitWarps = 8;
+constexpr int kRgThreads = 32 * (kRgEpiWarps + kRgSplitWarps + 2);
+constexpr int kRgMaxStages = 5;
+constexpr int kRgPrecisePanel = 64;  // columns: four accumulators, twice, in 512 columns of tensor memory
+constexpr int kRgSmemMax = 227 * 1024;
+constexpr int kRgEpiBytes = kRgEpiWarps * 2 * 32 * 128;  // two 32 x 32 blocks per warp
+
+struct RgShared {
+  unsigned long long raw[kRgMaxStages], split[kRgMaxStages], ready[kRgMaxStages], empty[kRgMaxStages];
+  unsigned long long acc_full[2], acc_empty[2], drained;
+  unsigned tmem_base;
+  int dead;
+};
+
+__host__ __device__ constexpr int rg_stage_bytes(int n) { return 2 * kTcRows * 128 + n * 128; }
+constexpr int rg_stages(int n) {
+  const int s = (kRgSmemMax - 2048 - kRgEpiBytes) / rg_stage_bytes(n);
+  return s < kRgMaxStages ? s : kRgMaxStages;
+}
+static_assert(rg_stages(256) >= 2, "a full-width tile needs two stages");
+
+__device__ __forceinline__ unsigned rg_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void rg_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Arrive on a barrier of this CTA / of the even CTA of the pair.  A release at cluster scope waits for the thread's accesses
+// to reach the other SM, which costs a splitting warp half of its time (N = K = 256, 2.1 M rows: 1 410 us with it); so those
+// arrive in their own CTA, and in the odd CTA one thread that has nothing else to do passes the arrival on.
+__device__ __forceinline__ void rg_arrive(unsigned long long *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+template <bool RELEASE>
+__device__ __forceinline__ void rg_arrive_leader(unsigned long long *bar) {
+  if (RELEASE)
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\t"
+        "mapa.shared::cluster.u32 a, %0, 0;\n\t"
+        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\t"
+        "mapa.shared::cluster.u32 a, %0, 0;\n\t"
+        "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+}
+// Bounded wait that also leaves when another role of the CTA has given up.  CLUSTER: threads of the other CTA arrive too.
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool rg_wait(unsigned long long *bar, unsigned parity, RgShared &s, int limit) {
+  const unsigned a = smem_u32(bar);
+  for (int i = 0; i < limit; ++i) {
+    unsigned done;
+    if (CLUSTER)
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(a), "r"(parity) : "memory");
+    else
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(a), "r"(parity) : "memory");
+    if (done) return true;
+    if (*reinterpret_cast<volatile int *>(&s.dead)) return false;
+  }
+  s.dead = 1;
+  return false;
+}
+__device__ __forceinline__ void rg_mma(unsigned d, unsigned long long da, unsigned long long db, unsigned idesc, unsigned acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
+}
+// Both CTAs' barriers at this offset are arrived on when the products issued so far have been computed.
+__device__ __forceinline__ void rg_commit(unsigned long long *bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                   smem_u32(bar)), "h"((unsigned short)3) : "memory");
+}
+
+// 32 columns of a warp's 32 tensor-memory lanes.  The registers hold them after tcgen05.wait::ld only: rg_loaded keeps the
+// compiler from using them before.
+__device__ __forceinline__ void rg_tmem_load(float (&v)[32], unsigned taddr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
+        "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]),
+        "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),
+        "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+      : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void rg_loaded(float (&v)[32]) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i) asm volatile("" : "+f"(v[i]));
+}
+
+// PRECISE: see above; n_pad <= 64.
+// n_pad: columns of W rounded up to 32 (rows of the split weight beyond n_real are zero).
+template <bool PRECISE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRgThreads, 1)
+row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_whi,
+                const __grid_constant__ CUtensorMap tm_wlo, const __grid_constant__ CUtensorMap tm_out, const RowGemmParams P) {
+  extern __shared__ char dyn[];
+  __shared__ RgShared s;
+  char *smem = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~(uintptr_t)1023);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const unsigned rank = rg_rank();
+  const int N = P.n_pad, half = N / 2, stage_bytes = rg_stage_bytes(N), stages = P.stages;
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  char *epi = smem + stages * stage_bytes;
+
+  if (tid == 0) {
+    for (int i = 0; i < stages; ++i) {
+      mbar_init(&s.raw[i], 1);
+      mbar_init(&s.split[i], kRgSplitWarps);      // (odd CTA)
+      mbar_init(&s.ready[i], kRgSplitWarps + 1);  // (even CTA)
+      mbar_init(&s.empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&s.acc_full[i], 1);
+      mbar_init(&s.acc_empty[i], 2 * kRgEpiWarps);
+    }
+    mbar_init(&s.drained, 1);
+    s.dead = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem_base)), "n"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  rg_cluster_sync();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+  if (warp == kRgEpiWarps + kRgSplitWarps) {
+    // ---- loads ----
+    if (lane == 0) {
+      int st = 0, issued = 0;
+      unsigned ph = 0;
+      bool ok = true;
+      for (int t = pair; t < P.tiles && ok; t += pairs) {
+        const int row = t * 2 * kTcRows + (int)rank * kTcRows;
+        for (int sl = 0; sl < P.n_slices; ++sl) {
+          if (issued >= stages && !(ok = rg_wait(&s.empty[st], ph ^ 1u, s, P.wait_limit))) break;
+          char *b = smem + st * stage_bytes;
+          mbar_expect_tx(&s.raw[st], (unsigned)((P.direct ? 0 : kTcRows * 128) + N * 128));
+          if (!P.direct) tma_load_2d(b, &tm_a, sl * kTcKSlice, row, &s.raw[st]);
+          tma_load_2d(b + 2 * kTcRows * 128, &tm_whi, sl * kTcKSlice, (int)rank * half, &s.raw[st]);
+          tma_load_2d(b + 2 * kTcRows * 128 + half * 128, &tm_wlo, sl * kTcKSlice, (int)rank * half, &s.raw[st]);
+          if (issued < stages) ++issued;
+          if (++st == stages) { st = 0; ph ^= 1u; }
+        }
+      }
+      // a copy still in flight must not outlive the CTA (only after a wait ran out is one possible)
+      if (s.dead)
+        for (int i = 0; i < issued; ++i)
+          for (int k = 0; k < P.wait_limit && !mbar_wait(&s.raw[i], (i < st ? ph : ph ^ 1u), 1); ++k) {}
+    }
+  } else if (warp == kRgEpiWarps + kRgSplitWarps + 1) {
+    // ---- products (even CTA); split stages passed on (odd CTA) ----
+    if (lane == 0 && rank == 1) {
+      int st = 0;
+      unsigned ph = 0;
+      bool ok = true;
+      for (int t = pair; t < P.tiles && ok; t += pairs)
+        for (int sl = 0; sl < P.n_slices; ++sl) {
+          if (!(ok = rg_wait(&s.split[st], ph, s, P.wait_limit))) break;
+          rg_arrive_leader<true>(&s.ready[st]);
+          if (++st == stages) { st = 0; ph ^= 1u; }
+        }
+    } else if (lane == 0) {
+      const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(N >> 3) << 17) | ((unsigned)(2 * kTcRows >> 4) << 24);
+      int st = 0, buf = 0, uses = 0;  // uses: accumulators handed out so far
+      unsigned ph = 0, acc_ph = 0;
+      bool ok = true;
+      auto take = [&]() {  // the accumulator has been read
+        if (uses >= 2 && !(ok = rg_wait<true>(&s.acc_empty[buf], acc_ph ^ 1u, s, P.wait_limit))) return false;
+        if (uses < 2) ++uses;
+        return true;
+      };
+      auto give = [&]() {
+        rg_commit(&s.acc_full[buf]);
+        buf ^= 1;
+        if (buf == 0) acc_ph ^= 1u;
+      };
+      for (int t = pair; t < P.tiles && ok; t += pairs) {
+        if (!PRECISE && !take()) break;
+        for (int sl = 0; sl < P.n_slices; ++sl) {
+          if (PRECISE && !take()) break;
+          if (!(ok = rg_wait<true>(&s.ready[st], ph, s, P.wait_limit))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const unsigned d = s.tmem_base + (unsigned)(buf * 256);
+          const unsigned b = smem_u32(smem + st * stage_bytes);
+          const unsigned ah = b, al = b + kTcRows * 128, wh = b + 2 * kTcRows * 128, wl = wh + half * 128;
+#pragma unroll
+          for (int j = 0; j < kTcKSlice / 8; ++j) {
+            const unsigned o = j * 32;  // eight TF32 values along K inside the swizzle row
+            if (PRECISE) {
+              rg_mma(d + j * 64, umma_desc_sw128(ah + o), umma_desc_sw128(wl + o), idesc, 0u);
+              rg_mma(d + j * 64, umma_desc_sw128(al + o), umma_desc_sw128(wh + o), idesc, 1u);
+              rg_mma(d + j * 64, umma_desc_sw128(ah + o), umma_desc_sw128(wh + o), idesc, 1u);
+            } else {
+              rg_mma(d, umma_desc_sw128(ah + o), umma_desc_sw128(wh + o), idesc, (sl | j) ? 1u : 0u);
+              rg_mma(d, umma_desc_sw128(ah + o), umma_desc_sw128(wl + o), idesc, 1u);
+              rg_mma(d, umma_desc_sw128(al + o), umma_desc_sw128(wh + o), idesc, 1u);
+            }
+          }
+          rg_commit(&s.empty[st]);
+          if (PRECISE || sl == P.n_slices - 1) give();
+          if (++st == stages) { st = 0; ph ^= 1u; }
+        }
+      }
+      if (!ok) {  // products still running read shared memory of both CTAs
+        rg_commit(&s.drained);
+        mbar_wait(&s.drained, 0, P.wait_limit);
+      }
+    }
+  } else if (warp >= kRgEpiWarps) {
+    // ---- split the raw rows: hi in place, lo beside it ----
+    const int w = tid - 32 * kRgEpiWarps;
+    int st = 0;
+    unsigned ph = 0;
+    bool ok = true;
+    for (int t = pair; t < P.tiles && ok; t += pairs)
+      for (int sl = 0; sl < P.n_slices; ++sl) {
+        if (!(ok = __all_sync(kFull, rg_wait(&s.raw[st], ph, s, P.wait_limit)))) break;  // (the warp leaves as one)
+        float4 *hi = reinterpret_cast<float4 *>(smem + st * stage_bytes), *lo = hi + kTcRows * 8;
+        float4 a[kTcRows * 8 / (32 * kRgSplitWarps)];
+        if (!P.direct) {
+#pragma unroll
+          for (int i = 0; i < kTcRows * 8 / (32 * kRgSplitWarps); ++i) a[i] = hi[w + i * 32 * kRgSplitWarps];
+        } else {  // rows that TMA cannot read: the same quads of the swizzled tile, value by value
+#pragma unroll
+          for (int i = 0; i < kTcRows * 8 / (32 * kRgSplitWarps); ++i) {
+            const int q = w + i * 32 * kRgSplitWarps, r = q >> 3, row = t * 2 * kTcRows + (int)rank * kTcRows + r;
+            const int k = sl * kTcKSlice + ((q & 7) ^ (r & 7)) * 4;
+            const float *x = P.x + (size_t)row * P.ld_x + k;
+            const bool in = row < P.m;
+            a[i] = make_float4(in && k < P.k ? __ldg(x) : 0.f, in && k + 1 < P.k ? __ldg(x + 1) : 0.f,
+                               in && k + 2 < P.k ? __ldg(x + 2) : 0.f, in && k + 3 < P.k ? __ldg(x + 3) : 0.f);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < kTcRows * 8 / (32 * kRgSplitWarps); ++i) {
+          const float4 x = a[i];
+          const float4 h = make_float4(tf32_round(x.x), tf32_round(x.y), tf32_round(x.z), tf32_round(x.w));
+          hi[w + i * 32 * kRgSplitWarps] = h;
+          lo[w + i * 32 * kRgSplitWarps] = make_float4(tf32_round(x.x - h.x), tf32_round(x.y - h.y), tf32_round(x.z - h.z), tf32_round(x.w - h.w));
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read next by the tensor core
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) rg_arrive(rank == 0 ? &s.ready[st] : &s.split[st]);
+        if (++st == stages) { st = 0; ph ^= 1u; }
+      }
+  } else {
+    // ---- drain: warp w holds the rows 32 w .. 32 w + 31 of the CTA's half of the tile ----
+    int buf = 0, eb = 0;
+    unsigned acc_ph = 0;
+    bool ok = true;
+    const unsigned lanes = s.tmem_base + ((unsigned)(warp * 32) << 16);
+    auto release = [&]() {  // the accumulator has been read: its next use may overwrite it
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) rg_arrive_leader<false>(&s.acc_empty[buf]);  // (nothing in memory goes with it)
+    };
+    auto next = [&]() {
+      buf ^= 1;
+      if (buf == 0) acc_ph ^= 1u;
+    };
+    // 32 columns from c on of this lane's row
+    auto put = [&](const float (&x)[32], int c, int row0) {
+      float v[32];
+#pragma unroll
+      for (int q = 0; q < 32; ++q) v[q] = P.relu ? fmaxf(x[q], 0.f) : x[q];
+      if (P.tma_store) {
+        float4 *blk = reinterpret_cast<float4 *>(epi + (warp * 2 + eb) * 4096);
+        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the store before the last has left the buffer
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) blk[lane * 8 + (q ^ (lane & 7))] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0)
+          asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+                           (unsigned long long)&tm_out), "r"(smem_u32(blk)), "r"(c), "r"(row0) : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        eb ^= 1;
+      } else if (row0 + lane < P.m) {
+        float *d = P.out + (size_t)(row0 + lane) * P.ld_out + c;
+#pragma unroll
+        for (int q = 0; q < 32; ++q)
+          if (c + q < P.n_real) d[q] = v[q];
+      }
+    };
+    for (int t = pair; t < P.tiles && ok; t += pairs) {
+      const int row0 = t * 2 * kTcRows + (int)rank * kTcRows + warp * 32;
+      if (PRECISE) {
+        float acc[2][32];
+#pragma unroll
+        for (int q = 0; q < 32; ++q) acc[0][q] = acc[1][q] = 0.f;
+        for (int sl = 0; sl < P.n_slices; ++sl) {
+          if (!(ok = __all_sync(kFull, rg_wait(&s.acc_full[buf], acc_ph, s, P.wait_limit)))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (h * 32 >= N) break;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float a[32];
+              rg_tmem_load(a, lanes + (unsigned)(buf * 256 + j * 64 + h * 32));
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+              rg_loaded(a);
+#pragma unroll
+              for (int q = 0; q < 32; ++q) acc[h][q] += a[q];
+            }
+          }
+          release();
+          next();
+        }
+        if (!ok) break;
+        if (row0 < P.m) {
+          put(acc[0], 0, row0);
+          if (P.n_real > 32) put(acc[1], 32, row0);
+        }
+      } else {
+        if (!(ok = __all_sync(kFull, rg_wait(&s.acc_full[buf], acc_ph, s, P.wait_limit)))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int c = 0; c < N; c += 32) {
+          float v[32];
+          rg_tmem_load(v, lanes + (unsigned)(buf * 256 + c));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          rg_loaded(v);
+          if (c + 32 >= N) release();
+          if (c < P.n_real && row0 < P.m) put(v, c, row0);
+        }
+        next();
+      }
+    }
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (tid == 0 && s.dead) atomicExch(P.error, 1);
+  rg_cluster_sync();
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(s.tmem_base), "n"(512) : "memory");
+  }
+}
+
+// hi / lo [n_pad][K] (K contiguous, rows from n on zero) from W [K][n], or from W [n][K] when w_transposed.
+__global__ void split_weight_pad_kernel(const float *__restrict__ W, int w_transposed, int K, int ldk, int n, int n_pad,
+                                        float *__restrict__ hi, float *__restrict__ lo) {
+  const int total = n_pad * ldk;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int r = i / ldk, k = i - r * ldk;
+    float w = 0.f;
+    if (r < n && k < K) w = w_transposed ? __ldg(W + (size_t)r * K + k) : __ldg(W + (size_t)k * n + r);
+    const float h = tf32_round(w);
+    hi[i] = h;
+    lo[i] = tf32_round(w - h);
+  }
+}
+
+}  // namespace
+
+bool row_gemm_supported(int n) { return n >= 1 && n <= kTcMaxN; }
+int row_gemm_pad_n(int n) { return (n + 31) / 32 * 32; }  // cta_group::2 takes multiples of 32
+int row_gemm_pad_k(int k) { return (k + 3) / 4 * 4; }
+
+cudaError_t row_gemm_split(const float *W, int w_transposed, int K, int n, float *hi, float *lo, cudaStream_t s) {
+  const int ldk = row_gemm_pad_k(K), n_pad = row_gemm_pad_n(n);
+  split_weight_pad_kernel<<<std::min((n_pad * ldk + 255) / 256, 148 * 4), 256, 0, s>>>(W, w_transposed, K, ldk, n, n_pad, hi, lo);
+  return cudaGetLastError();
+}
+
+static int launch_panel(const float *X, int m, int K, int ld_x, const float *hi, const float *lo, int n, float *out, int ld_out, bool relu,
+                        bool precise, int *error, int wait_limit, int sm_count, cudaStream_t s) {
+  const int n_pad = row_gemm_pad_n(n), ldk = row_gemm_pad_k(K);
+  CUtensorMap ma, mh, ml, mo;
+  RowGemmParams P;
+  P.x = X; P.k = K; P.ld_x = ld_x;
+  P.direct = ld_x % 4 != 0 || (reinterpret_cast<uintptr_t>(X) & 15) != 0;
+  int rc = tc_make_map(&mh, hi, n_pad, ldk, n_pad / 2, ldk);
+  if (rc == TF_OK) rc = tc_make_map(&ml, lo, n_pad, ldk, n_pad / 2, ldk);
+  P.m = m; P.n_pad = n_pad; P.n_real = n; P.n_slices = (K + kTcKSlice - 1) / kTcKSlice;
+  P.tiles = (m + 2 * kTcRows - 1) / (2 * kTcRows);
+  P.stages = rg_stages(n_pad);
+  P.out = out; P.ld_out = ld_out; P.relu = relu ? 1 : 0;
+  P.tma_store = ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  P.error = error; P.wait_limit = wait_limit;
+  if (rc != TF_OK) return rc;
+  ma = mo = mh;  // (not used by the variants that have no map of their own)
+  if (!P.direct) rc = tc_make_map(&ma, X, m, K, kTcRows, ld_x);
+  if (rc == TF_OK && P.tma_store) rc = tc_make_map(&mo, out, m, n, 32, ld_out);
+  if (rc != TF_OK) return rc;
+  const size_t smem = (size_t)P.stages * rg_stage_bytes(n_pad) + kRgEpiBytes + 1024;
+  auto f = precise ? row_gemm_kernel<true> : row_gemm_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute((const void *)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) {
+    f<<<2 * std::max(1, std::min(P.tiles, sm_count / 2)), kRgThreads, smem, s>>>(ma, mh, ml, mo, P);
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) return tf::fail(TF_ERR_CUDA, std::string("row_gemm: ") + cudaGetErrorString(e));
+  return TF_OK;
+}
+
+int row_gemm(const float *X, int m, int K, int ld_x, const float *hi, const float *lo, int n, float *out, int ld_out, bool relu,
+             int *error, int wait_limit, int sm_count, cudaStream_t s) {
+  const bool precise = !tc_supported(K, n);
+  const int panel = precise ? kRgPrecisePanel : n;
+  for (int c = 0; c < n; c += panel) {
+    const size_t off = (size_t)c * row_gemm_pad_k(K);
+    const int rc = launch_panel(X, m, K, ld_x, hi + off, lo + off, std::min(panel, n - c), out + c, ld_out, relu, precise, error,
+                                wait_limit, sm_count, s);
+    if (rc != TF_OK) return rc;
+  }
+  return TF_OK;
+}
+
+}  // namespace tfk

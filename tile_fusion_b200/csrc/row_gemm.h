@@ -1,0 +1,25 @@
+// T = B * W for a tall B on the tensor cores (row_gemm.cu): the dense product of a GeMM-SpMM chain in a launch of its own.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace tfk {
+
+struct RowGemmParams {
+  const float *x;  // read directly where rows do not start on 16-byte boundaries (`direct`)
+  float *out;
+  int *error;
+  int m, n_real, n_pad, n_slices, tiles, stages, ld_out, k, ld_x;
+  int direct, relu, tma_store, wait_limit;
+};
+
+bool row_gemm_supported(int n);  // n <= 256 columns
+int row_gemm_pad_n(int n);       // rows of the split weight
+int row_gemm_pad_k(int k);       // floats per row of it
+// hi, lo: row_gemm_pad_n(n) x row_gemm_pad_k(K) floats each.  W is K x n, or n x K when w_transposed.
+cudaError_t row_gemm_split(const float *W, int w_transposed, int K, int n, float *hi, float *lo, cudaStream_t s);
+// out[m][ld_out] (n columns written) = X[m][ld_x] (K columns read) * W, optionally max(0, .); hi, lo as row_gemm_split leaves
+// them.  Rows of X on 16-byte boundaries come by TMA, others value by value; rows of `out` leave likewise.
+int row_gemm(const float *X, int m, int K, int ld_x, const float *hi, const float *lo, int n, float *out, int ld_out, bool relu,
+             int *error, int wait_limit, int sm_count, cudaStream_t s);
+
+}  // namespace tfk
