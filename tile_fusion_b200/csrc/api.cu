@@ -108,7 +108,7 @@ struct DevGather {
     partial_ld = (std::max(n_cols, max_cols) + 3) / 4 * 4;
     const int panels = (partial_ld + 127) / 128;  // the most any width up to that is read in
     if (n_seg > 1) make_segments(g, A.m, n_seg);
-    if (!g.rows.empty()) g.rows.push_back(0);  // a group looks one row ahead
+    if (!g.rows.empty()) g.rows.resize(g.rows.size() + 2, 0);  // a group looks one row ahead (with the row of Q, two)
     int rc = cols.upload(reinterpret_cast<const int *>(g.cols.get()), g.n_entries);
     if (rc == TF_OK) rc = vals.upload(g.vals.get(), g.n_entries);
     if (rc == TF_OK) rc = units.upload(reinterpret_cast<const int4 *>(g.units.data()), g.units.size());
@@ -1132,6 +1132,14 @@ int tf_plan_sddmm_spmm(const tf_csr *A, int kq, int nv, const tf_plan_opts *opts
   cudaGetDevice(&p->device);
   p->chain = 2; p->mode = TF_MODE_STREAM;
   p->m = A->m; p->n_cols = nv; p->k_dim = kq;
+  if (tfk::sddmm_gather_supported(kq, nv) && o.rows_per_block == 0 && o.ctas_per_sm == 0) {
+    p->second.m = A->m; p->second.n = A->n;
+    rc = p->g_second.build(*A, 4 * tfk::sddmm_group(kq, nv), nv, sm_count);  // (units for as many groups of that size)
+    if (rc == TF_OK) rc = zero_state(*p);
+    if (rc != TF_OK) return rc;
+    *out = p.release();
+    return TF_OK;
+  }
   rc = p->second.upload(*A);
   if (rc != TF_OK) return rc;
   p->first_is_second = true;
@@ -1252,6 +1260,14 @@ int tf_exec_sddmm_spmm(tf_plan *p, const float *Q, const float *K, const float *
   if (p->chain != 2) return fail(TF_ERR_ARG, "tf_exec_sddmm_spmm: plan was built for another chain");
   int rc = set_device(*p);
   if (rc != TF_OK) return rc;
+  if (p->g_second.on) {
+    const DevGather &g = p->g_second;
+    const tfk::GatherParams G = gather_params(g, V, p->n_cols, D, p->n_cols, p->n_cols);
+    TF_CUDA(tfk::launch_rows_fix(g.empty.p, g.n_empty, p->n_cols, D, false, (cudaStream_t)stream));
+    TF_CUDA(tfk::launch_sddmm_gather(G, Q, K, p->k_dim, p->m, (cudaStream_t)stream));
+    p->launches = 1;
+    return TF_OK;
+  }
   tfk::Params P = base_params(*p);
   P.in0 = Q; P.in1 = K; P.in2 = V; P.out = D;
   return run_phases(*p, P, 1, 1, (cudaStream_t)stream);

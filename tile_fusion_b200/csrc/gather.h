@@ -64,6 +64,10 @@ struct GatherParams {
 int gather_group(int n_cols);
 // vec_in / vec_out: rows of X / of the result start on 16-byte boundaries.
 cudaError_t launch_gather(int group, bool vec_in, bool vec_out, const GatherParams &p, cudaStream_t s);
+// D = (A .* (Q K^T)) V over the same units (sddmm_gather.cu): V is p.dense, D p.out, both of n_cols columns; m rows of Q.
+bool sddmm_gather_supported(int kq, int nv);  // both up to 128
+int sddmm_group(int kq, int nv);              // lanes that work on a unit
+cudaError_t launch_sddmm_gather(const GatherParams &p, const float *Q, const float *K, int kq, int m, cudaStream_t s);
 // dst[r][0:ld] = src[r][0:n_cols], the rest zero: rows of a width that is no multiple of four made readable as float4.
 cudaError_t launch_pad_rows(const float *src, long long rows, int n_cols, int ld, float *dst, cudaStream_t s);
 
