@@ -135,7 +135,8 @@ typedef struct {
                              (every nonzero names the row's own grid point or one of its six neighbours):
                              0 = run the plane-marching kernel, which keeps the intermediate in shared memory,
                              <0 = never (general CSR path).  GeMM-SpMM plans on such an operator use the same
-                             kernel as the consumer of the dense product's rows (0) or the balanced gather (<0) */
+                             kernel as the consumer of the dense product's rows (0) or the balanced gather (<0).
+                             The same switch covers the executor that marches along the lines of a 2-D five-point operator. */
   int exchange;           /* tf_multi_plan only: 0 = halo rows are written by the copy engines straight into the
                              neighbours' memory (CUDA IPC) where every rank is a process of its own on one host,
                              else ncclSend / ncclRecv; <0 = always ncclSend / ncclRecv (every rank must say the same) */

@@ -19,6 +19,7 @@
 #include "kernels.cuh"
 #include "lattice_march.h"
 #include "launch.h"
+#include "line_march.h"
 #include "row_gemm.h"
 #include "tf_internal.h"
 
@@ -226,6 +227,13 @@ struct tf_plan {
     struct Slab { int item_begin, item_end, z_begin, z_end; };
     std::vector<Slab> slabs;
   } march;
+  // line-marching executor (both operators are five-point operators on one 2-D grid)
+  struct Lines {
+    bool on = false, same = false;
+    int nx = 0, ny = 0, tiles = 0;
+    DevBuf<unsigned> words_f, words_a;
+    tfk::LineParams par;
+  } lines;
   // schedule mode
   DevBuf<int> s_ptr2, s_id, s_type, s_ker;
   int s_n1 = 0;
@@ -535,6 +543,50 @@ int make_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &F, const tf_csr 
   return TF_OK;
 }
 
+// Line-marching executor: taken when both operators of an SpMM-SpMM chain are five-point operators on one 2-D grid.
+int build_lines(tf_plan &p, const tf_csr &F, const tf_csr &A, bool same, int sm_count) {
+  tf::LineOp f, a;
+  tf::analyse_line_operator(A.m, A.n, A.ap, A.ai, A.ax, a);
+  if (!a.ok) return TF_OK;
+  if (!same) {
+    tf::analyse_line_operator(F.m, F.n, F.ap, F.ai, F.ax, f);
+    if (!f.ok || f.nx != a.nx) return TF_OK;
+  }
+  const tf::LineOp &first = same ? a : f;
+  tf_plan::Lines &L = p.lines;
+  L.same = same;
+  L.nx = a.nx; L.ny = a.ny; L.tiles = a.tiles;
+  int rc = L.words_a.upload(a.words);
+  if (rc == TF_OK && !same) rc = L.words_f.upload(f.words);
+  if (rc == TF_OK) rc = zero_state(p);
+  if (rc != TF_OK) return rc;
+  std::memset(&L.par, 0, sizeof(L.par));
+  std::memcpy(L.par.dict_f, first.dict.data(), first.dict.size() * sizeof(float));
+  std::memcpy(L.par.dict_a, a.dict.data(), a.dict.size() * sizeof(float));
+  L.par.none_f = 0x01010101u * (unsigned)first.n_classes;
+  L.par.none_a = 0x01010101u * (unsigned)a.n_classes;
+  L.par.words_a = L.words_a.p;
+  L.par.words_f = same ? L.words_a.p : L.words_f.p;
+  L.par.nx = L.nx; L.par.ny = L.ny; L.par.tiles = L.tiles; L.par.n_cols = p.n_cols;
+  p.sm_count = sm_count;
+  L.on = true;
+  return TF_OK;
+}
+
+// The lines [y_begin, y_end) of D.
+int run_lines(tf_plan &p, const float *C, float *D, int y_begin, int y_end, cudaStream_t s) {
+  const bool vec = p.n_cols % 4 == 0;
+  if (vec && !(aligned(C, 16) && aligned(D, 16)))
+    return fail(TF_ERR_ARG, "this plan reads rows as 16-byte vectors and needs 16-byte aligned dense operands "
+                            "(build the plan with tile_slots < 0 otherwise)");
+  tfk::LineParams P = p.lines.par;
+  P.in = C; P.out = D;
+  P.y_begin = y_begin; P.y_end = y_end;
+  TF_CUDA(tfk::launch_line_march(P, vec, p.lines.same, p.sm_count, s));
+  p.launches = 1;
+  return TF_OK;
+}
+
 // GeMM-SpMM on the balanced gather.  The two products may be taken in either order, D = A (B C) = (A B) C: the sparse
 // product reads one row of its operand per nonzero, so it is given the narrower one -- B where k < n_cols, else B C.
 // (Rows of B that do not start on 16-byte boundaries would be gathered value by value; then B C comes first.  So it does
@@ -618,6 +670,16 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
   if (rc != TF_OK) return rc;
   pp.max_ctas = p->grid;
   pp.slack_blocks = o.mode == TF_MODE_UNFUSED ? (1 << 30) : o.slack_blocks;
+  if (chain == 0 && F && o.mode == TF_MODE_STREAM && o.lattice_march >= 0 && o.ring_bytes <= 0 && o.halo_rows == 0 && o.n_boundary == 0 &&
+      o.rows_per_block == 0 && o.slack_blocks < 0 && o.ctas_per_sm == 0 && o.tile_slots == 0 && o.tile_max_bz == 0 &&
+      o.tile_double_buffer == 0 && o.tile_pipeline == 0) {
+    rc = build_lines(*p, *F, *A, F == A, sm_count);
+    if (rc != TF_OK) return rc;
+    if (p->lines.on) {
+      *out = p.release();
+      return TF_OK;
+    }
+  }
   // gather tiles: 16-byte staging copies need rows that are multiples of 4 floats
   tf::Tiling pt, ct;
   // a tile holds one row per 4 lanes... of the CTA that runs it: 256 rows (sparse chains) or 512 (GeMM-SpMM)
@@ -949,43 +1011,46 @@ int run_host_pipeline(tf_plan &p, tfk::Params &P, const float *h_in, long long i
   return TF_OK;
 }
 
-// The same pipeline for plane-marching plans: one launch per slab of planes.  A slab [za, zb) reads the planes
-// za - 2 .. zb + 1 of C and completes the planes [za, zb) of D, so the copies run two planes ahead of the kernel
-// and the output leaves slab by slab.  Pageable arrays go piece by piece through rings of pinned slots
-// (host_stage.h).
+// The same pipeline for plans that march: one launch per slab of planes (of lines on a 2-D grid).  A slab
+// [za, zb) reads the planes za - 2 .. zb + 1 of C and completes the planes [za, zb) of D, so the copies run two planes
+// ahead of the kernel and the output leaves slab by slab.  Pageable arrays go piece by piece through rings of
+// pinned slots (host_stage.h).
 int run_host_march(tf_plan &p, const float *h_in, float *d_in, float *h_out, float *d_out) {
   tf_plan::March &M = p.march;
-  if (!p.s_h2d) {
-    TF_CUDA(cudaStreamCreateWithFlags(&p.s_h2d, cudaStreamNonBlocking));
-    TF_CUDA(cudaStreamCreateWithFlags(&p.s_run, cudaStreamNonBlocking));
-    TF_CUDA(cudaStreamCreateWithFlags(&p.s_d2h, cudaStreamNonBlocking));
-  }
-  const int ns = (int)M.slabs.size();
+  TF_TRY(ensure_streams(p));
+  const bool lines = p.lines.on;
+  const int nz = lines ? p.lines.ny : M.nz;
+  const long long plane_rows = lines ? p.lines.nx : (long long)M.nx * M.ny;
+  // (lines: slabs of 2 MB, at most 32 -- smaller copies cost more than what they overlap)
+  const int ns = lines ? (int)std::max<long long>(1, std::min<long long>({32, nz / 8, (long long)p.m * p.n_cols * 4 >> 21}))
+                               : (int)M.slabs.size();
+  auto at = [&](int z) { return (size_t)std::min<long long>(p.m, z * plane_rows) * p.n_cols; };  // first float of plane z
   while ((int)p.ev_in.size() < ns) {
     cudaEvent_t a, b;
     TF_CUDA(cudaEventCreateWithFlags(&a, cudaEventDisableTiming));
     TF_CUDA(cudaEventCreateWithFlags(&b, cudaEventDisableTiming));
     p.ev_in.push_back(a); p.ev_run.push_back(b);
   }
-  const size_t plane = (size_t)M.nx * M.ny * p.n_cols, plane_bytes = plane * sizeof(float);
   int rc = begin_host_pipe(p, h_in, h_out);
   if (rc != TF_OK) return rc;
   int planes_in = 0;
   long long launches = 0;
   for (int sl = 0; sl < ns; ++sl) {
-    const tf_plan::March::Slab &g = M.slabs[sl];
-    const int need = std::min(M.nz, g.z_end + 2);
+    const int z_begin = lines ? (int)((long long)nz * sl / ns) : M.slabs[sl].z_begin;
+    const int z_end = lines ? (int)((long long)nz * (sl + 1) / ns) : M.slabs[sl].z_end;
+    const int need = std::min(nz, z_end + 2);
     if (need > planes_in)
-      TF_CUDA(p.host_pipe->upload(d_in + plane * planes_in, h_in + plane * planes_in, plane_bytes * (size_t)(need - planes_in), p.s_h2d));
+      TF_CUDA(p.host_pipe->upload(d_in + at(planes_in), h_in + at(planes_in), (at(need) - at(planes_in)) * sizeof(float), p.s_h2d));
     planes_in = std::max(planes_in, need);
     TF_CUDA(cudaEventRecord(p.ev_in[sl], p.s_h2d));
     TF_CUDA(cudaStreamWaitEvent(p.s_run, p.ev_in[sl], 0));
-    rc = run_march(p, d_in, d_out, g.item_begin, g.item_end, false, p.s_run);
+    rc = lines ? run_lines(p, d_in, d_out, z_begin, z_end, p.s_run)
+               : run_march(p, d_in, d_out, M.slabs[sl].item_begin, M.slabs[sl].item_end, false, p.s_run);
     if (rc != TF_OK) return rc;
     launches += p.launches;
     TF_CUDA(cudaEventRecord(p.ev_run[sl], p.s_run));
     TF_CUDA(cudaStreamWaitEvent(p.s_d2h, p.ev_run[sl], 0));
-    TF_CUDA(p.host_pipe->download(h_out + plane * g.z_begin, d_out + plane * g.z_begin, plane_bytes * (size_t)(g.z_end - g.z_begin), p.s_d2h));
+    TF_CUDA(p.host_pipe->download(h_out + at(z_begin), d_out + at(z_begin), (at(z_end) - at(z_begin)) * sizeof(float), p.s_d2h));
   }
   p.launches = launches;
   TF_CUDA(p.host_pipe->finish());
@@ -1165,7 +1230,7 @@ int tf_plan_info(const tf_plan *p, long long info[8]) {
   info[2] = p->hp.n_cons;
   info[3] = p->hp.ring_rows;
   info[4] = p->march.on ? p->march.grid : (p->pipe ? p->pipe_grid : p->grid);
-  info[5] = p->march.on ? tfk::kMarchThreads : (p->pipe ? 672 : (p->dyn_smem > 0 ? tfk::tiled_threads(p->chain) : tfk::kThreads));
+  info[5] = p->march.on || p->lines.on ? tfk::kMarchThreads : (p->pipe ? 672 : (p->dyn_smem > 0 ? tfk::tiled_threads(p->chain) : tfk::kThreads));
   info[6] = p->launches;
   info[7] = p->hp.inter_rows;
   return TF_OK;
@@ -1212,6 +1277,7 @@ int tf_exec_spmm_spmm(tf_plan *p, const float *C, float *D, void *stream) {
   if (p->halo_rows || p->sendbuf.n) return fail(TF_ERR_ARG, "tf_exec_spmm_spmm: plan has halo rows, drive it with tf_exec_phase");
   int rc = set_device(*p);
   if (rc != TF_OK) return rc;
+  if (p->lines.on) return run_lines(*p, C, D, 0, p->lines.ny, (cudaStream_t)stream);
   if (march_usable(*p, C, D)) return run_march(*p, C, D, 0, p->march.n_items, false, (cudaStream_t)stream);
   if (p->g_second.on) return run_gather_spmm_spmm(*p, C, D, (cudaStream_t)stream);
   tfk::Params P = base_params(*p);
@@ -1302,6 +1368,10 @@ int tf_exec_phase(tf_plan *p, int phase, const float *in0, const float *in1, int
   if (phase > 0 && p->chain == 0 && march_usable(*p, in0, D))
     return phase == 1 ? run_march(*p, in0, D, 0, p->march.n_phase1, false, (cudaStream_t)stream)
                       : run_march(*p, in0, D, p->march.n_phase1, p->march.n_items, true, (cudaStream_t)stream);
+  if (p->lines.on) {  // no exchange: phase 1 is the whole chain
+    p->launches = 0;
+    return phase == 1 ? run_lines(*p, in0, D, 0, p->lines.ny, (cudaStream_t)stream) : TF_OK;
+  }
   if (p->g_second.on) {  // no exchange: phase 1 is the whole chain
     p->launches = 0;
     if (phase != 1) return TF_OK;
@@ -1408,12 +1478,12 @@ int tf_spmm_spmm_host(tf_plan *p, const float *C, float *D) {
   int rc = set_device(*p);
   if (rc != TF_OK) return rc;
   const size_t nd = (size_t)p->m * p->n_cols;
-  if (!p->march.slabs.empty()) {
+  if (!p->march.slabs.empty() || (p->lines.on && nd * sizeof(float) >= ((size_t)1 << 20))) {
     const size_t nin = (size_t)p->first_cols * p->n_cols;
     if (p->h_in0.n < nin) rc = p->h_in0.alloc(nin);
     if (rc == TF_OK && p->h_out.n < nd) rc = p->h_out.alloc(nd);
     if (rc != TF_OK) return rc;
-    if (march_usable(*p, p->h_in0.p, p->h_out.p)) {
+    if (p->lines.on || march_usable(*p, p->h_in0.p, p->h_out.p)) {
       rc = run_host_march(*p, C, p->h_in0.p, D, p->h_out.p);
       if (rc != TF_OK) return rc;
       return tf_plan_status(p, nullptr);
