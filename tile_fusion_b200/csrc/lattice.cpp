@@ -37,10 +37,12 @@ struct VecHash {
 }  // namespace
 
 int analyse_lattice_operator(int m, int ncols, const int *ap, const int *ai, const float *ax, int halo_rows,
-                             LatticeOp &out) {
+                             LatticeOp &out, bool allow_odd) {
   out = LatticeOp();
   const Lattice L = detect_lattice(m, ap, ai);
-  if (L.dims != 3 || L.nx < 2 || L.ny < 2 || L.nx % 2 != 0) return TF_OK;  // (the executor reads x in pairs)
+  if (L.dims != 3 || L.nx < 2 || L.ny < 2) return TF_OK;
+  const bool odd = L.nx % 2 != 0;  // (the executor reads x in pairs and patches up the point behind the last one)
+  if (odd && !(allow_odd && halo_rows == 0 && m == ncols)) return TF_OK;
   const long long plane = (long long)L.nx * L.ny;
   if (plane <= L.nx || m % plane != 0) return TF_OK;
   const int nx = L.nx, ny = L.ny, nz = (int)(m / plane);
@@ -98,6 +100,11 @@ int analyse_lattice_operator(int m, int ncols, const int *ap, const int *ai, con
           seen |= 1u << slot;
           std::memcpy(&k.w[slot], &ax[j], 4);
         }
+        // an extent that is odd is taken only where every neighbour is named, so that no coefficient in the grid is a zero
+        // that stands for none (other operators run on the general path, which multiplies what is stored)
+        if (odd && seen != ((z > 0 ? 1u : 0u) | (y > 0 ? 2u : 0u) | (x > 0 ? 4u : 0u) | 8u | (x < nx - 1 ? 16u : 0u) |
+                            (y < ny - 1 ? 32u : 0u) | (z < nz - 1 ? 64u : 0u)))
+          return TF_OK;
         auto it = ids.find(k);
         int id;
         if (it == ids.end()) {

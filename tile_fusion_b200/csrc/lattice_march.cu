@@ -33,6 +33,8 @@
 
 #include <type_traits>
 
+#include <algorithm>
+
 #include "lattice_march.h"
 
 namespace tfk {
@@ -69,6 +71,19 @@ __device__ __forceinline__ void tma_load_plane(unsigned smem, const CUtensorMap 
       "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
       ::"r"(smem), "l"((unsigned long long)tm), "r"(bar), "r"(col), "r"(xh), "r"(0), "r"(y), "r"(z)
       : "memory");
+}
+
+// The planes of C as a CTA loads them.  Where nx is odd, the pair of the last point of a line holds the first point of the
+// next line; patch_plane clears it.  Behind the very last line there is nothing to read at all, so the last plane has a map
+// of its own that ends one line earlier, and patch_plane brings that line.
+struct PlaneMaps {
+  const CUtensorMap *all, *last;
+};
+template <bool ODD>
+__device__ __forceinline__ void load_plane(unsigned smem, const PlaneMaps &tm, int col, int xh, int y, int z, unsigned bar,
+                                           const MarchParams &P) {
+  const bool last = ODD && z == P.nz - 1;
+  tma_load_plane(smem, last ? tm.last : tm.all, col, xh, y, last ? 0 : z, bar);
 }
 
 // Rectangles of P x (rows) row chunks of 64 bytes are kept as [y][x % 2][x / 2][64 B]: byte offset of
@@ -168,6 +183,7 @@ struct ClassColumn {
 struct Shared {
   unsigned cbuf, tbuf;       // C stages, the two planes of T
   unsigned full;             // mbarriers, 8 bytes each: one per C stage (the plane has landed)
+  unsigned fixbar;           // one phase per patched plane: every warp has written its part
   unsigned tbar;             // one phase per step: every warp has stored its rows of T(k-1) (and read C(k))
   volatile int *abort;
 };
@@ -214,8 +230,24 @@ __device__ __forceinline__ int lead_in(int zs, const MarchParams &P) {
   return (zs == 0 && P.z_shift == 0 && P.t_lo == nullptr) ? 0 : 2;
 }
 
+// nx odd: completes the plane of C in stage `cb` (see load_plane) where the rectangle of the tile reaches behind the last
+// point of a line or, in the last plane, to the last line.  One thread per 16 bytes.
+__device__ __forceinline__ void patch_plane(unsigned cb, int x0, int y0, int c0col, bool fix_x, bool fix_y, const MarchParams &P) {
+  const int tid = threadIdx.x, c4 = tid & 3, i = tid >> 2;  // 32 groups of four lanes
+  if (fix_x && i < H + 4) sts4(cb, i * (PC * 64) + xoff<PC>(P.nx - x0 + 2) + c4 * 16, zero4());
+  if (fix_y && i < W + 4) {
+    const int x = x0 - 2 + i, col = c0col + 4 * c4;
+    float4 v = zero4();
+    if (x >= 0 && x < P.nx && col < P.n_cols)
+      v = __ldg(reinterpret_cast<const float4 *>(P.c + ((size_t)P.nx * P.ny * P.nz - P.nx + x) * P.n_cols + col));
+    sts4(cb, (P.ny - 1 - y0 + 2) * (PC * 64) + xoff<PC>(i) + c4 * 16, v);
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the stage is filled by TMA again later
+}
+
 // State a CTA carries from item to item.
 struct CtaState {
+  unsigned n_fix;  // planes patched so far: phases of fixbar
   unsigned n_use;  // steps taken so far: step n uses C stage n % stages (parity of n / stages) and phase n of tbar
   unsigned n_iss;  // plane loads issued so far (kept by thread 0, which issues them)
 };
@@ -227,7 +259,8 @@ static_assert(W == 16 && H == 8 && kMarchThreads == 128 && kMarchCols == 16,
 
 // One work item, seen by one thread: its 2 x 2 patch of the tile at (x, y) (both products) and kRing single
 // rows of the ring of T around the tile at (rx[r], ry[r]) (first product only; `ring` = this warp has any).
-__device__ __forceinline__ bool run_item(const CUtensorMap *tm_c, const MarchParams &P, const Shared &S, CtaState &cs,
+template <bool ODD>
+__device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParams &P, const Shared &S, CtaState &cs,
                                          int x0, int y0, int zs, int ze, int c0col, int x, int y, bool ring,
                                          const int (&rx)[kRing], const int (&ry)[kRing], bool pair_x,
                                          const volatile int *next, int &prefetched) {
@@ -280,6 +313,9 @@ __device__ __forceinline__ bool run_item(const CUtensorMap *tm_c, const MarchPar
   for (int r = 0; r < kRing; ++r) { rA[r] = zero4(); accR[r] = zero4(); czpR[r] = 0.f; }
   unsigned wrA = ring ? cr_col.at(kfirst, P.nz, plane_words, zero_f) : 0u, wrB;
   unsigned wfA = cf_col.at(kfirst, P.nz, plane_words, zero_f), wfB;
+  // (odd) Rows of T(k-1) that do not exist: they are zero, not a product with it, so that an infinity in C stays where it
+  // belongs.  (On even extents such a product is taken: 4 % of the time otherwise, 550 -> 575 us at 128^3, 128 columns.)
+  unsigned deadT = 0xffffffffu, deadR = 3u;
   unsigned waA = zero_a, waB;  // classes of the second operator's rows of plane k - 1
 
   // One step: plane C(k) arrives.  (cprev, tprev, rprev, wf, wa, wr) were written by the step before;
@@ -291,6 +327,16 @@ __device__ __forceinline__ bool run_item(const CUtensorMap *tm_c, const MarchPar
     const unsigned stage = cs.n_use % kMarchStages;
     if (!wait_or_abort(S.full + 8 * stage, (cs.n_use / kMarchStages) & 1u, P.wait_limit, S.abort)) return false;
     const unsigned cb = S.cbuf + stage * kMarchCBytes;
+    if (ODD && k >= 0 && k < P.nz) {
+      const bool fix_x = P.nx < x0 + W + 2, fix_y = k == P.nz - 1 && P.ny - 1 < y0 + H + 2;  // (both are >= the tile's origin)
+      if (fix_x || fix_y) {
+        patch_plane(cb, x0, y0, c0col, fix_x, fix_y, P);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(S.fixbar);
+        if (!wait_or_abort(S.fixbar, cs.n_fix & 1u, P.wait_limit, S.abort)) return false;
+        ++cs.n_fix;
+      }
+    }
     float4 nb[8];
     const unsigned baseC = cb + boC;
     load_own<PC, 2>(baseC, own);
@@ -307,6 +353,11 @@ __device__ __forceinline__ bool run_item(const CUtensorMap *tm_c, const MarchPar
       tcur[j] = fma4(czpT[j], own[j], accT[j]);
       if (halo) tcur[j] = halo_row(halo, x + (j & 1), y + (j >> 1), col, P);
     }
+    if (ODD && deadT) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (deadT >> (8 * j) & 1u) tcur[j] = zero4();
+    }
     const unsigned baseT = tb + boT;
     // (the buffer of T(k-1) was last read in step k-2; this thread has waited for every warp's arrival of
     // step k-1, which each warp gives after its reads of step k-2)
@@ -314,6 +365,8 @@ __device__ __forceinline__ bool run_item(const CUtensorMap *tm_c, const MarchPar
     sts4i<co<PT, 1>(0) + PT * 64>(baseT, tcur[2]); sts4i<co<PT, 1>(1) + PT * 64>(baseT, tcur[3]);
     if (ring) {
       float4 t0 = fma4(czpR[0], rown[0], accR[0]), t1 = fma4(czpR[1], rown[1], accR[1]);
+      if (ODD && (deadR & 1u)) t0 = zero4();
+      if (ODD && (deadR & 2u)) t1 = zero4();
       if (halo) { t0 = halo_row(halo, rx[0], ry[0], col, P); t1 = halo_row(halo, rx[1], ry[1], col, P); }
       sts4(tb, rT, t0);
       if (pair_x) sts4i<kX1T>(tb + rT, t1); else sts4i<kY1T>(tb + rT, t1);
@@ -336,10 +389,12 @@ __device__ __forceinline__ bool run_item(const CUtensorMap *tm_c, const MarchPar
     // T(k): everything but the z+ product
     if (k >= zs - 1 && k <= ze) {
       patch_start(accT, czpT, P.dict_f, wf, cprev, own, nb);
+      if (ODD) deadT = __vcmpeq4(wf, zero_f);
       if (ring) {
         // (the ring rows' neighbours are read only now, when the patch's are no longer needed; the stage is
         // refilled one step later, see below)
         const unsigned cls0 = (wr >> rsh0) & 255u;
+        if (ODD) deadR = (cls0 == (zero_f & 255u) ? 1u : 0u) | (((wr >> (rsh0 + (pair_x ? 8u : 16u))) & 255u) == (zero_f & 255u) ? 2u : 0u);
         if (pair_x) {
           // the group's two ring rows are neighbours in x: each is the other's x- / x+ row
           const unsigned cls1 = (wr >> (rsh0 + 8u)) & 255u;
@@ -370,14 +425,14 @@ __device__ __forceinline__ bool run_item(const CUtensorMap *tm_c, const MarchPar
       if (ahead < steps) {
         ++cs.n_iss;
         mbar_expect_tx(S.full + 8 * prev_stage, kMarchCBytes);
-        tma_load_plane(S.cbuf + prev_stage * kMarchCBytes, tm_c, c0col, x0 / 2 - 1, y0 - 2, kfirst + ahead + P.z_shift,
-                       S.full + 8 * prev_stage);
+        load_plane<ODD>(S.cbuf + prev_stage * kMarchCBytes, tm_c, c0col, x0 / 2 - 1, y0 - 2, kfirst + ahead + P.z_shift,
+                   S.full + 8 * prev_stage, P);
       } else if (steps >= kMarchStages && next[0]) {   // (a shorter item left stages unarmed: no hand-over)
         ++cs.n_iss;
         ++prefetched;
         mbar_expect_tx(S.full + 8 * prev_stage, kMarchCBytes);
-        tma_load_plane(S.cbuf + prev_stage * kMarchCBytes, tm_c, next[4], next[1] / 2 - 1, next[2] - 2,
-                       next[3] + (ahead - steps) + P.z_shift, S.full + 8 * prev_stage);
+        load_plane<ODD>(S.cbuf + prev_stage * kMarchCBytes, tm_c, next[4], next[1] / 2 - 1, next[2] - 2,
+                   next[3] + (ahead - steps) + P.z_shift, S.full + 8 * prev_stage, P);
       }
     }
     // D(k-1): everything but the z+ product, from T(k-2) (registers), T(k-1) (registers and neighbours)
@@ -406,8 +461,11 @@ __device__ __forceinline__ bool run_item(const CUtensorMap *tm_c, const MarchPar
 
 }  // namespace
 
+// ODD: the x extent is odd.
+template <bool ODD>
 __global__ void __launch_bounds__(kMarchThreads, kMarchCtasPerSm)
-lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const MarchParams P) {
+lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_last, const MarchParams P) {
+  const PlaneMaps maps{&tm_c, &tm_last};
   extern __shared__ char dyn[];
   __shared__ int ctl[2];
   __shared__ int nxt[5];
@@ -416,12 +474,14 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const MarchParams
   S.tbuf = S.cbuf + kMarchStages * kMarchCBytes;
   S.full = S.tbuf + 2 * kMarchTBytes;
   S.tbar = S.full + 8 * kMarchStages;
+  S.fixbar = S.tbar + 8;
   S.abort = &ctl[1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
     for (int s = 0; s < kMarchStages; ++s) mbar_init(S.full + 8 * s, 1);
     mbar_init(S.tbar, kMarchThreads / 32);
+    mbar_init(S.fixbar, kMarchThreads / 32);
     ctl[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -450,7 +510,7 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const MarchParams
   asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
   const bool idle = (int)smid >= P.first_idle_sm;
 
-  CtaState cs{0u, 0u};
+  CtaState cs{0u, 0u, 0u};
   bool failed = false;
   // Thread 0 holds the ticket of the item after the current one and keeps that item's origin in shared memory:
   // the last steps of an item already fetch the first planes of the next (`pre` of them).
@@ -481,7 +541,7 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const MarchParams
       for (int s = pre; s < min(kMarchStages, steps); ++s) {
         const unsigned stage = (cs.n_use + s) % kMarchStages;
         mbar_expect_tx(S.full + 8 * stage, kMarchCBytes);
-        tma_load_plane(S.cbuf + stage * kMarchCBytes, &tm_c, c0col, x0 / 2 - 1, y0 - 2, kfirst + s + P.z_shift, S.full + 8 * stage);
+        load_plane<ODD>(S.cbuf + stage * kMarchCBytes, maps, c0col, x0 / 2 - 1, y0 - 2, kfirst + s + P.z_shift, S.full + 8 * stage, P);
       }
       cs.n_iss = cs.n_use + min(kMarchStages, steps);
       pre = 0;
@@ -489,7 +549,7 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const MarchParams
     int rx[kRing], ry[kRing];
 #pragma unroll
     for (int r = 0; r < kRing; ++r) { rx[r] = x0 + rdx[r]; ry[r] = y0 + rdy[r]; }
-    if (!run_item(&tm_c, P, S, cs, x0, y0, zs, ze, c0col, x0 + 2 * pi, y0 + 2 * warp, ring, rx, ry, warp < 2, nxt, pre)) { failed = true; break; }
+    if (!run_item<ODD>(maps, P, S, cs, x0, y0, zs, ze, c0col, x0 + 2 * pi, y0 + 2 * warp, ring, rx, ry, warp < 2, nxt, pre)) { failed = true; break; }
   }
   if (failed && tid == 0) atomicExch(&P.st->error, 1);
   // A thread that gave up has raised the CTA's abort flag; the others notice it in their own bounded waits
@@ -515,7 +575,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, long long planes) {
+int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, int lines, long long planes) {
   static EncodeTiledFn fn = nullptr;
   if (!fn) {
     void *p = nullptr;
@@ -525,9 +585,10 @@ int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny,
       fn = (EncodeTiledFn)p;
   }
   if (!fn) return -1;
-  // (column, x / 2, x % 2, y, plane): nx is even, so row x = 2 * (x / 2) + x % 2 of a y-line
+  // (column, x / 2, x % 2, y, plane): row x = 2 * (x / 2) + x % 2 of a y-line; where nx is odd the last pair of a line ends
+  // with the first row of the next
   const cuuint64_t row = (cuuint64_t)n_cols * 4;
-  cuuint64_t gdim[5] = {(cuuint64_t)n_cols, (cuuint64_t)(nx / 2), 2, (cuuint64_t)ny, (cuuint64_t)planes};
+  cuuint64_t gdim[5] = {(cuuint64_t)n_cols, (cuuint64_t)((nx + 1) / 2), 2, (cuuint64_t)lines, (cuuint64_t)planes};
   cuuint64_t gstride[4] = {2 * row, row, row * nx, row * nx * ny};
   cuuint32_t box[5] = {(cuuint32_t)kMarchCols, (cuuint32_t)((kMarchW + 4) / 2), 2, (cuuint32_t)(kMarchH + 4), 1};
   cuuint32_t estr[5] = {1, 1, 1, 1, 1};
@@ -538,22 +599,24 @@ int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny,
 }
 
 // CTAs of the kernel that fit one SM (0 on error).  The first call also raises the kernel's shared-memory limits.
-int march_ctas_per_sm() {
+template <bool ODD>
+static int ctas_per_sm() {
   static int occ = -1;
   if (occ >= 0) return occ;
-  const void *fn = (const void *)lattice_march_kernel;
+  const void *fn = (const void *)lattice_march_kernel<ODD>;
   int n = 0;
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMarchSmemBytes) != cudaSuccess ||
       cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, lattice_march_kernel, kMarchThreads, kMarchSmemBytes) != cudaSuccess)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kMarchThreads, kMarchSmemBytes) != cudaSuccess)
     return 0;
   occ = n;
   return occ;
 }
+int march_ctas_per_sm() { return std::min(ctas_per_sm<false>(), ctas_per_sm<true>()); }
 
-cudaError_t launch_lattice_march(int grid, const CUtensorMap &tm_c, const MarchParams &p, cudaStream_t s) {
+cudaError_t launch_lattice_march(int grid, const CUtensorMap &tm_c, const CUtensorMap &tm_last, const MarchParams &p, cudaStream_t s) {
   if (march_ctas_per_sm() <= 0) return cudaErrorLaunchOutOfResources;
-  lattice_march_kernel<<<grid, kMarchThreads, kMarchSmemBytes, s>>>(tm_c, p);
+  (p.c ? lattice_march_kernel<true> : lattice_march_kernel<false>)<<<grid, kMarchThreads, kMarchSmemBytes, s>>>(tm_c, tm_last, p);
   return cudaGetLastError();
 }
 

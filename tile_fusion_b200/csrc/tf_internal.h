@@ -72,7 +72,7 @@ struct LatticeOp {
 // halo_lo / halo_hi: rows of source planes that are not addressed as shifted lattice neighbours but are
 // appended after the m local rows (the second operator of a partitioned chain): lower plane first.
 int analyse_lattice_operator(int m, int ncols, const int *ap, const int *ai, const float *ax, int halo_rows,
-                             LatticeOp &out);
+                             LatticeOp &out, bool allow_odd = false);
 
 // Work items of the plane-marching executor: an x-y tile, a range of planes and a column chunk each.
 struct MarchItem {
