@@ -220,6 +220,10 @@ int tf_exec_gemm_spmm(tf_plan *p, const float *B, const float *W, int w_transpos
 int tf_exec_sddmm_spmm(tf_plan *p, const float *Q, const float *K, const float *V, float *D,
                        void *stream);
 
+/* out = A * X with the plan's A, X and out n_cols wide (at most the widest dense operand of the plan): the sparse product
+ * of a layer's backward pass (binding-project/src/Functions.cpp:1192-1244) on the operator that its forward pass uses. */
+int tf_exec_spmm(tf_plan *p, const float *X, int n_cols, float *out, void *stream);
+
 /* Multi-GPU phases of a plan built with boundary_rows / halo_rows:
  *   phase 0  produce the boundary rows of the intermediate (then send them),
  *   phase 1  everything that needs no halo row,

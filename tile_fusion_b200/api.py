@@ -272,6 +272,11 @@ class Plan:
         check(_lib.lib().tf_exec_sddmm_spmm(self._h, Qd.data_ptr(), Kd.data_ptr(), Vd.data_ptr(), Dd.data_ptr(),
                                             stream if stream is not None else _stream_ptr()))
 
+    def spmm(self, Xd, outd, stream=None):
+        """out = A X with the plan's operator A."""
+        check(_lib.lib().tf_exec_spmm(self._h, Xd.data_ptr(), Xd.shape[1], outd.data_ptr(),
+                                      stream if stream is not None else _stream_ptr()))
+
     def phase(self, phase, in0, in1=None, out=None, w_transposed=False, relu=False, stream=None):
         check(_lib.lib().tf_exec_phase(self._h, int(phase), in0.data_ptr(), in1.data_ptr() if in1 is not None else None,
                                        int(w_transposed), int(relu), out.data_ptr() if out is not None else None,

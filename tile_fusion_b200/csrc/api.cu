@@ -1343,6 +1343,19 @@ int tf_exec_sddmm_spmm(tf_plan *p, const float *Q, const float *K, const float *
   return run_phases(*p, P, 1, 1, (cudaStream_t)stream);
 }
 
+int tf_exec_spmm(tf_plan *p, const float *X, int n_cols, float *out, void *stream) {
+  if (!p || !X || !out) return fail(TF_ERR_ARG, "tf_exec_spmm: null argument");
+  if (n_cols <= 0) return fail(TF_ERR_ARG, "tf_exec_spmm: bad width");
+  int rc = set_device(*p);
+  if (rc != TF_OK) return rc;
+  const cudaStream_t s = (cudaStream_t)stream;
+  if (p->g_second.on && n_cols <= p->g_second.partial_ld)
+    return run_gather(p->g_second, X, n_cols, n_cols % 4 == 0 && aligned(X, 16), out, n_cols, n_cols % 4 == 0 && aligned(out, 16),
+                      n_cols, false, s);
+  if (!p->second.ap.n) return fail(TF_ERR_UNSUPPORTED, "tf_exec_spmm: wider than the plan's dense operands");
+  return tf_spmm_dev(p->second.ap.p, p->second.ai.p, p->second.ax.p, p->m, X, n_cols, out, stream);
+}
+
 int tf_exec_phase(tf_plan *p, int phase, const float *in0, const float *in1, int w_transposed, int relu,
                   float *D, void *stream) {
   if (!p || !in0) return fail(TF_ERR_ARG, "tf_exec_phase: null argument");

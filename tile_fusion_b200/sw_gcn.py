@@ -16,7 +16,7 @@ reference's layers do (``gcn-e2e-training/FusedGCNLayer.py:10-11``), everything 
 take part in autograd: the backward is the reference's (``src/Functions.cpp:819-1043``, ``:1192-1244``),
 ``dX = (A dY) W`` and ``dW = (A dY)^T X`` -- like the reference it multiplies by ``A``, not ``A^T``, i.e. it
 assumes the symmetric adjacency of a GCN.  The forward runs the library's fused GeMM-SpMM executor; the sparse
-product of the backward runs the library's CSR SpMM, its two dense products are plain library GEMMs.
+product of the backward runs on the same plan's operator, its two dense products are plain library GEMMs.
 
 The schedule tensors have the reference's layout (level pointers, per-partition kernel boundaries, row ids) and
 come from the library's inspector for the same cache budget; the GPU executor plans its own tiles and does not
@@ -28,7 +28,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from . import _lib, api
+from . import api
 
 _LIB = torch.library.Library("sw_gcn", "DEF")
 _plans: dict = {}
@@ -64,13 +64,11 @@ def _plan(adj, k, n, unfused=False):
     return p
 
 
-def _spmm(adj, x):
-    """A @ x with the library's CSR SpMM."""
-    _, _, (ap, ai, ax) = _csr_of(adj)
+def _spmm(plan, x):
+    """A @ x with the operator of a layer's plan."""
     x = x.contiguous().float()
-    out = torch.empty((adj.shape[0], x.shape[1]), device=x.device, dtype=torch.float32)
-    _lib.check(_lib.lib().tf_spmm_dev(ap.data_ptr(), ai.data_ptr(), ax.data_ptr(), adj.shape[0], x.data_ptr(), x.shape[1],
-                                      out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    out = torch.empty((x.shape[0], x.shape[1]), device=x.device, dtype=torch.float32)
+    plan.spmm(x, out)
     return out
 
 
@@ -84,14 +82,14 @@ class _FusedGeMMSpMM(torch.autograd.Function):
         w = weight.contiguous().float()
         out = torch.empty((adj.shape[0], w.shape[0]), device=x.device, dtype=torch.float32)
         _plan(adj, x.shape[1], w.shape[0], unfused).gemm_spmm(x, w, out, w_transposed=True)
-        ctx.adj = adj
+        ctx.adj, ctx.unfused = adj, unfused
         ctx.save_for_backward(x, w)
         return out
 
     @staticmethod
     def backward(ctx, grad_out):
         x, w = ctx.saved_tensors
-        ag = _spmm(ctx.adj, grad_out)                      # A dY (the reference multiplies by A: symmetric adjacency)
+        ag = _spmm(_plan(ctx.adj, x.shape[1], w.shape[0], ctx.unfused), grad_out)  # A dY (the reference multiplies by A: symmetric adjacency)
         grad_x = ag @ w if ctx.needs_input_grad[1] else None
         grad_w = ag.t() @ x if ctx.needs_input_grad[2] else None
         return None, grad_x, grad_w, None
