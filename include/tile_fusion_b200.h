@@ -224,6 +224,11 @@ int tf_exec_sddmm_spmm(tf_plan *p, const float *Q, const float *K, const float *
  * of a layer's backward pass (binding-project/src/Functions.cpp:1192-1244) on the operator that its forward pass uses. */
 int tf_exec_spmm(tf_plan *p, const float *X, int n_cols, float *out, void *stream);
 
+/* out (na x nb) = A^T * B for A m x na and B m x nb, device pointers, fp32: the weight gradient of a layer
+ * (binding-project/src/Functions.cpp:1192-1244).  `work` holds tf_atb_work_floats(m, na, nb) floats of scratch. */
+int tf_atb_dev(const float *A, int na, const float *B, int nb, int m, float *out, float *work, long long work_floats, void *stream);
+long long tf_atb_work_floats(int m, int na, int nb);
+
 /* Multi-GPU phases of a plan built with boundary_rows / halo_rows:
  *   phase 0  produce the boundary rows of the intermediate (then send them),
  *   phase 1  everything that needs no halo row,

@@ -16,7 +16,8 @@ reference's layers do (``gcn-e2e-training/FusedGCNLayer.py:10-11``), everything 
 take part in autograd: the backward is the reference's (``src/Functions.cpp:819-1043``, ``:1192-1244``),
 ``dX = (A dY) W`` and ``dW = (A dY)^T X`` -- like the reference it multiplies by ``A``, not ``A^T``, i.e. it
 assumes the symmetric adjacency of a GCN.  The forward runs the library's fused GeMM-SpMM executor; the sparse
-product of the backward runs on the same plan's operator, its two dense products are plain library GEMMs.
+product of the backward runs on the same plan's operator, the weight gradient -- a sum over all rows -- on a kernel
+of the library's own, the other dense product is a plain library GEMM.
 
 The schedule tensors have the reference's layout (level pointers, per-partition kernel boundaries, row ids) and
 come from the library's inspector for the same cache budget; the GPU executor plans its own tiles and does not
@@ -28,7 +29,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from . import api
+from . import _lib, api
 
 _LIB = torch.library.Library("sw_gcn", "DEF")
 _plans: dict = {}
@@ -72,6 +73,19 @@ def _spmm(plan, x):
     return out
 
 
+def _weight_grad(a, b):
+    """a.T @ b for two tall matrices: a sum over all rows.  (With a graph to record, by the operator that records.)"""
+    if torch.is_grad_enabled():
+        return a.t() @ b
+    L = _lib.lib()
+    m, na, nb = a.shape[0], a.shape[1], b.shape[1]
+    out = torch.empty((na, nb), device=a.device, dtype=torch.float32)
+    work = torch.empty(L.tf_atb_work_floats(m, na, nb), device=a.device, dtype=torch.float32)
+    _lib.check(L.tf_atb_dev(a.data_ptr(), na, b.data_ptr(), nb, m, out.data_ptr(), work.data_ptr(), work.numel(),
+                            torch.cuda.current_stream().cuda_stream))
+    return out
+
+
 class _FusedGeMMSpMM(torch.autograd.Function):
     """Forward D = A (X W^T) on the fused executor; backward as FusedGeMMSpMMROAdj::backward
     (binding-project/src/Functions.cpp:1192-1244)."""
@@ -91,7 +105,7 @@ class _FusedGeMMSpMM(torch.autograd.Function):
         x, w = ctx.saved_tensors
         ag = _spmm(_plan(ctx.adj, x.shape[1], w.shape[0], ctx.unfused), grad_out)  # A dY (the reference multiplies by A: symmetric adjacency)
         grad_x = ag @ w if ctx.needs_input_grad[1] else None
-        grad_w = ag.t() @ x if ctx.needs_input_grad[2] else None
+        grad_w = _weight_grad(ag, x) if ctx.needs_input_grad[2] else None
         return None, grad_x, grad_w, None
 
 
