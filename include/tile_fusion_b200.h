@@ -136,7 +136,8 @@ typedef struct {
                              0 = run the plane-marching kernel, which keeps the intermediate in shared memory,
                              <0 = never (general CSR path).  GeMM-SpMM plans on such an operator use the same
                              kernel as the consumer of the dense product's rows (0) or the balanced gather (<0).
-                             The same switch covers the executor that marches along the lines of a 2-D five-point operator. */
+                             The same switch covers the executors that march along the lines of a 2-D five-point operator
+                             and down the blocks of a banded one. */
   int exchange;           /* tf_multi_plan only: 0 = halo rows are written by the copy engines straight into the
                              neighbours' memory (CUDA IPC) where every rank is a process of its own on one host,
                              else ncclSend / ncclRecv; <0 = always ncclSend / ncclRecv (every rank must say the same) */

@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 
+#include "band_march.h"
 #include "gather.h"
 #include "gemm_tc_host.h"
 #include "host_stage.h"
@@ -234,6 +235,12 @@ struct tf_plan {
     DevBuf<unsigned> words_f, words_a;
     tfk::LineParams par;
   } lines;
+  // band-marching executor (both operators are banded)
+  struct Band {
+    int block = 0;  // rows per block; 0: not taken
+    DevBuf<int> quads_f, quads_a;
+    tfk::BandParams par;
+  } band;
   // schedule mode
   DevBuf<int> s_ptr2, s_id, s_type, s_ker;
   int s_n1 = 0;
@@ -591,6 +598,53 @@ int run_lines(tf_plan &p, const float *C, float *D, int y_begin, int y_end, cuda
   return TF_OK;
 }
 
+// Band-marching executor: taken when both operators of an SpMM-SpMM chain are banded and no grid was recognised.
+int build_band(tf_plan &p, const tf_csr &F, const tf_csr &A, bool same, int sm_count) {
+  int reach_a = 0, pairs_a = 0, reach_f = 0, pairs_f = 0;
+  if (!tf::band_shape(A.m, A.n, A.ap, A.ai, &reach_a, &pairs_a)) return TF_OK;
+  reach_f = reach_a; pairs_f = pairs_a;
+  if (!same && !tf::band_shape(F.m, F.n, F.ap, F.ai, &reach_f, &pairs_f)) return TF_OK;
+  const int block = std::max(reach_a, reach_f) <= 64 ? 64 : 128;
+  if (tfk::band_smem(block, pairs_f, pairs_a, same) > 226 * 1024) return TF_OK;
+  tf_plan::Band &K = p.band;
+  tf::BandOp op;
+  tf::build_band_operator(F.m, F.ap, F.ai, F.ax, block, pairs_f, op);
+  int rc = K.quads_f.upload(op.quads);
+  if (rc == TF_OK && !same) {
+    tf::build_band_operator(A.m, A.ap, A.ai, A.ax, block, pairs_a, op);
+    rc = K.quads_a.upload(op.quads);
+  }
+  if (rc == TF_OK) rc = zero_state(p);
+  if (rc != TF_OK) return rc;
+  std::memset(&K.par, 0, sizeof(K.par));
+  K.par.quads_f = reinterpret_cast<const int4 *>(K.quads_f.p);
+  K.par.quads_a = same ? K.par.quads_f : reinterpret_cast<const int4 *>(K.quads_a.p);
+  K.par.pairs_f = pairs_f; K.par.pairs_a = pairs_a;
+  K.par.same = same;
+  K.par.m = A.m; K.par.n_cols = p.n_cols;
+  K.block = block;
+  p.sm_count = sm_count;
+  return TF_OK;
+}
+
+// The blocks [block_begin, block_end) of rows of D.
+int run_band(tf_plan &p, const float *C, float *D, int block_begin, int block_end, cudaStream_t s) {
+  if (!(aligned(C, 16) && aligned(D, 16)))
+    return fail(TF_ERR_ARG, "this plan reads rows as 16-byte vectors and needs 16-byte aligned dense operands "
+                            "(build the plan with tile_slots < 0 otherwise)");
+  CUtensorMap tm;
+  TF_TRY(tfk::band_make_map(&tm, C, p.m, p.n_cols, p.band.block));
+  tfk::BandParams P = p.band.par;
+  P.out = D;
+  P.error = &p.state.p->error;
+  P.wait_limit = p.spin_limit;
+  P.block_begin = block_begin; P.block_end = block_end;
+  TF_CUDA(tfk::launch_band_march(tm, p.band.block, P, p.sm_count, s));
+  p.launches = 1;
+  return TF_OK;
+}
+int band_blocks(const tf_plan &p) { return (p.m + p.band.block - 1) / p.band.block; }
+
 // GeMM-SpMM on the balanced gather.  The two products may be taken in either order, D = A (B C) = (A B) C: the sparse
 // product reads one row of its operand per nonzero, so it is given the narrower one -- B where k < n_cols, else B C.
 // (Rows of B that do not start on 16-byte boundaries would be gathered value by value; then B C comes first.  So it does
@@ -730,6 +784,19 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
       rc = finish_plan(*p, o, sm_count, false);  // the staging buffer lowers the resident CTA count
       if (rc != TF_OK) return rc;
       pp.max_ctas = p->grid;
+    }
+  }
+  if (want_pipe && F && o.mode == TF_MODE_STREAM && o.lattice_march >= 0 && o.halo_rows == 0 && o.n_boundary == 0 && o.rows_per_block == 0 &&
+      o.slack_blocks < 0 && o.ctas_per_sm == 0 && o.tile_slots == 0 && o.tile_max_bz == 0 && o.tile_pipeline == 0) {
+    tf::LatticeOp grid;  // (star stencils on a 3-D grid march plane by plane)
+    rc = tf::analyse_lattice_operator(A->m, A->n, A->ap, A->ai, A->ax, 0, grid, true);
+    if (rc == TF_OK && !grid.ok) rc = build_band(*p, *F, *A, F == A, sm_count);
+    if (rc != TF_OK) return rc;
+    if (p->band.block) {
+      p->tile_info[0] = pt.bx; p->tile_info[1] = pt.by; p->tile_info[2] = pt.bz; p->tile_info[3] = pt.tiles();
+      p->tile_info[4] = ct.bx; p->tile_info[5] = ct.by; p->tile_info[6] = ct.bz; p->tile_info[7] = ct.tiles();
+      *out = p.release();
+      return TF_OK;
     }
   }
   // dense producer on the tensor cores: 128-row tiles, its K slices live in the same dynamic buffer
@@ -1015,18 +1082,18 @@ int run_host_pipeline(tf_plan &p, tfk::Params &P, const float *h_in, long long i
   return TF_OK;
 }
 
-// The same pipeline for plans that march: one launch per slab of planes (of lines on a 2-D grid).  A slab
-// [za, zb) reads the planes za - 2 .. zb + 1 of C and completes the planes [za, zb) of D, so the copies run two planes
-// ahead of the kernel and the output leaves slab by slab.  Pageable arrays go piece by piece through rings of
+// The same pipeline for plans that march: one launch per slab of planes (of lines on a 2-D grid, of blocks of rows down a
+// band).  A slab [za, zb) reads the planes za - 2 .. zb + 1 of C and completes the planes [za, zb) of D, so the copies run
+// two planes ahead of the kernel and the output leaves slab by slab.  Pageable arrays go piece by piece through rings of
 // pinned slots (host_stage.h).
 int run_host_march(tf_plan &p, const float *h_in, float *d_in, float *h_out, float *d_out) {
   tf_plan::March &M = p.march;
   TF_TRY(ensure_streams(p));
-  const bool lines = p.lines.on;
-  const int nz = lines ? p.lines.ny : M.nz;
-  const long long plane_rows = lines ? p.lines.nx : (long long)M.nx * M.ny;
-  // (lines: slabs of 2 MB, at most 32 -- smaller copies cost more than what they overlap)
-  const int ns = lines ? (int)std::max<long long>(1, std::min<long long>({32, nz / 8, (long long)p.m * p.n_cols * 4 >> 21}))
+  const bool lines = p.lines.on, band = p.band.block != 0;
+  const int nz = lines ? p.lines.ny : (band ? band_blocks(p) : M.nz);
+  const long long plane_rows = lines ? p.lines.nx : (band ? p.band.block : (long long)M.nx * M.ny);
+  // (lines and blocks: slabs of 2 MB, at most 32 -- smaller copies cost more than what they overlap)
+  const int ns = lines || band ? (int)std::max<long long>(1, std::min<long long>({32, nz / 8, (long long)p.m * p.n_cols * 4 >> 21}))
                                : (int)M.slabs.size();
   auto at = [&](int z) { return (size_t)std::min<long long>(p.m, z * plane_rows) * p.n_cols; };  // first float of plane z
   while ((int)p.ev_in.size() < ns) {
@@ -1040,8 +1107,8 @@ int run_host_march(tf_plan &p, const float *h_in, float *d_in, float *h_out, flo
   int planes_in = 0;
   long long launches = 0;
   for (int sl = 0; sl < ns; ++sl) {
-    const int z_begin = lines ? (int)((long long)nz * sl / ns) : M.slabs[sl].z_begin;
-    const int z_end = lines ? (int)((long long)nz * (sl + 1) / ns) : M.slabs[sl].z_end;
+    const int z_begin = lines || band ? (int)((long long)nz * sl / ns) : M.slabs[sl].z_begin;
+    const int z_end = lines || band ? (int)((long long)nz * (sl + 1) / ns) : M.slabs[sl].z_end;
     const int need = std::min(nz, z_end + 2);
     if (need > planes_in)
       TF_CUDA(p.host_pipe->upload(d_in + at(planes_in), h_in + at(planes_in), (at(need) - at(planes_in)) * sizeof(float), p.s_h2d));
@@ -1049,7 +1116,8 @@ int run_host_march(tf_plan &p, const float *h_in, float *d_in, float *h_out, flo
     TF_CUDA(cudaEventRecord(p.ev_in[sl], p.s_h2d));
     TF_CUDA(cudaStreamWaitEvent(p.s_run, p.ev_in[sl], 0));
     rc = lines ? run_lines(p, d_in, d_out, z_begin, z_end, p.s_run)
-               : run_march(p, d_in, d_out, M.slabs[sl].item_begin, M.slabs[sl].item_end, false, p.s_run);
+               : (band ? run_band(p, d_in, d_out, z_begin, z_end, p.s_run)
+                       : run_march(p, d_in, d_out, M.slabs[sl].item_begin, M.slabs[sl].item_end, false, p.s_run));
     if (rc != TF_OK) return rc;
     launches += p.launches;
     TF_CUDA(cudaEventRecord(p.ev_run[sl], p.s_run));
@@ -1282,6 +1350,7 @@ int tf_exec_spmm_spmm(tf_plan *p, const float *C, float *D, void *stream) {
   int rc = set_device(*p);
   if (rc != TF_OK) return rc;
   if (p->lines.on) return run_lines(*p, C, D, 0, p->lines.ny, (cudaStream_t)stream);
+  if (p->band.block) return run_band(*p, C, D, 0, band_blocks(*p), (cudaStream_t)stream);
   if (march_usable(*p, C, D)) return run_march(*p, C, D, 0, p->march.n_items, false, (cudaStream_t)stream);
   if (p->g_second.on) return run_gather_spmm_spmm(*p, C, D, (cudaStream_t)stream);
   tfk::Params P = base_params(*p);
@@ -1389,6 +1458,10 @@ int tf_exec_phase(tf_plan *p, int phase, const float *in0, const float *in1, int
     p->launches = 0;
     return phase == 1 ? run_lines(*p, in0, D, 0, p->lines.ny, (cudaStream_t)stream) : TF_OK;
   }
+  if (p->band.block) {
+    p->launches = 0;
+    return phase == 1 ? run_band(*p, in0, D, 0, band_blocks(*p), (cudaStream_t)stream) : TF_OK;
+  }
   if (p->g_second.on) {  // no exchange: phase 1 is the whole chain
     p->launches = 0;
     if (phase != 1) return TF_OK;
@@ -1495,12 +1568,12 @@ int tf_spmm_spmm_host(tf_plan *p, const float *C, float *D) {
   int rc = set_device(*p);
   if (rc != TF_OK) return rc;
   const size_t nd = (size_t)p->m * p->n_cols;
-  if (!p->march.slabs.empty() || (p->lines.on && nd * sizeof(float) >= ((size_t)1 << 20))) {
+  if (!p->march.slabs.empty() || ((p->lines.on || p->band.block) && nd * sizeof(float) >= ((size_t)1 << 20))) {
     const size_t nin = (size_t)p->first_cols * p->n_cols;
     if (p->h_in0.n < nin) rc = p->h_in0.alloc(nin);
     if (rc == TF_OK && p->h_out.n < nd) rc = p->h_out.alloc(nd);
     if (rc != TF_OK) return rc;
-    if (p->lines.on || march_usable(*p, p->h_in0.p, p->h_out.p)) {
+    if (p->lines.on || p->band.block || march_usable(*p, p->h_in0.p, p->h_out.p)) {
       rc = run_host_march(*p, C, p->h_in0.p, D, p->h_out.p);
       if (rc != TF_OK) return rc;
       return tf_plan_status(p, nullptr);

@@ -1,0 +1,164 @@
+// SpMM-SpMM on banded operators (band_march.h): D = A * (F * C), one launch, T = F * C in shared memory.
+//
+// A CTA takes 32 dense columns (128 bytes of a row) and a range of rows and marches down the band in blocks of as many rows
+// as a nonzero can be away from the diagonal (64, or 128).  A ring of four blocks of C and one of four blocks of T hold
+// whatever a row can name: in step s the CTA computes block s of T from the blocks s - 1 .. s + 1 of C and block s - 2 of D
+// from the blocks s - 3 .. s - 1 of T, while TMA brings block s + 2 of C and the nonzeros of the rows of that block (a ring
+// of five, because block s - 2 is still being read).  The two products of a step do not depend on each other, so a step has
+// one barrier.
+// A warp works on four rows at a time, eight lanes with a float4 each per row: a quarter-warp reads one row of 128 bytes,
+// which is free of bank conflicts whatever rows are named.  What bounds the kernel is that shared memory pipe: one
+// wavefront per nonzero, product and 32 columns, and an eighth of one for the nonzero itself.  (Read from global memory,
+// the nonzeros took their warps to L2 for every four rows, since the rings leave no L1: 168 us instead of 104 for
+// n = 200 003, 12 nonzeros within 40 of the diagonal, 96 columns; the tile pipeline takes 150.)
+// Products are added in CSR order with fused multiply-adds from zero, and nothing is multiplied that is not stored, so
+// results are bit for bit those of the CSR executors.
+#include <algorithm>
+
+#include "band_march.h"
+#include "gemm_tc.cuh"
+#include "gemm_tc_host.h"
+
+namespace tfk {
+
+namespace {
+
+constexpr int kBandThreads = 512, kBandSlots = 5;
+
+// Four rows of one product: row (lane >> 3) of the four that start at `row`, this lane's four columns.  ring: the operand;
+// quads: the nonzeros of the block that the rows belong to.
+template <int S>
+__device__ __forceinline__ float4 band_row(const int4 *quads, int pairs, int row, const char *ring, int lane) {
+  constexpr unsigned mask = 4u * S * 128u - 1;
+  const int r = row + (lane >> 3);
+  const int4 *q = quads + (r & (S - 1));
+  const int base = r * 128;  // (modulo the ring, which is a power of two)
+  const char *col = ring + (lane & 7) * 16;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int k = 0; k < pairs; ++k) {
+    const int4 e = q[k * S];
+    const float4 x = *reinterpret_cast<const float4 *>(col + ((unsigned)(base + (e.x & ~1)) & mask));
+    const float4 y = *reinterpret_cast<const float4 *>(col + ((unsigned)(base + (e.z & ~1)) & mask));
+    if (!(e.x & 1)) {
+      const float v = __int_as_float(e.y);
+      acc.x = fmaf(v, x.x, acc.x); acc.y = fmaf(v, x.y, acc.y); acc.z = fmaf(v, x.z, acc.z); acc.w = fmaf(v, x.w, acc.w);
+    }
+    if (!(e.z & 1)) {
+      const float v = __int_as_float(e.w);
+      acc.x = fmaf(v, y.x, acc.x); acc.y = fmaf(v, y.y, acc.y); acc.z = fmaf(v, y.z, acc.z); acc.w = fmaf(v, y.w, acc.w);
+    }
+  }
+  return acc;
+}
+
+__device__ __forceinline__ void bulk_load(void *smem, const void *src, unsigned bytes, unsigned long long *bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+
+template <int S>
+__global__ void __launch_bounds__(kBandThreads, S == 64 ? 2 : 1)
+band_march_kernel(const __grid_constant__ CUtensorMap tm_c, const BandParams P) {
+  constexpr unsigned kRing = 4u * S * 128u;
+  constexpr int kWarps = kBandThreads / 32;
+  extern __shared__ char dyn[];
+  __shared__ unsigned long long full[4];
+  char *c_ring = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~(uintptr_t)1023);
+  char *t_ring = c_ring + kRing;
+  const unsigned bytes_f = (unsigned)P.pairs_f * S * 16, bytes_a = P.same ? 0u : (unsigned)P.pairs_a * S * 16;
+  char *f_ring = t_ring + kRing, *a_ring = P.same ? f_ring : f_ring + kBandSlots * bytes_f;
+  const unsigned step_a = P.same ? bytes_f : bytes_a;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int chunk = blockIdx.x % P.chunks, seg = blockIdx.x / P.chunks;
+  const int jb = P.block_begin + seg * P.seg_blocks, je = min(P.block_end, jb + P.seg_blocks);
+  const int col0 = chunk * 32, col = col0 + (lane & 7) * 4;
+  const int first = max(0, jb - 2), end = min(P.blocks, je + 2);  // blocks of C that the segment reads
+  if (tid == 0) {
+    for (int i = 0; i < 4; ++i) mbar_init(&full[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  auto load = [&](int b) {
+    unsigned long long *bar = &full[b & 3];
+    mbar_expect_tx(bar, S * 128 + bytes_f + bytes_a);
+    tma_load_2d(c_ring + (size_t)(b & 3) * (S * 128), &tm_c, col0, b * S, bar);
+    bulk_load(f_ring + (b % kBandSlots) * bytes_f, P.quads_f + (size_t)b * P.pairs_f * S, bytes_f, bar);
+    if (bytes_a) bulk_load(a_ring + (b % kBandSlots) * bytes_a, P.quads_a + (size_t)b * P.pairs_a * S, bytes_a, bar);
+  };
+  int issued = first;
+  if (tid == 0)
+    for (; issued < min(end, jb + 1); ++issued) load(issued);
+  int landed = first;  // blocks that have arrived
+  bool ok = true;
+  for (int s = jb - 1; s <= je + 1; ++s) {
+    if (tid == 0 && s + 2 >= issued && s + 2 < end) { load(s + 2); issued = s + 3; }
+    for (; ok && landed < min(end, s + 2); ++landed)
+      ok = mbar_wait(&full[landed & 3], (unsigned)((landed - first) >> 2) & 1u, P.wait_limit);
+    if (ok && s >= 0 && s < P.blocks && s <= je) {
+      const int4 *quads = reinterpret_cast<const int4 *>(f_ring + (s % kBandSlots) * bytes_f);
+#pragma unroll
+      for (int q = 0; q < S / 4; q += kWarps) {
+        const int row = s * S + 4 * (q + warp);
+        const float4 t = band_row<S>(quads, P.pairs_f, row, c_ring, lane);
+        *reinterpret_cast<float4 *>(t_ring + ((unsigned)((row + (lane >> 3)) * 128) & (kRing - 1)) + (lane & 7) * 16) = t;
+      }
+    }
+    if (ok && s - 2 >= jb) {
+      const int4 *quads = reinterpret_cast<const int4 *>(a_ring + ((s - 2) % kBandSlots) * step_a);
+#pragma unroll
+      for (int q = 0; q < S / 4; q += kWarps) {
+        const int row = (s - 2) * S + 4 * (q + warp), mine = row + (lane >> 3);
+        const float4 d = band_row<S>(quads, P.same ? P.pairs_f : P.pairs_a, row, t_ring, lane);
+        if (mine < P.m && col < P.n_cols) *reinterpret_cast<float4 *>(P.out + (size_t)mine * P.n_cols + col) = d;
+      }
+    }
+    if (__syncthreads_or(!ok)) { ok = false; break; }
+  }
+  if (!ok && tid == 0) {
+    // a wait ran out: no copy may outlive the CTA, so wait (again with a limit) for those in flight
+    for (int b = max(first, issued - 4); b < issued; ++b)
+      mbar_wait(&full[b & 3], (unsigned)((b - first) >> 2) & 1u, P.wait_limit);
+    atomicExch(P.error, 1);
+  }
+}
+
+}  // namespace
+
+int band_make_map(CUtensorMap *out, const float *c, long long rows, int n_cols, int block) {
+  return tc_make_map(out, c, rows, n_cols, block, n_cols, false);
+}
+
+size_t band_smem(int block, int pairs_f, int pairs_a, bool same) {
+  return 1024 + (size_t)block * (2 * 4 * 128 + kBandSlots * 16 * (size_t)(pairs_f + (same ? 0 : pairs_a)));
+}
+
+template <int S>
+static cudaError_t launch(const CUtensorMap &tm_c, BandParams &p, int sm_count, cudaStream_t s) {
+  p.chunks = (p.n_cols + 31) / 32;
+  p.blocks = (p.m + S - 1) / S;
+  const int n = p.block_end - p.block_begin;
+  if (n <= 0) return cudaSuccess;
+  const size_t smem = band_smem(S, p.pairs_f, p.pairs_a, p.same);
+  const long long resident = (long long)sm_count * (S == 64 && smem <= 112 * 1024 ? 2 : 1);
+  // A segment of n blocks of D takes n + 3 steps; as many segments as give the fewest steps over the rounds of resident CTAs.
+  long long best = -1;
+  for (int k = 1; k <= n; ++k) {
+    const int len = (n + k - 1) / k;
+    const long long segs = (n + len - 1) / len, rounds = (segs * p.chunks + resident - 1) / resident;
+    const long long t = rounds * (len + 3);
+    if (best < 0 || t < best) { best = t; p.seg_blocks = len; }
+    if (len == 1) break;
+  }
+  cudaError_t e = cudaFuncSetAttribute((const void *)band_march_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const long long ctas = (long long)((n + p.seg_blocks - 1) / p.seg_blocks) * p.chunks;
+  band_march_kernel<S><<<(unsigned)ctas, kBandThreads, smem, s>>>(tm_c, p);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_band_march(const CUtensorMap &tm_c, int block, BandParams &p, int sm_count, cudaStream_t s) {
+  return block == 64 ? launch<64>(tm_c, p, sm_count, s) : launch<128>(tm_c, p, sm_count, s);
+}
+
+}  // namespace tfk
