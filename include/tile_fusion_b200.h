@@ -365,6 +365,9 @@ int tf_permute_csr(int m, const int *ap, const int *ai, const float *ax, const i
  * the process on a bad file; here a bad file is TF_ERR_ARG / TF_ERR_UNSUPPORTED with a message. */
 int tf_read_matrix(const char *path, int expand_symmetric, int *m, int *n, long long *nnz, int **ap, int **ai,
                    float **ax);
+/* Checksum over every step-th column id and value of a CSR matrix, in order (the plan cache of the README-level
+ * executors keys on it).  0 for bad arguments.  No counterpart in the reference. */
+unsigned long long tf_csr_checksum(const int *ai, const float *ax, long long nnz, long long step);
 /* Dense matrix from a Matrix Market array file (the feature matrices of the GCN demos,
  * get_dense_matrix_from_parameter, Fusion_Utils.cpp:274-283), returned row-major (malloc'd, tf_free). */
 int tf_read_dense_mtx(const char *path, int *rows, int *cols, float **data);

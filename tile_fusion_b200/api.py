@@ -15,6 +15,7 @@ stream).  Everything executes in the CUDA library; there is no CPU fallback.
 from __future__ import annotations
 
 import ctypes as C
+import math
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -60,8 +61,8 @@ class CSRMatrix:
         make a new CSRMatrix for new values."""
         nnz = self.nnz
         step = max(1, nnz // 2048)
-        return (self.M, self.N, nnz, int(self.Ai[::step].astype(np.int64).sum()),
-                self.Ax[::step].tobytes().__hash__(), self.Ap.ctypes.data, self.Ai.ctypes.data, self.Ax.ctypes.data)
+        ai, ax = self.Ai.ctypes.data, self.Ax.ctypes.data
+        return self.M, self.N, nnz, _lib.lib().tf_csr_checksum(ai, ax, nnz, step), self.Ap.ctypes.data, ai, ax
 
 
 class Matrix:
@@ -77,7 +78,7 @@ class Matrix:
             if not (Data.is_cuda and Data.is_contiguous() and Data.dtype.is_floating_point and Data.element_size() == 4):
                 raise ValueError("Matrix: device data must be a contiguous float32 CUDA tensor")
             self.on_device = True
-        if int(np.prod(Data.shape)) != self.M * self.N:
+        if math.prod(Data.shape) != self.M * self.N:
             raise ValueError("Matrix: Data must hold M*N values")
         self.Data = Data
 
@@ -335,7 +336,8 @@ def spMMSpMMExecutor(A: CSRMatrix, B: CSRMatrix, C_: Matrix, D: Matrix, schedule
         raise ValueError("spMMSpMMExecutor: C and D must both be host or both be device data")
     m = _mode_for(schedule, mode)
     same = B is A
-    key = ("ss", A.fingerprint(), B.fingerprint(), C_.N, m, id(schedule) if m == MODE_SCHEDULE else 0)
+    fa = A.fingerprint()
+    key = ("ss", fa, fa if same else B.fingerprint(), C_.N, m, id(schedule) if m == MODE_SCHEDULE else 0)
     plan = _cached_plan(key, lambda: Plan("spmm_spmm", A, B=None if same else B, n_cols=C_.N, mode=m,
                                           schedule=schedule if m == MODE_SCHEDULE else None))
     if C_.on_device:
