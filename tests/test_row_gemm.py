@@ -66,3 +66,30 @@ def test_grid_host_call_in_pieces(built_lib, dims, k, n_cols):
         np.testing.assert_array_equal(dh, d.cpu().numpy())
     plan.close()
     _check(t, n, k, n_cols, 3, relu=True)[0].close()
+
+
+@pytest.mark.parametrize("dims", [(16, 8, 2), (18, 9, 5), (17, 10, 9), (33, 17, 6), (101, 66, 3)])
+@pytest.mark.parametrize("k,n_cols", [(64, 64), (20, 100), (17, 4), (128, 256)])
+def test_grid_one_product_march(built_lib, dims, k, n_cols):
+    """3-D grids: the sparse product on the one-product march.  Bit for bit the balanced gather (the same dense product in
+    front of either), even and odd x extents, with and without the ReLU, tiles and chunks cut off by the grid and the width."""
+    import torch
+    t = synth.laplacian(dims)
+    n = len(t[0]) - 1
+    A = api.CSRMatrix(n, n, *t)
+    b, w = torch.from_numpy(synth.uniform(5, (n, k))).cuda(), torch.from_numpy(synth.uniform(6, (k, n_cols))).cuda()
+    plans = [api.Plan("gemm_spmm", A, k=k, n_cols=n_cols, lattice_march=lm) for lm in (0, -1)]
+    assert plans[0].info()["threads"] == 128 and plans[1].info()["threads"] != 128
+    for relu in (False, True):
+        out = []
+        for p in plans:
+            d = torch.full((n, n_cols), float("nan"), device="cuda")
+            for _ in range(2):
+                p.gemm_spmm(b, w, d, relu=relu)
+            p.status()
+            out.append(d)
+        assert torch.equal(*out)
+        want = _scipy(t, n) @ (b.double() @ w.double()).cpu().numpy()
+        common.assert_close(out[0].cpu().numpy(), np.maximum(want, 0) if relu else want, f"{dims} {k} {n_cols}")
+    for p in plans:
+        p.close()

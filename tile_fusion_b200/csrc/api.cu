@@ -217,6 +217,8 @@ struct tf_plan {
     DevBuf<unsigned> pcls_f, pcls_a;
     std::vector<float> dict_f, dict_a;   // host copies: the dictionaries travel as kernel parameters
     DevBuf<int4> items;
+    DevBuf<int4> star_items;         // GeMM-SpMM in two launches: the items of the one-product kernel
+    int n_star = 0;
     int first_idle_sm = INT_MAX;
     int n_boundary = 0;              // rows of the neighbours' halo that this rank produces (phase 0)
     DevBuf<int> b_ap, b_ai;
@@ -389,6 +391,15 @@ void build_segments(tf_plan &p, int n_seg);
 
 static_assert(tf::kMarchMaxClasses == tfk::kMarchMaxClassesDev, "host and device class limits differ");
 
+std::vector<int4> march_items_raw(const std::vector<tf::MarchItem> &items) {
+  std::vector<int4> raw(2 * items.size());
+  for (size_t i = 0; i < items.size(); ++i) {
+    raw[2 * i] = make_int4(items[i].x0, items[i].y0, items[i].zs, items[i].ze);
+    raw[2 * i + 1] = make_int4(items[i].c0, items[i].flags, 0, 0);
+  }
+  return raw;
+}
+
 // Plane-marching executor: taken when both operators of an SpMM-SpMM chain are star stencils on the same
 // grid (lattice.cpp).  The general plan is built as well and serves calls whose operands are not 16-byte
 // aligned.
@@ -456,13 +467,7 @@ int build_march(tf_plan &p, const tf_csr *Fp, const tf_csr &A, int halo_rows, in
       M.slabs.push_back(tf_plan::March::Slab{b, (int)M.host_items.size(), za, zb});
     }
   }
-  std::vector<int4> raw(2 * M.host_items.size());
-  for (size_t i = 0; i < M.host_items.size(); ++i) {
-    const tf::MarchItem &it = M.host_items[i];
-    raw[2 * i] = make_int4(it.x0, it.y0, it.zs, it.ze);
-    raw[2 * i + 1] = make_int4(it.c0, it.flags, 0, 0);
-  }
-  rc = M.items.upload(raw);
+  rc = M.items.upload(march_items_raw(M.host_items));
   if (rc == TF_OK) rc = M.pcls_f.upload(lf.patch_cls);
   M.dict_f = lf.dict;
   M.same = Fp == &A && halo_rows == 0;
@@ -528,6 +533,30 @@ int run_march(tf_plan &p, const float *C, float *D, int item_begin, int item_end
   const bool keep_free = !with_halo && p.halo_rows > 0;
   Q.first_idle_sm = keep_free ? M.first_idle_sm : INT_MAX;
   TF_CUDA(tfk::launch_lattice_march(keep_free ? M.grid : std::min(M.grid, std::max(1, item_end - item_begin)), tm, tm_last, Q, s));
+  p.launches = 1;
+  return TF_OK;
+}
+
+// D = A * T with the one-product march, T in the plan's intermediate (with a row to spare behind it).
+int run_star(tf_plan &p, float *D, bool relu, cudaStream_t s) {
+  tf_plan::March &M = p.march;
+  CUtensorMap tm;
+  const int mr = tfk::march_make_map(&tm, p.inter.p, p.n_cols, M.nx, M.ny, M.ny, M.nz, tfk::kMarchH + 2);
+  if (mr != 0) return fail(TF_ERR_CUDA, "cuTensorMapEncodeTiled failed for the intermediate (code " + std::to_string(mr) + ")");
+  tfk::MarchParams Q;
+  std::memset(&Q, 0, sizeof(Q));
+  Q.pcls_a = M.pcls_a.p;
+  std::memcpy(Q.dict_a, M.dict_a.data(), std::min(sizeof(Q.dict_a), M.dict_a.size() * sizeof(float)));
+  Q.ncls_a = M.ncls_a;
+  Q.out = D;
+  Q.items = M.star_items.p;
+  Q.item_end = M.n_star;
+  Q.st = M.st.p;
+  Q.nx = M.nx; Q.ny = M.ny; Q.nz = M.nz;
+  Q.pnx = (M.nx + 1) / 2; Q.pny = (M.ny + 1) / 2;
+  Q.n_cols = p.n_cols;
+  Q.wait_limit = p.spin_limit;
+  TF_CUDA(tfk::launch_star_march(std::min(M.n_star, p.sm_count * tfk::star_ctas_per_sm()), tm, Q, relu, s));
   p.launches = 1;
   return TF_OK;
 }
@@ -655,7 +684,7 @@ int make_gemm_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &A, const tf
   p->ld_t = (width + 3) / 4 * 4;
   const size_t wn = (size_t)tfk::row_gemm_pad_n(p->n_cols) * tfk::row_gemm_pad_k(p->k_dim);
   int rc = p->g_second.build(A, width, std::max(p->k_dim, p->n_cols), sm_count, tiled ? 16 : 0);
-  if (rc == TF_OK) rc = p->inter.alloc((size_t)p->m * p->ld_t);
+  if (rc == TF_OK) rc = p->inter.alloc((size_t)(p->m + 1) * p->ld_t);  // (the one-product march may read one row more)
   if (rc == TF_OK) rc = p->w_hi.alloc(wn);
   if (rc == TF_OK) rc = p->w_lo.alloc(wn);
   if (rc == TF_OK) rc = zero_state(*p);
@@ -665,6 +694,15 @@ int make_gemm_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &A, const tf
   if (tiled && o.lattice_march >= 0 && p->n_cols % 4 == 0) {
     rc = build_march(*p, nullptr, A, 0, sm_count, {});
     if (rc != TF_OK) return rc;
+    tf_plan::March &M = p->march;
+    if (M.on) {
+      std::vector<tf::MarchItem> items;
+      tf::build_march_items(M.nx, M.ny, 0, M.nz, p->n_cols, tfk::kMarchW, tfk::kMarchH, tfk::kMarchCols,
+                            sm_count * tfk::star_ctas_per_sm(), 1, items);
+      rc = M.star_items.upload(march_items_raw(items));
+      if (rc != TF_OK) return rc;
+      M.n_star = (int)items.size();
+    }
   }
   p->sm_count = sm_count;
   *out = p.release();
@@ -1360,7 +1398,7 @@ int tf_exec_spmm_spmm(tf_plan *p, const float *C, float *D, void *stream) {
 
 // GeMM-SpMM on a grid operator: the dense producer writes all rows of T (one launch of the tensor-core kernel), the
 // marching kernel consumes them (items [item_begin, item_end)).
-int run_gemm_march(tf_plan &p, const float *B, const float *W, int w_transposed, float *D, bool produce, int item_begin,
+int run_gemm_march(tf_plan &p, const float *B, const float *W, int w_transposed, bool relu, float *D, bool produce, int item_begin,
                    int item_end, bool with_halo, cudaStream_t s) {
   long long launches = 0;
   if (produce) {
@@ -1370,13 +1408,18 @@ int run_gemm_march(tf_plan &p, const float *B, const float *W, int w_transposed,
     if (rc != TF_OK) return rc;
     launches = 2;   // weight split + producer
   }
+  if (p.march.n_star > 0) {
+    int rc = run_star(p, D, relu, s);
+    p.launches += launches;
+    return rc;
+  }
   int rc = run_march(p, p.inter.p, D, item_begin, item_end, with_halo, s);
   p.launches += launches;
   return rc;
 }
 
 bool gemm_march_usable(const tf_plan &p, const float *B, const float *D, int relu) {
-  return p.chain == 1 && p.march.on && p.march.identity_first && !relu && aligned(B, 16) && aligned(D, 16);
+  return p.chain == 1 && p.march.on && p.march.identity_first && (!relu || p.march.n_star > 0) && aligned(B, 16) && aligned(D, 16);
 }
 
 int tf_exec_gemm_spmm(tf_plan *p, const float *B, const float *W, int w_transposed, int relu, float *D,
@@ -1387,7 +1430,7 @@ int tf_exec_gemm_spmm(tf_plan *p, const float *B, const float *W, int w_transpos
   int rc = set_device(*p);
   if (rc != TF_OK) return rc;
   if (gemm_march_usable(*p, B, D, relu))
-    return run_gemm_march(*p, B, W, w_transposed, D, true, 0, p->march.n_items, false, (cudaStream_t)stream);
+    return run_gemm_march(*p, B, W, w_transposed, relu != 0, D, true, 0, p->march.n_items, false, (cudaStream_t)stream);
   if (p->g_second.on) return run_gather_gemm_spmm(*p, B, W, w_transposed, relu != 0, D, (cudaStream_t)stream);
   tfk::Params P = base_params(*p);
   P.in0 = B; P.in1 = W; P.out = D; P.w_transposed = w_transposed; P.relu = relu;
@@ -1447,9 +1490,13 @@ int tf_exec_phase(tf_plan *p, int phase, const float *in0, const float *in1, int
     p->launches = 1;
     return TF_OK;
   }
+  if (phase == 2 && p->march.n_star > 0) {  // no exchange: phase 1 was the whole chain
+    p->launches = 0;
+    return TF_OK;
+  }
   if (phase > 0 && gemm_march_usable(*p, in0, D, relu))
-    return phase == 1 ? run_gemm_march(*p, in0, in1, w_transposed, D, true, 0, p->march.n_phase1, false, (cudaStream_t)stream)
-                      : run_gemm_march(*p, in0, in1, w_transposed, D, false, p->march.n_phase1, p->march.n_items, true,
+    return phase == 1 ? run_gemm_march(*p, in0, in1, w_transposed, relu != 0, D, true, 0, p->march.n_phase1, false, (cudaStream_t)stream)
+                      : run_gemm_march(*p, in0, in1, w_transposed, relu != 0, D, false, p->march.n_phase1, p->march.n_items, true,
                                        (cudaStream_t)stream);
   if (phase > 0 && p->chain == 0 && march_usable(*p, in0, D))
     return phase == 1 ? run_march(*p, in0, D, 0, p->march.n_phase1, false, (cudaStream_t)stream)

@@ -571,11 +571,126 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   }
 }
 
+// ---------------------------------------------------------------------------------------------------------------------
+// One product, D = A * T, for a star stencil on a 3-D grid: the sparse half of a GeMM-SpMM chain.  The same tiles, patches
+// and plane loads as above, but T is the plane that arrives (one point of rim instead of two, no ring, no exchange): a step
+// adds the z+ product to the rows of plane k - 1, stores them and starts those of plane k.  Memory bounds it, so what counts
+// is how many planes are on their way: four stages and four CTAs per SM.
+// Where nx is odd the point behind the last one of a line is set to zero as it is read; T ends with a spare row, which the
+// last pair of the last line reaches.
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int kStarStages = 4, kStarCtas = 4;
+constexpr int PS = W + 4, kStarBytes = PS * (H + 2) * kMarchCols * 4;  // x from x0 - 2 on (pairs), y from y0 - 1
+constexpr size_t kStarSmem = (size_t)kStarStages * kStarBytes + 2 * kStarStages * 8 + 1024;
+
+__global__ void __launch_bounds__(kMarchThreads, kStarCtas)
+star_march_kernel(const __grid_constant__ CUtensorMap tm, const MarchParams P, int relu) {
+  extern __shared__ char dyn[];
+  __shared__ int ctl[2];
+  const unsigned buf = (smem_u32(dyn) + 1023u) & ~1023u, full = buf + kStarStages * kStarBytes, empty = full + 8 * kStarStages;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, pi = lane >> 2, c4 = lane & 3;
+  volatile int *abort = &ctl[1];
+  if (tid == 0) {
+    for (int s = 0; s < kStarStages; ++s) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, kMarchThreads / 32); }
+    ctl[1] = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  unsigned n_use = 0, n_iss = 0;  // planes read, planes asked for (thread 0) so far
+  const int plane_words = P.pnx * P.pny;
+  const unsigned zero_a = 0x01010101u * (unsigned)P.ncls_a;
+  const size_t drow = (size_t)P.nx * P.n_cols, dplane = drow * P.ny;
+  for (;;) {
+    if (tid == 0) ctl[0] = atomicAdd(&P.st->ticket, 1);
+    __syncthreads();
+    const int it = P.item_begin + ctl[0];
+    if (it >= P.item_end) break;
+    const int4 ia = __ldg(P.items + 2 * it), ib = __ldg(P.items + 2 * it + 1);
+    const int x0 = ia.x, y0 = ia.y, zs = ia.z, ze = ia.w, c0col = ib.x;
+    const int steps = ze - zs + 2;  // planes zs - 1 .. ze
+    const int x = x0 + 2 * pi, y = y0 + 2 * warp, col = c0col + 4 * c4;
+    auto issue = [&](int step) {
+      const unsigned st = n_iss % kStarStages;
+      ++n_iss;
+      mbar_expect_tx(full + 8 * st, kStarBytes);
+      tma_load_plane(buf + st * kStarBytes, &tm, c0col, x0 / 2 - 1, y0 - 1, zs - 1 + step, full + 8 * st);
+    };
+    int asked = 0;  // (thread 0) planes of this item asked for
+    bool ok = true;
+    // a stage is filled again once every warp has read what was in it
+    auto refill = [&](int upto) {
+      for (; ok && asked < min(upto, steps); ++asked) {
+        if (n_iss >= (unsigned)kStarStages) ok = wait_or_abort(empty + 8 * (n_iss % kStarStages), (n_iss / kStarStages - 1) & 1u, P.wait_limit, abort);
+        if (ok) issue(asked);
+      }
+    };
+    unsigned live = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (x + (j & 1) < P.nx && y + (j >> 1) < P.ny && col < P.n_cols) live |= 1u << j;
+    const bool cut = x + 1 >= P.nx;  // the patch's second column does not exist
+    ClassColumn cls;
+    cls.init(P.pcls_a, x, y, P.nx, P.ny, P.pnx);
+    float *dptr = P.out + ((size_t)y * P.nx + x) * P.n_cols + col + (long long)(zs - 2) * (long long)dplane;
+    const int base0 = (y - y0 + 1) * (PS * 64) + pi * 64 + c4 * 16;
+    float4 prev[4], acc[4];
+    float czp[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { prev[j] = acc[j] = zero4(); czp[j] = 0.f; }
+    unsigned word = cls.at(zs - 1, P.nz, plane_words, zero_a), next = cls.at(zs, P.nz, plane_words, zero_a);
+    for (int step = 0; step < steps && ok; ++step) {
+      const int k = zs - 1 + step;
+      if (tid == 0) refill(step + kStarStages - 1);
+      const unsigned st = n_use % kStarStages;
+      if (!ok || !wait_or_abort(full + 8 * st, (n_use / kStarStages) & 1u, P.wait_limit, abort)) { ok = false; break; }
+      ++n_use;
+      const unsigned base = buf + st * kStarBytes + base0;
+      float4 own[4], nb[8];
+      load_own<PS, 2>(base, own);
+      load_nb<PS, 2>(base, nb);
+      if (cut) own[1] = own[3] = zero4();
+      const unsigned after = cls.at(k + 2, P.nz, plane_words, zero_a);
+      if (k - 1 >= zs) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float4 d = fma4(czp[j], own[j], acc[j]);
+          if (relu) d = make_float4(fmaxf(d.x, 0.f), fmaxf(d.y, 0.f), fmaxf(d.z, 0.f), fmaxf(d.w, 0.f));
+          if (live >> j & 1u) *reinterpret_cast<float4 *>(dptr + (j & 1) * (size_t)P.n_cols + (j >> 1) * drow) = d;
+        }
+      }
+      if (k >= zs && k < ze) patch_start(acc, czp, P.dict_a, word, prev, own, nb);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty + 8 * st);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) prev[j] = own[j];
+      word = next;
+      next = after;
+      dptr += dplane;
+    }
+    if (__syncthreads_or(!ok)) break;
+  }
+  // after a wait that ran out: copies still in flight must land before the shared memory is given up
+  __syncthreads();
+  if (tid == 0) {
+    if (ctl[1]) {
+      atomicExch(&P.st->error, 1);
+      for (unsigned q = n_iss > kStarStages ? n_iss - kStarStages : 0; q != n_iss; ++q)
+        mbar_wait(full + 8 * (q % kStarStages), (q / kStarStages) & 1u, P.wait_limit);
+    }
+    __threadfence();
+    const int f = atomicAdd(&P.st->finished, 1);
+    if (f == (int)gridDim.x - 1) {
+      P.st->ticket = 0;
+      P.st->finished = 0;
+      __threadfence();
+    }
+  }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, int lines, long long planes) {
+int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, int lines, long long planes, int box_lines) {
   static EncodeTiledFn fn = nullptr;
   if (!fn) {
     void *p = nullptr;
@@ -590,7 +705,7 @@ int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny,
   const cuuint64_t row = (cuuint64_t)n_cols * 4;
   cuuint64_t gdim[5] = {(cuuint64_t)n_cols, (cuuint64_t)((nx + 1) / 2), 2, (cuuint64_t)lines, (cuuint64_t)planes};
   cuuint64_t gstride[4] = {2 * row, row, row * nx, row * nx * ny};
-  cuuint32_t box[5] = {(cuuint32_t)kMarchCols, (cuuint32_t)((kMarchW + 4) / 2), 2, (cuuint32_t)(kMarchH + 4), 1};
+  cuuint32_t box[5] = {(cuuint32_t)kMarchCols, (cuuint32_t)((kMarchW + 4) / 2), 2, (cuuint32_t)box_lines, 1};
   cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<float *>(c), gdim, gstride, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -617,6 +732,15 @@ int march_ctas_per_sm() { return std::min(ctas_per_sm<false>(), ctas_per_sm<true
 cudaError_t launch_lattice_march(int grid, const CUtensorMap &tm_c, const CUtensorMap &tm_last, const MarchParams &p, cudaStream_t s) {
   if (march_ctas_per_sm() <= 0) return cudaErrorLaunchOutOfResources;
   (p.c ? lattice_march_kernel<true> : lattice_march_kernel<false>)<<<grid, kMarchThreads, kMarchSmemBytes, s>>>(tm_c, tm_last, p);
+  return cudaGetLastError();
+}
+
+int star_ctas_per_sm() { return kStarCtas; }
+
+cudaError_t launch_star_march(int grid, const CUtensorMap &tm, const MarchParams &p, bool relu, cudaStream_t s) {
+  cudaError_t e = cudaFuncSetAttribute((const void *)star_march_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStarSmem);
+  if (e != cudaSuccess) return e;
+  star_march_kernel<<<grid, kMarchThreads, kStarSmem, s>>>(tm, p, relu ? 1 : 0);
   return cudaGetLastError();
 }
 

@@ -44,10 +44,15 @@ struct MarchParams {
 };
 
 // Tensor map of C as a 5-D fp32 tensor (n_cols, ceil(nx / 2), 2, lines, planes) whose planes are nx * ny rows apart,
-// box = 16 columns x (W+4)/2 x 2 x (H+4) x 1.
-int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, int lines, long long planes);
+// box = 16 columns x (W+4)/2 x 2 x box_lines x 1.
+int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, int lines, long long planes,
+                   int box_lines = kMarchH + 4);
 int march_ctas_per_sm();
 // tm_last: the last plane without its last line where nx is odd, else as tm_c.
 cudaError_t launch_lattice_march(int grid, const CUtensorMap &tm_c, const CUtensorMap &tm_last, const MarchParams &p, cudaStream_t s);
+
+// One product D = A * T (p.out, p.pcls_a, p.dict_a): tm is a map of T with boxes of kMarchH + 2 lines.
+int star_ctas_per_sm();
+cudaError_t launch_star_march(int grid, const CUtensorMap &tm, const MarchParams &p, bool relu, cudaStream_t s);
 
 }  // namespace tfk
