@@ -62,7 +62,8 @@ class CSRMatrix:
         nnz = self.nnz
         step = max(1, nnz // 2048)
         ai, ax = self.Ai.ctypes.data, self.Ax.ctypes.data
-        return self.M, self.N, nnz, _lib.lib().tf_csr_checksum(ai, ax, nnz, step), self.Ap.ctypes.data, ai, ax
+        h = _lib.lib().tf_csr_checksum(ai, ax, nnz, step)
+        return self.M, self.N, nnz, h >> 32, h & 0xffffffff, self.Ap.ctypes.data, ai, ax
 
 
 class Matrix:
