@@ -38,7 +38,7 @@ constexpr int kRgSmemMax = 227 * 1024;
 constexpr int kRgEpiBytes = kRgEpiWarps * 2 * 32 * 128;  // two 32 x 32 blocks per warp
 
 struct RgShared {
-  unsigned long long raw[kRgMaxStages], split[kRgMaxStages], ready[kRgMaxStages], empty[kRgMaxStages];
+  unsigned long long raw[kRgMaxStages], ready[kRgMaxStages], empty[kRgMaxStages];
   unsigned long long acc_full[2], acc_empty[2], drained;
   unsigned tmem_base;
   int dead;
@@ -59,24 +59,16 @@ __device__ __forceinline__ unsigned rg_rank() {
 __device__ __forceinline__ void rg_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Arrive on a barrier of this CTA / of the even CTA of the pair.  A release at cluster scope waits for the thread's accesses
-// to reach the other SM, which costs a splitting warp half of its time (N = K = 256, 2.1 M rows: 1 410 us with it); so those
-// arrive in their own CTA, and in the odd CTA one thread that has nothing else to do passes the arrival on.
-__device__ __forceinline__ void rg_arrive(unsigned long long *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-template <bool RELEASE>
+// Arrive on the barrier of the even CTA of the pair.  What goes with the arrival is shared memory that the tensor cores read
+// through the async proxy: fence.proxy.async has completed the writes there before, each in its own SM.  (A release at
+// cluster scope would order the thread's other accesses too and costs a splitting warp half of its time: N = K = 256,
+// 2.1 M rows: 1 410 us with it, 1 228 with one thread of the odd CTA that passes local arrivals on, 1 075 like this, as
+// CUTLASS's ClusterBarrier::arrive has it.)
 __device__ __forceinline__ void rg_arrive_leader(unsigned long long *bar) {
-  if (RELEASE)
-    asm volatile(
-        "{\n\t.reg .b32 a;\n\t"
-        "mapa.shared::cluster.u32 a, %0, 0;\n\t"
-        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar)) : "memory");
-  else
-    asm volatile(
-        "{\n\t.reg .b32 a;\n\t"
-        "mapa.shared::cluster.u32 a, %0, 0;\n\t"
-        "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+  asm volatile(
+      "{\n\t.reg .b32 a;\n\t"
+      "mapa.shared::cluster.u32 a, %0, 0;\n\t"
+      "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar)) : "memory");
 }
 // Bounded wait that also leaves when another role of the CTA has given up.  CLUSTER: threads of the other CTA arrive too.
 template <bool CLUSTER = false>
@@ -148,8 +140,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   if (tid == 0) {
     for (int i = 0; i < stages; ++i) {
       mbar_init(&s.raw[i], 1);
-      mbar_init(&s.split[i], kRgSplitWarps);      // (odd CTA)
-      mbar_init(&s.ready[i], kRgSplitWarps + 1);  // (even CTA)
+      mbar_init(&s.ready[i], 2 * kRgSplitWarps);
       mbar_init(&s.empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -188,24 +179,17 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           if (++st == stages) { st = 0; ph ^= 1u; }
         }
       }
+      // the tensor core's arrivals on the stages of this CTA come from the other one too: the last of them must be in before
+      // the CTA may end
+      for (int i = 0; ok && i < issued; ++i) ok = rg_wait(&s.empty[i], i < st ? ph : ph ^ 1u, s, P.wait_limit);
       // a copy still in flight must not outlive the CTA (only after a wait ran out is one possible)
       if (s.dead)
         for (int i = 0; i < issued; ++i)
           for (int k = 0; k < P.wait_limit && !mbar_wait(&s.raw[i], (i < st ? ph : ph ^ 1u), 1); ++k) {}
     }
   } else if (warp == kRgEpiWarps + kRgSplitWarps + 1) {
-    // ---- products (even CTA); split stages passed on (odd CTA) ----
-    if (lane == 0 && rank == 1) {
-      int st = 0;
-      unsigned ph = 0;
-      bool ok = true;
-      for (int t = pair; t < P.tiles && ok; t += pairs)
-        for (int sl = 0; sl < P.n_slices; ++sl) {
-          if (!(ok = rg_wait(&s.split[st], ph, s, P.wait_limit))) break;
-          rg_arrive_leader<true>(&s.ready[st]);
-          if (++st == stages) { st = 0; ph ^= 1u; }
-        }
-    } else if (lane == 0) {
+    // ---- products (even CTA) ----
+    if (lane == 0 && rank == 0) {
       const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(N >> 3) << 17) | ((unsigned)(2 * kTcRows >> 4) << 24);
       int st = 0, buf = 0, uses = 0;  // uses: accumulators handed out so far
       unsigned ph = 0, acc_ph = 0;
@@ -287,7 +271,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read next by the tensor core
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) rg_arrive(rank == 0 ? &s.ready[st] : &s.split[st]);
+        if (lane == 0) rg_arrive_leader(&s.ready[st]);
         if (++st == stages) { st = 0; ph ^= 1u; }
       }
   } else {
@@ -299,7 +283,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     auto release = [&]() {  // the accumulator has been read: its next use may overwrite it
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) rg_arrive_leader<false>(&s.acc_empty[buf]);  // (nothing in memory goes with it)
+      if (lane == 0) rg_arrive_leader(&s.acc_empty[buf]);
     };
     auto next = [&]() {
       buf ^= 1;
