@@ -14,8 +14,10 @@
 // The tensor core cuts off what it adds to an accumulator instead of rounding it, so a chain of K / 8 sums drifts (rel.
 // error 2e-6 at K = 256, ten times that of fp32 FMAs).  Widths and depths that the ticket executor's tensor-core tile does
 // not take have always been multiplied with fp32 FMAs; for them the kernel has a second form that is as exact as those:
-// panels of up to 64 columns, an accumulator of its own for each K step of 8 (the small products first), and the four of a
-// slice are read back and added in registers.
+// panels of up to 64 columns, whose four accumulators are read back and added in registers after every slice.
+// The plain form keeps its chains short where tensor memory has room: up to 128 columns the K steps of a slice go round two
+// accumulators, up to 64 round four, the small products first (K = 256: rel. error 1.9e-6 with one, 8.8e-7 with two, 4.6e-7
+// with four; 262 144 rows, K = N = 64: 33.6 us with one, 36.3 with four).
 // All waits are bounded: the one that runs out sets the error flag, and every role leaves.
 #include "row_gemm.h"
 
@@ -135,6 +137,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   const unsigned rank = rg_rank();
   const int N = P.n_pad, half = N / 2, stage_bytes = rg_stage_bytes(N), stages = P.stages;
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int accs = PRECISE ? 4 : P.accs, acc_cols = PRECISE ? 64 : 256 / P.accs;  // accumulators of a tile, columns from one to the next
   char *epi = smem + stages * stage_bytes;
 
   if (tid == 0) {
@@ -213,17 +216,23 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           const unsigned d = s.tmem_base + (unsigned)(buf * 256);
           const unsigned b = smem_u32(smem + st * stage_bytes);
           const unsigned ah = b, al = b + kTcRows * 128, wh = b + 2 * kTcRows * 128, wl = wh + half * 128;
+          const unsigned fresh = PRECISE || sl == 0;
+          auto mma = [&](int j, int term, unsigned add) {  // K step j (eight TF32 values inside the swizzle row) of lo*hi, hi*lo, hi*hi
+            const unsigned o = j * 32;
+            rg_mma(d + (unsigned)((j & (accs - 1)) * acc_cols), umma_desc_sw128((term == 0 ? al : ah) + o),
+                   umma_desc_sw128((term == 1 ? wl : wh) + o), idesc, add);
+          };
+          if (accs > 1) {
 #pragma unroll
-          for (int j = 0; j < kTcKSlice / 8; ++j) {
-            const unsigned o = j * 32;  // eight TF32 values along K inside the swizzle row
-            if (PRECISE) {
-              rg_mma(d + j * 64, umma_desc_sw128(ah + o), umma_desc_sw128(wl + o), idesc, 0u);
-              rg_mma(d + j * 64, umma_desc_sw128(al + o), umma_desc_sw128(wh + o), idesc, 1u);
-              rg_mma(d + j * 64, umma_desc_sw128(ah + o), umma_desc_sw128(wh + o), idesc, 1u);
-            } else {
-              rg_mma(d, umma_desc_sw128(ah + o), umma_desc_sw128(wh + o), idesc, (sl | j) ? 1u : 0u);
-              rg_mma(d, umma_desc_sw128(ah + o), umma_desc_sw128(wl + o), idesc, 1u);
-              rg_mma(d, umma_desc_sw128(al + o), umma_desc_sw128(wh + o), idesc, 1u);
+            for (int term = 0; term < 3; ++term)
+#pragma unroll
+              for (int j = 0; j < kTcKSlice / 8; ++j) mma(j, term, fresh && term == 0 && j < accs ? 0u : 1u);
+          } else {  // in the order of gemm_tc.cuh: the same bits
+#pragma unroll
+            for (int j = 0; j < kTcKSlice / 8; ++j) {
+              mma(j, 2, fresh && j == 0 ? 0u : 1u);
+              mma(j, 1, 1u);
+              mma(j, 0, 1u);
             }
           }
           rg_commit(&s.empty[st]);
@@ -352,6 +361,14 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           rg_tmem_load(v, lanes + (unsigned)(buf * 256 + c));
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           rg_loaded(v);
+          for (int i = 1; i < accs; ++i) {
+            float a[32];
+            rg_tmem_load(a, lanes + (unsigned)(buf * 256 + i * acc_cols + c));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            rg_loaded(a);
+#pragma unroll
+            for (int q = 0; q < 32; ++q) v[q] += a[q];
+          }
           if (c + 32 >= N) release();
           if (c < P.n_real && row0 < P.m) put(v, c, row0);
         }
@@ -409,6 +426,7 @@ static int launch_panel(const float *X, int m, int K, int ld_x, const float *hi,
   P.m = m; P.n_pad = n_pad; P.n_real = n; P.n_slices = (K + kTcKSlice - 1) / kTcKSlice;
   P.tiles = (m + 2 * kTcRows - 1) / (2 * kTcRows);
   P.stages = rg_stages(n_pad);
+  P.accs = n_pad <= 64 ? 4 : (n_pad <= 128 ? 2 : 1);
   P.out = out; P.ld_out = ld_out; P.relu = relu ? 1 : 0;
   P.tma_store = ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   P.error = error; P.wait_limit = wait_limit;

@@ -8,7 +8,7 @@ struct RowGemmParams {
   const float *x;  // read directly where rows do not start on 16-byte boundaries (`direct`)
   float *out;
   int *error;
-  int m, n_real, n_pad, n_slices, tiles, stages, ld_out, k, ld_x;
+  int m, n_real, n_pad, n_slices, tiles, stages, accs, ld_out, k, ld_x;
   int direct, relu, tma_store, wait_limit;
 };
 
