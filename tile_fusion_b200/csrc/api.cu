@@ -102,9 +102,9 @@ struct DevGather {
     }
   }
   // n_cols: width of the dense operand the units are cut for; max_cols: widest one the operator will meet
-  int build(const tf_csr &A, int n_cols, int max_cols, int sm_count, int n_seg = 0) {
+  int build(const tf_csr &A, int n_cols, int max_cols, int sm_count, int n_seg = 0, int resident = tfk::kGatherResident) {
     tf::GatherPlan g;
-    tf::build_gather_plan(A.m, A.ap, A.ai, A.ax, sm_count * (tfk::kGatherResident / tfk::gather_group(n_cols)), g);
+    tf::build_gather_plan(A.m, A.ap, A.ai, A.ax, sm_count * (resident / tfk::gather_group(n_cols)), g);
     n_units = (int)g.units.size();
     n_empty = (int)g.empty_rows.size();
     partial_ld = (std::max(n_cols, max_cols) + 3) / 4 * 4;
@@ -1309,7 +1309,7 @@ int tf_plan_sddmm_spmm(const tf_csr *A, int kq, int nv, const tf_plan_opts *opts
   p->m = A->m; p->n_cols = nv; p->k_dim = kq;
   if (tfk::sddmm_gather_supported(kq, nv) && o.rows_per_block == 0 && o.ctas_per_sm == 0) {
     p->second.m = A->m; p->second.n = A->n;
-    rc = p->g_second.build(*A, 4 * tfk::sddmm_group(kq, nv), nv, sm_count);  // (units for as many groups of that size)
+    rc = p->g_second.build(*A, 4 * tfk::sddmm_group(kq, nv), nv, sm_count, 0, tfk::kSddmmResident);  // (units for groups of that size)
     if (rc == TF_OK) rc = zero_state(*p);
     if (rc != TF_OK) return rc;
     *out = p.release();

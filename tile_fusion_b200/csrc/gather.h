@@ -42,6 +42,7 @@ void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int
 namespace tfk {
 
 constexpr int kGatherResident = 768;  // threads of the gather kernel resident per SM
+constexpr int kSddmmResident = 512;   // and of the SDDMM kernel
 
 struct GatherParams {
   const int *cols;      // column | end bit

@@ -11,10 +11,13 @@ void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int
   out = GatherPlan();
   const long long nnz = ap[m];
   const long long cost = nnz + 2LL * m;
-  // One unit per resident group where that gives units of 32 to 256 nonzeros.  Shorter ones spend their time on the three
-  // dependent reads in front of the first product, longer ones leave the device idle at the end (R-MAT n = 200 000,
-  // degree 20, 64 columns, both products: 192 us with at most 128, 183 with 256, 253 with 512).
-  const int target = (int)std::min<long long>(256, std::max<long long>(32, cost / std::max(1, groups)));
+  // As many units as make whole rounds of the resident groups, of at most about 256 nonzeros: units take about equally long,
+  // so a round that only some groups have a unit in costs a whole one.  Shorter units spend their time on the three dependent
+  // reads in front of the first product (R-MAT n = 200 000, degree 20, 64 columns, both products: 192 us with 128, 183 with
+  // 256, 253 with 512, before the rounds were whole), so at least 32.  A unit is closed by the row that does not fit any more:
+  // half a row's cost, and three hundredths for luck, keep the last round from spilling over.
+  const double share = (double)cost / std::max(1, groups), rounds = std::max(1.0, std::ceil(share / 256));
+  const int target = (int)std::max(32.0, std::ceil(share / rounds * 1.03 + 0.5 * cost / std::max(1, m)));
   // A row at least this long is cut.  (Cutting only from twice that on: the same on large graphs, 25.4 instead of 22.7 us
   // at n = 20 000, where one long row is what the launch waits for.)
   const int long_row = target;
