@@ -17,7 +17,7 @@
 // Products of a row are added in CSR order with fused multiply-adds from zero, as in the reference's row loop
 // (SpMM_SpMM.cpp:211-248); only rows that were cut are added in pieces.
 //
-// Measured (R-MAT, n = 200 000, degree 20, both products of a chain): 64 columns 183 us (11.7 TB/s of row reads), where
+// Measured (R-MAT, n = 200 000, degree 20, both products of a chain): 64 columns 180 us (11.9 TB/s of row reads), where
 // the ticket executor took 784 (58 % of its warps' time at barriers behind long rows); 128 columns 306 us, 14 TB/s, which
 // is what L2 gives.  Eight reads in flight and three CTAs per SM: four CTAs spill (229 us), four reads and five CTAs 193.
 #include <algorithm>
