@@ -35,6 +35,10 @@ namespace {
 constexpr int kRgEpiWarps = 4, kRgSplitWarps = 8;
 constexpr int kRgThreads = 32 * (kRgEpiWarps + kRgSplitWarps + 2);
 constexpr int kRgMaxStages = 5;
+// Slices of B that are on their way to L2 in front of the loads, where a tile has many (2.1 M rows, K = N = 256: 1 085 us
+// without, 1 044 with 3; 8 and 20 are slower than 3; 500 009 rows, 256 -> 47: 234 and 229; where it has four or fewer the
+// request costs 1 to 2 %).
+constexpr int kRgAhead = 3, kRgAheadSlices = 8;
 constexpr int kRgPrecisePanel = 64;  // columns: four accumulators, twice, in 512 columns of tensor memory
 constexpr int kRgSmemMax = 227 * 1024;
 constexpr int kRgEpiBytes = kRgEpiWarps * 2 * 32 * 128;  // two 32 x 32 blocks per warp
@@ -169,9 +173,20 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       int st = 0, issued = 0;
       unsigned ph = 0;
       bool ok = true;
+      int pt = pair, psl = 0;
+      auto prefetch = [&]() {
+        if (P.direct || P.n_slices < kRgAheadSlices || pt >= P.tiles) return;
+        const int row = pt * 2 * kTcRows + (int)rank * kTcRows;
+        if (row < P.m)
+          asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"((unsigned long long)&tm_a),
+                       "r"(psl * kTcKSlice), "r"(row) : "memory");
+        if (++psl == P.n_slices) { psl = 0; pt += pairs; }
+      };
+      for (int i = 0; i < kRgAhead; ++i) prefetch();
       for (int t = pair; t < P.tiles && ok; t += pairs) {
         const int row = t * 2 * kTcRows + (int)rank * kTcRows;
         for (int sl = 0; sl < P.n_slices; ++sl) {
+          prefetch();
           if (issued >= stages && !(ok = rg_wait(&s.empty[st], ph ^ 1u, s, P.wait_limit))) break;
           char *b = smem + st * stage_bytes;
           mbar_expect_tx(&s.raw[st], (unsigned)((P.direct ? 0 : kTcRows * 128) + N * 128));
