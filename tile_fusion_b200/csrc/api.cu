@@ -826,9 +826,11 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
   }
   if (want_pipe && F && o.mode == TF_MODE_STREAM && o.lattice_march >= 0 && o.halo_rows == 0 && o.n_boundary == 0 && o.rows_per_block == 0 &&
       o.slack_blocks < 0 && o.ctas_per_sm == 0 && o.tile_slots == 0 && o.tile_max_bz == 0 && o.tile_pipeline == 0) {
-    tf::LatticeOp grid;  // (star stencils on a 3-D grid march plane by plane)
-    rc = tf::analyse_lattice_operator(A->m, A->n, A->ap, A->ai, A->ax, 0, grid, true);
-    if (rc == TF_OK && !grid.ok) rc = build_band(*p, *F, *A, F == A, sm_count);
+    tf::LatticeOp grid;  // (star stencils on a 3-D grid march plane by plane; looked for only where there is a band at all)
+    int reach = 0, pairs = 0;
+    const bool band = tf::band_shape(A->m, A->n, A->ap, A->ai, &reach, &pairs);
+    if (band) rc = tf::analyse_lattice_operator(A->m, A->n, A->ap, A->ai, A->ax, 0, grid, true);
+    if (rc == TF_OK && band && !grid.ok) rc = build_band(*p, *F, *A, F == A, sm_count);
     if (rc != TF_OK) return rc;
     if (p->band.block) {
       p->tile_info[0] = pt.bx; p->tile_info[1] = pt.by; p->tile_info[2] = pt.bz; p->tile_info[3] = pt.tiles();
