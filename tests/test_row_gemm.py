@@ -93,3 +93,45 @@ def test_grid_one_product_march(built_lib, dims, k, n_cols):
         common.assert_close(out[0].cpu().numpy(), np.maximum(want, 0) if relu else want, f"{dims} {k} {n_cols}")
     for p in plans:
         p.close()
+
+
+# both forms of the dense product, the sparse product in front of it, and the ticket executor's tile
+@pytest.mark.parametrize("k,n_cols,opts", [(64, 64, {}), (128, 256, {}), (64, 47, {}), (33, 64, {}), (32, 64, {}), (64, 64, {"ctas_per_sm": 1})])
+@pytest.mark.parametrize("bits", [0x7FFFFFFF, 0xFFFFFFFF, 0x7FC00000, 0x7F800001])
+def test_nan_stays_nan(built_lib, k, n_cols, opts, bits):
+    """A NaN of any payload -- 0x7FFFFFFF is the one that arithmetic on the GPU gives -- in B, in the weight, or made by the
+    gather in front of the dense product (0 * infinity) makes a NaN of every result that it enters, and of no other."""
+    import torch
+    n = 700
+    ap, ai, ax = _graph(n, 5, empty={0, n - 1}, hubs=((9, 600),))
+    hole = int(ai[ap[20]])  # row 20 multiplies the row of B that holds infinities by a zero
+    ax[ap[20]] = 0.0
+    A = _scipy((ap, ai, ax), n)
+    plan = api.Plan("gemm_spmm", api.CSRMatrix(n, n, ap, ai, ax), k=k, n_cols=n_cols, **opts)
+    b, w = torch.from_numpy(synth.uniform(3, (n, k))).cuda(), torch.from_numpy(synth.uniform(4, (k, n_cols))).cuda()
+    nan = torch.tensor([bits - (1 << 32) if bits >> 31 else bits], dtype=torch.int32, device="cuda").view(torch.float32)
+
+    def run(b, w):
+        d = torch.zeros((n, n_cols), device="cuda")
+        plan.gemm_spmm(b, w, d)
+        plan.status()
+        return d.cpu().numpy()
+
+    bn = b.clone()
+    bn[5, k - 1:], bn[300, 3:4] = nan, nan
+    hit = np.zeros(n, bool)
+    for r in (5, 300):
+        hit |= np.asarray((A[:, [r]] != 0).todense()).ravel()
+    hit |= np.isin(np.arange(n), [20]) & (hole in (5, 300))
+    got = run(bn, w)
+    np.testing.assert_array_equal(np.isnan(got), np.broadcast_to(hit[:, None], got.shape))
+    wn = w.clone()
+    wn[2, n_cols - 1:] = nan
+    got = run(b, wn)
+    want = np.zeros(got.shape, bool)
+    want[np.diff(ap) > 0, n_cols - 1] = True
+    np.testing.assert_array_equal(np.isnan(got), want)
+    bi = b.clone()
+    bi[hole, 1] = float("inf")
+    assert np.isnan(run(bi, w)[20]).all()
+    plan.close()

@@ -20,7 +20,7 @@ __global__ void split_weight_kernel(const float *__restrict__ W, int w_transpose
     const float w = w_transposed ? W[i] : W[(size_t)k * N + n];
     const float h = tf32_round(w);
     hi[i] = h;
-    lo[i] = tf32_round(w - h);
+    lo[i] = w - h;
   }
 }
 

@@ -1,6 +1,6 @@
 // T = B * W (optionally max(0, .)) for a tall fp32 B on the 5th-generation tensor cores, 3xTF32 inside.
 //
-// The arithmetic is that of gemm_tc.cuh, product by product: every operand is split as x = hi + lo, both rounded to TF32,
+// The arithmetic is that of gemm_tc.cuh, product by product: every operand is split as x = hi + lo, hi rounded to TF32,
 // and hi*hi + hi*lo + lo*hi is accumulated in fp32 in tensor memory.  What differs is that nothing waits for anything it
 // does not need:
 //   * Two CTAs on neighbouring SMs work on one tile of 256 rows with tcgen05.mma.cta_group::2.  Each holds 128 rows of B
@@ -290,7 +290,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           const float4 x = a[i];
           const float4 h = make_float4(tf32_round(x.x), tf32_round(x.y), tf32_round(x.z), tf32_round(x.w));
           hi[w + i * 32 * kRgSplitWarps] = h;
-          lo[w + i * 32 * kRgSplitWarps] = make_float4(tf32_round(x.x - h.x), tf32_round(x.y - h.y), tf32_round(x.z - h.z), tf32_round(x.w - h.w));
+          lo[w + i * 32 * kRgSplitWarps] = make_float4(x.x - h.x, x.y - h.y, x.z - h.z, x.w - h.w);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read next by the tensor core
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -413,7 +413,7 @@ __global__ void split_weight_pad_kernel(const float *__restrict__ W, int w_trans
     if (r < n && k < K) w = w_transposed ? __ldg(W + (size_t)r * K + k) : __ldg(W + (size_t)k * n + r);
     const float h = tf32_round(w);
     hi[i] = h;
-    lo[i] = tf32_round(w - h);
+    lo[i] = w - h;
   }
 }
 
