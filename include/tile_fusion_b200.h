@@ -127,6 +127,11 @@ typedef struct {
   int tensor_cores;       /* GeMM-SpMM dense product: 0 = tcgen05 3xTF32, in a launch of its own in front of (or, on
                              graphs with k < n_cols, behind) the sparse product up to N = 256, inside the ticket executor
                              where one of its options is given, K % 4 == 0 and N % 16 == 0;
+                             >0 = the same, with the sums of the ticket executor: A (B W), never (A B) W, one accumulator
+                             per tile, rows of 256 to 4096 nonzeros cut where its warps cut them.  Bit for bit its result
+                             where K % 4 == 0 and N % 16 == 0 (rows beyond 4096 nonzeros it adds up in no fixed order).
+                             For layers that are trained: a rounding error decides on which side of a ReLU an activation
+                             falls, and the gradient jumps there;
                              <0 = always the fp32 CUDA-core tile */
   int tile_pipeline;      /* SpMM-SpMM with both operators tiled and no ring requested: 0 = run the tiles on
                              the role-split pipeline (one CTA per SM: staging warps copy the next column

@@ -78,3 +78,25 @@ def test_other_operators(built_lib):
         common.assert_close(got.cpu().numpy(), want, "sw_gcn forward variants")
     af = torch.sparse.mm(adj, x)
     common.assert_close(torch.ops.sw_gcn.cachedSpMMGeMM(af, w, 4).cpu().numpy(), want, "cachedSpMMGeMM")
+
+
+@pytest.mark.parametrize("k,n_cols", [(64, 64), (32, 128), (128, 128), (100, 256), (36, 16)])
+def test_layers_keep_the_order_of_their_sums(built_lib, k, n_cols):
+    """Bit for bit the ticket executor's activations, whichever of k and n_cols is the larger: one that rounding puts on the
+    other side of zero is another gradient.  Rows around the 256 nonzeros that its warps share, up to the 4096 that a CTA takes."""
+    import torch
+    import tile_fusion_b200.sw_gcn  # noqa: F401
+    from tests.test_gather import _graph
+    from tile_fusion_b200 import api
+    n = 5000
+    t = _graph(n, 5, empty={0, 7, n - 1}, hubs=((9, 4096), (11, 255), (12, 256), (13, 257), (400, 513), (4000, 3000), (4001, 64)))
+    adj = torch.sparse_csr_tensor(*(torch.from_numpy(x) for x in t), size=(n, n)).cuda()
+    x, w = torch.from_numpy(synth.normal(2, (n, k))).cuda(), torch.from_numpy(synth.glorot(3, n_cols, k)).cuda()
+    ticket = api.Plan("gemm_spmm", api.CSRMatrix(n, n, *t), k=k, n_cols=n_cols, rows_per_block=128)
+    assert ticket.info()["items"] > 0
+    want = torch.full((n, n_cols), float("nan"), device="cuda")
+    ticket.gemm_spmm(x, w, want, w_transposed=True)
+    ticket.status()
+    with torch.no_grad():
+        assert torch.equal(torch.ops.sw_gcn.fusedGeMMSpMM(adj, x, w, [], 4), want)
+    ticket.close()

@@ -102,9 +102,10 @@ struct DevGather {
     }
   }
   // n_cols: width of the dense operand the units are cut for; max_cols: widest one the operator will meet
-  int build(const tf_csr &A, int n_cols, int max_cols, int sm_count, int n_seg = 0, int resident = tfk::kGatherResident) {
+  int build(const tf_csr &A, int n_cols, int max_cols, int sm_count, int n_seg = 0, int resident = tfk::kGatherResident,
+            bool ticket_sums = false) {
     tf::GatherPlan g;
-    tf::build_gather_plan(A.m, A.ap, A.ai, A.ax, sm_count * (resident / tfk::gather_group(n_cols)), g);
+    tf::build_gather_plan(A.m, A.ap, A.ai, A.ax, sm_count * (resident / tfk::gather_group(n_cols)), ticket_sums, g);
     n_units = (int)g.units.size();
     n_empty = (int)g.empty_rows.size();
     partial_ld = (std::max(n_cols, max_cols) + 3) / 4 * 4;
@@ -197,6 +198,7 @@ struct tf_plan {
   int ld_t = 0;              // floats per row of the intermediate: n_cols rounded up to whole float4
   DevBuf<float> g_pad;       // rows of C of a width that is no multiple of four, padded to ld_t
   bool spmm_first = false;   // GeMM-SpMM on the balanced gather: D = (A B) C instead of A (B C)
+  bool ticket_sums = false;  // every sum in the order of the ticket executor (tensor_cores > 0)
   size_t dyn_smem = 0;
   int tile_slots = 0;
   bool pipe = false;  // every item of phases 1 and 2 is a gather tile: run them on the tile pipeline
@@ -679,11 +681,12 @@ int band_blocks(const tf_plan &p) { return (p.m + p.band.block - 1) / p.band.blo
 // (Rows of B that do not start on 16-byte boundaries would be gathered value by value; then B C comes first.  So it does
 // on grids and bands: with a handful of nonzeros a row there is little to choose, and every consumer gives the same bits.)
 int make_gemm_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &A, const tf_plan_opts &o, bool tiled, int sm_count, tf_plan **out) {
-  p->spmm_first = !tiled && p->k_dim % 4 == 0 && p->k_dim < p->n_cols;
+  p->ticket_sums = o.tensor_cores > 0;
+  p->spmm_first = !tiled && !p->ticket_sums && p->k_dim % 4 == 0 && p->k_dim < p->n_cols;
   const int width = p->spmm_first ? p->k_dim : p->n_cols;
   p->ld_t = (width + 3) / 4 * 4;
   const size_t wn = (size_t)tfk::row_gemm_pad_n(p->n_cols) * tfk::row_gemm_pad_k(p->k_dim);
-  int rc = p->g_second.build(A, width, std::max(p->k_dim, p->n_cols), sm_count, tiled ? 16 : 0);
+  int rc = p->g_second.build(A, width, std::max(p->k_dim, p->n_cols), sm_count, tiled ? 16 : 0, tfk::kGatherResident, p->ticket_sums);
   if (rc == TF_OK) rc = p->inter.alloc((size_t)(p->m + 1) * p->ld_t);  // (the one-product march may read one row more)
   if (rc == TF_OK) rc = p->w_hi.alloc(wn);
   if (rc == TF_OK) rc = p->w_lo.alloc(wn);
@@ -1266,9 +1269,10 @@ int run_gather_gemm_spmm(tf_plan &p, const float *B, const float *W, int w_trans
   p.launches = 3;
   if (p.spmm_first) {
     TF_TRY(run_gather(p.g_second, B, k, aligned(B, 16), p.inter.p, p.ld_t, true, k, false, s));
-    return tfk::row_gemm(p.inter.p, p.m, k, p.ld_t, p.w_hi.p, p.w_lo.p, n, D, n, relu, &p.state.p->error, p.spin_limit, p.sm_count, s);
+    return tfk::row_gemm(p.inter.p, p.m, k, p.ld_t, p.w_hi.p, p.w_lo.p, n, D, n, relu, false, &p.state.p->error, p.spin_limit, p.sm_count, s);
   }
-  TF_TRY(tfk::row_gemm(B, p.m, k, k, p.w_hi.p, p.w_lo.p, n, p.inter.p, p.ld_t, false, &p.state.p->error, p.spin_limit, p.sm_count, s));
+  TF_TRY(tfk::row_gemm(B, p.m, k, k, p.w_hi.p, p.w_lo.p, n, p.inter.p, p.ld_t, false, p.ticket_sums, &p.state.p->error, p.spin_limit,
+                       p.sm_count, s));
   return run_gather(p.g_second, p.inter.p, p.ld_t, true, D, n, out16, n, relu, s);
 }
 
@@ -1405,8 +1409,8 @@ int run_gemm_march(tf_plan &p, const float *B, const float *W, int w_transposed,
   long long launches = 0;
   if (produce) {
     TF_CUDA(tfk::row_gemm_split(W, w_transposed, p.k_dim, p.n_cols, p.w_hi.p, p.w_lo.p, s));
-    int rc = tfk::row_gemm(B, p.m, p.k_dim, p.k_dim, p.w_hi.p, p.w_lo.p, p.n_cols, p.inter.p, p.n_cols, false, &p.march.st.p[0].error,
-                           p.spin_limit, p.sm_count, s);
+    int rc = tfk::row_gemm(B, p.m, p.k_dim, p.k_dim, p.w_hi.p, p.w_lo.p, p.n_cols, p.inter.p, p.n_cols, false, p.ticket_sums,
+                           &p.march.st.p[0].error, p.spin_limit, p.sm_count, s);
     if (rc != TF_OK) return rc;
     launches = 2;   // weight split + producer
   }
@@ -1592,7 +1596,7 @@ static int run_host_gemm_gather(tf_plan &p, const float *B, int w_transposed, bo
       TF_CUDA(cudaEventRecord(p.ev_in[s], p.s_h2d));
       TF_CUDA(cudaStreamWaitEvent(p.s_run, p.ev_in[s], 0));
       TF_TRY(tfk::row_gemm(src, (int)(in_to - in_done), k, k, p.w_hi.p, p.w_lo.p, n, p.inter.p + in_done * p.ld_t, p.ld_t, false,
-                           &p.state.p->error, p.spin_limit, p.sm_count, p.s_run));
+                           p.ticket_sums, &p.state.p->error, p.spin_limit, p.sm_count, p.s_run));
       in_done = in_to;
       ++p.launches;
     }

@@ -34,8 +34,9 @@ struct GatherPlan {
   size_t n_entries = 0;
   int n_slots = 0;
 };
-// `groups`: lane groups resident on the device, which sets how finely the work is cut.
-void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int groups, GatherPlan &out);
+// `groups`: lane groups resident on the device, which sets how finely the work is cut.  ticket_sums: rows are cut where the
+// warps of the ticket executor's CTA cut them and nowhere else, so that the sums are added in its order.
+void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int groups, bool ticket_sums, GatherPlan &out);
 
 }  // namespace tf
 

@@ -5,10 +5,11 @@
 #include <thread>
 
 #include "gather.h"
+#include "tf_internal.h"
 
 namespace tf {
 
-void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int groups, GatherPlan &out) {
+void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int groups, bool ticket_sums, GatherPlan &out) {
   out = GatherPlan();
   const long long nnz = ap[m];
   const long long cost = nnz + 2LL * m;
@@ -21,7 +22,7 @@ void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int
   const int target = (int)std::max(32.0, std::ceil(share / rounds * 1.03 + 0.5 * cost / std::max(1, m)));
   // A row at least this long is cut.  (Cutting only from twice that on: the same on large graphs, 25.4 instead of 22.7 us
   // at n = 20 000, where one long row is what the launch waits for.)
-  const int long_row = target;
+  const int long_row = ticket_sums ? kHeavyRowNnz : target;
   // rows and pieces first (nonzero ranges), entries afterwards
   struct Range { int pos, j0, j1, heavy; };
   std::vector<Range> plain, pieces;
@@ -40,13 +41,23 @@ void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int
     if (listed) out.rows.push_back(r);
     if (len >= long_row) {
       close();
-      // pieces of about sqrt(len): the group that adds them up last reads as many partial rows as a piece has gathers
-      const int piece = std::max(target, std::min(512, (int)std::sqrt((double)len)));
-      const int n = (len + piece - 1) / piece;
-      out.heavy.push_back(GatherHeavy{r, out.n_slots, n, 0});
-      for (int k = 0; k < n; ++k)
-        pieces.push_back(Range{out.n_slots++, ap[r] + (int)((long long)len * k / n),
-                               ap[r] + (int)((long long)len * (k + 1) / n), (int)out.heavy.size() - 1});
+      const int first_slot = out.n_slots;
+      auto piece_of = [&](int j0, int j1) { pieces.push_back(Range{out.n_slots++, j0, j1, (int)out.heavy.size()}); };
+      if (ticket_sums) {
+        // the ticket executor gives such a row to the 16 warps of a CTA in runs of whole 32 nonzeros, one beyond kSegmentNnz
+        // to several CTAs, each its segment
+        const int n_seg = (len + kSegmentNnz - 1) / kSegmentNnz, seg = (len + n_seg - 1) / n_seg;
+        for (int s0 = ap[r]; s0 < ap[r + 1]; s0 += seg) {
+          const int s1 = std::min(ap[r + 1], s0 + seg), per = ((s1 - s0 + 15) / 16 + 31) / 32 * 32;
+          for (int j = s0; j < s1; j += per) piece_of(j, std::min(s1, j + per));
+        }
+      } else {
+        // pieces of about sqrt(len): the group that adds them up last reads as many partial rows as a piece has gathers
+        const int piece = std::max(target, std::min(512, (int)std::sqrt((double)len)));
+        const int n = (len + piece - 1) / piece;
+        for (int k = 0; k < n; ++k) piece_of(ap[r] + (int)((long long)len * k / n), ap[r] + (int)((long long)len * (k + 1) / n));
+      }
+      out.heavy.push_back(GatherHeavy{r, first_slot, out.n_slots - first_slot, 0});
     } else {
       if (open_cost > 0 && open_cost + len + 2 > target) close();
       if (open_cost == 0) open = Range{pos, ap[r], ap[r], -1};

@@ -430,7 +430,7 @@ cudaError_t row_gemm_split(const float *W, int w_transposed, int K, int n, float
 }
 
 static int launch_panel(const float *X, int m, int K, int ld_x, const float *hi, const float *lo, int n, float *out, int ld_out, bool relu,
-                        bool precise, int *error, int wait_limit, int sm_count, cudaStream_t s) {
+                        bool precise, bool one_acc, int *error, int wait_limit, int sm_count, cudaStream_t s) {
   const int n_pad = row_gemm_pad_n(n), ldk = row_gemm_pad_k(K);
   CUtensorMap ma, mh, ml, mo;
   RowGemmParams P;
@@ -441,7 +441,7 @@ static int launch_panel(const float *X, int m, int K, int ld_x, const float *hi,
   P.m = m; P.n_pad = n_pad; P.n_real = n; P.n_slices = (K + kTcKSlice - 1) / kTcKSlice;
   P.tiles = (m + 2 * kTcRows - 1) / (2 * kTcRows);
   P.stages = rg_stages(n_pad);
-  P.accs = n_pad <= 64 ? 4 : (n_pad <= 128 ? 2 : 1);
+  P.accs = one_acc || n_pad > 128 ? 1 : (n_pad > 64 ? 2 : 4);
   P.out = out; P.ld_out = ld_out; P.relu = relu ? 1 : 0;
   P.tma_store = ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   P.error = error; P.wait_limit = wait_limit;
@@ -462,12 +462,12 @@ static int launch_panel(const float *X, int m, int K, int ld_x, const float *hi,
 }
 
 int row_gemm(const float *X, int m, int K, int ld_x, const float *hi, const float *lo, int n, float *out, int ld_out, bool relu,
-             int *error, int wait_limit, int sm_count, cudaStream_t s) {
+             bool one_acc, int *error, int wait_limit, int sm_count, cudaStream_t s) {
   const bool precise = !tc_supported(K, n);
   const int panel = precise ? kRgPrecisePanel : n;
   for (int c = 0; c < n; c += panel) {
     const size_t off = (size_t)c * row_gemm_pad_k(K);
-    const int rc = launch_panel(X, m, K, ld_x, hi + off, lo + off, std::min(panel, n - c), out + c, ld_out, relu, precise, error,
+    const int rc = launch_panel(X, m, K, ld_x, hi + off, lo + off, std::min(panel, n - c), out + c, ld_out, relu, precise, one_acc, error,
                                 wait_limit, sm_count, s);
     if (rc != TF_OK) return rc;
   }

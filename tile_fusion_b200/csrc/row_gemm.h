@@ -19,7 +19,8 @@ int row_gemm_pad_k(int k);       // floats per row of it
 cudaError_t row_gemm_split(const float *W, int w_transposed, int K, int n, float *hi, float *lo, cudaStream_t s);
 // out[m][ld_out] (n columns written) = X[m][ld_x] (K columns read) * W, optionally max(0, .); hi, lo as row_gemm_split leaves
 // them.  Rows of X on 16-byte boundaries come by TMA, others value by value; rows of `out` leave likewise.
+// one_acc: one accumulator per tile whatever the width, as the ticket executor has it (the same bits as its tile, where there is one).
 int row_gemm(const float *X, int m, int K, int ld_x, const float *hi, const float *lo, int n, float *out, int ld_out, bool relu,
-             int *error, int wait_limit, int sm_count, cudaStream_t s);
+             bool one_acc, int *error, int wait_limit, int sm_count, cudaStream_t s);
 
 }  // namespace tfk
