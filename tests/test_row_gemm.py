@@ -135,3 +135,29 @@ def test_nan_stays_nan(built_lib, k, n_cols, opts, bits):
     bi[hole, 1] = float("inf")
     assert np.isnan(run(bi, w)[20]).all()
     plan.close()
+
+
+# fewer terms than the precise form is taken for, and shapes the tensor-core tile does not take: FMAs in the order of the terms
+@pytest.mark.parametrize("k,n_cols", [(1, 1), (3, 64), (17, 16), (17, 256), (31, 225), (28, 20), (8, 7)])
+@pytest.mark.parametrize("m", [1, 127, 130, 80_011])
+def test_few_terms_are_fmas(built_lib, m, k, n_cols):
+    """Bit for bit the ticket executor's CUDA-core tile (n_cols <= k or k off the multiples of four: no sparse product in front),
+    infinities included, on rows and results off the 16-byte grid too."""
+    import torch
+    rng = np.random.default_rng(m + k)
+    t = (np.arange(m + 1, dtype=np.int32), rng.permutation(m).astype(np.int32), rng.uniform(1, 2, m).astype(np.float32))
+    b, w = synth.uniform(3, (m, k)), synth.uniform(4, (k, n_cols))
+    b[m // 2, k - 1], w[0, 0] = np.inf, -np.inf
+    A = api.CSRMatrix(m, m, *t)
+    for off, wt, relu in ((0, False, False), (1, True, True)):
+        bd = torch.empty(m * k + off, device="cuda")[off:].view(m, k).copy_(torch.from_numpy(b))
+        wd = torch.from_numpy(np.ascontiguousarray(w.T) if wt else w).cuda()
+        out = []
+        for opts in ({"tile_slots": -1}, {"tile_slots": -1, "tensor_cores": -1}):
+            plan = api.Plan("gemm_spmm", A, k=k, n_cols=n_cols, **opts)
+            out.append(torch.full((m * n_cols + off,), 7.0, device="cuda")[off:].view(m, n_cols))
+            plan.gemm_spmm(bd, wd, out[-1], w_transposed=wt, relu=relu)
+            plan.status()
+            plan.close()
+        assert torch.equal(torch.isnan(out[0]), torch.isnan(out[1]))
+        assert torch.equal(out[0].nan_to_num(), out[1].nan_to_num())

@@ -1266,13 +1266,14 @@ int run_gather_gemm_spmm(tf_plan &p, const float *B, const float *W, int w_trans
     return fail(TF_ERR_ARG, "this plan (gather tiles or tensor-core producer) needs 16-byte aligned dense operands "
                             "(build the plan with tile_slots < 0 and tensor_cores < 0 otherwise)");
   TF_CUDA(tfk::row_gemm_split(W, w_transposed, k, n, p.w_hi.p, p.w_lo.p, s));
-  p.launches = 3;
+  p.launches = tfk::row_gemm_form(k, n) == tfk::kRowFma ? 2 : 3;
   if (p.spmm_first) {
     TF_TRY(run_gather(p.g_second, B, k, aligned(B, 16), p.inter.p, p.ld_t, true, k, false, s));
-    return tfk::row_gemm(p.inter.p, p.m, k, p.ld_t, p.w_hi.p, p.w_lo.p, n, D, n, relu, false, &p.state.p->error, p.spin_limit, p.sm_count, s);
+    return tfk::row_gemm(p.inter.p, p.m, k, p.ld_t, W, w_transposed, p.w_hi.p, p.w_lo.p, n, D, n, relu, false, &p.state.p->error,
+                         p.spin_limit, p.sm_count, s);
   }
-  TF_TRY(tfk::row_gemm(B, p.m, k, k, p.w_hi.p, p.w_lo.p, n, p.inter.p, p.ld_t, false, p.ticket_sums, &p.state.p->error, p.spin_limit,
-                       p.sm_count, s));
+  TF_TRY(tfk::row_gemm(B, p.m, k, k, W, w_transposed, p.w_hi.p, p.w_lo.p, n, p.inter.p, p.ld_t, false, p.ticket_sums,
+                       &p.state.p->error, p.spin_limit, p.sm_count, s));
   return run_gather(p.g_second, p.inter.p, p.ld_t, true, D, n, out16, n, relu, s);
 }
 
@@ -1409,10 +1410,10 @@ int run_gemm_march(tf_plan &p, const float *B, const float *W, int w_transposed,
   long long launches = 0;
   if (produce) {
     TF_CUDA(tfk::row_gemm_split(W, w_transposed, p.k_dim, p.n_cols, p.w_hi.p, p.w_lo.p, s));
-    int rc = tfk::row_gemm(B, p.m, p.k_dim, p.k_dim, p.w_hi.p, p.w_lo.p, p.n_cols, p.inter.p, p.n_cols, false, p.ticket_sums,
-                           &p.march.st.p[0].error, p.spin_limit, p.sm_count, s);
+    int rc = tfk::row_gemm(B, p.m, p.k_dim, p.k_dim, W, w_transposed, p.w_hi.p, p.w_lo.p, p.n_cols, p.inter.p, p.n_cols, false,
+                           p.ticket_sums, &p.march.st.p[0].error, p.spin_limit, p.sm_count, s);
     if (rc != TF_OK) return rc;
-    launches = 2;   // weight split + producer
+    launches = tfk::row_gemm_form(p.k_dim, p.n_cols) == tfk::kRowFma ? 1 : 2;   // (weight split and) dense product
   }
   if (p.march.n_star > 0) {
     int rc = run_star(p, D, relu, s);
@@ -1595,8 +1596,8 @@ static int run_host_gemm_gather(tf_plan &p, const float *B, int w_transposed, bo
       TF_CUDA(p.host_pipe->upload(src, B + in_done * k, (size_t)(in_to - in_done) * k * 4, p.s_h2d));
       TF_CUDA(cudaEventRecord(p.ev_in[s], p.s_h2d));
       TF_CUDA(cudaStreamWaitEvent(p.s_run, p.ev_in[s], 0));
-      TF_TRY(tfk::row_gemm(src, (int)(in_to - in_done), k, k, p.w_hi.p, p.w_lo.p, n, p.inter.p + in_done * p.ld_t, p.ld_t, false,
-                           p.ticket_sums, &p.state.p->error, p.spin_limit, p.sm_count, p.s_run));
+      TF_TRY(tfk::row_gemm(src, (int)(in_to - in_done), k, k, p.h_in1.p, w_transposed, p.w_hi.p, p.w_lo.p, n,
+                           p.inter.p + in_done * p.ld_t, p.ld_t, false, p.ticket_sums, &p.state.p->error, p.spin_limit, p.sm_count, p.s_run));
       in_done = in_to;
       ++p.launches;
     }

@@ -13,8 +13,9 @@
 //   * The grid is one pair per two SMs and walks the tiles.
 // The tensor core cuts off what it adds to an accumulator instead of rounding it, so a chain of K / 8 sums drifts (rel.
 // error 2e-6 at K = 256, ten times that of fp32 FMAs).  Widths and depths that the ticket executor's tensor-core tile does
-// not take have always been multiplied with fp32 FMAs; for them the kernel has a second form that is as exact as those:
-// panels of up to 64 columns, whose four accumulators are read back and added in registers after every slice.
+// not take have always been multiplied with fp32 FMAs; for them the kernel has a second form that is as exact as those from
+// 32 terms on: panels of up to 64 columns, whose four accumulators are read back and added in registers after every slice.
+// Fewer terms are multiplied with FMAs still, by row_fma_kernel.
 // The plain form keeps its chains short where tensor memory has room: up to 128 columns the K steps of a slice go round two
 // accumulators, up to 64 round four, the small products first (K = 256: rel. error 1.9e-6 with one, 8.8e-7 with two, 4.6e-7
 // with four; 262 144 rows, K = N = 64: 33.6 us with one, 36.3 with four).
@@ -39,6 +40,10 @@ constexpr int kRgMaxStages = 5;
 // without, 1 044 with 3; 8 and 20 are slower than 3; 500 009 rows, 256 -> 47: 234 and 229; where it has four or fewer the
 // request costs 1 to 2 %).
 constexpr int kRgAhead = 3, kRgAheadSlices = 8;
+// Terms from which on the precise form's error is no larger than that of fp32 FMAs (40 000 rows, rel.: 9.2e-8 and 1.03e-7 on
+// uniform operands, 1.02e-7 and 1.03e-7 on normal ones, 6.1e-8 and 8.3e-8 on positive ones; 17 terms: 8.6e-8 and 7.6e-8);
+// shapes of fewer that the tensor-core tile does not take are multiplied with those.
+constexpr int kRgPreciseMinK = 32;
 constexpr int kRgPrecisePanel = 64;  // columns: four accumulators, twice, in 512 columns of tensor memory
 constexpr int kRgSmemMax = 227 * 1024;
 constexpr int kRgEpiBytes = kRgEpiWarps * 2 * 32 * 128;  // two 32 x 32 blocks per warp
@@ -403,6 +408,64 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   }
 }
 
+// out = X * W for few terms (K < kRgPreciseMinK) with fp32 FMAs in the order of the terms, as the ticket executor's CUDA-core
+// tile has them: the same bits.  W stays in shared memory, a CTA walks tiles of 128 rows (transposed, so that a thread reads
+// four of a term at once), a thread computes 8 rows x 4 columns at a time: three reads for 32 FMAs.  The result, written once,
+// bounds it.  (Whole GeMM-SpMM calls, 17 terms, 128 x 128 x 64 points: 64 columns 262 us, 205 with the precise form, 1 127 on
+// the ticket executor; 256 columns 768, 853 and 2 728.)
+constexpr int kFmaThreads = 256, kFmaRows = 128, kFmaLd = kFmaRows + 4;
+static_assert((256 + kFmaLd) * (kRgPreciseMinK - 1) * 4 <= 48 * 1024, "W and the rows fit the shared memory every launch has");
+__global__ void __launch_bounds__(kFmaThreads)
+row_fma_kernel(const float *__restrict__ X, int m, int K, int ld_x, const float *__restrict__ W, int w_transposed, int n,
+               float *__restrict__ out, int ld_out, int relu, bool vec) {
+  extern __shared__ float4 fma_smem[];
+  const int quads = (n + 3) / 4, tid = threadIdx.x;
+  float *w = reinterpret_cast<float *>(fma_smem), *x = w + 4 * quads * K;  // W [K][4 * quads], the rows [K][kFmaLd]
+  for (int i = tid; i < 4 * quads * K; i += kFmaThreads) {
+    const int k = i / (4 * quads), c = i - k * 4 * quads;
+    w[i] = c < n ? __ldg(w_transposed ? W + (size_t)c * K + k : W + (size_t)k * n + c) : 0.f;
+  }
+  for (long long r0 = (long long)blockIdx.x * kFmaRows; r0 < m; r0 += (long long)gridDim.x * kFmaRows) {
+    __syncthreads();  // W is complete, or the rows of the tile before have been read
+    for (int i = tid; i < kFmaRows * K; i += kFmaThreads) {
+      const int r = i / K, k = i - r * K;
+      x[k * kFmaLd + r] = r0 + r < m ? __ldg(X + (size_t)(r0 + r) * ld_x + k) : 0.f;
+    }
+    __syncthreads();
+    for (int i = tid; i < quads * (kFmaRows / 8); i += kFmaThreads) {
+      const int g = i / quads, q = i - g * quads;
+      float4 acc[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float *xg = x + 8 * g, *wq = w + 4 * q;
+      for (int k = 0; k < K; ++k, xg += kFmaLd, wq += 4 * quads) {
+        const float4 b = *reinterpret_cast<const float4 *>(wq);
+        const float4 lo = *reinterpret_cast<const float4 *>(xg), hi = *reinterpret_cast<const float4 *>(xg + 4);
+        const float a[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          acc[j].x = fmaf(a[j], b.x, acc[j].x); acc[j].y = fmaf(a[j], b.y, acc[j].y);
+          acc[j].z = fmaf(a[j], b.z, acc[j].z); acc[j].w = fmaf(a[j], b.w, acc[j].w);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (r0 + 8 * g + j >= m) break;
+        float4 v = acc[j];
+        if (relu) v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+        float *o = out + (size_t)(r0 + 8 * g + j) * ld_out + 4 * q;
+        if (vec && 4 * q + 3 < n) *reinterpret_cast<float4 *>(o) = v;
+        else {
+          o[0] = v.x;
+          if (4 * q + 1 < n) o[1] = v.y;
+          if (4 * q + 2 < n) o[2] = v.z;
+          if (4 * q + 3 < n) o[3] = v.w;
+        }
+      }
+    }
+  }
+}
+
 // hi / lo [n_pad][K] (K contiguous, rows from n on zero) from W [K][n], or from W [n][K] when w_transposed.
 __global__ void split_weight_pad_kernel(const float *__restrict__ W, int w_transposed, int K, int ldk, int n, int n_pad,
                                         float *__restrict__ hi, float *__restrict__ lo) {
@@ -423,10 +486,24 @@ bool row_gemm_supported(int n) { return n >= 1 && n <= kTcMaxN; }
 int row_gemm_pad_n(int n) { return (n + 31) / 32 * 32; }  // cta_group::2 takes multiples of 32
 int row_gemm_pad_k(int k) { return (k + 3) / 4 * 4; }
 
+RowGemmForm row_gemm_form(int K, int n) { return tc_supported(K, n) ? kRowTile : (K >= kRgPreciseMinK ? kRowPrecise : kRowFma); }
+
 cudaError_t row_gemm_split(const float *W, int w_transposed, int K, int n, float *hi, float *lo, cudaStream_t s) {
+  if (row_gemm_form(K, n) == kRowFma) return cudaSuccess;
   const int ldk = row_gemm_pad_k(K), n_pad = row_gemm_pad_n(n);
   split_weight_pad_kernel<<<std::min((n_pad * ldk + 255) / 256, 148 * 4), 256, 0, s>>>(W, w_transposed, K, ldk, n, n_pad, hi, lo);
   return cudaGetLastError();
+}
+
+static int launch_fma(const float *X, int m, int K, int ld_x, const float *W, int w_transposed, int n, float *out, int ld_out, bool relu,
+                      int sm_count, cudaStream_t s) {
+  const int quads = (n + 3) / 4;
+  const size_t smem = (size_t)(4 * quads + kFmaLd) * K * 4;
+  const bool vec = ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  row_fma_kernel<<<std::max(1, std::min((m + kFmaRows - 1) / kFmaRows, sm_count * 4)), kFmaThreads, smem, s>>>(
+      X, m, K, ld_x, W, w_transposed, n, out, ld_out, relu ? 1 : 0, vec);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? TF_OK : tf::fail(TF_ERR_CUDA, std::string("row_gemm: ") + cudaGetErrorString(e));
 }
 
 static int launch_panel(const float *X, int m, int K, int ld_x, const float *hi, const float *lo, int n, float *out, int ld_out, bool relu,
@@ -461,9 +538,11 @@ static int launch_panel(const float *X, int m, int K, int ld_x, const float *hi,
   return TF_OK;
 }
 
-int row_gemm(const float *X, int m, int K, int ld_x, const float *hi, const float *lo, int n, float *out, int ld_out, bool relu,
-             bool one_acc, int *error, int wait_limit, int sm_count, cudaStream_t s) {
-  const bool precise = !tc_supported(K, n);
+int row_gemm(const float *X, int m, int K, int ld_x, const float *W, int w_transposed, const float *hi, const float *lo, int n,
+             float *out, int ld_out, bool relu, bool one_acc, int *error, int wait_limit, int sm_count, cudaStream_t s) {
+  const RowGemmForm form = row_gemm_form(K, n);
+  if (form == kRowFma) return launch_fma(X, m, K, ld_x, W, w_transposed, n, out, ld_out, relu, sm_count, s);
+  const bool precise = form == kRowPrecise;
   const int panel = precise ? kRgPrecisePanel : n;
   for (int c = 0; c < n; c += panel) {
     const size_t off = (size_t)c * row_gemm_pad_k(K);
