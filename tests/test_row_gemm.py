@@ -161,3 +161,33 @@ def test_few_terms_are_fmas(built_lib, m, k, n_cols):
             plan.close()
         assert torch.equal(torch.isnan(out[0]), torch.isnan(out[1]))
         assert torch.equal(out[0].nan_to_num(), out[1].nan_to_num())
+
+
+@pytest.mark.parametrize("m,k,n_cols,off", [(700, 33, 128, 0), (700, 64, 47, 0), (129, 36, 33, 1), (300, 300, 225, 0), (1, 50, 70, 1)])
+def test_infinities_of_the_precise_form(built_lib, m, k, n_cols, off):
+    """Shapes that FMAs always took: an infinity in B or in the weight, and a number that rounds to one in TF32, give what FMAs
+    give -- the infinity, the finite sum, no number only where infinities meet their negatives or a zero."""
+    import torch
+    rng = np.random.default_rng(m + k)
+    t = (np.arange(m + 1, dtype=np.int32), rng.permutation(m).astype(np.int32), np.ones(m, np.float32))
+    b, w = synth.uniform(3, (m, k)), synth.uniform(4, (k, n_cols))
+    big = np.float32(3.4027e38)  # finite; its nearest TF32 number is not
+    b[0, 1], b[m // 2, k - 1], b[m // 3, 0], b[m // 3, 2] = np.inf, -np.inf, np.inf, np.inf
+    b[m // 5, 3] = big
+    w[1, 4], w[k - 1, 5], w[:, n_cols - 1] = 0.0, np.inf, np.abs(w[:, n_cols - 1]) + 1e-3
+    w[3] *= 1e-3
+    plan = api.Plan("gemm_spmm", api.CSRMatrix(m, m, *t), k=k, n_cols=n_cols)
+    bd = torch.empty(m * k + off, device="cuda")[off:].view(m, k).copy_(torch.from_numpy(b))
+    for wt in (False, True):
+        d = torch.zeros(m * n_cols + off, device="cuda")[off:].view(m, n_cols)
+        plan.gemm_spmm(bd, torch.from_numpy(np.ascontiguousarray(w.T) if wt else w).cuda(), d, w_transposed=wt)
+        plan.status()
+        with np.errstate(invalid="ignore"):
+            want = (b.astype(np.float64) @ w.astype(np.float64))[t[1]]
+        got = d.cpu().numpy()
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+        np.testing.assert_array_equal(np.where(np.isinf(got), got, 0), np.where(np.isinf(want), want, 0))
+        fin = np.isfinite(want)
+        scale = np.where(fin, np.abs(want), 0).max(1, keepdims=True)  # (a row of sums of up to 300 terms, each sum within 6e-7 of it)
+        assert (np.where(fin, np.abs(got - want), 0) <= 1e-6 * scale).all()
+    plan.close()

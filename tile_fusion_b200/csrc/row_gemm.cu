@@ -320,6 +320,21 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     };
     // 32 columns from c on of this lane's row
     auto put = [&](const float (&x)[32], int c, int row0) {
+      // (PRECISE) A sum that is no finite number is taken once more with FMAs: the halves of an infinity, or of a number that
+      // rounding carries to one, give infinity - infinity where FMAs give the infinity, or the finite sum.
+      unsigned odd = 0;
+      if (PRECISE) {
+#pragma unroll
+        for (int q = 0; q < 32; ++q)
+          if (!isfinite(x[q]) && c + q < P.n_real && row0 + lane < P.m) odd |= 1u << q;
+      }
+      auto exact = [&](int col) {  // (one addition at a time: rare, and registers are short)
+        const float *xr = P.x + (size_t)(row0 + lane) * P.ld_x, *wc = P.w + (size_t)col * P.w_c;
+        float sum = 0.f;
+#pragma unroll 1
+        for (int k = 0; k < P.k; ++k) sum = fmaf(__ldg(xr + k), __ldg(wc + (size_t)k * P.w_k), sum);
+        return P.relu ? fmaxf(sum, 0.f) : sum;
+      };
       float v[32];
 #pragma unroll
       for (int q = 0; q < 32; ++q) v[q] = P.relu ? fmaxf(x[q], 0.f) : x[q];
@@ -329,6 +344,10 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         __syncwarp();
 #pragma unroll
         for (int q = 0; q < 8; ++q) blk[lane * 8 + (q ^ (lane & 7))] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        for (; PRECISE && odd; odd &= odd - 1) {
+          const int q = __ffs(odd) - 1;
+          reinterpret_cast<float *>(blk + lane * 8 + (q / 4 ^ (lane & 7)))[q % 4] = exact(c + q);
+        }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0)
@@ -341,6 +360,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 #pragma unroll
         for (int q = 0; q < 32; ++q)
           if (c + q < P.n_real) d[q] = v[q];
+        for (; PRECISE && odd; odd &= odd - 1) d[__ffs(odd) - 1] = exact(c + __ffs(odd) - 1);
       }
     };
     for (int t = pair; t < P.tiles && ok; t += pairs) {
@@ -506,12 +526,13 @@ static int launch_fma(const float *X, int m, int K, int ld_x, const float *W, in
   return e == cudaSuccess ? TF_OK : tf::fail(TF_ERR_CUDA, std::string("row_gemm: ") + cudaGetErrorString(e));
 }
 
-static int launch_panel(const float *X, int m, int K, int ld_x, const float *hi, const float *lo, int n, float *out, int ld_out, bool relu,
+static int launch_panel(const float *X, int m, int K, int ld_x, const float *W, int w_k, int w_c, const float *hi, const float *lo, int n, float *out, int ld_out, bool relu,
                         bool precise, bool one_acc, int *error, int wait_limit, int sm_count, cudaStream_t s) {
   const int n_pad = row_gemm_pad_n(n), ldk = row_gemm_pad_k(K);
   CUtensorMap ma, mh, ml, mo;
   RowGemmParams P;
   P.x = X; P.k = K; P.ld_x = ld_x;
+  P.w = W; P.w_k = w_k; P.w_c = w_c;
   P.direct = ld_x % 4 != 0 || (reinterpret_cast<uintptr_t>(X) & 15) != 0;
   int rc = tc_make_map(&mh, hi, n_pad, ldk, n_pad / 2, ldk);
   if (rc == TF_OK) rc = tc_make_map(&ml, lo, n_pad, ldk, n_pad / 2, ldk);
@@ -546,8 +567,9 @@ int row_gemm(const float *X, int m, int K, int ld_x, const float *W, int w_trans
   const int panel = precise ? kRgPrecisePanel : n;
   for (int c = 0; c < n; c += panel) {
     const size_t off = (size_t)c * row_gemm_pad_k(K);
-    const int rc = launch_panel(X, m, K, ld_x, hi + off, lo + off, std::min(panel, n - c), out + c, ld_out, relu, precise, one_acc, error,
-                                wait_limit, sm_count, s);
+    const int w_k = w_transposed ? 1 : n, w_c = w_transposed ? K : 1;
+    const int rc = launch_panel(X, m, K, ld_x, W + (size_t)c * w_c, w_k, w_c, hi + off, lo + off, std::min(panel, n - c), out + c, ld_out,
+                                relu, precise, one_acc, error, wait_limit, sm_count, s);
     if (rc != TF_OK) return rc;
   }
   return TF_OK;

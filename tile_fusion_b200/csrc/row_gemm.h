@@ -5,11 +5,12 @@
 namespace tfk {
 
 struct RowGemmParams {
-  const float *x;  // read directly where rows do not start on 16-byte boundaries (`direct`)
+  const float *x;  // read directly where rows do not start on 16-byte boundaries (`direct`), and by the precise form's exact sums
+  const float *w;  // (the latter) the weight from the panel's first column on: element (k, c) at k * w_k + c * w_c
   float *out;
   int *error;
   int m, n_real, n_pad, n_slices, tiles, stages, accs, ld_out, k, ld_x;
-  int direct, relu, tma_store, wait_limit;
+  int direct, relu, tma_store, wait_limit, w_k, w_c;
 };
 
 bool row_gemm_supported(int n);  // n <= 256 columns
