@@ -191,3 +191,33 @@ def test_infinities_of_the_precise_form(built_lib, m, k, n_cols, off):
         scale = np.where(fin, np.abs(want), 0).max(1, keepdims=True)  # (a row of sums of up to 300 terms, each sum within 6e-7 of it)
         assert (np.where(fin, np.abs(got - want), 0) <= 1e-6 * scale).all()
     plan.close()
+
+
+@pytest.mark.parametrize("dims", [(16, 8, 6), (17, 10, 5)])
+@pytest.mark.parametrize("k,n_cols", [(64, 64), (33, 48), (17, 20)])
+def test_grid_with_missing_couplings(built_lib, dims, k, n_cols):
+    """A 3-D grid some of whose rows do not name a neighbour: nothing is multiplied that is not stored, so what is no finite
+    number in a row of B reaches the rows that name it and no others."""
+    import torch
+    ap, ai, ax = synth.laplacian(dims)
+    n = len(ap) - 1
+    rows = np.repeat(np.arange(n), np.diff(ap))
+    keep = (rows == ai) | (np.random.default_rng(1).uniform(size=len(ai)) > 0.1)
+    ap = np.concatenate([[0], np.cumsum(np.bincount(rows[keep], minlength=n))]).astype(np.int32)
+    ai, ax = ai[keep], ax[keep]
+    b, w = synth.uniform(5, (n, k)), synth.uniform(6, (k, n_cols))
+    b[np.arange(5, n, 50), 1] = np.inf
+    A = _scipy((ap, ai, ax), n)
+    hit = np.asarray(A.astype(bool)[:, 5::50].sum(1)).ravel() > 0
+    plan = api.Plan("gemm_spmm", api.CSRMatrix(n, n, ap, ai, ax), k=k, n_cols=n_cols)
+    for relu in (False, True):
+        d = torch.zeros((n, n_cols), device="cuda")
+        plan.gemm_spmm(torch.from_numpy(b).cuda(), torch.from_numpy(w).cuda(), d, relu=relu)
+        plan.status()
+        got = d.cpu().numpy()
+        assert np.isfinite(got[~hit]).all()
+        if not relu:
+            assert not np.isfinite(got[hit]).any()
+        want = A[~hit] @ np.where(np.isfinite(b), b, 0).astype(np.float64) @ w.astype(np.float64)
+        common.assert_close(got[~hit], np.maximum(want, 0) if relu else want, "rows without an infinity")
+    plan.close()

@@ -408,7 +408,10 @@ std::vector<int4> march_items_raw(const std::vector<tf::MarchItem> &items) {
 // Fp == null: the first operator is the identity (GeMM-SpMM: the dense producer has written T, and the marching
 // kernel computes D = A * (I * T); the products with the identity's zeros and its one are exact, so D is what the
 // CSR consumer gives).
-int build_march(tf_plan &p, const tf_csr *Fp, const tf_csr &A, int halo_rows, int sm_count, const std::vector<int> &boundary_rows) {
+// star: behind the dense product on the one-product march.  Taken only where every row names all of its neighbours: the march
+// multiplies a neighbour that is not named by zero, and an infinity there would not stay where it belongs.
+int build_march(tf_plan &p, const tf_csr *Fp, const tf_csr &A, int halo_rows, int sm_count, const std::vector<int> &boundary_rows,
+                bool star = false) {
   tf::LatticeOp lf, la;
   int rc = TF_OK;
   if (Fp) {
@@ -418,7 +421,7 @@ int build_march(tf_plan &p, const tf_csr *Fp, const tf_csr &A, int halo_rows, in
   if (Fp == &A && halo_rows == 0) la = lf;
   else {
     rc = tf::analyse_lattice_operator(A.m, A.n, A.ap, A.ai, A.ax, halo_rows, la, true);
-    if (rc != TF_OK || !la.ok) return rc;
+    if (rc != TF_OK || !la.ok || (star && !la.full)) return rc;
   }
   if (!Fp) {
     lf.ok = true; lf.nx = la.nx; lf.ny = la.ny; lf.nz = la.nz; lf.n_classes = 1;
@@ -695,7 +698,7 @@ int make_gemm_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &A, const tf
   p->hp.inter_rows = p->m;
   p->hp.n_cons = p->g_second.n_units;
   if (tiled && o.lattice_march >= 0 && p->n_cols % 4 == 0) {
-    rc = build_march(*p, nullptr, A, 0, sm_count, {});
+    rc = build_march(*p, nullptr, A, 0, sm_count, {}, true);
     if (rc != TF_OK) return rc;
     tf_plan::March &M = p->march;
     if (M.on) {

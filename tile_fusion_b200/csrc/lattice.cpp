@@ -73,6 +73,7 @@ int analyse_lattice_operator(int m, int ncols, const int *ap, const int *ai, con
   std::vector<VecKey> vecs;
   std::vector<long long> count;
   std::vector<uint8_t> cls((size_t)m);
+  bool full = true;
   for (int z = 0, r = 0; z < nz; ++z)
     for (int y = 0; y < ny; ++y)
       for (int x = 0; x < nx; ++x, ++r) {
@@ -102,9 +103,9 @@ int analyse_lattice_operator(int m, int ncols, const int *ap, const int *ai, con
         }
         // an extent that is odd is taken only where every neighbour is named, so that no coefficient in the grid is a zero
         // that stands for none (other operators run on the general path, which multiplies what is stored)
-        if (odd && seen != ((z > 0 ? 1u : 0u) | (y > 0 ? 2u : 0u) | (x > 0 ? 4u : 0u) | 8u | (x < nx - 1 ? 16u : 0u) |
-                            (y < ny - 1 ? 32u : 0u) | (z < nz - 1 ? 64u : 0u)))
-          return TF_OK;
+        full = full && seen == ((z > 0 ? 1u : 0u) | (y > 0 ? 2u : 0u) | (x > 0 ? 4u : 0u) | 8u | (x < nx - 1 ? 16u : 0u) |
+                            (y < ny - 1 ? 32u : 0u) | (z < nz - 1 ? 64u : 0u));
+        if (odd && !full) return TF_OK;
         auto it = ids.find(k);
         int id;
         if (it == ids.end()) {
@@ -138,6 +139,7 @@ int analyse_lattice_operator(int m, int ncols, const int *ap, const int *ai, con
   out.nx = nx; out.ny = ny; out.nz = nz;
   out.ghost_lo = ghost_lo; out.ghost_hi = ghost_hi;
   out.n_classes = nc;
+  out.full = full;
   out.ok = true;
   return TF_OK;
 }

@@ -63,6 +63,7 @@ Lattice detect_lattice(int m, const int *ap, const int *ai);
 constexpr int kMarchMaxClasses = 63;
 struct LatticeOp {
   bool ok = false;
+  bool full = false;               // every row names all of its neighbours in the grid
   int nx = 0, ny = 0, nz = 0;
   int ghost_lo = 0, ghost_hi = 0;  // planes of the source operand below / above the operator's own rows
   int n_classes = 0;               // distinct coefficient vectors; class n_classes is the all-zero vector
