@@ -86,3 +86,40 @@ def test_infinities_stay_where_they_are(built_lib):
     np.testing.assert_array_equal(np.isinf(got), np.isinf(want))
     assert not np.isnan(got).any()
     plan.close()
+
+
+@pytest.mark.parametrize("kind,n_cols", [("grid", 33), ("grid", 47), ("band", 47), ("two", 30), ("gaps", 41)])
+def test_host_call_in_pieces(built_lib, kind, n_cols):
+    """Host pointers on operators that name rows near their own, at widths that no march takes: the call runs in pieces, so that
+    copies and products overlap, and gives the bits of the device call.  Two operators of different reach; rows without nonzeros."""
+    import torch
+    n = 30_000
+    if kind == "grid":
+        t = synth.laplacian((32, 30, 31))
+        n = len(t[0]) - 1
+    else:
+        rng = np.random.default_rng(2)
+
+        def band(reach, per_row, empty=0):
+            r = np.repeat(np.arange(n), per_row)
+            c = np.clip(r + rng.integers(-reach, reach + 1, len(r)), 0, n - 1)
+            key = np.unique(r.astype(np.int64) * n + c)
+            key = key[(key // n) % 11 >= empty]
+            ap = np.concatenate([[0], np.cumsum(np.bincount(key // n, minlength=n))]).astype(np.int32)
+            return ap, (key % n).astype(np.int32), rng.uniform(-1, 1, len(key)).astype(np.float32)
+        t = band(40, 12, empty=3 if kind == "gaps" else 0)
+    A = api.CSRMatrix(n, n, *t)
+    F = api.CSRMatrix(n, n, *band(300, 5, empty=2)) if kind == "two" else None
+    c = synth.uniform(3, (n, n_cols))
+    plan = api.Plan("spmm_spmm", A, B=F, n_cols=n_cols)
+    d = torch.full((n, n_cols), float("nan"), device="cuda")
+    plan.spmm_spmm(torch.from_numpy(c).cuda(), d)
+    plan.status()
+    for _ in range(2):
+        dh = np.full((n, n_cols), np.nan, np.float32)
+        plan.spmm_spmm_host(c, dh)
+        assert plan.info()["launches"] > 16
+        np.testing.assert_array_equal(dh, d.cpu().numpy())
+    first = _scipy(t if F is None else (F.Ap, F.Ai, F.Ax), n)
+    common.assert_close(dh, _scipy(t, n) @ (first @ c.astype(np.float64)), kind)
+    plan.close()

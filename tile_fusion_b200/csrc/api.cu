@@ -85,24 +85,25 @@ struct DevGather {
   DevBuf<int4> units, heavy;
   DevBuf<int> rows, empty, cnt;
   DevBuf<float> partial;
-  // Runs of units in row order for the host-pointer calls, where no row is cut: units [unit_begin, unit_end) read rows
-  // < in_rows of the operand, and with them every row < out_rows of the result is final.
-  struct Seg { int unit_begin, unit_end; long long in_rows, out_rows; };
-  std::vector<Seg> segs;
-  void make_segments(const tf::GatherPlan &g, int m, int n_seg) {
+  // For the host-pointer calls, where no row is cut and units are in row order: units [0, u] read rows < in_rows[u] of the
+  // operand, and with them every row < out_rows[u] of the result is final.
+  std::vector<long long> in_rows, out_rows;
+  void follow_units(const tf::GatherPlan &g, int m) {
     const int n = (int)g.units.size();
-    if (!g.heavy.empty() || n < 2 * n_seg) return;
+    if (!g.heavy.empty()) return;
+    in_rows.resize(n);
+    out_rows.resize(n);
     long long need = 0;
-    for (int s = 0; s < n_seg; ++s) {
-      const int b = (int)((long long)n * s / n_seg), e = (int)((long long)n * (s + 1) / n_seg);
-      const size_t p1 = e < n ? (size_t)g.units[e].p0 : g.n_entries - tf::kGatherBatch;
-      for (size_t i = g.units[b].p0; i < p1; ++i) need = std::max<long long>(need, (g.cols[i] & ~tf::kGatherEnd) + 1LL);
-      const int pos = e < n ? g.units[e].pos : 0;
-      segs.push_back(Seg{b, e, need, e == n ? m : (g.rows.empty() ? pos : g.rows[pos])});
+    for (int u = 0; u < n; ++u) {
+      const size_t p1 = u + 1 < n ? (size_t)g.units[u + 1].p0 : g.n_entries - tf::kGatherBatch;
+      for (size_t i = g.units[u].p0; i < p1; ++i) need = std::max<long long>(need, (g.cols[i] & ~tf::kGatherEnd) + 1LL);
+      const int pos = u + 1 < n ? g.units[u + 1].pos : 0;
+      in_rows[u] = need;
+      out_rows[u] = u + 1 == n ? m : (g.rows.empty() ? pos : g.rows[pos]);
     }
   }
-  // n_cols: width of the dense operand the units are cut for; max_cols: widest one the operator will meet
-  int build(const tf_csr &A, int n_cols, int max_cols, int sm_count, int n_seg = 0, int resident = tfk::kGatherResident,
+  // n_cols: width of the dense operand the units are cut for; max_cols: widest one the operator will meet; follow: see above
+  int build(const tf_csr &A, int n_cols, int max_cols, int sm_count, bool follow = false, int resident = tfk::kGatherResident,
             bool ticket_sums = false) {
     tf::GatherPlan g;
     tf::build_gather_plan(A.m, A.ap, A.ai, A.ax, sm_count * (resident / tfk::gather_group(n_cols)), ticket_sums, g);
@@ -110,7 +111,7 @@ struct DevGather {
     n_empty = (int)g.empty_rows.size();
     partial_ld = (std::max(n_cols, max_cols) + 3) / 4 * 4;
     const int panels = (partial_ld + 127) / 128;  // the most any width up to that is read in
-    if (n_seg > 1) make_segments(g, A.m, n_seg);
+    if (follow) follow_units(g, A.m);
     if (!g.rows.empty()) g.rows.resize(g.rows.size() + 2, 0);  // a group looks one row ahead (with the row of Q, two)
     int rc = cols.upload(reinterpret_cast<const int *>(g.cols.get()), g.n_entries);
     if (rc == TF_OK) rc = vals.upload(g.vals.get(), g.n_entries);
@@ -197,6 +198,8 @@ struct tf_plan {
   DevGather g_first, g_second;
   int ld_t = 0;              // floats per row of the intermediate: n_cols rounded up to whole float4
   DevBuf<float> g_pad;       // rows of C of a width that is no multiple of four, padded to ld_t
+  struct Piece { int f_begin, f_end, begin, end; long long in_rows, out_rows; };  // units of the first and second operator
+  std::vector<Piece> pieces;  // see make_gather_pieces
   bool spmm_first = false;   // GeMM-SpMM on the balanced gather: D = (A B) C instead of A (B C)
   bool ticket_sums = false;  // every sum in the order of the ticket executor (tensor_cores > 0)
   size_t dyn_smem = 0;
@@ -566,16 +569,41 @@ int run_star(tf_plan &p, float *D, bool relu, cudaStream_t s) {
   return TF_OK;
 }
 
+// Pieces of a host-pointer call on operators that name rows near their own (grids, bands): the rows of the input that a piece
+// needs arrive while the one before is computed, and finished rows leave while the next one is.  None where a row is cut or
+// where the first piece already needs more than half of the input (graphs).
+void make_gather_pieces(tf_plan &p, int n) {
+  const DevGather &g = p.g_second, &f = p.first_is_second ? p.g_second : p.g_first;
+  const bool two = p.chain == 0;  // the rows of T are made by units of the first operator
+  const int units = (int)g.in_rows.size();
+  if (units < 2 * n || (two && f.in_rows.empty())) return;
+  tf_plan::Piece q{0, 0, 0, 0, 0, 0};
+  for (int s = 0; s < n; ++s) {
+    q.begin = q.end;
+    q.f_begin = q.f_end;
+    q.end = (int)((long long)units * (s + 1) / n);
+    q.in_rows = g.in_rows[q.end - 1];
+    q.out_rows = g.out_rows[q.end - 1];
+    if (two) {
+      while (q.f_end < (int)f.out_rows.size() && (q.f_end == 0 || f.out_rows[q.f_end - 1] < q.in_rows)) ++q.f_end;
+      q.in_rows = f.in_rows[q.f_end - 1];
+    }
+    p.pieces.push_back(q);
+  }
+  if (2 * p.pieces[0].in_rows > (two ? p.first_cols : p.m)) p.pieces.clear();
+}
+
 // The rest of a SpMM-SpMM plan that runs on the balanced gather.
 int make_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &F, const tf_csr &A, const tf_plan_opts &o, int sm_count,
                      tf_plan **out) {
   p->ld_t = (p->n_cols + 3) / 4 * 4;
-  int rc = p->g_second.build(A, p->n_cols, p->n_cols, sm_count);
-  if (rc == TF_OK && !p->first_is_second) rc = p->g_first.build(F, p->n_cols, p->n_cols, sm_count);
+  int rc = p->g_second.build(A, p->n_cols, p->n_cols, sm_count, true);
+  if (rc == TF_OK && !p->first_is_second) rc = p->g_first.build(F, p->n_cols, p->n_cols, sm_count, true);
   if (rc == TF_OK) rc = p->inter.alloc((size_t)p->m * p->ld_t);
   if (rc == TF_OK && p->ld_t != p->n_cols) rc = p->g_pad.alloc((size_t)p->first_cols * p->ld_t);
   if (rc == TF_OK) rc = zero_state(*p);
   if (rc != TF_OK) return rc;
+  make_gather_pieces(*p, 16);
   p->hp.inter_rows = p->m;
   p->hp.n_prod = (p->first_is_second ? p->g_second : p->g_first).n_units;
   p->hp.n_cons = p->g_second.n_units;
@@ -689,12 +717,13 @@ int make_gemm_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &A, const tf
   const int width = p->spmm_first ? p->k_dim : p->n_cols;
   p->ld_t = (width + 3) / 4 * 4;
   const size_t wn = (size_t)tfk::row_gemm_pad_n(p->n_cols) * tfk::row_gemm_pad_k(p->k_dim);
-  int rc = p->g_second.build(A, width, std::max(p->k_dim, p->n_cols), sm_count, tiled ? 16 : 0, tfk::kGatherResident, p->ticket_sums);
+  int rc = p->g_second.build(A, width, std::max(p->k_dim, p->n_cols), sm_count, tiled, tfk::kGatherResident, p->ticket_sums);
   if (rc == TF_OK) rc = p->inter.alloc((size_t)(p->m + 1) * p->ld_t);  // (the one-product march may read one row more)
   if (rc == TF_OK) rc = p->w_hi.alloc(wn);
   if (rc == TF_OK) rc = p->w_lo.alloc(wn);
   if (rc == TF_OK) rc = zero_state(*p);
   if (rc != TF_OK) return rc;
+  make_gather_pieces(*p, 16);
   p->hp.inter_rows = p->m;
   p->hp.n_cons = p->g_second.n_units;
   if (tiled && o.lattice_march >= 0 && p->n_cols % 4 == 0) {
@@ -1319,7 +1348,7 @@ int tf_plan_sddmm_spmm(const tf_csr *A, int kq, int nv, const tf_plan_opts *opts
   p->m = A->m; p->n_cols = nv; p->k_dim = kq;
   if (tfk::sddmm_gather_supported(kq, nv) && o.rows_per_block == 0 && o.ctas_per_sm == 0) {
     p->second.m = A->m; p->second.n = A->n;
-    rc = p->g_second.build(*A, 4 * tfk::sddmm_group(kq, nv), nv, sm_count, 0, tfk::kSddmmResident);  // (units for groups of that size)
+    rc = p->g_second.build(*A, 4 * tfk::sddmm_group(kq, nv), nv, sm_count, false, tfk::kSddmmResident);  // (units for groups of that size)
     if (rc == TF_OK) rc = zero_state(*p);
     if (rc != TF_OK) return rc;
     *out = p.release();
@@ -1575,36 +1604,49 @@ static int run_host_whole(tf_plan &p, const float *C, size_t nin, float *D, size
   return TF_OK;
 }
 
-// GeMM-SpMM whose operator names rows near its own (grids, bands): rows of B arrive in pieces, each piece's rows of the
-// dense product follow, then the rows of D that have all they need, which leave while the next piece arrives.
-static int run_host_gemm_gather(tf_plan &p, const float *B, int w_transposed, bool relu, float *D) {
-  const DevGather &g = p.g_second;
-  const int ns = (int)g.segs.size(), n = p.n_cols, k = p.k_dim;
+// Both chains on the pieces of a plan (make_gather_pieces): rows of the input (B or C) arrive in pieces, the rows of T that a
+// piece can make follow, then the rows of D that have all they need, which leave while the next piece arrives.
+static int run_host_pieces(tf_plan &p, const float *in, int w_transposed, bool relu, float *D) {
+  const DevGather &g = p.g_second, &f = p.first_is_second ? p.g_second : p.g_first;
+  const bool gemm = p.chain == 1;
+  const int ns = (int)p.pieces.size(), n = p.n_cols, k = gemm ? p.k_dim : p.n_cols;  // k: width of the input
   while ((int)p.ev_in.size() < ns) {
     cudaEvent_t a, b;
     TF_CUDA(cudaEventCreateWithFlags(&a, cudaEventDisableTiming));
     TF_CUDA(cudaEventCreateWithFlags(&b, cudaEventDisableTiming));
     p.ev_in.push_back(a); p.ev_run.push_back(b);
   }
-  TF_TRY(begin_host_pipe(p, B, D));
-  TF_CUDA(tfk::row_gemm_split(p.h_in1.p, w_transposed, k, n, p.w_hi.p, p.w_lo.p, p.s_run));
+  TF_TRY(begin_host_pipe(p, in, D));
+  if (gemm) TF_CUDA(tfk::row_gemm_split(p.h_in1.p, w_transposed, k, n, p.w_hi.p, p.w_lo.p, p.s_run));
+  else TF_CUDA(tfk::launch_rows_fix(f.empty.p, f.n_empty, p.ld_t, p.inter.p, false, p.s_run));
   TF_CUDA(tfk::launch_rows_fix(g.empty.p, g.n_empty, n, p.h_out.p, false, p.s_run));
+  const bool pad = p.g_pad.n != 0, vec = pad || n % 4 == 0;  // (the buffers of the call start on 16-byte boundaries)
   long long in_done = 0, out_done = 0;
   p.launches = 1;
   for (int s = 0; s < ns; ++s) {
-    const DevGather::Seg &sg = g.segs[s];
-    const long long in_to = s == ns - 1 ? p.m : std::max(in_done, sg.in_rows);
+    const tf_plan::Piece &sg = p.pieces[s];
+    const long long in_to = gemm && s == ns - 1 ? p.m : std::max(in_done, sg.in_rows);
     if (in_to > in_done) {
       float *src = p.h_in0.p + in_done * k;
-      TF_CUDA(p.host_pipe->upload(src, B + in_done * k, (size_t)(in_to - in_done) * k * 4, p.s_h2d));
+      TF_CUDA(p.host_pipe->upload(src, in + in_done * k, (size_t)(in_to - in_done) * k * 4, p.s_h2d));
       TF_CUDA(cudaEventRecord(p.ev_in[s], p.s_h2d));
       TF_CUDA(cudaStreamWaitEvent(p.s_run, p.ev_in[s], 0));
-      TF_TRY(tfk::row_gemm(src, (int)(in_to - in_done), k, k, p.h_in1.p, w_transposed, p.w_hi.p, p.w_lo.p, n,
-                           p.inter.p + in_done * p.ld_t, p.ld_t, false, p.ticket_sums, &p.state.p->error, p.spin_limit, p.sm_count, p.s_run));
+      if (gemm) {
+        TF_TRY(tfk::row_gemm(src, (int)(in_to - in_done), k, k, p.h_in1.p, w_transposed, p.w_hi.p, p.w_lo.p, n,
+                             p.inter.p + in_done * p.ld_t, p.ld_t, false, p.ticket_sums, &p.state.p->error, p.spin_limit, p.sm_count, p.s_run));
+        ++p.launches;
+      } else if (pad) {
+        TF_CUDA(tfk::launch_pad_rows(src, in_to - in_done, n, p.ld_t, p.g_pad.p + in_done * p.ld_t, p.s_run));
+        ++p.launches;
+      }
       in_done = in_to;
+    }
+    if (!gemm && sg.f_end > sg.f_begin) {
+      TF_TRY(run_gather(f, pad ? p.g_pad.p : p.h_in0.p, pad ? p.ld_t : n, vec, p.inter.p, p.ld_t, true, vec ? p.ld_t : n, false, p.s_run,
+                        sg.f_begin, sg.f_end));
       ++p.launches;
     }
-    TF_TRY(run_gather(g, p.inter.p, p.ld_t, true, p.h_out.p, n, n % 4 == 0, n, relu, p.s_run, sg.unit_begin, sg.unit_end));
+    TF_TRY(run_gather(g, p.inter.p, p.ld_t, true, p.h_out.p, n, n % 4 == 0, n, relu, p.s_run, sg.begin, sg.end));
     ++p.launches;
     if (sg.out_rows > out_done) {
       TF_CUDA(cudaEventRecord(p.ev_run[s], p.s_run));
@@ -1651,8 +1693,10 @@ int tf_spmm_spmm_host(tf_plan *p, const float *C, float *D) {
     const size_t nin = (size_t)p->first_cols * p->n_cols;
     if (p->h_in0.n < nin) rc = p->h_in0.alloc(nin);
     if (rc == TF_OK && p->h_out.n < nd) rc = p->h_out.alloc(nd);
+    if (rc == TF_OK) rc = ensure_streams(*p);
     if (rc == TF_OK)
-      rc = run_host_whole(*p, C, nin, D, nd, [&] { return run_gather_spmm_spmm(*p, p->h_in0.p, p->h_out.p, p->s_run); });
+      rc = !p->pieces.empty() ? run_host_pieces(*p, C, 0, false, D)
+                              : run_host_whole(*p, C, nin, D, nd, [&] { return run_gather_spmm_spmm(*p, p->h_in0.p, p->h_out.p, p->s_run); });
     if (rc != TF_OK) return rc;
     return tf_plan_status(p, nullptr);
   }
@@ -1690,7 +1734,7 @@ int tf_gemm_spmm_host(tf_plan *p, const float *B, const float *W, int w_transpos
     if (rc != TF_OK) return rc;
     TF_TRY(ensure_streams(*p));
     TF_TRY(stage_in(p->h_in1, W, (size_t)p->k_dim * p->n_cols, p->s_run));  // the weight first, on the stream that uses it
-    if (!p->g_second.segs.empty()) rc = run_host_gemm_gather(*p, B, w_transposed, relu != 0, D);
+    if (!p->pieces.empty()) rc = run_host_pieces(*p, B, w_transposed, relu != 0, D);
     else
       rc = run_host_whole(*p, B, nin, D, nd, [&] {
         return run_gather_gemm_spmm(*p, p->h_in0.p, p->h_in1.p, w_transposed, relu != 0, p->h_out.p, p->s_run);
