@@ -178,6 +178,10 @@ void tf_free(void *p);
  * row}.  No counterpart in the reference. */
 int tf_tiling_preview(const tf_csr *A, int tile_slots, int tile_max_bz, int **row_ptr, int **rows,
                       int **halo_ptr, int **halo, int *n_tiles, int info[4]);
+/* Host-only: the length of the segments into which the executors that march down a band or along the lines of a grid cut n
+ * steps of `columns` columns for `resident` workers, a segment of len steps costing len + lead.  No counterpart in the
+ * reference. */
+int tf_segment_preview(int n, long long columns, long long resident, int lead, int min_len);
 /* Host-only: how the library sees operator A (m x n CSR, of which the last `halo_rows` columns are halo rows
  * appended after the local ones) as a star stencil on a 3-D grid in natural order -- the form the
  * plane-marching executor runs from.  info = {recognised, nx, ny, nz, source planes below, source planes above,

@@ -18,6 +18,7 @@
 #include "band_march.h"
 #include "gemm_tc.cuh"
 #include "gemm_tc_host.h"
+#include "segments.h"
 
 namespace tfk {
 
@@ -141,15 +142,7 @@ static cudaError_t launch(const CUtensorMap &tm_c, BandParams &p, int sm_count, 
   if (n <= 0) return cudaSuccess;
   const size_t smem = band_smem(S, p.pairs_f, p.pairs_a, p.same);
   const long long resident = (long long)sm_count * (S == 64 && smem <= 112 * 1024 ? 2 : 1);
-  // A segment of n blocks of D takes n + 3 steps; as many segments as give the fewest steps over the rounds of resident CTAs.
-  long long best = -1;
-  for (int k = 1; k <= n; ++k) {
-    const int len = (n + k - 1) / k;
-    const long long segs = (n + len - 1) / len, rounds = (segs * p.chunks + resident - 1) / resident;
-    const long long t = rounds * (len + 3);
-    if (best < 0 || t < best) { best = t; p.seg_blocks = len; }
-    if (len == 1) break;
-  }
+  p.seg_blocks = tf::segment_length(n, p.chunks, resident, 3, 1);  // a segment of n blocks of D takes n + 3 steps
   cudaError_t e = cudaFuncSetAttribute((const void *)band_march_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const long long ctas = (long long)((n + p.seg_blocks - 1) / p.seg_blocks) * p.chunks;

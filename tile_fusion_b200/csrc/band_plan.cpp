@@ -4,6 +4,8 @@
 #include <cstring>
 
 #include "band_march.h"
+#include "segments.h"
+#include "tf_internal.h"
 
 namespace tf {
 
@@ -38,3 +40,9 @@ void build_band_operator(int m, const int *ap, const int *ai, const float *ax, i
 }
 
 }  // namespace tf
+
+// Host-only view of the segment length, for tests.
+extern "C" int tf_segment_preview(int n, long long columns, long long resident, int lead, int min_len) {
+  if (n <= 0 || columns <= 0 || resident <= 0 || lead <= 0 || min_len <= 0) return TF_ERR_ARG;
+  return tf::segment_length(n, columns, resident, lead, min_len);
+}

@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "line_march.h"
+#include "segments.h"
 
 namespace tfk {
 
@@ -226,17 +227,9 @@ cudaError_t launch_line_march(LineParams &p, bool vec, bool same, int sm_count, 
   LineFn f = vec ? (same ? (LineFn)line_march_kernel<4, true> : (LineFn)line_march_kernel<4, false>)
                  : (same ? (LineFn)line_march_kernel<1, true> : (LineFn)line_march_kernel<1, false>);
   p.chunks = (p.n_cols + 15) / 16;
-  // A segment of n lines costs n + 4 steps.  The number of segments is the one for which the steps of the rounds that the
-  // resident warps take are fewest.
+  // a segment of n lines costs n + 4 steps; four lines at least
   const long long columns = (long long)p.tiles * p.chunks, resident = (long long)sm_count * line_ctas(vec) * kLineWarps;
-  long long best = -1;
-  for (int n = 1; n <= lines; ++n) {
-    const int len = (lines + n - 1) / n;
-    if (n > 1 && len < 4) break;
-    const long long segs = (lines + len - 1) / len, rounds = (columns * segs + resident - 1) / resident;
-    const long long t = rounds * (len + 4);
-    if (best < 0 || t < best) { best = t; p.seg_len = len; }
-  }
+  p.seg_len = tf::segment_length(lines, columns, resident, 4, 4);
   const long long items = columns * ((lines + p.seg_len - 1) / p.seg_len);
   if (items > 0x7fffffff) return cudaErrorInvalidValue;
   p.n_items = (int)items;
