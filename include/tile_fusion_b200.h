@@ -233,6 +233,10 @@ int tf_exec_sddmm_spmm(tf_plan *p, const float *Q, const float *K, const float *
 /* out = A * X with the plan's A, X and out n_cols wide (at most the widest dense operand of the plan): the sparse product
  * of a layer's backward pass (binding-project/src/Functions.cpp:1192-1244) on the operator that its forward pass uses. */
 int tf_exec_spmm(tf_plan *p, const float *X, int n_cols, float *out, void *stream);
+/* The same with scratch of the caller's (device memory, 16-byte aligned, tf_exec_spmm_work_bytes of it) instead of the plan's,
+ * so that it may run beside other calls on the plan, on any stream; tf_exec_spmm, like the other executors, may not. */
+int tf_exec_spmm_work(tf_plan *p, const float *X, int n_cols, float *out, void *work, size_t work_bytes, void *stream);
+size_t tf_exec_spmm_work_bytes(const tf_plan *p);
 
 /* out (na x nb) = A^T * B for A m x na and B m x nb, device pointers, fp32: the weight gradient of a layer
  * (binding-project/src/Functions.cpp:1192-1244).  `work` holds tf_atb_work_floats(m, na, nb) floats of scratch. */

@@ -100,3 +100,31 @@ def test_layers_keep_the_order_of_their_sums(built_lib, k, n_cols):
     with torch.no_grad():
         assert torch.equal(torch.ops.sw_gcn.fusedGeMMSpMM(adj, x, w, [], 4), want)
     ticket.close()
+
+
+def test_backward_on_two_streams(built_lib):
+    """Two models on one adjacency share its plan; the sparse products of their backward passes run beside one another, long rows
+    (cut into pieces that are counted) included."""
+    import torch
+    import tile_fusion_b200.sw_gcn as sw
+    from tests.test_gather import _graph
+    n, k, c = 4000, 48, 64
+    t = _graph(n, 5, hubs=[(r, 1500 + r) for r in range(0, 400, 10)])
+    adj = torch.sparse_csr_tensor(*(torch.from_numpy(x) for x in t), size=(n, n)).cuda()
+    plan = sw._plan(adj, k, c)
+    assert sw._lib.lib().tf_exec_spmm_work_bytes(plan._h) > 0
+    gs = [torch.from_numpy(synth.uniform(s, (n, c))).cuda() for s in (1, 2)]
+    want = [sw._spmm(plan, g) for g in gs]
+    streams = [torch.cuda.Stream() for _ in gs]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        got = []
+        for s, g in zip(streams, gs):
+            with torch.cuda.stream(s):
+                got.append([sw._spmm(plan, g) for _ in range(4)])
+        torch.cuda.synchronize()
+        for outs, w in zip(got, want):
+            assert all(torch.equal(o, w) for o in outs)
+    # scratch that is too small is refused
+    x, w = gs[0], torch.empty(16, dtype=torch.uint8, device="cuda")
+    assert sw._lib.lib().tf_exec_spmm_work(plan._h, x.data_ptr(), c, want[0].data_ptr(), w.data_ptr(), 16, None) == sw._lib.TF_ERR_ARG

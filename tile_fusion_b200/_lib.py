@@ -43,7 +43,7 @@ EXPORTS = [
     "tf_schedule_free", "tf_plan_spmm_spmm", "tf_plan_gemm_spmm", "tf_plan_sddmm_spmm", "tf_plan_free",
     "tf_plan_info", "tf_plan_status", "tf_exec_spmm_spmm", "tf_exec_gemm_spmm", "tf_exec_sddmm_spmm",
     "tf_exec_phase", "tf_plan_intermediate", "tf_plan_exchange_buffers", "tf_spmm_spmm_host", "tf_gemm_spmm_host",
-    "tf_sddmm_spmm_host", "tf_exec_spmm", "tf_csr_checksum", "tf_atb_dev", "tf_atb_work_floats", "tf_spmm_dev", "tf_fill_uniform", "tf_fill_normal", "tf_plan_preview", "tf_free", "tf_plan_set_wait_limit", "tf_tiling_preview", "tf_segment_preview", "tf_plan_tile_info", "tf_spmm_spmm_noalloc",
+    "tf_sddmm_spmm_host", "tf_exec_spmm", "tf_exec_spmm_work", "tf_exec_spmm_work_bytes", "tf_csr_checksum", "tf_atb_dev", "tf_atb_work_floats", "tf_spmm_dev", "tf_fill_uniform", "tf_fill_normal", "tf_plan_preview", "tf_free", "tf_plan_set_wait_limit", "tf_tiling_preview", "tf_segment_preview", "tf_plan_tile_info", "tf_spmm_spmm_noalloc",
     "tf_noalloc_max_floats", "tf_gemm_tc_dev", "tf_lattice_preview", "tf_comm_unique_id", "tf_comm_create",
     "tf_comm_from_nccl", "tf_comm_free", "tf_multi_plan", "tf_multi_free", "tf_multi_info", "tf_multi_plan_handle",
     "tf_multi_exec", "tf_multi_status", "tf_multi_trace", "tf_partition_layout", "tf_read_matrix", "tf_read_dense_mtx",
@@ -93,6 +93,9 @@ def lib() -> C.CDLL:
     L.tf_gemm_spmm_host.argtypes = [vp, vp, vp, i, i, vp]
     L.tf_sddmm_spmm_host.argtypes = [vp, vp, vp, vp, vp]
     L.tf_exec_spmm.argtypes = [vp, vp, i, vp, vp]
+    L.tf_exec_spmm_work.argtypes = [vp, vp, i, vp, vp, C.c_size_t, vp]
+    L.tf_exec_spmm_work_bytes.argtypes = [vp]
+    L.tf_exec_spmm_work_bytes.restype = C.c_size_t
     L.tf_atb_work_floats.argtypes = [i, i, i]
     L.tf_atb_work_floats.restype = C.c_longlong
     L.tf_atb_dev.argtypes = [vp, i, vp, i, i, vp, vp, C.c_longlong, vp]

@@ -275,9 +275,16 @@ class Plan:
                                             stream if stream is not None else _stream_ptr()))
 
     def spmm(self, Xd, outd, stream=None):
-        """out = A X with the plan's operator A."""
-        check(_lib.lib().tf_exec_spmm(self._h, Xd.data_ptr(), Xd.shape[1], outd.data_ptr(),
-                                      stream if stream is not None else _stream_ptr()))
+        """out = A X with the plan's operator A, beside whatever else runs on the plan: what the product keeps between its
+        groups is scratch of the call."""
+        import torch
+        L = _lib.lib()
+        n = L.tf_exec_spmm_work_bytes(self._h)
+        s = torch.cuda.current_stream() if stream is None else torch.cuda.ExternalStream(stream)
+        with torch.cuda.stream(s):
+            work = torch.empty(n, dtype=torch.uint8, device=outd.device) if n else None
+        check(L.tf_exec_spmm_work(self._h, Xd.data_ptr(), Xd.shape[1], outd.data_ptr(), work.data_ptr() if n else None, n,
+                                  s.cuda_stream))
 
     def phase(self, phase, in0, in1=None, out=None, w_transposed=False, relu=False, stream=None):
         check(_lib.lib().tf_exec_phase(self._h, int(phase), in0.data_ptr(), in1.data_ptr() if in1 is not None else None,

@@ -79,7 +79,7 @@ struct DevCsr {
 // Operator of the balanced gather (gather.cu).
 struct DevGather {
   bool on = false;
-  int n_units = 0, n_empty = 0, partial_ld = 0;
+  int n_units = 0, n_empty = 0, partial_ld = 0, n_slots = 0;
   DevBuf<int> cols;
   DevBuf<float> vals;
   DevBuf<int4> units, heavy;
@@ -109,6 +109,7 @@ struct DevGather {
     tf::build_gather_plan(A.m, A.ap, A.ai, A.ax, sm_count * (resident / tfk::gather_group(n_cols)), ticket_sums, g);
     n_units = (int)g.units.size();
     n_empty = (int)g.empty_rows.size();
+    n_slots = g.n_slots;
     partial_ld = (std::max(n_cols, max_cols) + 3) / 4 * 4;
     const int panels = (partial_ld + 127) / 128;  // the most any width up to that is read in
     if (follow) follow_units(g, A.m);
@@ -126,6 +127,10 @@ struct DevGather {
     on = true;
     return TF_OK;
   }
+  // What a product keeps between its groups, for a caller's buffer in the place of the plan's own: the counters of the cut rows,
+  // then their partial sums.
+  size_t scratch_counters() const { return (cnt.n * sizeof(int) + 255) / 256 * 256; }
+  size_t scratch_bytes() const { return heavy.n ? scratch_counters() + (size_t)n_slots * partial_ld * sizeof(float) : 0; }
 };
 
 }  // namespace
@@ -1265,8 +1270,13 @@ tfk::GatherParams gather_params(const DevGather &g, const float *X, int ld_in, f
 }
 // (a run of units: the caller has seen to the empty rows)
 int run_gather(const DevGather &g, const float *X, int ld_in, bool vec_in, float *Y, int ld_out, bool vec_out, int n_cols,
-               bool relu, cudaStream_t s, int unit_begin = 0, int unit_end = -1) {
+               bool relu, cudaStream_t s, int unit_begin = 0, int unit_end = -1, void *scratch = nullptr) {
   tfk::GatherParams P = gather_params(g, X, ld_in, Y, ld_out, n_cols);
+  if (scratch && g.heavy.n) {
+    P.heavy_cnt = (int *)scratch;
+    P.partial = (float *)((char *)scratch + g.scratch_counters());
+    TF_CUDA(cudaMemsetAsync(scratch, 0, g.cnt.n * sizeof(int), s));
+  }
   const int group = tfk::gather_group(n_cols);
   P.panel_w = vec_in ? 4 * group : 128;
   P.relu = relu ? 1 : 0;
@@ -1494,15 +1504,23 @@ int tf_exec_sddmm_spmm(tf_plan *p, const float *Q, const float *K, const float *
   return run_phases(*p, P, 1, 1, (cudaStream_t)stream);
 }
 
+size_t tf_exec_spmm_work_bytes(const tf_plan *p) { return p && p->g_second.on ? p->g_second.scratch_bytes() : 0; }
+
 int tf_exec_spmm(tf_plan *p, const float *X, int n_cols, float *out, void *stream) {
+  return tf_exec_spmm_work(p, X, n_cols, out, nullptr, 0, stream);
+}
+
+int tf_exec_spmm_work(tf_plan *p, const float *X, int n_cols, float *out, void *work, size_t work_bytes, void *stream) {
   if (!p || !X || !out) return fail(TF_ERR_ARG, "tf_exec_spmm: null argument");
+  if (work && (work_bytes < tf_exec_spmm_work_bytes(p) || !aligned(work, 16)))
+    return fail(TF_ERR_ARG, "tf_exec_spmm_work: work space too small or not on a 16-byte boundary");
   if (n_cols <= 0) return fail(TF_ERR_ARG, "tf_exec_spmm: bad width");
   int rc = set_device(*p);
   if (rc != TF_OK) return rc;
   const cudaStream_t s = (cudaStream_t)stream;
   if (p->g_second.on && n_cols <= p->g_second.partial_ld)
     return run_gather(p->g_second, X, n_cols, n_cols % 4 == 0 && aligned(X, 16), out, n_cols, n_cols % 4 == 0 && aligned(out, 16),
-                      n_cols, false, s);
+                      n_cols, false, s, 0, -1, work);
   if (!p->second.ap.n) return fail(TF_ERR_UNSUPPORTED, "tf_exec_spmm: wider than the plan's dense operands");
   return tf_spmm_dev(p->second.ap.p, p->second.ai.p, p->second.ax.p, p->m, X, n_cols, out, stream);
 }
