@@ -128,3 +128,19 @@ def test_backward_on_two_streams(built_lib):
     # scratch that is too small is refused
     x, w = gs[0], torch.empty(16, dtype=torch.uint8, device="cuda")
     assert sw._lib.lib().tf_exec_spmm_work(plan._h, x.data_ptr(), c, want[0].data_ptr(), w.data_ptr(), 16, None) == sw._lib.TF_ERR_ARG
+
+
+@pytest.mark.parametrize("n,k,c", [(300, 4100, 4099), (9000, 32, 7), (9000, 32, 12), (5000, 1433, 16), (2000, 602, 256), (600, 1, 40), (600, 64, 1)])
+def test_weight_gradient_of_any_size(built_lib, n, k, c):
+    """Layers of more than 2^24 weights, of one feature or class, of few entries and of many: dW against fp64, as before the
+    library had a kernel of its own for it."""
+    import torch
+    import tile_fusion_b200.sw_gcn  # noqa: F401
+    g = synth.rmat_gcn(6, n, 8)
+    adj = torch.sparse_csr_tensor(*(torch.from_numpy(t) for t in g), size=(n, n)).cuda()
+    x = torch.from_numpy(synth.normal(2, (n, k))).cuda()
+    w = torch.from_numpy(synth.glorot(3, c, k)).cuda().requires_grad_(True)
+    dy = torch.from_numpy(synth.uniform(4, (n, c))).cuda()
+    torch.ops.sw_gcn.fusedGeMMSpMM(adj, x, w, [], 4).backward(dy)
+    want = (adj.to_dense().double() @ dy.double()).t() @ x.double()
+    common.assert_close(w.grad.cpu().numpy(), want.cpu().numpy(), "dW")

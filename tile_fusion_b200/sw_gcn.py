@@ -76,12 +76,27 @@ def _spmm(plan, x):
     return out
 
 
+def _own_weight_grad(m, na, nb):
+    """Whether the library's own kernel takes a weight gradient of na x nb over m rows.  Its tiles are 64 or 128 x 128 and
+    it gains by cutting the rows into as many ranges as the device holds.  So not: one row or column (a matrix-vector product:
+    120 001 rows, 1 x 256: 103 us, torch 43); so few entries that a tile is mostly padding (16 x 16: 58 and 43, 500 009 rows:
+    207 and 107; 7 x 64: 58 and 154, 209 and 110); so many tiles that few ranges are left (512 x 512: 1 289 and 1 245, 12 tiles
+    of 16 x 1433: 619 and 541, at 20 000 rows 115 and 179), above all of few rows (1 000 rows, 256 x 602: 29 and 21); and
+    nothing beyond 2^24 entries, which it does not take at all."""
+    entries, tiles = na * nb, -(-na // (64 if na <= 64 else 128)) * -(-nb // 128)
+    if na == 1 or nb == 1 or entries > 1 << 24:
+        return False
+    if (entries <= 320 and m >= 8192) or (entries <= 512 and m >= 1 << 18):
+        return False
+    return tiles <= 8 or (tiles <= 10 and m >= 4096) or (tiles < 16 and 4096 <= m < 65536)
+
+
 def _weight_grad(a, b):
     """a.T @ b for two tall matrices: a sum over all rows.  (With a graph to record, by the operator that records.)"""
-    if torch.is_grad_enabled():
+    m, na, nb = a.shape[0], a.shape[1], b.shape[1]
+    if torch.is_grad_enabled() or not _own_weight_grad(m, na, nb):
         return a.t() @ b
     L = _lib.lib()
-    m, na, nb = a.shape[0], a.shape[1], b.shape[1]
     out = torch.empty((na, nb), device=a.device, dtype=torch.float32)
     work = torch.empty(L.tf_atb_work_floats(m, na, nb), device=a.device, dtype=torch.float32)
     _lib.check(L.tf_atb_dev(a.data_ptr(), na, b.data_ptr(), nb, m, out.data_ptr(), work.data_ptr(), work.numel(),
