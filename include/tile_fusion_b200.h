@@ -247,7 +247,9 @@ long long tf_atb_work_floats(int m, int na, int nb);
  *   phase 0  produce the boundary rows of the intermediate (then send them),
  *   phase 1  everything that needs no halo row,
  *   phase 2  the consumer rows that read halo rows (after the receive).
- * tf_plan_intermediate gives the device buffer: local rows first, then halo rows. */
+ * tf_plan_intermediate gives the device buffer: local rows first, then halo rows, `cols` floats apart.  Plans whose executor
+ * leaves no intermediate in memory do so from this call on, at the cost of it (the plane march of 3-D grids with an even x
+ * extent excepted: it never has).  Not beside a running call. */
 int tf_exec_phase(tf_plan *p, int phase, const float *in0, const float *in1, int w_transposed, int relu,
                   float *D, void *stream);
 int tf_plan_intermediate(tf_plan *p, float **dev_ptr, long long *rows, int *cols);

@@ -205,6 +205,7 @@ struct tf_plan {
   DevBuf<float> g_pad;       // rows of C of a width that is no multiple of four, padded to ld_t
   struct Piece { int f_begin, f_end, begin, end; long long in_rows, out_rows; };  // units of the first and second operator
   std::vector<Piece> pieces;  // see make_gather_pieces
+  bool keep_t = false;       // the caller asked for the intermediate: every call leaves it in `inter`
   bool spmm_first = false;   // GeMM-SpMM on the balanced gather: D = (A B) C instead of A (B C)
   bool ticket_sums = false;  // every sum in the order of the ticket executor (tensor_cores > 0)
   size_t dyn_smem = 0;
@@ -712,6 +713,63 @@ int run_band(tf_plan &p, const float *C, float *D, int block_begin, int block_en
 }
 int band_blocks(const tf_plan &p) { return (p.m + p.band.block - 1) / p.band.block; }
 
+// The CSR arrays of an operator that a plan holds as line words or band quads only, for the calls that need them after all.
+int restore_csr(tf_plan &p, bool second) {
+  DevCsr &out = second || p.first_is_second ? p.second : p.first;
+  if (out.ap.n) return TF_OK;
+  std::vector<int> ap(1, 0), ai;
+  std::vector<float> ax;
+  auto fetch = [](auto &host, const auto &dev) {
+    host.resize(dev.n);
+    return cudaMemcpy(host.data(), dev.p, dev.n * sizeof(*dev.p), cudaMemcpyDeviceToHost);
+  };
+  if (p.lines.on) {
+    const tf_plan::Lines &L = p.lines;
+    std::vector<unsigned> words;
+    TF_CUDA(fetch(words, second || L.same ? L.words_a : L.words_f));
+    const float *dict = reinterpret_cast<const float *>(second || L.same ? L.par.dict_a : L.par.dict_f);
+    for (int y = 0; y < L.ny; ++y)
+      for (int x = 0; x < L.nx; ++x) {
+        const int t = x / tf::kLineOut, i = x - t * tf::kLineOut + 2, r = y * L.nx + x;
+        const unsigned cls = words[((size_t)y * L.tiles + t) * 8 + i / 4] >> (8 * (i & 3)) & 255u;
+        const int off[5] = {-L.nx, -1, 0, 1, L.nx};
+        const bool in[5] = {y > 0, x > 0, true, x < L.nx - 1, y < L.ny - 1};
+        for (int q = 0; q < 5; ++q)
+          if (in[q]) { ai.push_back(r + off[q]); ax.push_back(dict[8 * (size_t)cls + q]); }
+        ap.push_back((int)ai.size());
+      }
+  } else {
+    const tf_plan::Band &K = p.band;
+    const bool a = second || K.par.same;
+    const int pairs = a && !K.par.same ? K.par.pairs_a : K.par.pairs_f;
+    std::vector<int> quads;
+    TF_CUDA(fetch(quads, a && !K.par.same ? K.quads_a : K.quads_f));
+    for (int r = 0; r < p.m; ++r) {
+      for (int k = 0; k < 2 * pairs; ++k) {
+        const int *q = &quads[4 * (((size_t)(r / K.block) * pairs + k / 2) * K.block + r % K.block) + 2 * (k & 1)];
+        if (q[0] & 1) continue;  // no nonzero
+        ai.push_back(r + q[0] / 128);
+        float v;
+        std::memcpy(&v, &q[1], 4);
+        ax.push_back(v);
+      }
+      ap.push_back((int)ai.size());
+    }
+  }
+  tf_csr h;
+  std::memset(&h, 0, sizeof(h));
+  h.m = p.m; h.n = p.m;
+  h.ap = ap.data(); h.ai = ai.data(); h.ax = ax.data();
+  return out.upload(h);
+}
+
+// T of a march that leaves none behind, where the caller asked for it.
+int leave_intermediate(tf_plan &p, const float *C, cudaStream_t s) {
+  if (!p.keep_t) return TF_OK;
+  const DevCsr &f = p.first_is_second ? p.second : p.first;
+  return tf_spmm_dev(f.ap.p, f.ai.p, f.ax.p, p.m, C, p.n_cols, p.inter.p, s);
+}
+
 // GeMM-SpMM on the balanced gather.  The two products may be taken in either order, D = A (B C) = (A B) C: the sparse
 // product reads one row of its operand per nonzero, so it is given the narrower one -- B where k < n_cols, else B C.
 // (Rows of B that do not start on 16-byte boundaries would be gathered value by value; then B C comes first.  So it does
@@ -990,7 +1048,9 @@ tfk::Params base_params(tf_plan &p) {
 }
 
 bool aligned(const void *q, size_t a) { return (reinterpret_cast<uintptr_t>(q) % a) == 0; }
-bool march_usable(const tf_plan &p, const float *C, const float *D) { return p.march.on && aligned(C, 16) && aligned(D, 16); }
+bool march_usable(const tf_plan &p, const float *C, const float *D) {
+  return p.march.on && !(p.keep_t && p.march.nx % 2) && aligned(C, 16) && aligned(D, 16);
+}
 
 // vector width usable with the caller's pointers (plan-owned buffers are always aligned)
 void call_shape(const tf_plan &p, std::initializer_list<const void *> ptrs, int *vec, int *ch) {
@@ -1205,6 +1265,7 @@ int run_host_march(tf_plan &p, const float *h_in, float *d_in, float *h_out, flo
     TF_CUDA(p.host_pipe->download(h_out + at(z_begin), d_out + at(z_begin), (at(z_end) - at(z_begin)) * sizeof(float), p.s_d2h));
   }
   p.launches = launches;
+  if (lines || band) TF_TRY(leave_intermediate(p, d_in, p.s_run));
   TF_CUDA(p.host_pipe->finish());
   TF_CUDA(cudaStreamSynchronize(p.s_d2h));
   TF_CUDA(cudaStreamSynchronize(p.s_run));
@@ -1436,8 +1497,10 @@ int tf_exec_spmm_spmm(tf_plan *p, const float *C, float *D, void *stream) {
   if (p->halo_rows || p->sendbuf.n) return fail(TF_ERR_ARG, "tf_exec_spmm_spmm: plan has halo rows, drive it with tf_exec_phase");
   int rc = set_device(*p);
   if (rc != TF_OK) return rc;
-  if (p->lines.on) return run_lines(*p, C, D, 0, p->lines.ny, (cudaStream_t)stream);
-  if (p->band.block) return run_band(*p, C, D, 0, band_blocks(*p), (cudaStream_t)stream);
+  if (p->lines.on || p->band.block) {
+    TF_TRY(p->lines.on ? run_lines(*p, C, D, 0, p->lines.ny, (cudaStream_t)stream) : run_band(*p, C, D, 0, band_blocks(*p), (cudaStream_t)stream));
+    return leave_intermediate(*p, C, (cudaStream_t)stream);
+  }
   if (march_usable(*p, C, D)) return run_march(*p, C, D, 0, p->march.n_items, false, (cudaStream_t)stream);
   if (p->g_second.on) return run_gather_spmm_spmm(*p, C, D, (cudaStream_t)stream);
   tfk::Params P = base_params(*p);
@@ -1558,13 +1621,9 @@ int tf_exec_phase(tf_plan *p, int phase, const float *in0, const float *in1, int
   if (phase > 0 && p->chain == 0 && march_usable(*p, in0, D))
     return phase == 1 ? run_march(*p, in0, D, 0, p->march.n_phase1, false, (cudaStream_t)stream)
                       : run_march(*p, in0, D, p->march.n_phase1, p->march.n_items, true, (cudaStream_t)stream);
-  if (p->lines.on) {  // no exchange: phase 1 is the whole chain
+  if (p->lines.on || p->band.block) {  // no exchange: phase 1 is the whole chain
     p->launches = 0;
-    return phase == 1 ? run_lines(*p, in0, D, 0, p->lines.ny, (cudaStream_t)stream) : TF_OK;
-  }
-  if (p->band.block) {
-    p->launches = 0;
-    return phase == 1 ? run_band(*p, in0, D, 0, band_blocks(*p), (cudaStream_t)stream) : TF_OK;
+    return phase == 1 ? tf_exec_spmm_spmm(p, in0, D, stream) : TF_OK;
   }
   if (p->g_second.on) {  // no exchange: phase 1 is the whole chain
     p->launches = 0;
@@ -1579,6 +1638,19 @@ int tf_exec_phase(tf_plan *p, int phase, const float *in0, const float *in1, int
 
 int tf_plan_intermediate(tf_plan *p, float **dev_ptr, long long *rows, int *cols) {
   if (!p) return fail(TF_ERR_ARG, "tf_plan_intermediate: null plan");
+  if (!p->keep_t) {  // executors that leave no T = F C (T = B W) in memory do so from now on
+    TF_TRY(set_device(*p));
+    if (p->spmm_first) {
+      p->ld_t = (p->n_cols + 3) / 4 * 4;
+      TF_TRY(p->inter.alloc((size_t)(p->m + 1) * p->ld_t));
+      p->spmm_first = false;
+    } else if (p->lines.on || p->band.block) {
+      TF_TRY(restore_csr(*p, false));
+      TF_TRY(p->inter.alloc((size_t)p->m * p->n_cols));
+      p->hp.inter_rows = p->m;
+    }
+    p->keep_t = true;
+  }
   if (dev_ptr) *dev_ptr = p->inter.p;
   if (rows) *rows = p->hp.inter_rows;
   if (cols) *cols = p->ld_t ? p->ld_t : p->n_cols;

@@ -266,7 +266,7 @@ int setup_direct_exchange(tf_multi &M, const std::vector<long long> &bounds, con
   float *base = nullptr;
   long long rows = 0;
   int cols = 0;
-  int rc = tf_plan_intermediate(M.plan, &base, &rows, &cols);
+  int rc = M.halobuf ? tf_plan_intermediate(M.plan, &base, &rows, &cols) : TF_OK;
   if (rc != TF_OK) return rc;
   bool can = allow_direct;
   if (M.halobuf && base) {
