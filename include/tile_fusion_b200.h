@@ -230,8 +230,9 @@ int tf_exec_gemm_spmm(tf_plan *p, const float *B, const float *W, int w_transpos
 int tf_exec_sddmm_spmm(tf_plan *p, const float *Q, const float *K, const float *V, float *D,
                        void *stream);
 
-/* out = A * X with the plan's A, X and out n_cols wide (at most the widest dense operand of the plan): the sparse product
- * of a layer's backward pass (binding-project/src/Functions.cpp:1192-1244) on the operator that its forward pass uses. */
+/* out = A * X with the A of any plan, X and out n_cols wide: the sparse product of a layer's backward pass
+ * (binding-project/src/Functions.cpp:1192-1244) on the operator that its forward pass uses.  (Plans that march along lines or
+ * down a band copy their operator back to a CSR on the first call, which waits for the device.) */
 int tf_exec_spmm(tf_plan *p, const float *X, int n_cols, float *out, void *stream);
 /* The same with scratch of the caller's (device memory, 16-byte aligned, tf_exec_spmm_work_bytes of it) instead of the plan's,
  * so that it may run beside other calls on the plan, on any stream; tf_exec_spmm, like the other executors, may not. */

@@ -1581,10 +1581,16 @@ int tf_exec_spmm_work(tf_plan *p, const float *X, int n_cols, float *out, void *
   int rc = set_device(*p);
   if (rc != TF_OK) return rc;
   const cudaStream_t s = (cudaStream_t)stream;
-  if (p->g_second.on && n_cols <= p->g_second.partial_ld)
-    return run_gather(p->g_second, X, n_cols, n_cols % 4 == 0 && aligned(X, 16), out, n_cols, n_cols % 4 == 0 && aligned(out, 16),
-                      n_cols, false, s, 0, -1, work);
-  if (!p->second.ap.n) return fail(TF_ERR_UNSUPPORTED, "tf_exec_spmm: wider than the plan's dense operands");
+  if (p->g_second.on) {
+    const DevGather &g = p->g_second;
+    const bool in16 = n_cols % 4 == 0 && aligned(X, 16), out16 = n_cols % 4 == 0 && aligned(out, 16);
+    // (as many columns at a time as the partial sums of cut rows have room for; the first pass sees to the rows without nonzeros)
+    for (int c = 0; c < n_cols; c += g.partial_ld)
+      TF_TRY(run_gather(g, X + c, n_cols, in16, out + c, n_cols, out16, std::min(g.partial_ld, n_cols - c), false, s, 0,
+                        c ? g.n_units : -1, work));
+    return TF_OK;
+  }
+  if (!p->second.ap.n) TF_TRY(restore_csr(*p, true));
   return tf_spmm_dev(p->second.ap.p, p->second.ai.p, p->second.ax.p, p->m, X, n_cols, out, stream);
 }
 
