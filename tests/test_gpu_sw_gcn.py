@@ -144,3 +144,25 @@ def test_weight_gradient_of_any_size(built_lib, n, k, c):
     torch.ops.sw_gcn.fusedGeMMSpMM(adj, x, w, [], 4).backward(dy)
     want = (adj.to_dense().double() @ dy.double()).t() @ x.double()
     common.assert_close(w.grad.cpu().numpy(), want.cpu().numpy(), "dW")
+
+
+@pytest.mark.parametrize("index,value", [("int32", "float32"), ("int64", "float32"), ("int64", "float64")])
+def test_adjacency_is_held_and_not_copied(built_lib, index, value):
+    """The cache knows an adjacency by where it lies, so it holds it -- another of the same sizes is another one -- but keeps no
+    second copy on the device: what a first call on an adjacency leaves allocated is its plan's and the output's."""
+    import torch
+    import tile_fusion_b200.sw_gcn as sw
+    n = 3000
+    g = synth.rmat_gcn(6, n, 12)
+    x, w = torch.from_numpy(synth.normal(2, (n, 32))).cuda(), torch.from_numpy(synth.glorot(3, 48, 32)).cuda()
+    for scale in (1.0, 2.0, 3.0):
+        parts = [torch.from_numpy(g[0]).to(getattr(torch, index)).cuda(), torch.from_numpy(g[1]).to(getattr(torch, index)).cuda(),
+                 (torch.from_numpy(g[2]) * scale).to(getattr(torch, value)).cuda()]
+        adj = torch.sparse_csr_tensor(*parts, size=(n, n))
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        out = torch.ops.sw_gcn.fusedGeMMSpMM(adj, x, w, [], 4)
+        assert torch.cuda.memory_allocated() - before <= out.numel() * 4 + 512
+        want = adj.to_dense().double() @ (x.double() @ w.double().t())
+        common.assert_close(out.cpu().numpy(), want.cpu().numpy(), f"scale {scale}")
+        del adj, parts, out, want

@@ -36,7 +36,8 @@ _plans: dict = {}
 
 
 def _csr_of(adj: torch.Tensor):
-    """(key, CSRMatrix on the host, device arrays) of a sparse-CSR adjacency; cached per tensor storage."""
+    """(key, CSRMatrix on the host) of a sparse-CSR adjacency; cached per tensor storage.  The entry holds the tensors
+    themselves, whatever their types, so that no other adjacency can come to lie where a cached one lay."""
     if adj.layout != torch.sparse_csr:
         raise ValueError("sw_gcn: the adjacency must be a torch sparse CSR tensor")
     crow, col, val = adj.crow_indices(), adj.col_indices(), adj.values()
@@ -45,19 +46,17 @@ def _csr_of(adj: torch.Tensor):
     if hit is None:
         A = api.CSRMatrix(adj.shape[0], adj.shape[1], crow.to(torch.int32).cpu().numpy(), col.to(torch.int32).cpu().numpy(),
                           val.to(torch.float32).cpu().numpy())
-        dev = (crow.to(torch.int32).cuda().contiguous(), col.to(torch.int32).cuda().contiguous(),
-               val.to(torch.float32).cuda().contiguous())
         if len(_plans) > 64:
             for p in list(_plans.values()):
                 if isinstance(p, api.Plan):
                     p.close()
             _plans.clear()
-        hit = _plans[("csr", key)] = (A, dev)
-    return key, hit[0], hit[1]
+        hit = _plans[("csr", key)] = (A, (crow, col, val))
+    return key, hit[0]
 
 
 def _plan(adj, k, n, unfused=False):
-    key, A, _ = _csr_of(adj)
+    key, A = _csr_of(adj)
     pk = ("plan", key, k, n, unfused)
     p = _plans.get(pk)
     if p is None:
@@ -142,7 +141,7 @@ class _CachedSpMMGeMM(torch.autograd.Function):
 
 
 def _schedule_tensors(adj, kind, **prm):
-    _, A, _ = _csr_of(adj)
+    _, A = _csr_of(adj)
     s = api.inspector(A, prm.pop("threads"), kind=kind, **prm)
     level = torch.from_numpy(np.concatenate([s.ptr1, np.zeros(max(0, 3 - len(s.ptr1)), np.int32)])[:3].astype(np.int32))
     mix = torch.from_numpy(np.concatenate([np.zeros(2, np.int32), s.ker_begin]).astype(np.int32)) if s.ker_begin is not None \
