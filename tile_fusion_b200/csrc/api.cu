@@ -673,7 +673,7 @@ int build_band(tf_plan &p, const tf_csr &F, const tf_csr &A, bool same, int sm_c
   reach_f = reach_a; pairs_f = pairs_a;
   if (!same && !tf::band_shape(F.m, F.n, F.ap, F.ai, &reach_f, &pairs_f)) return TF_OK;
   const int block = std::max(reach_a, reach_f) <= 64 ? 64 : 128;
-  if (tfk::band_smem(block, pairs_f, pairs_a, same) > 226 * 1024) return TF_OK;
+  if (tfk::band_smem(block, pairs_f, pairs_a, same) > tfk::kBandSmemMax) return TF_OK;
   tf_plan::Band &K = p.band;
   tf::BandOp op;
   tf::build_band_operator(F.m, F.ap, F.ai, F.ax, block, pairs_f, op);

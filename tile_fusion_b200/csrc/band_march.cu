@@ -126,6 +126,8 @@ band_march_kernel(const __grid_constant__ CUtensorMap tm_c, const BandParams P) 
 
 }  // namespace
 
+static_assert(kBandSmemMax <= 227 * 1024 - 64, "with the four barriers, what a CTA has");
+
 int band_make_map(CUtensorMap *out, const float *c, long long rows, int n_cols, int block) {
   return tc_make_map(out, c, rows, n_cols, block, n_cols, false);
 }
@@ -143,7 +145,9 @@ static cudaError_t launch(const CUtensorMap &tm_c, BandParams &p, int sm_count, 
   const size_t smem = band_smem(S, p.pairs_f, p.pairs_a, p.same);
   const long long resident = (long long)sm_count * (S == 64 && smem <= 112 * 1024 ? 2 : 1);
   p.seg_blocks = tf::segment_length(n, p.chunks, resident, 3, 1);  // a segment of n blocks of D takes n + 3 steps
-  cudaError_t e = cudaFuncSetAttribute((const void *)band_march_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // (the limit is the kernel's, not the call's: the same for all operators, so that threads with different plans don't lower it
+  // for one another)
+  cudaError_t e = cudaFuncSetAttribute((const void *)band_march_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBandSmemMax);
   if (e != cudaSuccess) return e;
   const long long ctas = (long long)((n + p.seg_blocks - 1) / p.seg_blocks) * p.chunks;
   band_march_kernel<S><<<(unsigned)ctas, kBandThreads, smem, s>>>(tm_c, p);

@@ -37,7 +37,8 @@ struct BandParams {
 
 // Tensor map of C: boxes of 32 columns x `block` rows.
 int band_make_map(CUtensorMap *out, const float *c, long long rows, int n_cols, int block);
-// Shared memory of the kernel for these widths; plans whose operators need more than a CTA has are not made.
+// Shared memory of the kernel for these widths; plans whose operators need more than kBandSmemMax are not made.
+constexpr int kBandSmemMax = 226 * 1024;
 size_t band_smem(int block, int pairs_f, int pairs_a, bool same);
 // Fills in chunks, blocks and seg_blocks and launches.
 cudaError_t launch_band_march(const CUtensorMap &tm_c, int block, BandParams &p, int sm_count, cudaStream_t s);

@@ -550,7 +550,9 @@ static int launch_panel(const float *X, int m, int K, int ld_x, const float *W, 
   if (rc != TF_OK) return rc;
   const size_t smem = (size_t)P.stages * rg_stage_bytes(n_pad) + kRgEpiBytes + 1024;
   auto f = precise ? row_gemm_kernel<true> : row_gemm_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute((const void *)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // (the limit is the kernel's, not the call's: the same for all widths, so that threads with different plans don't lower it
+  // for one another)
+  cudaError_t e = cudaFuncSetAttribute((const void *)f, cudaFuncAttributeMaxDynamicSharedMemorySize, kRgSmemMax - 1024);
   if (e == cudaSuccess) {
     f<<<2 * std::max(1, std::min(P.tiles, sm_count / 2)), kRgThreads, smem, s>>>(ma, mh, ml, mo, P);
     e = cudaGetLastError();
