@@ -33,14 +33,14 @@ __device__ __forceinline__ float4 band_row(const int4 *quads, int pairs, int row
   constexpr unsigned mask = 4u * S * 128u - 1;
   const int r = row + (lane >> 3);
   const int4 *q = quads + (r & (S - 1));
-  const int base = r * 128;  // (modulo the ring, which is a power of two)
+  const unsigned base = (unsigned)r * 128u;  // (modulo the ring, which is a power of two; the row count is not bounded by it)
   const char *col = ring + (lane & 7) * 16;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
   for (int k = 0; k < pairs; ++k) {
     const int4 e = q[k * S];
-    const float4 x = *reinterpret_cast<const float4 *>(col + ((unsigned)(base + (e.x & ~1)) & mask));
-    const float4 y = *reinterpret_cast<const float4 *>(col + ((unsigned)(base + (e.z & ~1)) & mask));
+    const float4 x = *reinterpret_cast<const float4 *>(col + ((base + (unsigned)(e.x & ~1)) & mask));
+    const float4 y = *reinterpret_cast<const float4 *>(col + ((base + (unsigned)(e.z & ~1)) & mask));
     if (!(e.x & 1)) {
       const float v = __int_as_float(e.y);
       acc.x = fmaf(v, x.x, acc.x); acc.y = fmaf(v, x.y, acc.y); acc.z = fmaf(v, x.z, acc.z); acc.w = fmaf(v, x.w, acc.w);
@@ -102,7 +102,7 @@ band_march_kernel(const __grid_constant__ CUtensorMap tm_c, const BandParams P) 
       for (int q = 0; q < S / 4; q += kWarps) {
         const int row = s * S + 4 * (q + warp);
         const float4 t = band_row<S>(quads, P.pairs_f, row, c_ring, lane);
-        *reinterpret_cast<float4 *>(t_ring + ((unsigned)((row + (lane >> 3)) * 128) & (kRing - 1)) + (lane & 7) * 16) = t;
+        *reinterpret_cast<float4 *>(t_ring + (((unsigned)(row + (lane >> 3)) * 128u) & (kRing - 1)) + (lane & 7) * 16) = t;
       }
     }
     if (ok && s - 2 >= jb) {
