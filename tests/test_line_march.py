@@ -92,3 +92,32 @@ def test_other_operators_are_declined(built_lib):
         plan = api.Plan("spmm_spmm", api.CSRMatrix(n, n, T.indptr.astype(np.int32), T.indices.astype(np.int32), data), n_cols=32)
         assert plan.info()["threads"] != 128
         plan.close()
+
+
+@pytest.mark.parametrize("dims,taken", [((1000, 2), True), ((511, 2), True), ((400, 2), False), ((1000, 3), False)])
+def test_two_long_lines_off_the_16_byte_grid(built_lib, dims, taken):
+    """Two long lines have no reuse that a gather tile could hold, and the executor that takes such operators reads rows wherever
+    they lie: so does this one.  Where tiles would be taken, operands off the 16-byte grid are refused as they ask."""
+    import torch
+    from tile_fusion_b200 import _lib
+    t = synth.laplacian(dims)
+    n, w = len(t[0]) - 1, 32
+    plan = api.Plan("spmm_spmm", _csr(t), n_cols=w)
+    old = api.Plan("spmm_spmm", _csr(t), n_cols=w, lattice_march=-1)
+    assert plan.info()["threads"] == 128
+    c = torch.from_numpy(synth.uniform(3, (n, w))).cuda()
+    d = torch.empty((n, w), device="cuda")
+    plan.spmm_spmm(c, d)
+    cu = torch.empty(n * w + 1, device="cuda")[1:].view(n, w).copy_(c)
+    du = torch.full((n * w + 1,), float("nan"), device="cuda")[1:].view(n, w)
+    for p in (plan, old):
+        if taken:
+            p.spmm_spmm(cu, du)
+            p.status()
+            assert torch.equal(du, d)
+            du.fill_(float("nan"))
+        else:
+            with pytest.raises(_lib.TileFusionError) as e:
+                p.spmm_spmm(cu, du)
+            assert e.value.code == _lib.TF_ERR_ARG
+        p.close()

@@ -244,6 +244,7 @@ struct tf_plan {
   // line-marching executor (both operators are five-point operators on one 2-D grid)
   struct Lines {
     bool on = false, same = false;
+    bool any_align = false;  // rows off the 16-byte grid are taken (value by value) instead of refused
     int nx = 0, ny = 0, tiles = 0;
     DevBuf<unsigned> words_f, words_a;
     tfk::LineParams par;
@@ -635,6 +636,12 @@ int build_lines(tf_plan &p, const tf_csr &F, const tf_csr &A, bool same, int sm_
   tf_plan::Lines &L = p.lines;
   L.same = same;
   L.nx = a.nx; L.ny = a.ny; L.tiles = a.tiles;
+  if (a.ny == 2) {  // two long lines: gather tiles decline them, and the executor behind those reads rows that lie anywhere
+    tf::Tiling t;
+    tf::build_tiling(A.m, A.ap, A.ai, tf::kPipeTileSlots, tf::kDefaultTileMaxBz, tf::kPipeTileRows, t);
+    if (!t.tiled) tf::build_tiling(A.m, A.ap, A.ai, tf::kDefaultTileSlotsSmall, tf::kDefaultTileMaxBz, tfk::tiled_threads(0), t);
+    L.any_align = !t.tiled;
+  }
   int rc = L.words_a.upload(a.words);
   if (rc == TF_OK && !same) rc = L.words_f.upload(f.words);
   if (rc == TF_OK) rc = zero_state(p);
@@ -654,8 +661,8 @@ int build_lines(tf_plan &p, const tf_csr &F, const tf_csr &A, bool same, int sm_
 
 // The lines [y_begin, y_end) of D.
 int run_lines(tf_plan &p, const float *C, float *D, int y_begin, int y_end, cudaStream_t s) {
-  const bool vec = p.n_cols % 4 == 0;
-  if (vec && !(aligned(C, 16) && aligned(D, 16)))
+  const bool on16 = aligned(C, 16) && aligned(D, 16), vec = p.n_cols % 4 == 0 && (on16 || !p.lines.any_align);
+  if (vec && !on16)
     return fail(TF_ERR_ARG, "this plan reads rows as 16-byte vectors and needs 16-byte aligned dense operands "
                             "(build the plan with tile_slots < 0 otherwise)");
   tfk::LineParams P = p.lines.par;
