@@ -221,3 +221,17 @@ def test_grid_with_missing_couplings(built_lib, dims, k, n_cols):
         want = A[~hit] @ np.where(np.isfinite(b), b, 0).astype(np.float64) @ w.astype(np.float64)
         common.assert_close(got[~hit], np.maximum(want, 0) if relu else want, "rows without an infinity")
     plan.close()
+
+
+@pytest.mark.parametrize("chain,n_cols", [("gemm_spmm", 96), ("spmm_spmm", 65)])
+def test_large_intermediate_stays_a_ring(built_lib, chain, n_cols):
+    """A plan on a grid (of one dimension here) keeps no more of T than the ring that the operator allows where all of it (and the padded rows of C of a
+    width that is no multiple of four) would take more than a 48th of the device's memory."""
+    import torch
+    free, mem = torch.cuda.mem_get_info()
+    t = synth.laplacian((int(1.05 * mem / 48 / (4 * n_cols * (1 if chain == "gemm_spmm" else 2))),))
+    n = len(t[0]) - 1
+    plan = api.Plan(chain, api.CSRMatrix(n, n, *t), k=17, n_cols=n_cols)
+    assert plan.info()["ring_rows"] > 0
+    assert free - torch.cuda.mem_get_info()[0] < 2 << 30  # operator and tiles, ring, weight
+    plan.close()

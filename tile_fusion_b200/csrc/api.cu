@@ -959,15 +959,35 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
     if (rc != TF_OK) return rc;
     pp.max_ctas = p->grid;
   }
+  // The launches of their own keep all of T (and where rows are padded, of C: `bytes` in all).  Where the ticket executor would
+  // keep a ring of at most 48 MB, that is memory a program may count on (its operands may fill the device), so more than a 48th
+  // of it (4 GB) is not taken.  (48 MB hold the ring of a grid up to about 100 columns: this is for some 10 M rows and more.)
+  auto keeps_whole = [&](size_t bytes, bool &whole) -> int {
+    size_t mem_free = 0, mem = 0;
+    TF_CUDA(cudaMemGetInfo(&mem_free, &mem));
+    whole = bytes <= mem / 48;
+    if (whole) return TF_OK;
+    TF_TRY(tf::build_stream_plan(pp, F ? F->ap : nullptr, F ? F->ai : nullptr, A->ap, A->ai, &pt, &ct, p->hp));
+    whole = p->hp.ring_rows == 0;  // (it would keep all of T as well)
+    if (whole) p->hp = tf::HostPlan();
+    return TF_OK;
+  };
   // No operator is tiled and nothing asks for the ticket executor's own knobs: the balanced gather runs the chain.
   if (chain == 0 && F && o.mode == TF_MODE_STREAM && !pt.tiled && !ct.tiled && o.ring_bytes <= 0 && o.halo_rows == 0 &&
-      o.n_boundary == 0 && o.rows_per_block == 0 && o.slack_blocks < 0 && o.ctas_per_sm == 0)
-    return make_gather_plan(p, *F, *A, o, sm_count, out);
+      o.n_boundary == 0 && o.rows_per_block == 0 && o.slack_blocks < 0 && o.ctas_per_sm == 0) {
+    const size_t ld = (n_cols + 3) / 4 * 4 * sizeof(float);
+    bool whole = false;
+    TF_TRY(keeps_whole(A->m * ld + (n_cols % 4 ? F->n * ld : 0), whole));
+    if (whole) return make_gather_plan(p, *F, *A, o, sm_count, out);
+  }
   p->tile_info[0] = pt.bx; p->tile_info[1] = pt.by; p->tile_info[2] = pt.bz; p->tile_info[3] = pt.tiles();
   p->tile_info[4] = ct.bx; p->tile_info[5] = ct.by; p->tile_info[6] = ct.bz; p->tile_info[7] = ct.tiles();
   if (chain == 1 && o.mode == TF_MODE_STREAM && o.tensor_cores >= 0 && tfk::row_gemm_supported(n_cols) &&
-      o.ring_bytes <= 0 && o.halo_rows == 0 && o.n_boundary == 0 && o.rows_per_block == 0 && o.slack_blocks < 0 && o.ctas_per_sm == 0)
-    return make_gemm_gather_plan(p, *A, o, ct.tiled, sm_count, out);
+      o.ring_bytes <= 0 && o.halo_rows == 0 && o.n_boundary == 0 && o.rows_per_block == 0 && o.slack_blocks < 0 && o.ctas_per_sm == 0) {
+    bool whole = false;
+    TF_TRY(keeps_whole((size_t)A->m * n_cols * sizeof(float), whole));
+    if (whole) return make_gemm_gather_plan(p, *A, o, ct.tiled, sm_count, out);
+  }
   rc = p->second.upload(*A);
   if (rc == TF_OK && F && F != A) rc = p->first.upload(*F);
   if (rc != TF_OK) return rc;
