@@ -782,7 +782,6 @@ int leave_intermediate(tf_plan &p, const float *C, cudaStream_t s) {
 // (Rows of B that do not start on 16-byte boundaries would be gathered value by value; then B C comes first.  So it does
 // on grids and bands: with a handful of nonzeros a row there is little to choose, and every consumer gives the same bits.)
 int make_gemm_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &A, const tf_plan_opts &o, bool tiled, int sm_count, tf_plan **out) {
-  p->ticket_sums = o.tensor_cores > 0;
   p->spmm_first = !tiled && !p->ticket_sums && p->k_dim % 4 == 0 && p->k_dim < p->n_cols;
   const int width = p->spmm_first ? p->k_dim : p->n_cols;
   p->ld_t = (width + 3) / 4 * 4;
@@ -848,6 +847,7 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
   cudaGetDevice(&p->device);
   p->chain = chain; p->mode = o.mode;
   p->m = A->m; p->n_cols = n_cols; p->k_dim = k_dim; p->halo_rows = o.halo_rows;
+  p->ticket_sums = chain == 1 && o.tensor_cores > 0;
   if (F) {
     p->first_cols = F->n;
     p->first_is_second = F == A;
