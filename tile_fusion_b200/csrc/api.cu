@@ -1477,7 +1477,13 @@ int tf_plan_info(const tf_plan *p, long long info[8]) {
   info[2] = p->hp.n_cons;
   info[3] = p->hp.ring_rows;
   info[4] = p->march.on ? p->march.grid : (p->pipe ? p->pipe_grid : p->grid);
-  info[5] = p->march.on || p->lines.on ? tfk::kMarchThreads : (p->pipe ? 672 : (p->dyn_smem > 0 ? tfk::tiled_threads(p->chain) : tfk::kThreads));
+  info[5] = p->march.on         ? tfk::kMarchThreads
+            : p->lines.on       ? 32 * tfk::kLineWarps
+            : p->band.block     ? tfk::kBandThreads
+            : p->pipe           ? 672
+            : p->g_second.on    ? tfk::kThreads
+            : p->dyn_smem > 0   ? tfk::tiled_threads(p->chain)
+                                : tfk::kThreads;
   info[6] = p->launches;
   info[7] = p->hp.inter_rows;
   return TF_OK;

@@ -24,7 +24,7 @@ namespace tfk {
 
 namespace {
 
-constexpr int kBandThreads = 512, kBandSlots = 5;
+constexpr int kBandSlots = 5;
 
 // Four rows of one product: row (lane >> 3) of the four that start at `row`, this lane's four columns.  ring: the operand;
 // quads: the nonzeros of the block that the rows belong to.

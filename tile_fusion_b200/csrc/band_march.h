@@ -37,6 +37,7 @@ struct BandParams {
 
 // Tensor map of C: boxes of 32 columns x `block` rows.
 int band_make_map(CUtensorMap *out, const float *c, long long rows, int n_cols, int block);
+constexpr int kBandThreads = 512;
 // Shared memory of the kernel for these widths; plans whose operators need more than kBandSmemMax are not made.
 constexpr int kBandSmemMax = 226 * 1024;
 size_t band_smem(int block, int pairs_f, int pairs_a, bool same);

@@ -21,7 +21,6 @@ namespace tfk {
 
 namespace {
 
-constexpr int kLineWarps = 4;
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int line_ctas(bool vec) { return vec ? 3 : 2; }  // resident per SM (with single columns a lane holds four times the points)
 

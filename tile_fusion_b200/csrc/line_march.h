@@ -27,6 +27,8 @@ void analyse_line_operator(int m, int n, const int *ap, const int *ai, const flo
 
 namespace tfk {
 
+constexpr int kLineWarps = 4;  // per CTA
+
 struct LineParams {
   const float *in;
   float *out;
