@@ -238,6 +238,11 @@ def print_reference(args):
         print(json.dumps({"impl": "reference", "unavailable": "the reference has no CPU executor for the composed graph chains "
                           "(2-layer GCN, SDDMM-SpMM); see cpu_baseline (kind port) of the GPU arm"}))
         return 0
+    from oracle.bindings import Ref
+    if not Ref.available():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's sources are not here to be compiled (oracle/_ref); the "
+                          "restatement in C is not the reference, see cpu_baseline (kind port) of the GPU arm"}))
+        return 0
     r = cpu_reference(args.workload, args.steps, max(args.warmup, 1))
     ms = 1e3 * float(np.mean(r["times"]))
     val = r["flops"] / (ms * 1e-3) / 1e9
