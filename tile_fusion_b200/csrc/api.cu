@@ -88,34 +88,89 @@ struct DevGather {
   // For the host-pointer calls, where no row is cut and units are in row order: units [0, u] read rows < in_rows[u] of the
   // operand, and with them every row < out_rows[u] of the result is final.
   std::vector<long long> in_rows, out_rows;
-  void follow_units(const tf::GatherPlan &g, int m) {
+  void follow_units(const tf::GatherPlan &g, int m, const int *ai) {
     const int n = (int)g.units.size();
     if (!g.heavy.empty()) return;
     in_rows.resize(n);
     out_rows.resize(n);
     long long need = 0;
     for (int u = 0; u < n; ++u) {
-      const size_t p1 = u + 1 < n ? (size_t)g.units[u + 1].p0 : g.n_entries - tf::kGatherBatch;
-      for (size_t i = g.units[u].p0; i < p1; ++i) need = std::max<long long>(need, (g.cols[i] & ~tf::kGatherEnd) + 1LL);
+      for (int j = g.ranges[u].j0; j < g.ranges[u].j1; ++j) need = std::max<long long>(need, ai[j] + 1LL);
       const int pos = u + 1 < n ? g.units[u + 1].pos : 0;
       in_rows[u] = need;
       out_rows[u] = u + 1 == n ? m : (g.rows.empty() ? pos : g.rows[pos]);
     }
   }
+  // The entries are made in pieces of 4 MB by up to four threads, each of which copies its pieces to the device.  (Arrays of all
+  // of them cost more in first touches than the copies take: an SDDMM plan of 8.4 M nonzeros 25.4 ms, like this 19.8.)
+  int upload_entries(const tf::GatherPlan &g, const tf_csr &A) {
+    int rc = cols.alloc(g.n_entries), dev = 0;
+    if (rc == TF_OK) rc = vals.alloc(g.n_entries);
+    if (rc != TF_OK) return rc;
+    TF_CUDA(cudaGetDevice(&dev));
+    constexpr size_t kPiece = (size_t)1 << 19;  // entries
+    const size_t n = g.units.size();
+    if (n == 0) {  // the batch behind the last unit
+      TF_CUDA(cudaMemset(cols.p, 0, cols.n * sizeof(int)));
+      TF_CUDA(cudaMemset(vals.p, 0, vals.n * sizeof(float)));
+      return TF_OK;
+    }
+    const size_t parts = g.n_entries < 2 * kPiece ? 1 : std::min<size_t>(4, std::max(1u, std::thread::hardware_concurrency() / 2));
+    auto at = [&](size_t u) { return u < n ? (size_t)g.units[u].p0 : g.n_entries; };  // where unit u begins, or all end
+    std::vector<cudaError_t> errors(parts, cudaSuccess);
+    auto part = [&](size_t k) {
+      cudaError_t &e = errors[k];
+      try {
+        std::unique_ptr<uint32_t[]> c;
+        std::unique_ptr<float[]> v;
+        size_t room = 0;
+        e = cudaSetDevice(dev);
+        size_t u = n * k / parts;
+        const size_t end = n * (k + 1) / parts;
+        while (u < end && e == cudaSuccess) {
+          size_t to = u + 1;
+          while (to < end && at(to + 1) - at(u) <= kPiece) ++to;
+          const size_t count = at(to) - at(u);
+          if (count > room) {
+            room = std::max(count, std::min(kPiece, g.n_entries));
+            c.reset(new uint32_t[room]);
+            v.reset(new float[room]);
+          }
+          tf::fill_gather_entries(g, A.m, A.ap, A.ai, A.ax, u, to, c.get(), v.get());
+          e = cudaMemcpy(cols.p + at(u), c.get(), count * sizeof(int), cudaMemcpyHostToDevice);
+          if (e == cudaSuccess) e = cudaMemcpy(vals.p + at(u), v.get(), count * sizeof(float), cudaMemcpyHostToDevice);
+          u = to;
+        }
+      } catch (const std::bad_alloc &) {
+        e = cudaErrorMemoryAllocation;
+      }
+    };
+    std::vector<std::thread> pool;
+    size_t started = 1;
+    try {
+      pool.reserve(parts);
+      for (; started < parts; ++started) pool.emplace_back(part, started);
+    } catch (const std::exception &) {  // no thread to be had: the rest is done here
+    }
+    part(0);
+    for (size_t k = started; k < parts; ++k) part(k);
+    for (std::thread &th : pool) th.join();
+    for (cudaError_t e : errors) TF_CUDA(e);
+    return TF_OK;
+  }
   // n_cols: width of the dense operand the units are cut for; max_cols: widest one the operator will meet; follow: see above
   int build(const tf_csr &A, int n_cols, int max_cols, int sm_count, bool follow = false, int resident = tfk::kGatherResident,
             bool ticket_sums = false) {
     tf::GatherPlan g;
-    tf::build_gather_plan(A.m, A.ap, A.ai, A.ax, sm_count * (resident / tfk::gather_group(n_cols)), ticket_sums, g);
+    tf::build_gather_plan(A.m, A.ap, sm_count * (resident / tfk::gather_group(n_cols)), ticket_sums, g);
     n_units = (int)g.units.size();
     n_empty = (int)g.empty_rows.size();
     n_slots = g.n_slots;
     partial_ld = (std::max(n_cols, max_cols) + 3) / 4 * 4;
     const int panels = (partial_ld + 127) / 128;  // the most any width up to that is read in
-    if (follow) follow_units(g, A.m);
+    if (follow) follow_units(g, A.m, A.ai);
     if (!g.rows.empty()) g.rows.resize(g.rows.size() + 2, 0);  // a group looks one row ahead (with the row of Q, two)
-    int rc = cols.upload(reinterpret_cast<const int *>(g.cols.get()), g.n_entries);
-    if (rc == TF_OK) rc = vals.upload(g.vals.get(), g.n_entries);
+    int rc = upload_entries(g, A);
     if (rc == TF_OK) rc = units.upload(reinterpret_cast<const int4 *>(g.units.data()), g.units.size());
     if (rc == TF_OK) rc = heavy.upload(reinterpret_cast<const int4 *>(g.heavy.data()), g.heavy.size());
     if (rc == TF_OK) rc = rows.upload(g.rows);

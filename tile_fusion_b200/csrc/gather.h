@@ -26,17 +26,20 @@ struct GatherPlan {
   std::vector<GatherHeavy> heavy;
   std::vector<int> rows;              // non-empty rows in order; left empty when every row has a nonzero
   std::vector<int> empty_rows;
-  // column | kGatherEnd and value of every nonzero, unit after unit, each unit filled up to whole batches with entries
-  // of value 0 that name its last column again (they follow the unit's last row end, so their sums go nowhere);
-  // one batch more at the end, because a group reads one batch ahead
-  std::unique_ptr<uint32_t[]> cols;
-  std::unique_ptr<float[]> vals;
-  size_t n_entries = 0;
+  struct Range { int pos, j0, j1, heavy; };
+  std::vector<Range> ranges;          // the nonzeros of every unit
+  size_t n_entries = 0;               // see fill_gather_entries
   int n_slots = 0;
 };
 // `groups`: lane groups resident on the device, which sets how finely the work is cut.  ticket_sums: rows are cut where the
 // warps of the ticket executor's CTA cut them and nowhere else, so that the sums are added in its order.
-void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int groups, bool ticket_sums, GatherPlan &out);
+void build_gather_plan(int m, const int *ap, int groups, bool ticket_sums, GatherPlan &out);
+// The entries of the units [u0, u1), those of u0 first: column | kGatherEnd and value of every nonzero, unit after unit, each
+// unit filled up to whole batches with entries of value 0 that name its last column again (they follow the unit's last row end,
+// so their sums go nowhere).  Behind the last unit there is one batch more, of zeros, because a group reads one batch ahead.
+// Returns their number.
+size_t fill_gather_entries(const GatherPlan &g, int m, const int *ap, const int *ai, const float *ax, size_t u0, size_t u1,
+                           uint32_t *cols, float *vals);
 
 }  // namespace tf
 

@@ -2,14 +2,13 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <thread>
 
 #include "gather.h"
 #include "tf_internal.h"
 
 namespace tf {
 
-void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int groups, bool ticket_sums, GatherPlan &out) {
+void build_gather_plan(int m, const int *ap, int groups, bool ticket_sums, GatherPlan &out) {
   out = GatherPlan();
   const long long nnz = ap[m];
   const long long cost = nnz + 2LL * m;
@@ -23,9 +22,8 @@ void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int
   // A row at least this long is cut.  (Cutting only from twice that on: the same on large graphs, 25.4 instead of 22.7 us
   // at n = 20 000, where one long row is what the launch waits for.)
   const int long_row = ticket_sums ? kHeavyRowNnz : target;
-  // rows and pieces first (nonzero ranges), entries afterwards
-  struct Range { int pos, j0, j1, heavy; };
-  std::vector<Range> plain, pieces;
+  using Range = GatherPlan::Range;
+  std::vector<Range> plain, &pieces = out.ranges;
   int pos = 0, open_cost = 0;
   Range open{0, 0, 0, -1};
   auto close = [&] {
@@ -80,44 +78,31 @@ void build_gather_plan(int m, const int *ap, const int *ai, const float *ax, int
     n += (size_t)batches * kGatherBatch;
   }
   out.n_entries = n + kGatherBatch;
-  out.cols.reset(new uint32_t[out.n_entries]);  // (left uninitialised: every entry is written below)
-  out.vals.reset(new float[out.n_entries]);
-  // units [u0, u1): every one writes its own entries, so ranges of them can be filled side by side
-  auto fill = [&](size_t u0, size_t u1) {
-    int row = -1;  // plain units come in row order: the row ends inside them are found by walking ap
-    for (size_t i = u0; i < u1; ++i) {
-      const Range &u = pieces[i];
-      const int len = u.j1 - u.j0;
-      size_t w = (size_t)out.units[i].p0;
-      std::memcpy(&out.cols[w], ai + u.j0, sizeof(int) * (size_t)len);
-      std::memcpy(&out.vals[w], ax + u.j0, sizeof(float) * (size_t)len);
-      if (u.heavy < 0) {
-        if (row < 0) row = (int)(std::upper_bound(ap, ap + m + 1, u.j0) - ap) - 1;  // the first row that ends behind j0
-        while (ap[row + 1] <= u.j0) ++row;
-        for (; row < m && ap[row + 1] <= u.j1; ++row)
-          if (ap[row + 1] > ap[row]) out.cols[w + (ap[row + 1] - 1 - u.j0)] |= kGatherEnd;
-      } else {
-        out.cols[w + len - 1] |= kGatherEnd;
-      }
-      w += len;
-      for (; w % kGatherBatch != 0; ++w) { out.cols[w] = (uint32_t)ai[u.j1 - 1]; out.vals[w] = 0.f; }
+}
+
+size_t fill_gather_entries(const GatherPlan &g, int m, const int *ap, const int *ai, const float *ax, size_t u0, size_t u1,
+                           uint32_t *cols, float *vals) {
+  size_t w = 0;
+  int row = -1;  // plain units come in row order: the row ends inside them are found by walking ap
+  for (size_t i = u0; i < u1; ++i) {
+    const GatherPlan::Range &u = g.ranges[i];
+    const int len = u.j1 - u.j0;
+    std::memcpy(cols + w, ai + u.j0, sizeof(int) * (size_t)len);
+    std::memcpy(vals + w, ax + u.j0, sizeof(float) * (size_t)len);
+    if (u.heavy < 0) {
+      if (row < 0) row = (int)(std::upper_bound(ap, ap + m + 1, u.j0) - ap) - 1;  // the first row that ends behind j0
+      while (ap[row + 1] <= u.j0) ++row;
+      for (; row < m && ap[row + 1] <= u.j1; ++row)
+        if (ap[row + 1] > ap[row]) cols[w + (ap[row + 1] - 1 - u.j0)] |= kGatherEnd;
+    } else {
+      cols[w + len - 1] |= kGatherEnd;
     }
-  };
-  // Most of the time goes into the first touch of the arrays (11.6 M nonzeros: 60 ms on one thread, 20 on four).
-  const size_t parts = nnz < (1 << 20) ? 1 : std::min<size_t>(8, std::max(1u, std::thread::hardware_concurrency() / 2));
-  auto part = [&](size_t k) { fill(pieces.size() * k / parts, pieces.size() * (k + 1) / parts); };
-  std::vector<std::thread> pool;
-  size_t started = 1;
-  try {
-    pool.reserve(parts);
-    for (; started < parts; ++started) pool.emplace_back(part, started);
-  } catch (const std::exception &) {  // no thread to be had: the rest is done here
+    w += len;
+    for (; w % kGatherBatch != 0; ++w) { cols[w] = (uint32_t)ai[u.j1 - 1]; vals[w] = 0.f; }
   }
-  part(0);
-  for (size_t k = started; k < parts; ++k) part(k);
-  for (std::thread &th : pool) th.join();
-  size_t w = n;
-  for (int k = 0; k < kGatherBatch; ++k, ++w) { out.cols[w] = 0; out.vals[w] = 0.f; }
+  if (u1 == g.ranges.size())
+    for (int k = 0; k < kGatherBatch; ++k, ++w) { cols[w] = 0; vals[w] = 0.f; }
+  return w;
 }
 
 }  // namespace tf
