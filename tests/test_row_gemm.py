@@ -235,3 +235,9 @@ def test_large_intermediate_stays_a_ring(built_lib, chain, n_cols):
     assert plan.info()["ring_rows"] > 0
     assert free - torch.cuda.mem_get_info()[0] < 2 << 30  # operator and tiles, ring, weight
     plan.close()
+
+
+@pytest.mark.parametrize("k,n_cols", [(64, 64), (64, 47)])
+@pytest.mark.parametrize("bits", [0x7FFFFFFF, 0x7F800001])
+def test_nan_stays_nan_in_the_sums_of_the_ticket_executor(built_lib, k, n_cols, bits):
+    test_nan_stays_nan(None, k, n_cols, {"tensor_cores": 1}, bits)

@@ -1450,7 +1450,7 @@ int run_gather_gemm_spmm(tf_plan &p, const float *B, const float *W, int w_trans
   if (p.dyn_smem > 0 && !(aligned(B, 16) && aligned(D, 16)))
     return fail(TF_ERR_ARG, "this plan (gather tiles or tensor-core producer) needs 16-byte aligned dense operands "
                             "(build the plan with tile_slots < 0 and tensor_cores < 0 otherwise)");
-  TF_CUDA(tfk::row_gemm_split(W, w_transposed, k, n, p.w_hi.p, p.w_lo.p, s));
+  TF_CUDA(tfk::row_gemm_split(W, w_transposed, k, n, p.ticket_sums, p.w_hi.p, p.w_lo.p, s));
   p.launches = tfk::row_gemm_form(k, n) == tfk::kRowFma ? 2 : 3;
   if (p.spmm_first) {
     TF_TRY(run_gather(p.g_second, B, k, aligned(B, 16), p.inter.p, p.ld_t, true, k, false, s));
@@ -1602,7 +1602,7 @@ int run_gemm_march(tf_plan &p, const float *B, const float *W, int w_transposed,
                    int item_end, bool with_halo, cudaStream_t s) {
   long long launches = 0;
   if (produce) {
-    TF_CUDA(tfk::row_gemm_split(W, w_transposed, p.k_dim, p.n_cols, p.w_hi.p, p.w_lo.p, s));
+    TF_CUDA(tfk::row_gemm_split(W, w_transposed, p.k_dim, p.n_cols, p.ticket_sums, p.w_hi.p, p.w_lo.p, s));
     int rc = tfk::row_gemm(B, p.m, p.k_dim, p.k_dim, W, w_transposed, p.w_hi.p, p.w_lo.p, p.n_cols, p.inter.p, p.n_cols, false,
                            p.ticket_sums, &p.march.st.p[0].error, p.spin_limit, p.sm_count, s);
     if (rc != TF_OK) return rc;
@@ -1801,7 +1801,7 @@ static int run_host_pieces(tf_plan &p, const float *in, int w_transposed, bool r
     p.ev_in.push_back(a); p.ev_run.push_back(b);
   }
   TF_TRY(begin_host_pipe(p, in, D));
-  if (gemm) TF_CUDA(tfk::row_gemm_split(p.h_in1.p, w_transposed, k, n, p.w_hi.p, p.w_lo.p, p.s_run));
+  if (gemm) TF_CUDA(tfk::row_gemm_split(p.h_in1.p, w_transposed, k, n, p.ticket_sums, p.w_hi.p, p.w_lo.p, p.s_run));
   else TF_CUDA(tfk::launch_rows_fix(f.empty.p, f.n_empty, p.ld_t, p.inter.p, false, p.s_run));
   TF_CUDA(tfk::launch_rows_fix(g.empty.p, g.n_empty, n, p.h_out.p, false, p.s_run));
   const bool pad = p.g_pad.n != 0, vec = pad || n % 4 == 0;  // (the buffers of the call start on 16-byte boundaries)

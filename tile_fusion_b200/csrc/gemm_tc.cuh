@@ -117,11 +117,10 @@ __device__ __forceinline__ void tc_end(TcShared &s) {
   }
 }
 
-// x rounded to TF32, for numbers.  A NaN may come out as a zero (0x7FFFFFFF, the one that arithmetic on the GPU gives, carries
-// into the sign), so the other half of a split, x - tf32_round(x), stays as it is: it is that NaN, and the product a NaN with
-// it.  Rounded as well it would vanish; the tensor core cuts its last bits off, which is 2^-22 of x.
+// x rounded to TF32.  A NaN stays as it is: the addition would carry 0x7FFFFFFF, the one that arithmetic on the GPU gives, into
+// the sign and leave a zero.
 __device__ __forceinline__ float tf32_round(float x) {
-  return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
+  return x == x ? __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u) : x;
 }
 
 // One tile of up to 128 rows.  `phase` carries the barrier parities across calls (bit 0: TMA,
@@ -155,7 +154,7 @@ __device__ __forceinline__ bool tc_gemm_rows(const CUtensorMap *tmA, const CUten
     for (int i = tid; i < kTcRows * kTcKSlice; i += NT) {
       const float a = a_hi[i], h = tf32_round(a);
       a_hi[i] = h;
-      a_lo[i] = a - h;  // (not rounded: see tf32_round)
+      a_lo[i] = a - h;  // (the tensor core cuts its last bits off)
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> async proxy (MMA) reads
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

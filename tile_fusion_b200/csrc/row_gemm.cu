@@ -1,8 +1,8 @@
 // T = B * W (optionally max(0, .)) for a tall fp32 B on the 5th-generation tensor cores, 3xTF32 inside.
 //
-// The arithmetic is that of gemm_tc.cuh, product by product: every operand is split as x = hi + lo, hi rounded to TF32,
-// and hi*hi + hi*lo + lo*hi is accumulated in fp32 in tensor memory.  What differs is that nothing waits for anything it
-// does not need:
+// The arithmetic is that of gemm_tc.cuh, product by product: every operand is split as x = hi + lo, both rounded to TF32
+// (lo only where that tile's bits are not asked for; 1 to 3 % of the error), and hi*hi + hi*lo + lo*hi is accumulated in
+// fp32 in tensor memory.  What differs is that nothing waits for anything it does not need:
 //   * Two CTAs on neighbouring SMs work on one tile of 256 rows with tcgen05.mma.cta_group::2.  Each holds 128 rows of B
 //     and half of the columns of W, so W crosses from L2 once per 256 rows, and the tensor core reads half of it from
 //     each SM's shared memory.  (One CTA with 128 rows and all of W would need 180 bytes per clock of shared memory at
@@ -295,7 +295,9 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           const float4 x = a[i];
           const float4 h = make_float4(tf32_round(x.x), tf32_round(x.y), tf32_round(x.z), tf32_round(x.w));
           hi[w + i * 32 * kRgSplitWarps] = h;
-          lo[w + i * 32 * kRgSplitWarps] = make_float4(x.x - h.x, x.y - h.y, x.z - h.z, x.w - h.w);
+          float4 l = make_float4(x.x - h.x, x.y - h.y, x.z - h.z, x.w - h.w);
+          if (!P.ticket) l = make_float4(tf32_round(l.x), tf32_round(l.y), tf32_round(l.z), tf32_round(l.w));
+          lo[w + i * 32 * kRgSplitWarps] = l;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read next by the tensor core
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -487,7 +489,7 @@ row_fma_kernel(const float *__restrict__ X, int m, int K, int ld_x, const float 
 }
 
 // hi / lo [n_pad][K] (K contiguous, rows from n on zero) from W [K][n], or from W [n][K] when w_transposed.
-__global__ void split_weight_pad_kernel(const float *__restrict__ W, int w_transposed, int K, int ldk, int n, int n_pad,
+__global__ void split_weight_pad_kernel(const float *__restrict__ W, int w_transposed, int K, int ldk, int n, int n_pad, bool ticket,
                                         float *__restrict__ hi, float *__restrict__ lo) {
   const int total = n_pad * ldk;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -496,7 +498,7 @@ __global__ void split_weight_pad_kernel(const float *__restrict__ W, int w_trans
     if (r < n && k < K) w = w_transposed ? __ldg(W + (size_t)r * K + k) : __ldg(W + (size_t)k * n + r);
     const float h = tf32_round(w);
     hi[i] = h;
-    lo[i] = w - h;
+    lo[i] = ticket ? w - h : tf32_round(w - h);
   }
 }
 
@@ -508,10 +510,11 @@ int row_gemm_pad_k(int k) { return (k + 3) / 4 * 4; }
 
 RowGemmForm row_gemm_form(int K, int n) { return tc_supported(K, n) ? kRowTile : (K >= kRgPreciseMinK ? kRowPrecise : kRowFma); }
 
-cudaError_t row_gemm_split(const float *W, int w_transposed, int K, int n, float *hi, float *lo, cudaStream_t s) {
+cudaError_t row_gemm_split(const float *W, int w_transposed, int K, int n, bool ticket, float *hi, float *lo, cudaStream_t s) {
   if (row_gemm_form(K, n) == kRowFma) return cudaSuccess;
+  ticket = ticket && row_gemm_form(K, n) == kRowTile;
   const int ldk = row_gemm_pad_k(K), n_pad = row_gemm_pad_n(n);
-  split_weight_pad_kernel<<<std::min((n_pad * ldk + 255) / 256, 148 * 4), 256, 0, s>>>(W, w_transposed, K, ldk, n, n_pad, hi, lo);
+  split_weight_pad_kernel<<<std::min((n_pad * ldk + 255) / 256, 148 * 4), 256, 0, s>>>(W, w_transposed, K, ldk, n, n_pad, ticket, hi, lo);
   return cudaGetLastError();
 }
 
@@ -527,19 +530,20 @@ static int launch_fma(const float *X, int m, int K, int ld_x, const float *W, in
 }
 
 static int launch_panel(const float *X, int m, int K, int ld_x, const float *W, int w_k, int w_c, const float *hi, const float *lo, int n, float *out, int ld_out, bool relu,
-                        bool precise, bool one_acc, int *error, int wait_limit, int sm_count, cudaStream_t s) {
+                        bool precise, bool ticket, int *error, int wait_limit, int sm_count, cudaStream_t s) {
   const int n_pad = row_gemm_pad_n(n), ldk = row_gemm_pad_k(K);
   CUtensorMap ma, mh, ml, mo;
   RowGemmParams P;
   P.x = X; P.k = K; P.ld_x = ld_x;
   P.w = W; P.w_k = w_k; P.w_c = w_c;
+  P.ticket = ticket ? 1 : 0;
   P.direct = ld_x % 4 != 0 || (reinterpret_cast<uintptr_t>(X) & 15) != 0;
   int rc = tc_make_map(&mh, hi, n_pad, ldk, n_pad / 2, ldk);
   if (rc == TF_OK) rc = tc_make_map(&ml, lo, n_pad, ldk, n_pad / 2, ldk);
   P.m = m; P.n_pad = n_pad; P.n_real = n; P.n_slices = (K + kTcKSlice - 1) / kTcKSlice;
   P.tiles = (m + 2 * kTcRows - 1) / (2 * kTcRows);
   P.stages = rg_stages(n_pad);
-  P.accs = one_acc || n_pad > 128 ? 1 : (n_pad > 64 ? 2 : 4);
+  P.accs = ticket || n_pad > 128 ? 1 : (n_pad > 64 ? 2 : 4);
   P.out = out; P.ld_out = ld_out; P.relu = relu ? 1 : 0;
   P.tma_store = ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   P.error = error; P.wait_limit = wait_limit;
@@ -562,16 +566,17 @@ static int launch_panel(const float *X, int m, int K, int ld_x, const float *W, 
 }
 
 int row_gemm(const float *X, int m, int K, int ld_x, const float *W, int w_transposed, const float *hi, const float *lo, int n,
-             float *out, int ld_out, bool relu, bool one_acc, int *error, int wait_limit, int sm_count, cudaStream_t s) {
+             float *out, int ld_out, bool relu, bool ticket, int *error, int wait_limit, int sm_count, cudaStream_t s) {
   const RowGemmForm form = row_gemm_form(K, n);
   if (form == kRowFma) return launch_fma(X, m, K, ld_x, W, w_transposed, n, out, ld_out, relu, sm_count, s);
   const bool precise = form == kRowPrecise;
+  ticket = ticket && !precise;
   const int panel = precise ? kRgPrecisePanel : n;
   for (int c = 0; c < n; c += panel) {
     const size_t off = (size_t)c * row_gemm_pad_k(K);
     const int w_k = w_transposed ? 1 : n, w_c = w_transposed ? K : 1;
     const int rc = launch_panel(X, m, K, ld_x, W + (size_t)c * w_c, w_k, w_c, hi + off, lo + off, std::min(panel, n - c), out + c, ld_out,
-                                relu, precise, one_acc, error, wait_limit, sm_count, s);
+                                relu, precise, ticket, error, wait_limit, sm_count, s);
     if (rc != TF_OK) return rc;
   }
   return TF_OK;
