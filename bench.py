@@ -344,7 +344,7 @@ def run_graph_workload(args):
             "clocks": clk.summary(),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": None, "peak_source": f"of {peak_kind}", "algorithmic_bytes_per_launch": nbytes,
-                         "kernel": "gather kernels (and row_gemm_kernel)", "kernel_ms": ms,
+                         "kernel": "sddmm_gather_kernel" if args.workload == "c4" else "gather_kernel and row_gemm_kernel", "kernel_ms": ms,
                          "gather_bytes_per_step": gather, "gather_gbs": gather / (ms * 1e-3) / 1e9,
                          "gather_note": "one dense row per nonzero through L2 -> SM; random rows, so the HBM figure does not bound "
                                         "this workload: read gather_gbs against the ~13 TB/s L2 -> SM row-gather rate of this GPU"},

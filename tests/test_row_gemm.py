@@ -1,8 +1,8 @@
 """GeMM-SpMM on the dense product of its own launch (csrc/row_gemm.cu) and the balanced gather, in either order.
 
 Bounds on the relative error, beside the tolerance of tests/common.py: shapes of the tensor-core tile (K a multiple of 4, N
-of 16) add K / 8 * 3 sums that are cut off at 2^-23: 2e-6 up to K = 256, as in test_gpu_tc.py.  All others are as exact as
-fp32 FMAs: per eight terms one sum cut off at 2^-23, then K / 8 rounded sums, each of random sign against the rest, and the
+of 16) add K / 8 * 3 sums that are cut off at 2^-23: 2e-6 up to K = 256, as in test_gpu_tc.py.  All others are fp32
+FMAs up to 31 terms and as exact as those beyond: per eight terms one sum cut off at 2^-23, then K / 8 rounded sums, each of random sign against the rest, and the
 dropped lo * lo terms at 2^-22 of a product: below 2^-22 + 2^-24 * sqrt(K / 8) < 6e-7 up to K = 300."""
 import numpy as np
 import pytest
