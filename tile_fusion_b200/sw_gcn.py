@@ -17,7 +17,7 @@ take part in autograd: the backward is the reference's (``src/Functions.cpp:819-
 ``dX = (A dY) W`` and ``dW = (A dY)^T X`` -- like the reference it multiplies by ``A``, not ``A^T``, i.e. it
 assumes the symmetric adjacency of a GCN.  The forward runs the library's fused GeMM-SpMM executor; the sparse
 product of the backward runs on the same plan's operator, the weight gradient -- a sum over all rows -- on a kernel
-of the library's own, the other dense product is a plain library GEMM.
+of the library's own where that is the faster one, the other dense product is a plain library GEMM.
 
 The schedule tensors have the reference's layout (level pointers, per-partition kernel boundaries, row ids) and
 come from the library's inspector for the same cache budget; the GPU executor plans its own tiles and does not
