@@ -74,6 +74,7 @@ __device__ __forceinline__ unsigned long long umma_desc_sw128(unsigned smem_addr
   d |= (unsigned long long)2 << 61;                         // SWIZZLE_128B
   return d;
 }
+constexpr int kUmmaStep = 32 >> 4;  // descriptors: 8 tf32 along K inside the swizzle row, in 16 bytes
 // Instruction descriptor: D fp32, A and B tf32, both K-major, M = 128, N = n.
 __device__ __forceinline__ unsigned umma_idesc_tf32(int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(kTcRows >> 4) << 24);
@@ -115,6 +116,19 @@ __device__ __forceinline__ void tc_end(TcShared &s) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s.tmem_base), "n"(kTcTmemCols) : "memory");
   }
+}
+
+// One lane of a warp that is not divergent, the same at every call.  What issues tcgen05.mma takes its operands from uniform
+// registers: under `if (elect_one())` in code that the whole warp runs they are computed there, while under `if (lane == 0)`
+// every operand is brought over by itself, which made a product of a CTA pair cost 154 cycles of its issuing thread (of one
+// CTA 199) whatever its size, instead of 39 (32 columns), 43 (64), 64 (128) and 128 (256).
+__device__ __forceinline__ bool elect_one() {
+  unsigned p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 
 // x rounded to TF32.  A NaN stays as it is: the addition would carry 0x7FFFFFFF, the one that arithmetic on the GPU gives, into
@@ -159,17 +173,21 @@ __device__ __forceinline__ bool tc_gemm_rows(const CUtensorMap *tmA, const CUten
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> async proxy (MMA) reads
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (tid == 0) {
+    if (__shfl_sync(kFull, warp, 0) == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const unsigned ah = smem_u32(a_hi), al = smem_u32(a_lo), wh = smem_u32(w_hi), wl = smem_u32(w_lo);
+      const unsigned long long ah = umma_desc_sw128(smem_u32(a_hi)), al = umma_desc_sw128(smem_u32(a_lo));
+      const unsigned long long wh = umma_desc_sw128(smem_u32(w_hi)), wl = umma_desc_sw128(smem_u32(w_lo));
+      if (elect_one()) {
 #pragma unroll
-      for (int j = 0; j < kTcKSlice / 8; ++j) {
-        const unsigned o = j * 32;  // 8 tf32 = 32 bytes along K inside the swizzle row
-        umma_tf32(tmem_d, umma_desc_sw128(ah + o), umma_desc_sw128(wh + o), idesc, (sl | j) ? 1u : 0u);
-        umma_tf32(tmem_d, umma_desc_sw128(ah + o), umma_desc_sw128(wl + o), idesc, 1u);
-        umma_tf32(tmem_d, umma_desc_sw128(al + o), umma_desc_sw128(wh + o), idesc, 1u);
+        for (int j = 0; j < kTcKSlice / 8; ++j) {
+          const int o = j * kUmmaStep;
+          umma_tf32(tmem_d, ah + o, wh + o, idesc, (sl | j) ? 1u : 0u);
+          umma_tf32(tmem_d, ah + o, wl + o, idesc, 1u);
+          umma_tf32(tmem_d, al + o, wh + o, idesc, 1u);
+        }
+        umma_commit(&s.bar_mma);
       }
-      umma_commit(&s.bar_mma);
+      __syncwarp();
     }
     // the slice buffers are reused by the next TMA: wait until the tensor core has read them
     if (!mbar_wait(&s.bar_mma, (phase >> 1) & 1u, wait_limit)) { s.ok = 0; }

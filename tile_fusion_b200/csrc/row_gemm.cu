@@ -8,7 +8,8 @@
 //     each SM's shared memory.  (One CTA with 128 rows and all of W would need 180 bytes per clock of shared memory at
 //     N = 256, 40 % more than there are.)
 //   * A warp keeps the TMA loads of K slices of 32 columns running ahead through a ring of stages, eight warps split
-//     the raw rows, one thread of the even CTA issues the products, four warps drain the accumulator of the tile before
+//     the raw rows, one warp of the even CTA issues the products (see elect_one: by a thread alone 2 % slower at K = N = 256,
+//     262 144 rows, K = N = 128: 65.0 us and 54.1; 500 009 rows, 256 -> 47: 243 and 198), four warps drain the accumulator of the tile before
 //     (two accumulators of up to 256 columns in tensor memory) and write it with TMA stores.
 //   * The grid is one pair per two SMs and walks the tiles.
 // The tensor core cuts off what it adds to an accumulator instead of rounding it, so a chain of K / 8 sums drifts (rel.
@@ -18,15 +19,15 @@
 // Fewer terms are multiplied with FMAs still, by row_fma_kernel.
 // The plain form keeps its chains short where tensor memory has room: up to 128 columns the K steps of a slice go round two
 // accumulators, up to 64 round four, the small products first (K = 256: rel. error 1.9e-6 with one, 8.8e-7 with two, 4.6e-7
-// with four; 262 144 rows, K = N = 64: 33.6 us with one, 36.3 with four).
+// with four; 262 144 rows, K = N = 64: 30.5 us with four).
 // All waits are bounded: the one that runs out sets the error flag, and every role leaves.
 #include "row_gemm.h"
 
 #include <algorithm>
 #include <string>
 
-#include "gemm_tc.cuh"
 #include "gemm_tc_host.h"
+#include "pair_mma.cuh"
 #include "tf_internal.h"
 
 namespace tfk {
@@ -62,77 +63,6 @@ constexpr int rg_stages(int n) {
 }
 static_assert(rg_stages(256) >= 2, "a full-width tile needs two stages");
 
-__device__ __forceinline__ unsigned rg_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void rg_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Arrive on the barrier of the even CTA of the pair.  What goes with the arrival is shared memory that the tensor cores read
-// through the async proxy: fence.proxy.async has completed the writes there before, each in its own SM.  (A release at
-// cluster scope would order the thread's other accesses too and costs a splitting warp half of its time: N = K = 256,
-// 2.1 M rows: 1 410 us with it, 1 228 with one thread of the odd CTA that passes local arrivals on, 1 075 like this, as
-// CUTLASS's ClusterBarrier::arrive has it.)
-__device__ __forceinline__ void rg_arrive_leader(unsigned long long *bar) {
-  asm volatile(
-      "{\n\t.reg .b32 a;\n\t"
-      "mapa.shared::cluster.u32 a, %0, 0;\n\t"
-      "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar)) : "memory");
-}
-// Bounded wait that also leaves when another role of the CTA has given up.  CLUSTER: threads of the other CTA arrive too.
-template <bool CLUSTER = false>
-__device__ __forceinline__ bool rg_wait(unsigned long long *bar, unsigned parity, RgShared &s, int limit) {
-  const unsigned a = smem_u32(bar);
-  for (int i = 0; i < limit; ++i) {
-    unsigned done;
-    if (CLUSTER)
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t"
-          "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(a), "r"(parity) : "memory");
-    else
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t"
-          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(a), "r"(parity) : "memory");
-    if (done) return true;
-    if (*reinterpret_cast<volatile int *>(&s.dead)) return false;
-  }
-  s.dead = 1;
-  return false;
-}
-__device__ __forceinline__ void rg_mma(unsigned d, unsigned long long da, unsigned long long db, unsigned idesc, unsigned acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
-}
-// Both CTAs' barriers at this offset are arrived on when the products issued so far have been computed.
-__device__ __forceinline__ void rg_commit(unsigned long long *bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-                   smem_u32(bar)), "h"((unsigned short)3) : "memory");
-}
-
-// 32 columns of a warp's 32 tensor-memory lanes.  The registers hold them after tcgen05.wait::ld only: rg_loaded keeps the
-// compiler from using them before.
-__device__ __forceinline__ void rg_tmem_load(float (&v)[32], unsigned taddr) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
-        "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]),
-        "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),
-        "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
-      : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void rg_loaded(float (&v)[32]) {
-#pragma unroll
-  for (int i = 0; i < 32; ++i) asm volatile("" : "+f"(v[i]));
-}
-
 // PRECISE: see above; n_pad <= 64.
 // n_pad: columns of W rounded up to 32 (rows of the split weight beyond n_real are zero).
 template <bool PRECISE>
@@ -142,8 +72,8 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   extern __shared__ char dyn[];
   __shared__ RgShared s;
   char *smem = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~(uintptr_t)1023);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const unsigned rank = rg_rank();
+  const int tid = threadIdx.x, warp = __shfl_sync(kFull, tid >> 5, 0), lane = tid & 31;  // (known to be uniform)
+  const unsigned rank = pair_rank();
   const int N = P.n_pad, half = N / 2, stage_bytes = rg_stage_bytes(N), stages = P.stages;
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int accs = PRECISE ? 4 : P.accs, acc_cols = PRECISE ? 64 : 256 / P.accs;  // accumulators of a tile, columns from one to the next
@@ -169,7 +99,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  rg_cluster_sync();
+  pair_sync();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
   if (warp == kRgEpiWarps + kRgSplitWarps) {
@@ -192,7 +122,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         const int row = t * 2 * kTcRows + (int)rank * kTcRows;
         for (int sl = 0; sl < P.n_slices; ++sl) {
           prefetch();
-          if (issued >= stages && !(ok = rg_wait(&s.empty[st], ph ^ 1u, s, P.wait_limit))) break;
+          if (issued >= stages && !(ok = pair_wait(&s.empty[st], ph ^ 1u, s.dead, P.wait_limit))) break;
           char *b = smem + st * stage_bytes;
           mbar_expect_tx(&s.raw[st], (unsigned)((P.direct ? 0 : kTcRows * 128) + N * 128));
           if (!P.direct) tma_load_2d(b, &tm_a, sl * kTcKSlice, row, &s.raw[st]);
@@ -204,64 +134,71 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       }
       // the tensor core's arrivals on the stages of this CTA come from the other one too: the last of them must be in before
       // the CTA may end
-      for (int i = 0; ok && i < issued; ++i) ok = rg_wait(&s.empty[i], i < st ? ph : ph ^ 1u, s, P.wait_limit);
+      for (int i = 0; ok && i < issued; ++i) ok = pair_wait(&s.empty[i], i < st ? ph : ph ^ 1u, s.dead, P.wait_limit);
       // a copy still in flight must not outlive the CTA (only after a wait ran out is one possible)
       if (s.dead)
         for (int i = 0; i < issued; ++i)
           for (int k = 0; k < P.wait_limit && !mbar_wait(&s.raw[i], (i < st ? ph : ph ^ 1u), 1); ++k) {}
     }
   } else if (warp == kRgEpiWarps + kRgSplitWarps + 1) {
-    // ---- products (even CTA) ----
-    if (lane == 0 && rank == 0) {
-      const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(N >> 3) << 17) | ((unsigned)(2 * kTcRows >> 4) << 24);
+    // ---- products (even CTA): the whole warp, see elect_one ----
+    if (rank == 0) {
+      const unsigned idesc = pair_idesc(N);
       int st = 0, buf = 0, uses = 0;  // uses: accumulators handed out so far
       unsigned ph = 0, acc_ph = 0;
       bool ok = true;
+      auto wait = [&](unsigned long long *bar, unsigned parity) {
+        return ok = __all_sync(kFull, pair_wait<true>(bar, parity, s.dead, P.wait_limit));
+      };
       auto take = [&]() {  // the accumulator has been read
-        if (uses >= 2 && !(ok = rg_wait<true>(&s.acc_empty[buf], acc_ph ^ 1u, s, P.wait_limit))) return false;
+        if (uses >= 2 && !wait(&s.acc_empty[buf], acc_ph ^ 1u)) return false;
         if (uses < 2) ++uses;
         return true;
       };
-      auto give = [&]() {
-        rg_commit(&s.acc_full[buf]);
-        buf ^= 1;
-        if (buf == 0) acc_ph ^= 1u;
-      };
+      const unsigned tmem = s.tmem_base;
       for (int t = pair; t < P.tiles && ok; t += pairs) {
         if (!PRECISE && !take()) break;
         for (int sl = 0; sl < P.n_slices; ++sl) {
           if (PRECISE && !take()) break;
-          if (!(ok = rg_wait<true>(&s.ready[st], ph, s, P.wait_limit))) break;
+          if (!wait(&s.ready[st], ph)) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const unsigned d = s.tmem_base + (unsigned)(buf * 256);
+          const unsigned d = tmem + (unsigned)(buf * 256);
           const unsigned b = smem_u32(smem + st * stage_bytes);
-          const unsigned ah = b, al = b + kTcRows * 128, wh = b + 2 * kTcRows * 128, wl = wh + half * 128;
+          const unsigned long long ah = umma_desc_sw128(b), al = umma_desc_sw128(b + kTcRows * 128);
+          const unsigned long long wh = umma_desc_sw128(b + 2 * kTcRows * 128), wl = umma_desc_sw128(b + 2 * kTcRows * 128 + half * 128);
           const unsigned fresh = PRECISE || sl == 0;
+          const bool last = PRECISE || sl == P.n_slices - 1;
           auto mma = [&](int j, int term, unsigned add) {  // K step j (eight TF32 values inside the swizzle row) of lo*hi, hi*lo, hi*hi
-            const unsigned o = j * 32;
-            rg_mma(d + (unsigned)((j & (accs - 1)) * acc_cols), umma_desc_sw128((term == 0 ? al : ah) + o),
-                   umma_desc_sw128((term == 1 ? wl : wh) + o), idesc, add);
+            pair_mma(d + (unsigned)((j & (accs - 1)) * acc_cols), (term == 0 ? al : ah) + j * kUmmaStep, (term == 1 ? wl : wh) + j * kUmmaStep,
+                     idesc, add);
           };
-          if (accs > 1) {
+          if (elect_one()) {
+            if (accs > 1) {
 #pragma unroll
-            for (int term = 0; term < 3; ++term)
+              for (int term = 0; term < 3; ++term)
 #pragma unroll
-              for (int j = 0; j < kTcKSlice / 8; ++j) mma(j, term, fresh && term == 0 && j < accs ? 0u : 1u);
-          } else {  // in the order of gemm_tc.cuh: the same bits
+                for (int j = 0; j < kTcKSlice / 8; ++j) mma(j, term, fresh && term == 0 && j < accs ? 0u : 1u);
+            } else {  // in the order of gemm_tc.cuh: the same bits
 #pragma unroll
-            for (int j = 0; j < kTcKSlice / 8; ++j) {
-              mma(j, 2, fresh && j == 0 ? 0u : 1u);
-              mma(j, 1, 1u);
-              mma(j, 0, 1u);
+              for (int j = 0; j < kTcKSlice / 8; ++j) {
+                mma(j, 2, fresh && j == 0 ? 0u : 1u);
+                mma(j, 1, 1u);
+                mma(j, 0, 1u);
+              }
             }
+            pair_commit(&s.empty[st]);
+            if (last) pair_commit(&s.acc_full[buf]);
           }
-          rg_commit(&s.empty[st]);
-          if (PRECISE || sl == P.n_slices - 1) give();
+          __syncwarp();
+          if (last) {
+            buf ^= 1;
+            if (buf == 0) acc_ph ^= 1u;
+          }
           if (++st == stages) { st = 0; ph ^= 1u; }
         }
       }
       if (!ok) {  // products still running read shared memory of both CTAs
-        rg_commit(&s.drained);
+        if (elect_one()) pair_commit(&s.drained);
         mbar_wait(&s.drained, 0, P.wait_limit);
       }
     }
@@ -273,7 +210,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     bool ok = true;
     for (int t = pair; t < P.tiles && ok; t += pairs)
       for (int sl = 0; sl < P.n_slices; ++sl) {
-        if (!(ok = __all_sync(kFull, rg_wait(&s.raw[st], ph, s, P.wait_limit)))) break;  // (the warp leaves as one)
+        if (!(ok = __all_sync(kFull, pair_wait(&s.raw[st], ph, s.dead, P.wait_limit)))) break;  // (the warp leaves as one)
         float4 *hi = reinterpret_cast<float4 *>(smem + st * stage_bytes), *lo = hi + kTcRows * 8;
         float4 a[kTcRows * 8 / (32 * kRgSplitWarps)];
         if (!P.direct) {
@@ -302,7 +239,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read next by the tensor core
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) rg_arrive_leader(&s.ready[st]);
+        if (lane == 0) pair_arrive_leader(&s.ready[st]);
         if (++st == stages) { st = 0; ph ^= 1u; }
       }
   } else {
@@ -314,7 +251,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     auto release = [&]() {  // the accumulator has been read: its next use may overwrite it
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) rg_arrive_leader(&s.acc_empty[buf]);
+      if (lane == 0) pair_arrive_leader(&s.acc_empty[buf]);
     };
     auto next = [&]() {
       buf ^= 1;
@@ -372,7 +309,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 #pragma unroll
         for (int q = 0; q < 32; ++q) acc[0][q] = acc[1][q] = 0.f;
         for (int sl = 0; sl < P.n_slices; ++sl) {
-          if (!(ok = __all_sync(kFull, rg_wait(&s.acc_full[buf], acc_ph, s, P.wait_limit)))) break;
+          if (!(ok = __all_sync(kFull, pair_wait(&s.acc_full[buf], acc_ph, s.dead, P.wait_limit)))) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -380,9 +317,9 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               float a[32];
-              rg_tmem_load(a, lanes + (unsigned)(buf * 256 + j * 64 + h * 32));
+              tmem_load32(a, lanes + (unsigned)(buf * 256 + j * 64 + h * 32));
               asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-              rg_loaded(a);
+              tmem_loaded(a);
 #pragma unroll
               for (int q = 0; q < 32; ++q) acc[h][q] += a[q];
             }
@@ -396,18 +333,18 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           if (P.n_real > 32) put(acc[1], 32, row0);
         }
       } else {
-        if (!(ok = __all_sync(kFull, rg_wait(&s.acc_full[buf], acc_ph, s, P.wait_limit)))) break;
+        if (!(ok = __all_sync(kFull, pair_wait(&s.acc_full[buf], acc_ph, s.dead, P.wait_limit)))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int c = 0; c < N; c += 32) {
           float v[32];
-          rg_tmem_load(v, lanes + (unsigned)(buf * 256 + c));
+          tmem_load32(v, lanes + (unsigned)(buf * 256 + c));
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          rg_loaded(v);
+          tmem_loaded(v);
           for (int i = 1; i < accs; ++i) {
             float a[32];
-            rg_tmem_load(a, lanes + (unsigned)(buf * 256 + i * acc_cols + c));
+            tmem_load32(a, lanes + (unsigned)(buf * 256 + i * acc_cols + c));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            rg_loaded(a);
+            tmem_loaded(a);
 #pragma unroll
             for (int q = 0; q < 32; ++q) v[q] += a[q];
           }
@@ -423,7 +360,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (tid == 0 && s.dead) atomicExch(P.error, 1);
-  rg_cluster_sync();
+  pair_sync();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(s.tmem_base), "n"(512) : "memory");
