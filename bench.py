@@ -541,6 +541,8 @@ def run_lattice_workload(name, args, ctx, headline):
     kernel = {128: "lattice_march_kernel", 672: "tile_pipeline_kernel"}.get(threads, "stream_kernel")
     if chain == "gemm_spmm" and threads == 128:
         kernel = "row_gemm_kernel (dense product) + " + ("star_march_kernel" if world == 1 else "lattice_march_kernel")
+    elif chain == "gemm_spmm" and threads == 480:
+        kernel = "spmm_gemm_kernel"
     elif chain == "gemm_spmm" and args.mode == "stream" and world == 1:
         kernel = "row_gemm_kernel (dense product) + gather_kernel"
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,

@@ -8,8 +8,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "libtilefusion_b200.so")
 SOURCES = ["kernels.cu", "api.cu", "inspector.cpp", "planner.cpp", "tiling.cpp", "noalloc.cu", "gemm_tc.cu", "tile_pipeline.cu", "lattice.cpp", "lattice_march.cu", "multi.cu", "io.cpp", "reorder.cpp",
-           "gather.cu", "gather_plan.cpp", "row_gemm.cu", "sddmm_gather.cu", "line_march.cu", "line_plan.cpp", "band_march.cu", "band_plan.cpp", "atb.cu"]
-HEADERS = ["kernels.cuh", "launch.h", "tf_internal.h", "gemm_tc.cuh", "gemm_tc_host.h", "lattice_march.h", "host_stage.h", "gather.h", "row_gemm.h", "line_march.h", "band_march.h", "segments.h", "pair_mma.cuh"]
+           "gather.cu", "gather_plan.cpp", "row_gemm.cu", "sddmm_gather.cu", "line_march.cu", "line_plan.cpp", "band_march.cu", "band_plan.cpp", "atb.cu", "spmm_gemm.cu", "spmm_gemm_plan.cpp"]
+HEADERS = ["kernels.cuh", "launch.h", "tf_internal.h", "gemm_tc.cuh", "gemm_tc_host.h", "lattice_march.h", "host_stage.h", "gather.h", "row_gemm.h", "line_march.h", "band_march.h", "segments.h", "spmm_gemm.h", "pair_mma.cuh"]
 
 
 def _stale() -> bool:

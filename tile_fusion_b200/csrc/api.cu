@@ -22,6 +22,7 @@
 #include "launch.h"
 #include "line_march.h"
 #include "row_gemm.h"
+#include "spmm_gemm.h"
 #include "tf_internal.h"
 
 namespace {
@@ -263,6 +264,8 @@ struct tf_plan {
   bool keep_t = false;       // the caller asked for the intermediate: every call leaves it in `inter`
   bool spmm_first = false;   // GeMM-SpMM on the balanced gather: D = (A B) C instead of A (B C)
   bool ticket_sums = false;  // every sum in the order of the ticket executor (tensor_cores > 0)
+  bool one_sums = false;     // (with spmm_first) those of the one launch, in two
+  tfk::RowGemmSums sums() const { return ticket_sums ? tfk::kSumsTicket : one_sums && spmm_first ? tfk::kSumsSpmmGemm : tfk::kSumsFree; }
   size_t dyn_smem = 0;
   int tile_slots = 0;
   bool pipe = false;  // every item of phases 1 and 2 is a gather tile: run them on the tile pipeline
@@ -310,6 +313,13 @@ struct tf_plan {
     DevBuf<int> quads_f, quads_a;
     tfk::BandParams par;
   } band;
+  // GeMM-SpMM in one launch
+  struct OneLaunch {
+    bool on = false;
+    tfk::SpmmGemmParams par = {};
+    DevBuf<float> coef;
+    std::vector<Piece> pieces;  // of a host-pointer call: bricks [begin, end)
+  } one;
   // schedule mode
   DevBuf<int> s_ptr2, s_id, s_type, s_ker;
   int s_n1 = 0;
@@ -832,17 +842,50 @@ int leave_intermediate(tf_plan &p, const float *C, cudaStream_t s) {
   return tf_spmm_dev(f.ap.p, f.ai.p, f.ax.p, p.m, C, p.n_cols, p.inter.p, s);
 }
 
+// GeMM-SpMM in one launch (spmm_gemm.cu): star stencils with every neighbour stored, shapes of the tensor-core tile.  It adds up
+// rows of B, so B should not be much wider than the result: on flat grids it is ahead up to K = 8 N (700 000 points, 128 -> 16:
+// 126 us and 131, 256 -> 16: 216 and 210), on 3-D grids up to 1.5 N (1 M points, 128 -> 128: 290 and 382, 100 -> 64: 271 and 253,
+// 128 -> 64: 258 and 251, 64 -> 16: 124 and 106).  Small grids keep the executors they had: there is a launch or two to gain
+// (4 913 points in 3-D, 64 -> 64: 9.0 us and 15.3), and callers compare the march with the gather bit for bit on them.
+int build_one_launch(tf_plan &p, const tf_csr &A) {
+  if (p.ticket_sums || !tfk::tc_supported(p.k_dim, p.n_cols) || A.m < (1 << 12)) return TF_OK;
+  tf::StarOp op;
+  tf::analyse_star_operator(A.m, A.n, A.ap, A.ai, A.ax, op);
+  if (!op.nx || (op.nz == 1 ? p.k_dim > 8 * p.n_cols : 2 * p.k_dim > 3 * p.n_cols || A.m < (1 << 15))) return TF_OK;
+  tf_plan::OneLaunch &O = p.one;
+  if (!tf::choose_bricks(op, tfk::spmm_gemm_points(p.k_dim, p.n_cols), O.par.grid)) return TF_OK;
+  if (op.uniform) std::copy(op.coef.begin(), op.coef.end(), O.par.uniform);
+  else TF_TRY(O.coef.upload(op.coef));
+  O.par.coef = O.coef.p;
+  // a host-pointer call goes layer by layer (on a flat grid row of bricks by row of bricks), up to 16 at a time
+  const tf::BrickGrid &g = O.par.grid;
+  const bool deep = g.nz > 1;
+  const int layers = deep ? g.bz() : g.by(), per = g.bricks() / layers, n = std::min(16, layers);
+  const long long points = (long long)g.nx * (deep ? g.ny : 1), thick = 1LL << (deep ? g.lz : g.ly);
+  for (int i = 0; i < n; ++i) {
+    const int a = (int)((long long)layers * i / n), b = (int)((long long)layers * (i + 1) / n);
+    O.pieces.push_back(tf_plan::Piece{0, 0, a * per, b * per, std::min<long long>(p.m, (b * thick + 1) * points), std::min<long long>(p.m, b * thick * points)});
+  }
+  O.on = true;
+  return TF_OK;
+}
+
 // GeMM-SpMM on the balanced gather.  The two products may be taken in either order, D = A (B C) = (A B) C: the sparse
 // product reads one row of its operand per nonzero, so it is given the narrower one -- B where k < n_cols, else B C.
 // (Rows of B that do not start on 16-byte boundaries would be gathered value by value; then B C comes first.  So it does
 // on grids and bands: with a handful of nonzeros a row there is little to choose, and every consumer gives the same bits.)
 int make_gemm_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &A, const tf_plan_opts &o, bool tiled, int sm_count, tf_plan **out) {
-  p->spmm_first = !tiled && !p->ticket_sums && p->k_dim % 4 == 0 && p->k_dim < p->n_cols;
+  if (p->mode == TF_MODE_UNFUSED) {  // what runs in one launch otherwise, in two
+    p->one.on = false;
+    p->spmm_first = p->one_sums = true;
+  } else {
+    p->spmm_first = !tiled && !p->ticket_sums && p->k_dim % 4 == 0 && p->k_dim < p->n_cols;
+  }
   const int width = p->spmm_first ? p->k_dim : p->n_cols;
   p->ld_t = (width + 3) / 4 * 4;
   const size_t wn = (size_t)tfk::row_gemm_pad_n(p->n_cols) * tfk::row_gemm_pad_k(p->k_dim);
-  int rc = p->g_second.build(A, width, std::max(p->k_dim, p->n_cols), sm_count, tiled, tfk::kGatherResident, p->ticket_sums);
-  if (rc == TF_OK) rc = p->inter.alloc((size_t)(p->m + 1) * p->ld_t);  // (the one-product march may read one row more)
+  int rc = p->g_second.build(A, width, std::max(p->k_dim, p->n_cols), sm_count, tiled && !p->one_sums, tfk::kGatherResident, p->ticket_sums);
+  if (rc == TF_OK && !p->one.on) rc = p->inter.alloc((size_t)(p->m + 1) * p->ld_t);  // (the one-product march may read one row more)
   if (rc == TF_OK) rc = p->w_hi.alloc(wn);
   if (rc == TF_OK) rc = p->w_lo.alloc(wn);
   if (rc == TF_OK) rc = zero_state(*p);
@@ -850,7 +893,7 @@ int make_gemm_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &A, const tf
   make_gather_pieces(*p, 16);
   p->hp.inter_rows = p->m;
   p->hp.n_cons = p->g_second.n_units;
-  if (tiled && o.lattice_march >= 0 && p->n_cols % 4 == 0) {
+  if (tiled && o.lattice_march >= 0 && p->n_cols % 4 == 0 && !p->one.on && !p->one_sums) {
     rc = build_march(*p, nullptr, A, 0, sm_count, {}, true);
     if (rc != TF_OK) return rc;
     tf_plan::March &M = p->march;
@@ -1037,11 +1080,15 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
   }
   p->tile_info[0] = pt.bx; p->tile_info[1] = pt.by; p->tile_info[2] = pt.bz; p->tile_info[3] = pt.tiles();
   p->tile_info[4] = ct.bx; p->tile_info[5] = ct.by; p->tile_info[6] = ct.bz; p->tile_info[7] = ct.tiles();
-  if (chain == 1 && o.mode == TF_MODE_STREAM && o.tensor_cores >= 0 && tfk::row_gemm_supported(n_cols) &&
-      o.ring_bytes <= 0 && o.halo_rows == 0 && o.n_boundary == 0 && o.rows_per_block == 0 && o.slack_blocks < 0 && o.ctas_per_sm == 0) {
-    bool whole = false;
-    TF_TRY(keeps_whole((size_t)A->m * n_cols * sizeof(float), whole));
-    if (whole) return make_gemm_gather_plan(p, *A, o, ct.tiled, sm_count, out);
+  // (The unfused mode takes the two products one after the other in the order in which the one launch takes them where that has
+  // one accumulator, so that it gives the same bits there.)
+  if (chain == 1 && (o.mode == TF_MODE_STREAM || (o.mode == TF_MODE_UNFUSED && n_cols > 128)) && o.tensor_cores >= 0 &&
+      tfk::row_gemm_supported(n_cols) && o.ring_bytes <= 0 && o.halo_rows == 0 && o.n_boundary == 0 && o.rows_per_block == 0 &&
+      o.slack_blocks < 0 && o.ctas_per_sm == 0) {
+    bool whole = o.mode == TF_MODE_UNFUSED;
+    if (!whole) TF_TRY(keeps_whole((size_t)A->m * n_cols * sizeof(float), whole));
+    if (whole && ct.tiled && o.lattice_march >= 0) TF_TRY(build_one_launch(*p, *A));
+    if (whole && (o.mode == TF_MODE_STREAM || p->one.on)) return make_gemm_gather_plan(p, *A, o, ct.tiled, sm_count, out);
   }
   rc = p->second.upload(*A);
   if (rc == TF_OK && F && F != A) rc = p->first.upload(*F);
@@ -1444,20 +1491,38 @@ int run_gather_spmm_spmm(tf_plan &p, const float *C, float *D, cudaStream_t s) {
   return run_gather(p.g_second, p.inter.p, p.ld_t, true, D, p.n_cols, p.n_cols % 4 == 0 && aligned(D, 16), p.n_cols, false, s);
 }
 
+// GeMM-SpMM in one launch; split: the weight may have changed since the launch before.
+int run_one_launch(tf_plan &p, const float *B, const float *W, int w_transposed, bool relu, float *D, int brick_begin, int brick_end, bool split,
+                   cudaStream_t s) {
+  p.launches = 1;
+  if (split && !tfk::spmm_gemm_resident(p.k_dim, p.n_cols)) {
+    TF_CUDA(tfk::row_gemm_split(W, w_transposed, p.k_dim, p.n_cols, tfk::kSumsFree, p.w_hi.p, p.w_lo.p, s));
+    p.launches = 2;
+  }
+  tfk::SpmmGemmParams P = p.one.par;
+  P.b = B; P.w = W; P.out = D;
+  P.k = p.k_dim; P.n = p.n_cols; P.w_transposed = w_transposed;
+  P.brick_begin = brick_begin; P.brick_end = brick_end;
+  P.relu = relu ? 1 : 0;
+  P.error = &p.state.p->error; P.wait_limit = p.spin_limit;
+  return tfk::spmm_gemm(P, p.w_hi.p, p.w_lo.p, p.sm_count, s);
+}
+
 int run_gather_gemm_spmm(tf_plan &p, const float *B, const float *W, int w_transposed, bool relu, float *D, cudaStream_t s) {
   const int n = p.n_cols, k = p.k_dim;
   const bool out16 = n % 4 == 0 && aligned(D, 16);
   if (p.dyn_smem > 0 && !(aligned(B, 16) && aligned(D, 16)))
     return fail(TF_ERR_ARG, "this plan (gather tiles or tensor-core producer) needs 16-byte aligned dense operands "
                             "(build the plan with tile_slots < 0 and tensor_cores < 0 otherwise)");
-  TF_CUDA(tfk::row_gemm_split(W, w_transposed, k, n, p.ticket_sums, p.w_hi.p, p.w_lo.p, s));
+  if (p.one.on && !p.keep_t) return run_one_launch(p, B, W, w_transposed, relu, D, 0, p.one.par.grid.bricks(), true, s);
+  TF_CUDA(tfk::row_gemm_split(W, w_transposed, k, n, p.sums(), p.w_hi.p, p.w_lo.p, s));
   p.launches = tfk::row_gemm_form(k, n) == tfk::kRowFma ? 2 : 3;
   if (p.spmm_first) {
     TF_TRY(run_gather(p.g_second, B, k, aligned(B, 16), p.inter.p, p.ld_t, true, k, false, s));
-    return tfk::row_gemm(p.inter.p, p.m, k, p.ld_t, W, w_transposed, p.w_hi.p, p.w_lo.p, n, D, n, relu, false, &p.state.p->error,
+    return tfk::row_gemm(p.inter.p, p.m, k, p.ld_t, W, w_transposed, p.w_hi.p, p.w_lo.p, n, D, n, relu, p.sums(), &p.state.p->error,
                          p.spin_limit, p.sm_count, s);
   }
-  TF_TRY(tfk::row_gemm(B, p.m, k, k, W, w_transposed, p.w_hi.p, p.w_lo.p, n, p.inter.p, p.ld_t, false, p.ticket_sums,
+  TF_TRY(tfk::row_gemm(B, p.m, k, k, W, w_transposed, p.w_hi.p, p.w_lo.p, n, p.inter.p, p.ld_t, false, p.sums(),
                        &p.state.p->error, p.spin_limit, p.sm_count, s));
   return run_gather(p.g_second, p.inter.p, p.ld_t, true, D, n, out16, n, relu, s);
 }
@@ -1535,6 +1600,7 @@ int tf_plan_info(const tf_plan *p, long long info[8]) {
   info[5] = p->march.on         ? tfk::kMarchThreads
             : p->lines.on       ? 32 * tfk::kLineWarps
             : p->band.block     ? tfk::kBandThreads
+            : p->one.on && !p->keep_t ? tfk::kSpmmGemmThreads
             : p->pipe           ? 672
             : p->g_second.on    ? tfk::kThreads
             : p->dyn_smem > 0   ? tfk::tiled_threads(p->chain)
@@ -1602,9 +1668,9 @@ int run_gemm_march(tf_plan &p, const float *B, const float *W, int w_transposed,
                    int item_end, bool with_halo, cudaStream_t s) {
   long long launches = 0;
   if (produce) {
-    TF_CUDA(tfk::row_gemm_split(W, w_transposed, p.k_dim, p.n_cols, p.ticket_sums, p.w_hi.p, p.w_lo.p, s));
+    TF_CUDA(tfk::row_gemm_split(W, w_transposed, p.k_dim, p.n_cols, p.sums(), p.w_hi.p, p.w_lo.p, s));
     int rc = tfk::row_gemm(B, p.m, p.k_dim, p.k_dim, W, w_transposed, p.w_hi.p, p.w_lo.p, p.n_cols, p.inter.p, p.n_cols, false,
-                           p.ticket_sums, &p.march.st.p[0].error, p.spin_limit, p.sm_count, s);
+                           p.sums(), &p.march.st.p[0].error, p.spin_limit, p.sm_count, s);
     if (rc != TF_OK) return rc;
     launches = tfk::row_gemm_form(p.k_dim, p.n_cols) == tfk::kRowFma ? 1 : 2;   // (weight split and) dense product
   }
@@ -1742,6 +1808,8 @@ int tf_plan_intermediate(tf_plan *p, float **dev_ptr, long long *rows, int *cols
       TF_TRY(restore_csr(*p, false));
       TF_TRY(p->inter.alloc((size_t)p->m * p->n_cols));
       p->hp.inter_rows = p->m;
+    } else if (p->one.on) {
+      TF_TRY(p->inter.alloc((size_t)(p->m + 1) * p->ld_t));
     }
     p->keep_t = true;
   }
@@ -1793,7 +1861,9 @@ static int run_host_whole(tf_plan &p, const float *C, size_t nin, float *D, size
 static int run_host_pieces(tf_plan &p, const float *in, int w_transposed, bool relu, float *D) {
   const DevGather &g = p.g_second, &f = p.first_is_second ? p.g_second : p.g_first;
   const bool gemm = p.chain == 1;
-  const int ns = (int)p.pieces.size(), n = p.n_cols, k = gemm ? p.k_dim : p.n_cols;  // k: width of the input
+  const bool one = p.one.on && !p.keep_t;
+  const std::vector<tf_plan::Piece> &pieces = one ? p.one.pieces : p.pieces;
+  const int ns = (int)pieces.size(), n = p.n_cols, k = gemm ? p.k_dim : p.n_cols;  // k: width of the input
   while ((int)p.ev_in.size() < ns) {
     cudaEvent_t a, b;
     TF_CUDA(cudaEventCreateWithFlags(&a, cudaEventDisableTiming));
@@ -1801,23 +1871,25 @@ static int run_host_pieces(tf_plan &p, const float *in, int w_transposed, bool r
     p.ev_in.push_back(a); p.ev_run.push_back(b);
   }
   TF_TRY(begin_host_pipe(p, in, D));
-  if (gemm) TF_CUDA(tfk::row_gemm_split(p.h_in1.p, w_transposed, k, n, p.ticket_sums, p.w_hi.p, p.w_lo.p, p.s_run));
+  if (one) {}
+  else if (gemm) TF_CUDA(tfk::row_gemm_split(p.h_in1.p, w_transposed, k, n, p.sums(), p.w_hi.p, p.w_lo.p, p.s_run));
   else TF_CUDA(tfk::launch_rows_fix(f.empty.p, f.n_empty, p.ld_t, p.inter.p, false, p.s_run));
   TF_CUDA(tfk::launch_rows_fix(g.empty.p, g.n_empty, n, p.h_out.p, false, p.s_run));
   const bool pad = p.g_pad.n != 0, vec = pad || n % 4 == 0;  // (the buffers of the call start on 16-byte boundaries)
   long long in_done = 0, out_done = 0;
   p.launches = 1;
   for (int s = 0; s < ns; ++s) {
-    const tf_plan::Piece &sg = p.pieces[s];
+    const tf_plan::Piece &sg = pieces[s];
     const long long in_to = gemm && s == ns - 1 ? p.m : std::max(in_done, sg.in_rows);
     if (in_to > in_done) {
       float *src = p.h_in0.p + in_done * k;
       TF_CUDA(p.host_pipe->upload(src, in + in_done * k, (size_t)(in_to - in_done) * k * 4, p.s_h2d));
       TF_CUDA(cudaEventRecord(p.ev_in[s], p.s_h2d));
       TF_CUDA(cudaStreamWaitEvent(p.s_run, p.ev_in[s], 0));
-      if (gemm) {
+      if (one) {
+      } else if (gemm) {
         TF_TRY(tfk::row_gemm(src, (int)(in_to - in_done), k, k, p.h_in1.p, w_transposed, p.w_hi.p, p.w_lo.p, n,
-                             p.inter.p + in_done * p.ld_t, p.ld_t, false, p.ticket_sums, &p.state.p->error, p.spin_limit, p.sm_count, p.s_run));
+                             p.inter.p + in_done * p.ld_t, p.ld_t, false, p.sums(), &p.state.p->error, p.spin_limit, p.sm_count, p.s_run));
         ++p.launches;
       } else if (pad) {
         TF_CUDA(tfk::launch_pad_rows(src, in_to - in_done, n, p.ld_t, p.g_pad.p + in_done * p.ld_t, p.s_run));
@@ -1830,8 +1902,10 @@ static int run_host_pieces(tf_plan &p, const float *in, int w_transposed, bool r
                         sg.f_begin, sg.f_end));
       ++p.launches;
     }
-    TF_TRY(run_gather(g, p.inter.p, p.ld_t, true, p.h_out.p, n, n % 4 == 0, n, relu, p.s_run, sg.begin, sg.end));
-    ++p.launches;
+    const long long before = p.launches;
+    if (one) TF_TRY(run_one_launch(p, p.h_in0.p, p.h_in1.p, w_transposed, relu, p.h_out.p, sg.begin, sg.end, s == 0, p.s_run));
+    else TF_TRY(run_gather(g, p.inter.p, p.ld_t, true, p.h_out.p, n, n % 4 == 0, n, relu, p.s_run, sg.begin, sg.end));
+    p.launches = before + 1;
     if (sg.out_rows > out_done) {
       TF_CUDA(cudaEventRecord(p.ev_run[s], p.s_run));
       TF_CUDA(cudaStreamWaitEvent(p.s_d2h, p.ev_run[s], 0));
@@ -1918,7 +1992,7 @@ int tf_gemm_spmm_host(tf_plan *p, const float *B, const float *W, int w_transpos
     if (rc != TF_OK) return rc;
     TF_TRY(ensure_streams(*p));
     TF_TRY(stage_in(p->h_in1, W, (size_t)p->k_dim * p->n_cols, p->s_run));  // the weight first, on the stream that uses it
-    if (!p->pieces.empty()) rc = run_host_pieces(*p, B, w_transposed, relu != 0, D);
+    if (!p->pieces.empty() || (p->one.on && !p->keep_t)) rc = run_host_pieces(*p, B, w_transposed, relu != 0, D);
     else
       rc = run_host_whole(*p, B, nin, D, nd, [&] {
         return run_gather_gemm_spmm(*p, p->h_in0.p, p->h_in1.p, w_transposed, relu != 0, p->h_out.p, p->s_run);

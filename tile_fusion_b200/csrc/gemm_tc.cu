@@ -87,8 +87,8 @@ extern "C" int tf_gemm_tc_dev(const float *B, const float *W, int w_transposed, 
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    e = tfk::row_gemm_split(W, w_transposed, K, N, false, hi, lo, s);
-    if (e == cudaSuccess) rc = tfk::row_gemm(B, m, K, K, W, w_transposed, hi, lo, N, T, N, false, false, err, 1 << 20, sms, s);
+    e = tfk::row_gemm_split(W, w_transposed, K, N, tfk::kSumsFree, hi, lo, s);
+    if (e == cudaSuccess) rc = tfk::row_gemm(B, m, K, K, W, w_transposed, hi, lo, N, T, N, false, tfk::kSumsFree, err, 1 << 20, sms, s);
     if (e == cudaSuccess && rc == TF_OK) e = cudaStreamSynchronize(s);
     int h_err = 0;
     if (e == cudaSuccess && rc == TF_OK) e = cudaMemcpy(&h_err, err, 4, cudaMemcpyDeviceToHost);

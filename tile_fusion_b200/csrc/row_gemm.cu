@@ -173,7 +173,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                      idesc, add);
           };
           if (elect_one()) {
-            if (accs > 1) {
+            if (accs > 1 || P.small_first) {
 #pragma unroll
               for (int term = 0; term < 3; ++term)
 #pragma unroll
@@ -233,7 +233,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           const float4 h = make_float4(tf32_round(x.x), tf32_round(x.y), tf32_round(x.z), tf32_round(x.w));
           hi[w + i * 32 * kRgSplitWarps] = h;
           float4 l = make_float4(x.x - h.x, x.y - h.y, x.z - h.z, x.w - h.w);
-          if (!P.ticket) l = make_float4(tf32_round(l.x), tf32_round(l.y), tf32_round(l.z), tf32_round(l.w));
+          if (!P.cut_low) l = make_float4(tf32_round(l.x), tf32_round(l.y), tf32_round(l.z), tf32_round(l.w));
           lo[w + i * 32 * kRgSplitWarps] = l;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read next by the tensor core
@@ -447,9 +447,9 @@ int row_gemm_pad_k(int k) { return (k + 3) / 4 * 4; }
 
 RowGemmForm row_gemm_form(int K, int n) { return tc_supported(K, n) ? kRowTile : (K >= kRgPreciseMinK ? kRowPrecise : kRowFma); }
 
-cudaError_t row_gemm_split(const float *W, int w_transposed, int K, int n, bool ticket, float *hi, float *lo, cudaStream_t s) {
+cudaError_t row_gemm_split(const float *W, int w_transposed, int K, int n, RowGemmSums sums, float *hi, float *lo, cudaStream_t s) {
   if (row_gemm_form(K, n) == kRowFma) return cudaSuccess;
-  ticket = ticket && row_gemm_form(K, n) == kRowTile;
+  const bool ticket = sums == kSumsTicket && row_gemm_form(K, n) == kRowTile;
   const int ldk = row_gemm_pad_k(K), n_pad = row_gemm_pad_n(n);
   split_weight_pad_kernel<<<std::min((n_pad * ldk + 255) / 256, 148 * 4), 256, 0, s>>>(W, w_transposed, K, ldk, n, n_pad, ticket, hi, lo);
   return cudaGetLastError();
@@ -467,20 +467,21 @@ static int launch_fma(const float *X, int m, int K, int ld_x, const float *W, in
 }
 
 static int launch_panel(const float *X, int m, int K, int ld_x, const float *W, int w_k, int w_c, const float *hi, const float *lo, int n, float *out, int ld_out, bool relu,
-                        bool precise, bool ticket, int *error, int wait_limit, int sm_count, cudaStream_t s) {
+                        bool precise, RowGemmSums sums, int *error, int wait_limit, int sm_count, cudaStream_t s) {
   const int n_pad = row_gemm_pad_n(n), ldk = row_gemm_pad_k(K);
   CUtensorMap ma, mh, ml, mo;
   RowGemmParams P;
   P.x = X; P.k = K; P.ld_x = ld_x;
   P.w = W; P.w_k = w_k; P.w_c = w_c;
-  P.ticket = ticket ? 1 : 0;
+  P.cut_low = sums != kSumsFree ? 1 : 0;
+  P.small_first = sums == kSumsSpmmGemm ? 1 : 0;
   P.direct = ld_x % 4 != 0 || (reinterpret_cast<uintptr_t>(X) & 15) != 0;
   int rc = tc_make_map(&mh, hi, n_pad, ldk, n_pad / 2, ldk);
   if (rc == TF_OK) rc = tc_make_map(&ml, lo, n_pad, ldk, n_pad / 2, ldk);
   P.m = m; P.n_pad = n_pad; P.n_real = n; P.n_slices = (K + kTcKSlice - 1) / kTcKSlice;
   P.tiles = (m + 2 * kTcRows - 1) / (2 * kTcRows);
   P.stages = rg_stages(n_pad);
-  P.accs = ticket || n_pad > 128 ? 1 : (n_pad > 64 ? 2 : 4);
+  P.accs = sums == kSumsTicket || n_pad > 128 ? 1 : (n_pad > 64 ? 2 : 4);
   P.out = out; P.ld_out = ld_out; P.relu = relu ? 1 : 0;
   P.tma_store = ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   P.error = error; P.wait_limit = wait_limit;
@@ -503,17 +504,17 @@ static int launch_panel(const float *X, int m, int K, int ld_x, const float *W, 
 }
 
 int row_gemm(const float *X, int m, int K, int ld_x, const float *W, int w_transposed, const float *hi, const float *lo, int n,
-             float *out, int ld_out, bool relu, bool ticket, int *error, int wait_limit, int sm_count, cudaStream_t s) {
+             float *out, int ld_out, bool relu, RowGemmSums sums, int *error, int wait_limit, int sm_count, cudaStream_t s) {
   const RowGemmForm form = row_gemm_form(K, n);
   if (form == kRowFma) return launch_fma(X, m, K, ld_x, W, w_transposed, n, out, ld_out, relu, sm_count, s);
   const bool precise = form == kRowPrecise;
-  ticket = ticket && !precise;
+  if (precise) sums = kSumsFree;
   const int panel = precise ? kRgPrecisePanel : n;
   for (int c = 0; c < n; c += panel) {
     const size_t off = (size_t)c * row_gemm_pad_k(K);
     const int w_k = w_transposed ? 1 : n, w_c = w_transposed ? K : 1;
     const int rc = launch_panel(X, m, K, ld_x, W + (size_t)c * w_c, w_k, w_c, hi + off, lo + off, std::min(panel, n - c), out + c, ld_out,
-                                relu, precise, ticket, error, wait_limit, sm_count, s);
+                                relu, precise, sums, error, wait_limit, sm_count, s);
     if (rc != TF_OK) return rc;
   }
   return TF_OK;
