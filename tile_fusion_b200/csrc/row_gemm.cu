@@ -9,17 +9,20 @@
 //     N = 256, 40 % more than there are.)
 //   * A warp keeps the TMA loads of K slices of 32 columns running ahead through a ring of stages, eight warps split
 //     the raw rows, one warp of the even CTA issues the products (see elect_one: by a thread alone 2 % slower at K = N = 256,
-//     262 144 rows, K = N = 128: 65.0 us and 54.1; 500 009 rows, 256 -> 47: 243 and 198), four warps drain the accumulator of the tile before
-//     (two accumulators of up to 256 columns in tensor memory) and write it with TMA stores.
+//     262 144 rows, K = N = 128: 65.0 us and 54.1; 500 009 rows, 256 -> 47: 243 and 198), four warps drain the accumulator of
+//     the tile before (two accumulators of up to 256 columns in tensor memory) and write it with TMA stores.  (Splitting warps
+//     in two teams with a slice each: no faster, and wrong where the stages are odd in number -- a team that visits a stage
+//     every other time cannot tell the phase before the last from the last.)
 //   * The grid is one pair per two SMs and walks the tiles.
 // The tensor core cuts off what it adds to an accumulator instead of rounding it, so a chain of K / 8 sums drifts (rel.
 // error 2e-6 at K = 256, ten times that of fp32 FMAs).  Widths and depths that the ticket executor's tensor-core tile does
 // not take have always been multiplied with fp32 FMAs; for them the kernel has a second form that is as exact as those from
-// 32 terms on: panels of up to 64 columns, whose four accumulators are read back and added in registers after every slice.
+// 32 terms on: panels of up to 64 columns, whose four accumulators are read back and added in registers after every slice, by eight
+// warps (500 009 rows, 256 -> 47: 193 us with four, 178 with eight, 155 with the split of rg_split, 3.9 TB/s of B and D).
 // Fewer terms are multiplied with FMAs still, by row_fma_kernel.
 // The plain form keeps its chains short where tensor memory has room: up to 128 columns the K steps of a slice go round two
 // accumulators, up to 64 round four, the small products first (K = 256: rel. error 1.9e-6 with one, 8.8e-7 with two, 4.6e-7
-// with four; 262 144 rows, K = N = 64: 30.5 us with four).
+// with four).
 // All waits are bounded: the one that runs out sets the error flag, and every role leaves.
 #include "row_gemm.h"
 
@@ -34,20 +37,21 @@ namespace tfk {
 
 namespace {
 
-constexpr int kRgEpiWarps = 4, kRgSplitWarps = 8;
-constexpr int kRgThreads = 32 * (kRgEpiWarps + kRgSplitWarps + 2);
+__host__ __device__ constexpr int rg_epi_warps(bool precise) { return precise ? 8 : 4; }
+constexpr int kRgSplitWarps = 8;
+__host__ __device__ constexpr int rg_threads(bool precise) { return 32 * (rg_epi_warps(precise) + kRgSplitWarps + 2); }
 constexpr int kRgMaxStages = 5;
-// Slices of B that are on their way to L2 in front of the loads, where a tile has many (2.1 M rows, K = N = 256: 1 085 us
-// without, 1 044 with 3; 8 and 20 are slower than 3; 500 009 rows, 256 -> 47: 234 and 229; where it has four or fewer the
-// request costs 1 to 2 %).
-constexpr int kRgAhead = 3, kRgAheadSlices = 8;
+// Slices of B that are on their way to L2 in front of the loads, where a tile has many or the product is narrow and leaves the
+// loads to bound it (2.1 M rows, K = N = 256: 1 085 us without, 1 044 with 3, 8 and 20 are slower than 3; 262 144 rows, 128 -> 128:
+// 52.8 and 48.5, 64 -> 64: 29.2 and 27.7, with 6 50.5 and 29.9; but 500 009 rows, 100 -> 256: 159 and 166).
+constexpr int kRgAhead = 3, kRgAheadSlices = 8, kRgAheadWidth = 128;
 // Terms from which on the precise form's error is no larger than that of fp32 FMAs (40 000 rows, rel.: 9.2e-8 and 1.03e-7 on
 // uniform operands, 1.02e-7 and 1.03e-7 on normal ones, 6.1e-8 and 8.3e-8 on positive ones; 17 terms: 8.6e-8 and 7.6e-8);
 // shapes of fewer that the tensor-core tile does not take are multiplied with those.
 constexpr int kRgPreciseMinK = 32;
 constexpr int kRgPrecisePanel = 64;  // columns: four accumulators, twice, in 512 columns of tensor memory
 constexpr int kRgSmemMax = 227 * 1024;
-constexpr int kRgEpiBytes = kRgEpiWarps * 2 * 32 * 128;  // two 32 x 32 blocks per warp
+constexpr int kRgEpiBytes = 8 * 32 * 128;  // 32 x 32 blocks: two per warp, one where eight warps drain
 
 struct RgShared {
   unsigned long long raw[kRgMaxStages], ready[kRgMaxStages], empty[kRgMaxStages];
@@ -63,12 +67,25 @@ constexpr int rg_stages(int n) {
 }
 static_assert(rg_stages(256) >= 2, "a full-width tile needs two stages");
 
+// x = hi + lo for the tensor core, which reads the first eleven bits of either.  hi is rounded to them by the addition (its last bits
+// need not be cleared); a NaN may be lost there, but not in lo.  lo is a power of two or has at most twelve bits: if the last of
+// them is set, lo / 2048 carries into the bit before (it is at least one unit there and less than two), if not, what it adds
+// is cut off again, so that lo is rounded like hi.  (Clearing hi, rounding lo like hi and looking for NaNs first took
+// eight instructions of the half-rate integer pipe, which bounded the splitting, instead of two.)
+constexpr float kRgRoundLow = 1.f + 1.f / 2048;
+__device__ __forceinline__ void rg_split(float x, float round_low, float &hi, float &lo) {
+  const unsigned h = __float_as_uint(x) + 0x1000u;
+  hi = __uint_as_float(h);
+  lo = (x - __uint_as_float(h & 0xffffe000u)) * round_low;
+}
+
 // PRECISE: see above; n_pad <= 64.
 // n_pad: columns of W rounded up to 32 (rows of the split weight beyond n_real are zero).
 template <bool PRECISE>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRgThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(rg_threads(PRECISE), 1)
 row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_whi,
                 const __grid_constant__ CUtensorMap tm_wlo, const __grid_constant__ CUtensorMap tm_out, const RowGemmParams P) {
+  constexpr int kRgEpiWarps = rg_epi_warps(PRECISE);
   extern __shared__ char dyn[];
   __shared__ RgShared s;
   char *smem = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~(uintptr_t)1023);
@@ -103,43 +120,49 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
   if (warp == kRgEpiWarps + kRgSplitWarps) {
-    // ---- loads ----
-    if (lane == 0) {
-      int st = 0, issued = 0;
-      unsigned ph = 0;
-      bool ok = true;
-      int pt = pair, psl = 0;
-      auto prefetch = [&]() {
-        if (P.direct || P.n_slices < kRgAheadSlices || pt >= P.tiles) return;
-        const int row = pt * 2 * kTcRows + (int)rank * kTcRows;
-        if (row < P.m)
-          asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"((unsigned long long)&tm_a),
-                       "r"(psl * kTcKSlice), "r"(row) : "memory");
-        if (++psl == P.n_slices) { psl = 0; pt += pairs; }
-      };
-      for (int i = 0; i < kRgAhead; ++i) prefetch();
-      for (int t = pair; t < P.tiles && ok; t += pairs) {
-        const int row = t * 2 * kTcRows + (int)rank * kTcRows;
-        for (int sl = 0; sl < P.n_slices; ++sl) {
-          prefetch();
-          if (issued >= stages && !(ok = pair_wait(&s.empty[st], ph ^ 1u, s.dead, P.wait_limit))) break;
-          char *b = smem + st * stage_bytes;
+    // ---- loads: the whole warp, see elect_one ----
+    int st = 0, issued = 0;
+    unsigned ph = 0;
+    bool ok = true;
+    auto wait = [&](unsigned long long *bar, unsigned parity) {
+      return ok = __all_sync(kFull, pair_wait(bar, parity, s.dead, P.wait_limit));
+    };
+    int pt = pair, psl = 0;
+    const bool ahead = !P.direct && (P.n_slices >= kRgAheadSlices || (P.n_slices > 1 && N <= kRgAheadWidth));
+    auto prefetch = [&]() {
+      if (!ahead || pt >= P.tiles) return;
+      const int row = pt * 2 * kTcRows + (int)rank * kTcRows;
+      if (row < P.m && elect_one())
+        asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"((unsigned long long)&tm_a),
+                     "r"(psl * kTcKSlice), "r"(row) : "memory");
+      __syncwarp();
+      if (++psl == P.n_slices) { psl = 0; pt += pairs; }
+    };
+    for (int i = 0; i < kRgAhead; ++i) prefetch();
+    for (int t = pair; t < P.tiles && ok; t += pairs) {
+      const int row = t * 2 * kTcRows + (int)rank * kTcRows;
+      for (int sl = 0; sl < P.n_slices; ++sl) {
+        prefetch();
+        if (issued >= stages && !wait(&s.empty[st], ph ^ 1u)) break;
+        char *b = smem + st * stage_bytes;
+        if (elect_one()) {
           mbar_expect_tx(&s.raw[st], (unsigned)((P.direct ? 0 : kTcRows * 128) + N * 128));
           if (!P.direct) tma_load_2d(b, &tm_a, sl * kTcKSlice, row, &s.raw[st]);
           tma_load_2d(b + 2 * kTcRows * 128, &tm_whi, sl * kTcKSlice, (int)rank * half, &s.raw[st]);
           tma_load_2d(b + 2 * kTcRows * 128 + half * 128, &tm_wlo, sl * kTcKSlice, (int)rank * half, &s.raw[st]);
-          if (issued < stages) ++issued;
-          if (++st == stages) { st = 0; ph ^= 1u; }
         }
+        __syncwarp();
+        if (issued < stages) ++issued;
+        if (++st == stages) { st = 0; ph ^= 1u; }
       }
-      // the tensor core's arrivals on the stages of this CTA come from the other one too: the last of them must be in before
-      // the CTA may end
-      for (int i = 0; ok && i < issued; ++i) ok = pair_wait(&s.empty[i], i < st ? ph : ph ^ 1u, s.dead, P.wait_limit);
-      // a copy still in flight must not outlive the CTA (only after a wait ran out is one possible)
-      if (s.dead)
-        for (int i = 0; i < issued; ++i)
-          for (int k = 0; k < P.wait_limit && !mbar_wait(&s.raw[i], (i < st ? ph : ph ^ 1u), 1); ++k) {}
     }
+    // the tensor core's arrivals on the stages of this CTA come from the other one too: the last of them must be in before
+    // the CTA may end
+    for (int i = 0; ok && i < issued; ++i) wait(&s.empty[i], i < st ? ph : ph ^ 1u);
+    // a copy still in flight must not outlive the CTA (only after a wait ran out is one possible)
+    if (!ok || s.dead)
+      for (int i = 0; i < issued; ++i)
+        for (int k = 0; k < P.wait_limit && !mbar_wait(&s.raw[i], (i < st ? ph : ph ^ 1u), 1); ++k) {}
   } else if (warp == kRgEpiWarps + kRgSplitWarps + 1) {
     // ---- products (even CTA): the whole warp, see elect_one ----
     if (rank == 0) {
@@ -205,6 +228,8 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   } else if (warp >= kRgEpiWarps) {
     // ---- split the raw rows: hi in place, lo beside it ----
     const int w = tid - 32 * kRgEpiWarps;
+    constexpr int kStep = 32 * kRgSplitWarps, kQuads = kTcRows * 8 / kStep;  // quads of a thread in a slice, from one to the next
+    const float round_low = P.cut_low ? 1.f : kRgRoundLow;
     int st = 0;
     unsigned ph = 0;
     bool ok = true;
@@ -212,14 +237,14 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       for (int sl = 0; sl < P.n_slices; ++sl) {
         if (!(ok = __all_sync(kFull, pair_wait(&s.raw[st], ph, s.dead, P.wait_limit)))) break;  // (the warp leaves as one)
         float4 *hi = reinterpret_cast<float4 *>(smem + st * stage_bytes), *lo = hi + kTcRows * 8;
-        float4 a[kTcRows * 8 / (32 * kRgSplitWarps)];
+        float4 a[kQuads];
         if (!P.direct) {
 #pragma unroll
-          for (int i = 0; i < kTcRows * 8 / (32 * kRgSplitWarps); ++i) a[i] = hi[w + i * 32 * kRgSplitWarps];
+          for (int i = 0; i < kQuads; ++i) a[i] = hi[w + i * kStep];
         } else {  // rows that TMA cannot read: the same quads of the swizzled tile, value by value
 #pragma unroll
-          for (int i = 0; i < kTcRows * 8 / (32 * kRgSplitWarps); ++i) {
-            const int q = w + i * 32 * kRgSplitWarps, r = q >> 3, row = t * 2 * kTcRows + (int)rank * kTcRows + r;
+          for (int i = 0; i < kQuads; ++i) {
+            const int q = w + i * kStep, r = q >> 3, row = t * 2 * kTcRows + (int)rank * kTcRows + r;
             const int k = sl * kTcKSlice + ((q & 7) ^ (r & 7)) * 4;
             const float *x = P.x + (size_t)row * P.ld_x + k;
             const bool in = row < P.m;
@@ -228,13 +253,12 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           }
         }
 #pragma unroll
-        for (int i = 0; i < kTcRows * 8 / (32 * kRgSplitWarps); ++i) {
-          const float4 x = a[i];
-          const float4 h = make_float4(tf32_round(x.x), tf32_round(x.y), tf32_round(x.z), tf32_round(x.w));
-          hi[w + i * 32 * kRgSplitWarps] = h;
-          float4 l = make_float4(x.x - h.x, x.y - h.y, x.z - h.z, x.w - h.w);
-          if (!P.cut_low) l = make_float4(tf32_round(l.x), tf32_round(l.y), tf32_round(l.z), tf32_round(l.w));
-          lo[w + i * 32 * kRgSplitWarps] = l;
+        for (int i = 0; i < kQuads; ++i) {
+          float4 h, l;
+          rg_split(a[i].x, round_low, h.x, l.x); rg_split(a[i].y, round_low, h.y, l.y);
+          rg_split(a[i].z, round_low, h.z, l.z); rg_split(a[i].w, round_low, h.w, l.w);
+          hi[w + i * kStep] = h;
+          lo[w + i * kStep] = l;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read next by the tensor core
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -243,11 +267,12 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         if (++st == stages) { st = 0; ph ^= 1u; }
       }
   } else {
-    // ---- drain: warp w holds the rows 32 w .. 32 w + 31 of the CTA's half of the tile ----
+    // ---- drain: warp w holds the rows 32 (w % 4) .. + 31 of the CTA's half of the tile (PRECISE: 32 columns of them) ----
+    const int quadrant = warp & 3, side = warp >> 2;
     int buf = 0, eb = 0;
     unsigned acc_ph = 0;
     bool ok = true;
-    const unsigned lanes = s.tmem_base + ((unsigned)(warp * 32) << 16);
+    const unsigned lanes = s.tmem_base + ((unsigned)(quadrant * 32) << 16);
     auto release = [&]() {  // the accumulator has been read: its next use may overwrite it
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -278,8 +303,9 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 #pragma unroll
       for (int q = 0; q < 32; ++q) v[q] = P.relu ? fmaxf(x[q], 0.f) : x[q];
       if (P.tma_store) {
-        float4 *blk = reinterpret_cast<float4 *>(epi + (warp * 2 + eb) * 4096);
-        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the store before the last has left the buffer
+        float4 *blk = reinterpret_cast<float4 *>(epi + (PRECISE ? warp : warp * 2 + eb) * 4096);
+        if (PRECISE) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the store before has left the buffer
+        else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");          // (there are two)
         __syncwarp();
 #pragma unroll
         for (int q = 0; q < 8; ++q) blk[lane * 8 + (q ^ (lane & 7))] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
@@ -289,7 +315,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0)
+        if (elect_one())
           asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
                            (unsigned long long)&tm_out), "r"(smem_u32(blk)), "r"(c), "r"(row0) : "memory");
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -303,35 +329,30 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       }
     };
     for (int t = pair; t < P.tiles && ok; t += pairs) {
-      const int row0 = t * 2 * kTcRows + (int)rank * kTcRows + warp * 32;
+      const int row0 = t * 2 * kTcRows + (int)rank * kTcRows + quadrant * 32;
       if (PRECISE) {
-        float acc[2][32];
+        float acc[32];
 #pragma unroll
-        for (int q = 0; q < 32; ++q) acc[0][q] = acc[1][q] = 0.f;
+        for (int q = 0; q < 32; ++q) acc[q] = 0.f;
         for (int sl = 0; sl < P.n_slices; ++sl) {
           if (!(ok = __all_sync(kFull, pair_wait(&s.acc_full[buf], acc_ph, s.dead, P.wait_limit)))) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (h * 32 >= N) break;
+          if (side * 32 < N) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               float a[32];
-              tmem_load32(a, lanes + (unsigned)(buf * 256 + j * 64 + h * 32));
+              tmem_load32(a, lanes + (unsigned)(buf * 256 + j * 64 + side * 32));
               asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
               tmem_loaded(a);
 #pragma unroll
-              for (int q = 0; q < 32; ++q) acc[h][q] += a[q];
+              for (int q = 0; q < 32; ++q) acc[q] += a[q];
             }
           }
           release();
           next();
         }
         if (!ok) break;
-        if (row0 < P.m) {
-          put(acc[0], 0, row0);
-          if (P.n_real > 32) put(acc[1], 32, row0);
-        }
+        if (row0 < P.m && side * 32 < P.n_real) put(acc, side * 32, row0);
       } else {
         if (!(ok = __all_sync(kFull, pair_wait(&s.acc_full[buf], acc_ph, s.dead, P.wait_limit)))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -496,7 +517,7 @@ static int launch_panel(const float *X, int m, int K, int ld_x, const float *W, 
   // for one another)
   cudaError_t e = cudaFuncSetAttribute((const void *)f, cudaFuncAttributeMaxDynamicSharedMemorySize, kRgSmemMax - 1024);
   if (e == cudaSuccess) {
-    f<<<2 * std::max(1, std::min(P.tiles, sm_count / 2)), kRgThreads, smem, s>>>(ma, mh, ml, mo, P);
+    f<<<2 * std::max(1, std::min(P.tiles, sm_count / 2)), rg_threads(precise), smem, s>>>(ma, mh, ml, mo, P);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) return tf::fail(TF_ERR_CUDA, std::string("row_gemm: ") + cudaGetErrorString(e));
