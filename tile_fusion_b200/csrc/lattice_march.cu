@@ -188,6 +188,15 @@ struct Shared {
   volatile int *abort;
 };
 
+// One lane of a converged warp (see elect_one in gemm_tc.cuh).
+__device__ __forceinline__ bool elect_lane() {
+  unsigned p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void mbar_arrive(unsigned bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -249,7 +258,7 @@ __device__ __forceinline__ void patch_plane(unsigned cb, int x0, int y0, int c0c
 struct CtaState {
   unsigned n_fix;  // planes patched so far: phases of fixbar
   unsigned n_use;  // steps taken so far: step n uses C stage n % stages (parity of n / stages) and phase n of tbar
-  unsigned n_iss;  // plane loads issued so far (kept by thread 0, which issues them)
+  unsigned n_iss;  // plane loads issued so far (kept by the first warp, which issues them)
 };
 
 // Rows of the ring of T around the tile that one 4-lane group computes besides its patch.
@@ -263,8 +272,8 @@ template <bool ODD>
 __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParams &P, const Shared &S, CtaState &cs,
                                          int x0, int y0, int zs, int ze, int c0col, int x, int y, bool ring,
                                          const int (&rx)[kRing], const int (&ry)[kRing], bool pair_x,
-                                         const volatile int *next, int &prefetched) {
-  const int tid = threadIdx.x, lane = tid & 31, c4 = lane & 3;
+                                         const volatile int *next, int &prefetched, bool loader) {
+  const int lane = threadIdx.x & 31, c4 = lane & 3;
   const int kfirst = zs - lead_in(zs, P), steps = ze - kfirst + 2;
   // byte offset of the patch's first y-row (at pi * 64 bytes into it, lane's 16 bytes included) in the C rectangle
   // (two points of rim: R0 = 2) and in the T rectangle (one point: R0 = 1)
@@ -419,20 +428,23 @@ __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParam
     // When this item has no such plane left, the stage takes a plane of the CTA's next item (thread 0 knows
     // it: next[] = {valid, x0, y0, first plane, first column}), so the stream of copies does not stop between
     // items.
-    if (step > 0 && tid == 0) {
+    if (step > 0 && loader) {
       const unsigned prev_stage = (cs.n_use - 1) % kMarchStages;
       const int ahead = step - 1 + kMarchStages;
-      if (ahead < steps) {
-        ++cs.n_iss;
-        mbar_expect_tx(S.full + 8 * prev_stage, kMarchCBytes);
-        load_plane<ODD>(S.cbuf + prev_stage * kMarchCBytes, tm_c, c0col, x0 / 2 - 1, y0 - 2, kfirst + ahead + P.z_shift,
-                   S.full + 8 * prev_stage, P);
-      } else if (steps >= kMarchStages && next[0]) {   // (a shorter item left stages unarmed: no hand-over)
-        ++cs.n_iss;
+      int lc = c0col, lx = x0, ly = y0, lz = kfirst + ahead;
+      bool go = ahead < steps;
+      if (!go && steps >= kMarchStages && next[0]) {   // (a shorter item left stages unarmed: no hand-over)
+        go = true;
         ++prefetched;
-        mbar_expect_tx(S.full + 8 * prev_stage, kMarchCBytes);
-        load_plane<ODD>(S.cbuf + prev_stage * kMarchCBytes, tm_c, next[4], next[1] / 2 - 1, next[2] - 2,
-                   next[3] + (ahead - steps) + P.z_shift, S.full + 8 * prev_stage, P);
+        lc = next[4]; lx = next[1]; ly = next[2]; lz = next[3] + (ahead - steps);
+      }
+      if (go) {
+        ++cs.n_iss;
+        if (elect_lane()) {
+          mbar_expect_tx(S.full + 8 * prev_stage, kMarchCBytes);
+          load_plane<ODD>(S.cbuf + prev_stage * kMarchCBytes, tm_c, lc, lx / 2 - 1, ly - 2, lz + P.z_shift, S.full + 8 * prev_stage, P);
+        }
+        __syncwarp();
       }
     }
     // D(k-1): everything but the z+ product, from T(k-2) (registers), T(k-1) (registers and neighbours)
@@ -476,7 +488,8 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   S.tbar = S.full + 8 * kMarchStages;
   S.fixbar = S.tbar + 8;
   S.abort = &ctl[1];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const bool loader = warp == 0;  // the warp that asks for the planes
 
   if (tid == 0) {
     for (int s = 0; s < kMarchStages; ++s) mbar_init(S.full + 8 * s, 1);
@@ -537,11 +550,14 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
     const int4 ia = __ldg(P.items + 2 * it), ib = __ldg(P.items + 2 * it + 1);
     const int x0 = ia.x, y0 = ia.y, zs = ia.z, ze = ia.w, c0col = ib.x;
     const int kfirst = zs - lead_in(zs, P), steps = ze - kfirst + 2;
-    if (tid == 0) {
+    if (loader) {
       for (int s = pre; s < min(kMarchStages, steps); ++s) {
         const unsigned stage = (cs.n_use + s) % kMarchStages;
-        mbar_expect_tx(S.full + 8 * stage, kMarchCBytes);
-        load_plane<ODD>(S.cbuf + stage * kMarchCBytes, maps, c0col, x0 / 2 - 1, y0 - 2, kfirst + s + P.z_shift, S.full + 8 * stage, P);
+        if (elect_lane()) {
+          mbar_expect_tx(S.full + 8 * stage, kMarchCBytes);
+          load_plane<ODD>(S.cbuf + stage * kMarchCBytes, maps, c0col, x0 / 2 - 1, y0 - 2, kfirst + s + P.z_shift, S.full + 8 * stage, P);
+        }
+        __syncwarp();
       }
       cs.n_iss = cs.n_use + min(kMarchStages, steps);
       pre = 0;
@@ -549,7 +565,7 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
     int rx[kRing], ry[kRing];
 #pragma unroll
     for (int r = 0; r < kRing; ++r) { rx[r] = x0 + rdx[r]; ry[r] = y0 + rdy[r]; }
-    if (!run_item<ODD>(maps, P, S, cs, x0, y0, zs, ze, c0col, x0 + 2 * pi, y0 + 2 * warp, ring, rx, ry, warp < 2, nxt, pre)) { failed = true; break; }
+    if (!run_item<ODD>(maps, P, S, cs, x0, y0, zs, ze, c0col, x0 + 2 * pi, y0 + 2 * warp, ring, rx, ry, warp < 2, nxt, pre, loader)) { failed = true; break; }
   }
   if (failed && tid == 0) atomicExch(&P.st->error, 1);
   // A thread that gave up has raised the CTA's abort flag; the others notice it in their own bounded waits
