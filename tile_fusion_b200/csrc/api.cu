@@ -1467,12 +1467,10 @@ int run_gather(const DevGather &g, const float *X, int ld_in, bool vec_in, float
     P.partial = (float *)((char *)scratch + g.scratch_counters());
     TF_CUDA(cudaMemsetAsync(scratch, 0, g.cnt.n * sizeof(int), s));
   }
-  const int group = tfk::gather_group(n_cols);
-  P.panel_w = vec_in ? 4 * group : 128;
   P.relu = relu ? 1 : 0;
   if (unit_end >= 0) { P.units += unit_begin; P.n_units = unit_end - unit_begin; }
   else TF_CUDA(tfk::launch_rows_fix(g.empty.p, g.n_empty, ld_out, Y, false, s));
-  TF_CUDA(tfk::launch_gather(group, vec_in, vec_out, P, s));
+  TF_CUDA(tfk::launch_gather(vec_in, vec_out, P, s));
   return TF_OK;
 }
 
@@ -1566,7 +1564,7 @@ int tf_plan_sddmm_spmm(const tf_csr *A, int kq, int nv, const tf_plan_opts *opts
   p->m = A->m; p->n_cols = nv; p->k_dim = kq;
   if (tfk::sddmm_gather_supported(kq, nv) && o.rows_per_block == 0 && o.ctas_per_sm == 0) {
     p->second.m = A->m; p->second.n = A->n;
-    rc = p->g_second.build(*A, 4 * tfk::sddmm_group(kq, nv), nv, sm_count, false, tfk::kSddmmResident);  // (units for groups of that size)
+    rc = p->g_second.build(*A, 4 * tfk::sddmm_group(kq, nv), nv, sm_count, false, tfk::sddmm_resident(kq, nv));  // (units for groups of that size)
     if (rc == TF_OK) rc = zero_state(*p);
     if (rc != TF_OK) return rc;
     *out = p.release();

@@ -19,7 +19,8 @@
 //
 // Measured (R-MAT, n = 200 000, degree 20, both products of a chain): 64 columns 180 us (11.9 TB/s of row reads), where
 // the ticket executor took 784 (58 % of its warps' time at barriers behind long rows); 128 columns 306 us, 14 TB/s, which
-// is what L2 gives.  Eight reads in flight and three CTAs per SM: four CTAs spill (229 us), four reads and five CTAs 193.
+// is what L2 gives.  Eight reads in flight and 24 warps per SM: 32 warps spill (229 us), four reads and 40 warps 193; in CTAs of 128
+// threads, which end earlier than those of 256: 100 columns (n = 500 009, degree 25) 443 -> 428 us, 48 242 -> 236.
 #include <algorithm>
 
 #include "gather.h"
@@ -29,22 +30,23 @@ namespace tfk {
 
 namespace {
 
-constexpr int kGatherThreads = 256;
+constexpr int kGatherThreads = 128, kGatherCtas = kGatherResident / kGatherThreads;
 constexpr int kBatch = tf::kGatherBatch;
 
-// Four columns of one lane: contiguous (VEC) or 32 apart, the last of them clamped to the last column that exists.
-template <bool VEC>
-__device__ __forceinline__ float4 load_quad(const float *p, int e1, int e2, int e3) {
+// The columns of one lane: four in a row (VEC), or E of them at the offsets `at`, those that do not exist clamped to one that does.
+template <bool VEC, int E>
+__device__ __forceinline__ float4 load_quad(const float *p, const int (&at)[4]) {
   if (VEC) return __ldg(reinterpret_cast<const float4 *>(p));
-  return make_float4(__ldg(p), __ldg(p + e1), __ldg(p + e2), __ldg(p + e3));
+  return make_float4(__ldg(p), E > 1 ? __ldg(p + at[1]) : 0.f, E > 2 ? __ldg(p + at[2]) : 0.f, E > 3 ? __ldg(p + at[3]) : 0.f);
 }
 __device__ __forceinline__ void fma_quad(float4 &a, float v, const float4 &x) {
   a.x = fmaf(v, x.x, a.x); a.y = fmaf(v, x.y, a.y); a.z = fmaf(v, x.z, a.z); a.w = fmaf(v, x.w, a.w);
 }
 
-// G: lanes per group.  VIN: rows of X are read as float4.  VOUT: rows of the result are written as float4.
-template <int G, bool VIN, bool VOUT>
-__global__ void __launch_bounds__(kGatherThreads, 3) gather_kernel(const GatherParams P) {
+// G: lanes per group.  VIN: rows of X are read as float4, else E columns per lane, G apart.  VOUT: rows of the result are written
+// as float4.
+template <int G, bool VIN, bool VOUT, int E = 4>
+__global__ void __launch_bounds__(kGatherThreads, kGatherCtas) gather_kernel(const GatherParams P) {
   static_assert(!VOUT || VIN, "strided columns are stored one by one");
   const int lane = threadIdx.x & (G - 1);
   const int panel = blockIdx.x / P.unit_blocks;
@@ -53,9 +55,9 @@ __global__ void __launch_bounds__(kGatherThreads, 3) gather_kernel(const GatherP
   const int c0 = panel * P.panel_w, c1 = min(P.n_cols, c0 + P.panel_w);
   // A lane without a column of its own reads the last one again instead of branching around every load.
   const int own = c0 + (VIN ? lane * 4 : lane);
-  const int left = c1 - own;  // columns of this lane that exist (VIN: from `own` on; else element e while 32 * e < left)
+  const int left = c1 - own;  // columns of this lane that exist (VIN: from `own` on; else element e while G * e < left)
   const int col = left > 0 ? own : (VIN ? (c1 - 1) & ~3 : c1 - 1);
-  const int e1 = 32 < left ? 32 : 0, e2 = 64 < left ? 64 : 0, e3 = 96 < left ? 96 : 0;
+  const int at[4] = {0, G < left ? G : 0, 2 * G < left ? 2 * G : 0, 3 * G < left ? 3 * G : 0};
   const int4 u = __ldg(P.units + unit);
   const bool piece = u.w >= 0;
   const float *src = P.dense + col;
@@ -70,14 +72,14 @@ __global__ void __launch_bounds__(kGatherThreads, 3) gather_kernel(const GatherP
 
   auto put = [&](float *o, bool clamp) {
     if (clamp) { acc.x = fmaxf(acc.x, 0.f); acc.y = fmaxf(acc.y, 0.f); acc.z = fmaxf(acc.z, 0.f); acc.w = fmaxf(acc.w, 0.f); }
-    constexpr int d = VIN ? 1 : 32;
+    constexpr int d = VIN ? 1 : G;
     if (VOUT) {
       if (left > 0) *reinterpret_cast<float4 *>(o) = acc;
     } else {
       if (0 < left) o[0] = acc.x;
-      if (d < left) o[d] = acc.y;
-      if (2 * d < left) o[2 * d] = acc.z;
-      if (3 * d < left) o[3 * d] = acc.w;
+      if (E > 1 && d < left) o[d] = acc.y;
+      if (E > 2 && 2 * d < left) o[2 * d] = acc.z;
+      if (E > 3 && 3 * d < left) o[3 * d] = acc.w;
     }
   };
 
@@ -96,7 +98,7 @@ __global__ void __launch_bounds__(kGatherThreads, 3) gather_kernel(const GatherP
     }
     float4 x[kBatch];
 #pragma unroll
-    for (int q = 0; q < kBatch; ++q) x[q] = load_quad<VIN>(src + (size_t)(unsigned)(c[q] & 0x7fffffff) * ld_in, e1, e2, e3);
+    for (int q = 0; q < kBatch; ++q) x[q] = load_quad<VIN, E>(src + (size_t)(unsigned)(c[q] & 0x7fffffff) * ld_in, at);
     pc += kBatch / 4;
 #pragma unroll
     for (int q = 0; q < kBatch / 4; ++q) {
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(kGatherThreads, 3) gather_kernel(const GatherP
 #pragma unroll
     for (int q = 0; q < kBatch; ++q) {
       const float *o = ps + (size_t)min(s + q, h.z - 1) * P.partial_ld;
-      x[q] = VIN ? __ldcg(reinterpret_cast<const float4 *>(o)) : make_float4(__ldcg(o), __ldcg(o + e1), __ldcg(o + e2), __ldcg(o + e3));
+      x[q] = VIN ? __ldcg(reinterpret_cast<const float4 *>(o)) : make_float4(__ldcg(o), __ldcg(o + at[1]), __ldcg(o + at[2]), __ldcg(o + at[3]));
     }
 #pragma unroll
     for (int q = 0; q < kBatch; ++q)
@@ -158,20 +160,38 @@ typedef void (*GatherFn)(const GatherParams);
 template <int G>
 GatherFn pick(bool vec_out) { return vec_out ? gather_kernel<G, true, true> : gather_kernel<G, true, false>; }
 
+// Rows read value by value: the lanes of a group and the columns of a lane, so that the fewest reads are made (a read brings G
+// columns of 32 / G rows), with as few lanes as that allows.  (R-MAT n = 500 009, degree 25: 7 columns 493 us as 32 x 4, where columns that
+// do not exist are read too, 106 like this; 31: 502 and 238, with 32 lanes 273; 47: 514 and 277; 57: 521 and 332, with 32 lanes 360.)
+struct Single {
+  int width, group;
+  GatherFn f;
+};
+const Single kSingles[] = {{8, 8, gather_kernel<8, false, false, 1>},    {16, 8, gather_kernel<8, false, false, 2>},
+                           {24, 8, gather_kernel<8, false, false, 3>},   {32, 8, gather_kernel<8, false, false, 4>},
+                           {48, 16, gather_kernel<16, false, false, 3>}, {64, 16, gather_kernel<16, false, false, 4>},
+                           {96, 32, gather_kernel<32, false, false, 3>}, {128, 32, gather_kernel<32, false, false, 4>}};
+
 }  // namespace
 
 // (R-MAT n = 500 000, degree 25, 32 columns: 377 us with 8 lanes, 703 with 16, 1 018 with 32.)
 int gather_group(int n_cols) { return n_cols <= 32 ? 8 : (n_cols <= 64 ? 16 : 32); }
 
-cudaError_t launch_gather(int group, bool vec_in, bool vec_out, const GatherParams &p, cudaStream_t s) {
+cudaError_t launch_gather(bool vec_in, bool vec_out, const GatherParams &p, cudaStream_t s) {
   if (p.n_units <= 0) return cudaSuccess;
   GatherFn f;
-  if (!vec_in) { f = gather_kernel<32, false, false>; group = 32; }
-  else if (group == 8) f = pick<8>(vec_out);
+  GatherParams q = p;
+  int group = gather_group(p.n_cols);
+  q.panel_w = vec_in ? 4 * group : 128;
+  if (!vec_in) {
+    const Single *w = kSingles;
+    while (w->width < std::min(p.n_cols, 128)) ++w;
+    f = w->f;
+    group = w->group;
+  } else if (group == 8) f = pick<8>(vec_out);
   else if (group == 16) f = pick<16>(vec_out);
   else f = pick<32>(vec_out);
-  GatherParams q = p;
-  q.panels = (p.n_cols + p.panel_w - 1) / p.panel_w;
+  q.panels = (p.n_cols + q.panel_w - 1) / q.panel_w;
   q.unit_blocks = (p.n_units + kGatherThreads / group - 1) / (kGatherThreads / group);
   f<<<q.unit_blocks * q.panels, kGatherThreads, 0, s>>>(q);
   return cudaGetLastError();

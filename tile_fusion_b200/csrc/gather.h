@@ -46,7 +46,6 @@ size_t fill_gather_entries(const GatherPlan &g, int m, const int *ap, const int 
 namespace tfk {
 
 constexpr int kGatherResident = 768;  // threads of the gather kernel resident per SM
-constexpr int kSddmmResident = 512;   // and of the SDDMM kernel
 
 struct GatherParams {
   const int *cols;      // column | end bit
@@ -60,18 +59,19 @@ struct GatherParams {
   float *out;
   int ld_in, ld_out, partial_ld;
   int n_cols;           // columns computed
-  int panel_w, panels;  // columns per pass over the units (four per lane of a group)
-  int n_units, unit_blocks;
+  int n_units;
+  int panel_w, panels, unit_blocks;  // (filled in by the launcher) columns per pass over the units, ...
   int relu;
 };
 
 // Lanes per group for a dense width: each lane owns four columns.
 int gather_group(int n_cols);
 // vec_in / vec_out: rows of X / of the result start on 16-byte boundaries.
-cudaError_t launch_gather(int group, bool vec_in, bool vec_out, const GatherParams &p, cudaStream_t s);
+cudaError_t launch_gather(bool vec_in, bool vec_out, const GatherParams &p, cudaStream_t s);
 // D = (A .* (Q K^T)) V over the same units (sddmm_gather.cu): V is p.dense, D p.out, both of n_cols columns; m rows of Q.
 bool sddmm_gather_supported(int kq, int nv);  // both up to 128
 int sddmm_group(int kq, int nv);              // lanes that work on a unit
+int sddmm_resident(int kq, int nv);           // threads of the kernel resident per SM
 cudaError_t launch_sddmm_gather(const GatherParams &p, const float *Q, const float *K, int kq, int m, cudaStream_t s);
 // dst[r][0:ld] = src[r][0:n_cols], the rest zero: rows of a width that is no multiple of four made readable as float4.
 cudaError_t launch_pad_rows(const float *src, long long rows, int n_cols, int ld, float *dst, cudaStream_t s);
