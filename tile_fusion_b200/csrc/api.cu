@@ -772,14 +772,15 @@ int run_band(tf_plan &p, const float *C, float *D, int block_begin, int block_en
   if (!(aligned(C, 16) && aligned(D, 16)))
     return fail(TF_ERR_ARG, "this plan reads rows as 16-byte vectors and needs 16-byte aligned dense operands "
                             "(build the plan with tile_slots < 0 otherwise)");
-  CUtensorMap tm;
+  CUtensorMap tm, tm_d;
   TF_TRY(tfk::band_make_map(&tm, C, p.m, p.n_cols, p.band.block));
+  TF_TRY(tfk::band_make_map(&tm_d, D, p.m, p.n_cols, 32));
   tfk::BandParams P = p.band.par;
   P.out = D;
   P.error = &p.state.p->error;
   P.wait_limit = p.spin_limit;
   P.block_begin = block_begin; P.block_end = block_end;
-  TF_CUDA(tfk::launch_band_march(tm, p.band.block, P, p.sm_count, s));
+  TF_CUDA(tfk::launch_band_march(tm, tm_d, p.band.block, P, p.sm_count, s));
   p.launches = 1;
   return TF_OK;
 }
@@ -1597,7 +1598,7 @@ int tf_plan_info(const tf_plan *p, long long info[8]) {
   info[4] = p->march.on ? p->march.grid : (p->pipe ? p->pipe_grid : p->grid);
   info[5] = p->march.on         ? tfk::kMarchThreads
             : p->lines.on       ? 32 * tfk::kLineWarps
-            : p->band.block     ? tfk::kBandThreads
+            : p->band.block     ? tfk::band_threads(p->band.block, p->band.par, p->sm_count)
             : p->one.on && !p->keep_t ? tfk::kSpmmGemmThreads
             : p->pipe           ? 672
             : p->g_second.on    ? tfk::kThreads

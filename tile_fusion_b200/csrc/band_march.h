@@ -35,13 +35,15 @@ struct BandParams {
   bool same;                   // one operator on both sides: quads_f is read for both products
 };
 
-// Tensor map of C: boxes of 32 columns x `block` rows.
+// Tensor map of C (of D): boxes of 32 columns x `block` rows.
 int band_make_map(CUtensorMap *out, const float *c, long long rows, int n_cols, int block);
 constexpr int kBandThreads = 512;
 // Shared memory of the kernel for these widths; plans whose operators need more than kBandSmemMax are not made.
 constexpr int kBandSmemMax = 226 * 1024;
 size_t band_smem(int block, int pairs_f, int pairs_a, bool same);
-// Fills in chunks, blocks and seg_blocks and launches.
-cudaError_t launch_band_march(const CUtensorMap &tm_c, int block, BandParams &p, int sm_count, cudaStream_t s);
+// Threads per CTA of the kernel that a plan runs on.
+int band_threads(int block, const BandParams &p, int sm_count);
+// Fills in chunks, blocks and seg_blocks and launches; tm_d: the map of D with boxes of 32 rows.
+cudaError_t launch_band_march(const CUtensorMap &tm_c, const CUtensorMap &tm_d, int block, BandParams &p, int sm_count, cudaStream_t s);
 
 }  // namespace tfk
