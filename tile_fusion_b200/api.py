@@ -36,6 +36,14 @@ def _f32(a):
     return np.ascontiguousarray(a, dtype=np.float32)
 
 
+def _ptr(a: np.ndarray) -> int:
+    """a.ctypes.data, which takes three times as long to say so (a read-only or empty array has to)."""
+    try:
+        return C.addressof(C.c_char.from_buffer(a))
+    except (TypeError, ValueError):
+        return a.ctypes.data
+
+
 class CSRMatrix:
     """CSRMatrix(M, N, Ap, Ai, Ax) -- README.md:37.  Host arrays, int32 / fp32, not copied if already so."""
 
@@ -60,10 +68,9 @@ class CSRMatrix:
         arrays refilled in place, get a new plan.  A change that touches none of the sampled entries is not seen:
         make a new CSRMatrix for new values."""
         nnz = self.nnz
-        step = max(1, nnz // 2048)
-        ai, ax = self.Ai.ctypes.data, self.Ax.ctypes.data
-        h = _lib.lib().tf_csr_checksum(ai, ax, nnz, step)
-        return self.M, self.N, nnz, h >> 32, h & 0xffffffff, self.Ap.ctypes.data, ai, ax
+        ap, ai, ax = _ptr(self.Ap), _ptr(self.Ai), _ptr(self.Ax)
+        h = _lib.lib().tf_csr_checksum(ai, ax, nnz, nnz // 2048 or 1)
+        return self.M, self.N, nnz, h >> 32, h & 0xffffffff, ap, ai, ax
 
 
 class Matrix:
@@ -184,9 +191,18 @@ def inspector(A: CSRMatrix, NumThreads: int, params: ScheduleParameters | None =
     return FusedSchedule(h.value, p)
 
 
+_torch = None
+
+
 def _stream_ptr():
-    import torch
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device, as torch.cuda.current_stream() gives it (which takes 3 us to say so)."""
+    global _torch
+    if _torch is None:
+        import torch
+        _torch = torch
+    if not _torch.cuda.is_initialized():
+        return _torch.cuda.current_stream().cuda_stream
+    return _torch._C._cuda_getCurrentRawStream(_torch._C._cuda_getDevice())
 
 
 class Plan:

@@ -178,19 +178,24 @@ extern "C" int tf_read_dense_mtx(const char *path, int *rows, int *cols, float *
   return TF_OK;
 }
 
-// Sampled checksum of a matrix: every step-th column id and value, in order.  Four chains, because one would wait for its
+// Sampled checksum of a matrix: every step-th column id and value, in order.  Eight chains, because one would wait for its
 // multiplications.
 extern "C" unsigned long long tf_csr_checksum(const int *ai, const float *ax, long long nnz, long long step) {
-  unsigned long long h[4] = {0x9E3779B97F4A7C15ull, 0xC2B2AE3D27D4EB4Full, 0x165667B19E3779F9ull, 0x27D4EB2F165667C5ull};
+  constexpr int kChains = 8;
+  unsigned long long h[kChains] = {0x9E3779B97F4A7C15ull, 0xC2B2AE3D27D4EB4Full, 0x165667B19E3779F9ull, 0x27D4EB2F165667C5ull,
+                                   0x85EBCA77C2B2AE63ull, 0xA0761D6478BD642Full, 0xE7037ED1A0B428DBull, 0x8EBC6AF09C88C6E3ull};
   if (!ai || !ax || step < 1) return 0;
-  int lane = 0;
-  for (long long j = 0; j < nnz; j += step, lane = (lane + 1) & 3) {
+  auto add = [&](int chain, long long j) {
     unsigned v;
     std::memcpy(&v, ax + j, 4);
     const unsigned long long w = (unsigned long long)(unsigned)ai[j] << 32 | v;
-    h[lane] = (h[lane] ^ w) * 0xBF58476D1CE4E5B9ull;
-    h[lane] ^= h[lane] >> 29;
-  }
+    h[chain] = (h[chain] ^ w) * 0xBF58476D1CE4E5B9ull;
+    h[chain] ^= h[chain] >> 29;
+  };
+  long long j = 0;
+  for (; j + (kChains - 1) * step < nnz; j += kChains * step)
+    for (int c = 0; c < kChains; ++c) add(c, j + c * step);
+  for (int c = 0; j < nnz; ++c, j += step) add(c, j);
   unsigned long long s = (unsigned long long)nnz;
   for (unsigned long long x : h) s = (s ^ x) * 0x94D049BB133111EBull, s ^= s >> 31;
   return s;
