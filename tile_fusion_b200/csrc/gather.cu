@@ -17,10 +17,17 @@
 // Products of a row are added in CSR order with fused multiply-adds from zero, as in the reference's row loop
 // (SpMM_SpMM.cpp:211-248); only rows that were cut are added in pieces.
 //
-// Measured (R-MAT, n = 200 000, degree 20, both products of a chain): 64 columns 180 us (11.9 TB/s of row reads), where
-// the ticket executor took 784 (58 % of its warps' time at barriers behind long rows); 128 columns 306 us, 14 TB/s, which
-// is what L2 gives.  Eight reads in flight and 24 warps per SM: 32 warps spill (229 us), four reads and 40 warps 193; in CTAs of 128
-// threads, which end earlier than those of 256: 100 columns (n = 500 009, degree 25) 443 -> 428 us, 48 242 -> 236.
+// A CTA is one warp.  Where a group is a whole warp (more than 64 columns) the entries are then the CTA's, so they and the addresses
+// of the rows are worked out once by the uniform datapath and not by every lane; and a warp that has finished makes room for the
+// next whatever its neighbours do.
+//
+// Measured (R-MAT, n = 500 009, degree 25, one product): 128 columns 383 us (17 TB/s of row reads, 15 % of them from L1), 100 columns
+// 368, in CTAs of four warps 440 and 428, of eight 454 and 443; 64 columns 242, 48 columns 237 (a row costs its 128-byte lines, whole
+// or not).  n = 200 000, degree 20, 64 columns, both products of a chain: 175 us, the ticket executor took 784 (58 % of its warps'
+// time at barriers behind long rows).
+// Eight reads in flight and 24 warps per SM: 28 warps 376 at 100 columns and slower at small sizes, 32 spill (307 at 64 columns); four
+// reads and 40 warps, or asking for half a batch again as soon as it has been added up (569 at 100 columns), are slower, and so are 32
+// lanes of two columns each for up to 64 (272; sixteen in flight 327).
 #include <algorithm>
 
 #include "gather.h"
@@ -30,7 +37,7 @@ namespace tfk {
 
 namespace {
 
-constexpr int kGatherThreads = 128, kGatherCtas = kGatherResident / kGatherThreads;
+constexpr int kGatherThreads = 32, kGatherCtas = kGatherResident / kGatherThreads;
 constexpr int kBatch = tf::kGatherBatch;
 
 // The columns of one lane: four in a row (VEC), or E of them at the offsets `at`, those that do not exist clamped to one that does.
