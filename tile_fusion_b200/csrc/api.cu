@@ -581,11 +581,12 @@ bool aligned(const void *q, size_t a);
 int run_march(tf_plan &p, const float *C, float *D, int item_begin, int item_end, bool with_halo, cudaStream_t s) {
   tf_plan::March &M = p.march;
   if (item_end <= item_begin) { p.launches = 0; return TF_OK; }
-  CUtensorMap tm, tm_last;
+  CUtensorMap tm, tm_odd;
   const bool odd = M.nx % 2 != 0;
-  int mr = tfk::march_make_map(&tm, C, p.n_cols, M.nx, M.ny, M.ny, odd ? M.planes_c - 1 : M.planes_c);
-  tm_last = tm;
-  if (odd && mr == 0) mr = tfk::march_make_map(&tm_last, C + (size_t)(M.nz - 1) * M.nx * M.ny * p.n_cols, p.n_cols, M.nx, M.ny, M.ny - 1, 1);
+  int mr = odd ? tfk::march_make_half_map(&tm, C, p.n_cols, M.nx, M.ny, M.planes_c, 0)
+               : tfk::march_make_map(&tm, C, p.n_cols, M.nx, M.ny, M.ny, M.planes_c);
+  tm_odd = tm;
+  if (odd && mr == 0) mr = tfk::march_make_half_map(&tm_odd, C, p.n_cols, M.nx, M.ny, M.planes_c, 1);
   if (mr != 0) return fail(TF_ERR_CUDA, "cuTensorMapEncodeTiled failed for the dense operand (code " + std::to_string(mr) + ")");
   tfk::MarchParams Q;
   std::memset(&Q, 0, sizeof(Q));
@@ -599,7 +600,6 @@ int run_march(tf_plan &p, const float *C, float *D, int item_begin, int item_end
   Q.st = M.st.p + (with_halo ? 1 : 0);
   Q.nx = M.nx; Q.ny = M.ny; Q.nz = M.nz;
   Q.pnx = (M.nx + 1) / 2; Q.pny = (M.ny + 1) / 2;
-  Q.c = odd ? C : nullptr;
   Q.n_cols = p.n_cols;
   Q.z_shift = M.z_shift;
   if (with_halo) {  // the received planes sit after the local rows of the intermediate: the lower neighbour's first
@@ -612,7 +612,7 @@ int run_march(tf_plan &p, const float *C, float *D, int item_begin, int item_end
   // phase 1 of a plan with neighbour ranks keeps the last SMs free; every other launch uses what it finds
   const bool keep_free = !with_halo && p.halo_rows > 0;
   Q.first_idle_sm = keep_free ? M.first_idle_sm : INT_MAX;
-  TF_CUDA(tfk::launch_lattice_march(keep_free ? M.grid : std::min(M.grid, std::max(1, item_end - item_begin)), tm, tm_last, Q, s));
+  TF_CUDA(tfk::launch_lattice_march(keep_free ? M.grid : std::min(M.grid, std::max(1, item_end - item_begin)), tm, tm_odd, Q, s));
   p.launches = 1;
   return TF_OK;
 }

@@ -72,24 +72,40 @@ __device__ __forceinline__ void tma_load_plane(unsigned smem, const CUtensorMap 
       ::"r"(smem), "l"((unsigned long long)tm), "r"(bar), "r"(col), "r"(xh), "r"(0), "r"(y), "r"(z)
       : "memory");
 }
-
-// The planes of C as a CTA loads them.  Where nx is odd, the pair of the last point of a line holds the first point of the
-// next line; patch_plane clears it.  Behind the very last line there is nothing to read at all, so the last plane has a map
-// of its own that ends one line earlier, and patch_plane brings that line.
-struct PlaneMaps {
-  const CUtensorMap *all, *last;
-};
-template <bool ODD>
-__device__ __forceinline__ void load_plane(unsigned smem, const PlaneMaps &tm, int col, int xh, int y, int z, unsigned bar,
-                                           const MarchParams &P) {
-  const bool last = ODD && z == P.nz - 1;
-  tma_load_plane(smem, last ? tm.last : tm.all, col, xh, y, last ? 0 : z, bar);
+// The points of a plane with even (odd) x: coordinates (column, x / 2, y, plane).
+__device__ __forceinline__ void tma_load_half(unsigned smem, const CUtensorMap *tm, int col, int xh, int y, int z, unsigned bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(smem), "l"((unsigned long long)tm), "r"(bar), "r"(col), "r"(xh), "r"(y), "r"(z)
+      : "memory");
 }
 
-// Rectangles of P x (rows) row chunks of 64 bytes are kept as [y][x % 2][x / 2][64 B]: byte offset of
-// column rx inside a y-row.
-template <int P>
-__device__ __forceinline__ int xoff(int rx) { return (rx & 1) * (P / 2 * 64) + (rx >> 1) * 64; }
+// The planes of C as a CTA loads them.  Where nx is even a plane is one box of (column, x / 2, x % 2, y, plane) and lands as
+// [y][x % 2][x / 2].  Where nx is odd, pairs of points would run on into the next line, so the points with even x and those with odd
+// x have maps of their own, whose lines are nx rows apart all the same, and a plane is two boxes, [x % 2][y][x / 2].
+// (127 x 128 x 128, 100 columns: 484 us; 579 with pairs that were mended in shared memory where they had run on.  128^3: 457.)
+struct PlaneMaps {
+  const CUtensorMap *all, *odd_x;
+};
+template <bool ODD>
+struct RectC {
+  static constexpr int row = ODD ? PC / 2 * 64 : PC * 64;                    // from a line to the next
+  static constexpr int par = ODD ? (H + 4) * (PC / 2 * 64) : PC / 2 * 64;    // from even x to odd x
+};
+template <bool ODD>
+__device__ __forceinline__ void load_plane(unsigned smem, const PlaneMaps &tm, int col, int xh, int y, int z, unsigned bar) {
+  if (ODD) {
+    tma_load_half(smem, tm.all, col, xh, y, z, bar);
+    tma_load_half(smem + RectC<true>::par, tm.odd_x, col, xh, y, z, bar);
+  } else {
+    tma_load_plane(smem, tm.all, col, xh, y, z, bar);
+  }
+}
+
+// Rectangles of row chunks of 64 bytes are kept as [y][x % 2][x / 2][64 B] (or see load_plane): byte offset of column rx inside a
+// y-row, PAR bytes from even to odd columns.
+template <int PAR>
+__device__ __forceinline__ int xoff(int rx) { return (rx & 1) * PAR + (rx >> 1) * 64; }
 
 // Shared memory is addressed by 32-bit shared-window addresses throughout (ld.shared / st.shared).
 __device__ __forceinline__ float4 lds4(unsigned buf, int off) {
@@ -123,21 +139,22 @@ __device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.
 // x0 - R0 the patch's columns a = -1 .. 2 sit at fixed byte distances co<P, R0>(a) from `base` = the address of
 // (column of x0 - R0 + 2 * pi ... i.e. pi * 64 bytes into the row, lane's 16 bytes included) of the patch's first
 // y-row: one register addresses all twelve loads of a patch.
-template <int P, int R0>
-__host__ __device__ constexpr int co(int a) { return ((R0 + a) & 1) * (P / 2 * 64) + ((R0 + a) >> 1) * 64; }
+template <int PAR, int R0>
+__host__ __device__ constexpr int co(int a) { return ((R0 + a) & 1) * PAR + ((R0 + a) >> 1) * 64; }
 
+// ROW: bytes from a y-row to the next.
 // nb: [0, 2) left column, [2, 4) right column, [4, 6) row below, [6, 8) row above.
-template <int P, int R0>
+template <int ROW, int PAR, int R0>
 __device__ __forceinline__ void load_nb(unsigned base, float4 (&nb)[8]) {
-  nb[0] = lds4i<co<P, R0>(-1)>(base);             nb[1] = lds4i<co<P, R0>(-1) + P * 64>(base);
-  nb[2] = lds4i<co<P, R0>(2)>(base);              nb[3] = lds4i<co<P, R0>(2) + P * 64>(base);
-  nb[4] = lds4i<co<P, R0>(0) - P * 64>(base);     nb[5] = lds4i<co<P, R0>(1) - P * 64>(base);
-  nb[6] = lds4i<co<P, R0>(0) + 2 * P * 64>(base); nb[7] = lds4i<co<P, R0>(1) + 2 * P * 64>(base);
+  nb[0] = lds4i<co<PAR, R0>(-1)>(base);          nb[1] = lds4i<co<PAR, R0>(-1) + ROW>(base);
+  nb[2] = lds4i<co<PAR, R0>(2)>(base);           nb[3] = lds4i<co<PAR, R0>(2) + ROW>(base);
+  nb[4] = lds4i<co<PAR, R0>(0) - ROW>(base);     nb[5] = lds4i<co<PAR, R0>(1) - ROW>(base);
+  nb[6] = lds4i<co<PAR, R0>(0) + 2 * ROW>(base); nb[7] = lds4i<co<PAR, R0>(1) + 2 * ROW>(base);
 }
-template <int P, int R0>
+template <int ROW, int PAR, int R0>
 __device__ __forceinline__ void load_own(unsigned base, float4 (&own)[4]) {
-  own[0] = lds4i<co<P, R0>(0)>(base);          own[1] = lds4i<co<P, R0>(1)>(base);
-  own[2] = lds4i<co<P, R0>(0) + P * 64>(base); own[3] = lds4i<co<P, R0>(1) + P * 64>(base);
+  own[0] = lds4i<co<PAR, R0>(0)>(base);       own[1] = lds4i<co<PAR, R0>(1)>(base);
+  own[2] = lds4i<co<PAR, R0>(0) + ROW>(base); own[3] = lds4i<co<PAR, R0>(1) + ROW>(base);
 }
 
 // Starts one row: acc = its first six products in sorted-column order -- z- (from `zm`, the same grid point one
@@ -183,7 +200,6 @@ struct ClassColumn {
 struct Shared {
   unsigned cbuf, tbuf;       // C stages, the two planes of T
   unsigned full;             // mbarriers, 8 bytes each: one per C stage (the plane has landed)
-  unsigned fixbar;           // one phase per patched plane: every warp has written its part
   unsigned tbar;             // one phase per step: every warp has stored its rows of T(k-1) (and read C(k))
   volatile int *abort;
 };
@@ -239,24 +255,8 @@ __device__ __forceinline__ int lead_in(int zs, const MarchParams &P) {
   return (zs == 0 && P.z_shift == 0 && P.t_lo == nullptr) ? 0 : 2;
 }
 
-// nx odd (101 x 67 x 83, 100 columns: 199 us, on the tile pipeline 284): completes the plane of C in stage `cb` (see load_plane) where the rectangle of the tile reaches behind the last
-// point of a line or, in the last plane, to the last line.  One thread per 16 bytes.
-__device__ __forceinline__ void patch_plane(unsigned cb, int x0, int y0, int c0col, bool fix_x, bool fix_y, const MarchParams &P) {
-  const int tid = threadIdx.x, c4 = tid & 3, i = tid >> 2;  // 32 groups of four lanes
-  if (fix_x && i < H + 4) sts4(cb, i * (PC * 64) + xoff<PC>(P.nx - x0 + 2) + c4 * 16, zero4());
-  if (fix_y && i < W + 4) {
-    const int x = x0 - 2 + i, col = c0col + 4 * c4;
-    float4 v = zero4();
-    if (x >= 0 && x < P.nx && col < P.n_cols)
-      v = __ldg(reinterpret_cast<const float4 *>(P.c + ((size_t)P.nx * P.ny * P.nz - P.nx + x) * P.n_cols + col));
-    sts4(cb, (P.ny - 1 - y0 + 2) * (PC * 64) + xoff<PC>(i) + c4 * 16, v);
-  }
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the stage is filled by TMA again later
-}
-
 // State a CTA carries from item to item.
 struct CtaState {
-  unsigned n_fix;  // planes patched so far: phases of fixbar
   unsigned n_use;  // steps taken so far: step n uses C stage n % stages (parity of n / stages) and phase n of tbar
   unsigned n_iss;  // plane loads issued so far (kept by the first warp, which issues them)
 };
@@ -278,20 +278,21 @@ __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParam
   // byte offset of the patch's first y-row (at pi * 64 bytes into it, lane's 16 bytes included) in the C rectangle
   // (two points of rim: R0 = 2) and in the T rectangle (one point: R0 = 1)
   const int pi64 = (x - x0) * 32 + c4 * 16;
-  const int boC = (y - y0 + 2) * (PC * 64) + pi64, boT = (y - y0 + 1) * (PT * 64) + pi64;
+  constexpr int kRow = RectC<ODD>::row, kPar = RectC<ODD>::par;
+  const int boC = (y - y0 + 2) * kRow + pi64, boT = (y - y0 + 1) * (PT * 64) + pi64;
   // The group's two ring rows are neighbours (in x below / above the tile, in y beside it) and lie in one 2 x 2 class
   // patch.  Offsets of the first row, of its left neighbour and of the right neighbour (of the second row when
   // the pair lies along x) in the C rectangle, of the first row in the T rectangle; the second row's follow by
   // constants.
-  const int ybr = (ry[0] - y0 + 2) * (PC * 64) + c4 * 16;
-  const int rC = ybr + xoff<PC>(rx[0] - x0 + 2), rL = ybr + xoff<PC>(rx[0] - x0 + 1);
-  const int rR = ybr + xoff<PC>(rx[0] - x0 + (pair_x ? 4 : 3));
-  const int rT = (ry[0] - y0 + 1) * (PT * 64) + xoff<PT>(rx[0] - x0 + 1) + c4 * 16;
+  const int ybr = (ry[0] - y0 + 2) * kRow + c4 * 16;
+  const int rC = ybr + xoff<kPar>(rx[0] - x0 + 2), rL = ybr + xoff<kPar>(rx[0] - x0 + 1);
+  const int rR = ybr + xoff<kPar>(rx[0] - x0 + (pair_x ? 4 : 3));
+  const int rT = (ry[0] - y0 + 1) * (PT * 64) + xoff<PT / 2 * 64>(rx[0] - x0 + 1) + c4 * 16;
   const unsigned rsh0 = 8u * (2u * (ry[0] & 1) + (rx[0] & 1));  // bit position of the first row's class in the class word
   ClassColumn cr_col;
   cr_col.init(P.pcls_f, rx[0], ry[0], P.nx, P.ny, P.pnx);
   // second row: distances in the C rectangle, in the T rectangle and in the class word
-  constexpr int kX1C = PC / 2 * 64, kY1C = PC * 64;       // x + 1 from an even column / y + 1
+  constexpr int kX1C = kPar, kY1C = kRow;                 // x + 1 from an even column / y + 1
   constexpr int kX1T = 64 - PT / 2 * 64, kY1T = PT * 64;  // x + 1 from an odd column / y + 1
   const int col = c0col + 4 * c4;
   // rows of the patch that exist and whose columns exist: bit j
@@ -336,20 +337,10 @@ __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParam
     const unsigned stage = cs.n_use % kMarchStages;
     if (!wait_or_abort(S.full + 8 * stage, (cs.n_use / kMarchStages) & 1u, P.wait_limit, S.abort)) return false;
     const unsigned cb = S.cbuf + stage * kMarchCBytes;
-    if (ODD && k >= 0 && k < P.nz) {
-      const bool fix_x = P.nx < x0 + W + 2, fix_y = k == P.nz - 1 && P.ny - 1 < y0 + H + 2;  // (both are >= the tile's origin)
-      if (fix_x || fix_y) {
-        patch_plane(cb, x0, y0, c0col, fix_x, fix_y, P);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(S.fixbar);
-        if (!wait_or_abort(S.fixbar, cs.n_fix & 1u, P.wait_limit, S.abort)) return false;
-        ++cs.n_fix;
-      }
-    }
     float4 nb[8];
     const unsigned baseC = cb + boC;
-    load_own<PC, 2>(baseC, own);
-    load_nb<PC, 2>(baseC, nb);
+    load_own<kRow, kPar, 2>(baseC, own);
+    load_nb<kRow, kPar, 2>(baseC, nb);
     if (ring) {
       rown[0] = lds4(cb, rC);
       rown[1] = pair_x ? lds4i<kX1C>(cb + rC) : lds4i<kY1C>(cb + rC);
@@ -370,8 +361,8 @@ __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParam
     const unsigned baseT = tb + boT;
     // (the buffer of T(k-1) was last read in step k-2; this thread has waited for every warp's arrival of
     // step k-1, which each warp gives after its reads of step k-2)
-    sts4i<co<PT, 1>(0)>(baseT, tcur[0]);           sts4i<co<PT, 1>(1)>(baseT, tcur[1]);
-    sts4i<co<PT, 1>(0) + PT * 64>(baseT, tcur[2]); sts4i<co<PT, 1>(1) + PT * 64>(baseT, tcur[3]);
+    sts4i<co<PT / 2 * 64, 1>(0)>(baseT, tcur[0]);           sts4i<co<PT / 2 * 64, 1>(1)>(baseT, tcur[1]);
+    sts4i<co<PT / 2 * 64, 1>(0) + PT * 64>(baseT, tcur[2]); sts4i<co<PT / 2 * 64, 1>(1) + PT * 64>(baseT, tcur[3]);
     if (ring) {
       float4 t0 = fma4(czpR[0], rown[0], accR[0]), t1 = fma4(czpR[1], rown[1], accR[1]);
       if (ODD && (deadR & 1u)) t0 = zero4();
@@ -407,16 +398,16 @@ __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParam
         if (pair_x) {
           // the group's two ring rows are neighbours in x: each is the other's x- / x+ row
           const unsigned cls1 = (wr >> (rsh0 + 8u)) & 255u;
-          const float4 ym0 = lds4i<-PC * 64>(cb + rC), xm0 = lds4(cb, rL), yp0 = lds4i<PC * 64>(cb + rC);
+          const float4 ym0 = lds4i<-kRow>(cb + rC), xm0 = lds4(cb, rL), yp0 = lds4i<kRow>(cb + rC);
           czpR[0] = row_start(accR[0], P.dict_f, cls0, rprev[0], ym0, xm0, rown[0], rown[1], yp0);
-          const float4 ym1 = lds4i<kX1C - PC * 64>(cb + rC), xp1 = lds4(cb, rR), yp1 = lds4i<kX1C + PC * 64>(cb + rC);
+          const float4 ym1 = lds4i<kX1C - kRow>(cb + rC), xp1 = lds4(cb, rR), yp1 = lds4i<kX1C + kRow>(cb + rC);
           czpR[1] = row_start(accR[1], P.dict_f, cls1, rprev[1], ym1, rown[0], rown[1], xp1, yp1);
         } else {
           // ... neighbours in y: each is the other's y- / y+ row
           const unsigned cls1 = (wr >> (rsh0 + 16u)) & 255u;
-          const float4 ym0 = lds4i<-PC * 64>(cb + rC), xm0 = lds4(cb, rL), xp0 = lds4(cb, rR);
+          const float4 ym0 = lds4i<-kRow>(cb + rC), xm0 = lds4(cb, rL), xp0 = lds4(cb, rR);
           czpR[0] = row_start(accR[0], P.dict_f, cls0, rprev[0], ym0, xm0, rown[0], xp0, rown[1]);
-          const float4 xm1 = lds4i<kY1C>(cb + rL), xp1 = lds4i<kY1C>(cb + rR), yp1 = lds4i<2 * PC * 64>(cb + rC);
+          const float4 xm1 = lds4i<kY1C>(cb + rL), xp1 = lds4i<kY1C>(cb + rR), yp1 = lds4i<2 * kRow>(cb + rC);
           czpR[1] = row_start(accR[1], P.dict_f, cls1, rprev[1], rown[0], xm1, rown[1], xp1, yp1);
         }
       }
@@ -442,7 +433,7 @@ __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParam
         ++cs.n_iss;
         if (elect_lane()) {
           mbar_expect_tx(S.full + 8 * prev_stage, kMarchCBytes);
-          load_plane<ODD>(S.cbuf + prev_stage * kMarchCBytes, tm_c, lc, lx / 2 - 1, ly - 2, lz + P.z_shift, S.full + 8 * prev_stage, P);
+          load_plane<ODD>(S.cbuf + prev_stage * kMarchCBytes, tm_c, lc, lx / 2 - 1, ly - 2, lz + P.z_shift, S.full + 8 * prev_stage);
         }
         __syncwarp();
       }
@@ -450,7 +441,7 @@ __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParam
     // D(k-1): everything but the z+ product, from T(k-2) (registers), T(k-1) (registers and neighbours)
     if (k - 1 >= zs && k - 1 < ze) {
       float4 tn[8];
-      load_nb<PT, 1>(baseT, tn);
+      load_nb<PT * 64, PT / 2 * 64, 1>(baseT, tn);
       patch_start(accD, czpD, P.dict_a, wa, tprev, tcur, tn);
     }
     ++cs.n_use;
@@ -476,8 +467,8 @@ __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParam
 // ODD: the x extent is odd.
 template <bool ODD>
 __global__ void __launch_bounds__(kMarchThreads, kMarchCtasPerSm)
-lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_last, const MarchParams P) {
-  const PlaneMaps maps{&tm_c, &tm_last};
+lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_odd, const MarchParams P) {
+  const PlaneMaps maps{&tm_c, &tm_odd};
   extern __shared__ char dyn[];
   __shared__ int ctl[2];
   __shared__ int nxt[5];
@@ -486,7 +477,6 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   S.tbuf = S.cbuf + kMarchStages * kMarchCBytes;
   S.full = S.tbuf + 2 * kMarchTBytes;
   S.tbar = S.full + 8 * kMarchStages;
-  S.fixbar = S.tbar + 8;
   S.abort = &ctl[1];
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const bool loader = warp == 0;  // the warp that asks for the planes
@@ -494,7 +484,6 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   if (tid == 0) {
     for (int s = 0; s < kMarchStages; ++s) mbar_init(S.full + 8 * s, 1);
     mbar_init(S.tbar, kMarchThreads / 32);
-    mbar_init(S.fixbar, kMarchThreads / 32);
     ctl[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -523,7 +512,7 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
   const bool idle = (int)smid >= P.first_idle_sm;
 
-  CtaState cs{0u, 0u, 0u};
+  CtaState cs{0u, 0u};
   bool failed = false;
   // Thread 0 holds the ticket of the item after the current one and keeps that item's origin in shared memory:
   // the last steps of an item already fetch the first planes of the next (`pre` of them).
@@ -555,7 +544,7 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
         const unsigned stage = (cs.n_use + s) % kMarchStages;
         if (elect_lane()) {
           mbar_expect_tx(S.full + 8 * stage, kMarchCBytes);
-          load_plane<ODD>(S.cbuf + stage * kMarchCBytes, maps, c0col, x0 / 2 - 1, y0 - 2, kfirst + s + P.z_shift, S.full + 8 * stage, P);
+          load_plane<ODD>(S.cbuf + stage * kMarchCBytes, maps, c0col, x0 / 2 - 1, y0 - 2, kfirst + s + P.z_shift, S.full + 8 * stage);
         }
         __syncwarp();
       }
@@ -662,8 +651,8 @@ star_march_kernel(const __grid_constant__ CUtensorMap tm, const MarchParams P, i
       ++n_use;
       const unsigned base = buf + st * kStarBytes + base0;
       float4 own[4], nb[8];
-      load_own<PS, 2>(base, own);
-      load_nb<PS, 2>(base, nb);
+      load_own<PS * 64, PS / 2 * 64, 2>(base, own);
+      load_nb<PS * 64, PS / 2 * 64, 2>(base, nb);
       if (cut) own[1] = own[3] = zero4();
       const unsigned after = cls.at(k + 2, P.nz, plane_words, zero_a);
       if (k - 1 >= zs) {
@@ -707,15 +696,19 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, int lines, long long planes, int box_lines) {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
+static EncodeTiledFn encode_fn() {
+  static EncodeTiledFn fn = [] {
     void *p = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (EncodeTiledFn)p;
-  }
+    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess
+               ? (EncodeTiledFn)p
+               : (EncodeTiledFn) nullptr;
+  }();
+  return fn;
+}
+
+int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, int lines, long long planes, int box_lines) {
+  EncodeTiledFn fn = encode_fn();
   if (!fn) return -1;
   // (column, x / 2, x % 2, y, plane): row x = 2 * (x / 2) + x % 2 of a y-line; where nx is odd the last pair of a line ends
   // with the first row of the next
@@ -725,6 +718,20 @@ int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny,
   cuuint32_t box[5] = {(cuuint32_t)kMarchCols, (cuuint32_t)((kMarchW + 4) / 2), 2, (cuuint32_t)box_lines, 1};
   cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<float *>(c), gdim, gstride, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : (int)r;
+}
+
+int march_make_half_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, long long planes, int odd_x) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return -1;
+  const cuuint64_t row = (cuuint64_t)n_cols * 4;
+  cuuint64_t gdim[4] = {(cuuint64_t)n_cols, (cuuint64_t)((nx + 1 - odd_x) / 2), (cuuint64_t)ny, (cuuint64_t)planes};
+  cuuint64_t gstride[3] = {2 * row, row * nx, row * nx * ny};
+  cuuint32_t box[4] = {(cuuint32_t)kMarchCols, (cuuint32_t)((kMarchW + 4) / 2), (cuuint32_t)(kMarchH + 4), 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(c) + (size_t)odd_x * n_cols, gdim, gstride, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : (int)r;
@@ -746,9 +753,9 @@ static int ctas_per_sm() {
 }
 int march_ctas_per_sm() { return std::min(ctas_per_sm<false>(), ctas_per_sm<true>()); }
 
-cudaError_t launch_lattice_march(int grid, const CUtensorMap &tm_c, const CUtensorMap &tm_last, const MarchParams &p, cudaStream_t s) {
+cudaError_t launch_lattice_march(int grid, const CUtensorMap &tm_c, const CUtensorMap &tm_odd, const MarchParams &p, cudaStream_t s) {
   if (march_ctas_per_sm() <= 0) return cudaErrorLaunchOutOfResources;
-  (p.c ? lattice_march_kernel<true> : lattice_march_kernel<false>)<<<grid, kMarchThreads, kMarchSmemBytes, s>>>(tm_c, tm_last, p);
+  (p.nx % 2 ? lattice_march_kernel<true> : lattice_march_kernel<false>)<<<grid, kMarchThreads, kMarchSmemBytes, s>>>(tm_c, tm_odd, p);
   return cudaGetLastError();
 }
 

@@ -14,7 +14,7 @@ constexpr int kMarchCtasPerSm = 2;          // two independent CTAs per SM: one 
 constexpr int kMarchCBytes = (kMarchW + 4) * (kMarchH + 4) * kMarchCols * 4;                          // 15 360
 constexpr int kMarchTBytes = ((kMarchW + 2) * (kMarchH + 2) * kMarchCols * 4 + 1023) / 1024 * 1024;  // 12 288
 constexpr int kMarchMaxClassesDev = 63;
-constexpr size_t kMarchSmemBytes = (size_t)kMarchStages * kMarchCBytes + 2 * kMarchTBytes + (kMarchStages + 2) * 8 + 1024;
+constexpr size_t kMarchSmemBytes = (size_t)kMarchStages * kMarchCBytes + 2 * kMarchTBytes + (kMarchStages + 1) * 8 + 1024;
 
 struct MarchState {
   int ticket;    // next item
@@ -34,7 +34,6 @@ struct MarchParams {
   int nx, ny, nz, pnx, pny, n_cols;
   int z_shift;                      // plane of C (in the tensor map) that holds the operand rows of plane 0
   int wait_limit;
-  const float *c;                   // the operand itself where nx is odd (null: it is even), see load_plane
   int first_idle_sm;                // CTAs that land on an SM with this id or a higher one leave at once (see api.cu)
   // Coefficient dictionaries, (classes + 1) x 2 float4 each: {z-, y-, x-, centre}, {x+, y+, z+, 0}.  They travel
   // as kernel parameters, i.e. in the constant bank: the four lanes that share a row -- usually the whole warp --
@@ -48,8 +47,10 @@ struct MarchParams {
 int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, int lines, long long planes,
                    int box_lines = kMarchH + 4);
 int march_ctas_per_sm();
-// tm_last: the last plane without its last line where nx is odd, else as tm_c.
-cudaError_t launch_lattice_march(int grid, const CUtensorMap &tm_c, const CUtensorMap &tm_last, const MarchParams &p, cudaStream_t s);
+// Where nx is odd: the points with even (odd) x as (n_cols, x / 2, y, plane), box = 16 columns x (W+4)/2 x (H+4) x 1.
+int march_make_half_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, long long planes, int odd_x);
+// Where nx is odd: tm_c and tm_odd are the half maps, else tm_c is march_make_map's.
+cudaError_t launch_lattice_march(int grid, const CUtensorMap &tm_c, const CUtensorMap &tm_odd, const MarchParams &p, cudaStream_t s);
 
 // One product D = A * T (p.out, p.pcls_a, p.dict_a): tm is a map of T with boxes of kMarchH + 2 lines.
 int star_ctas_per_sm();
