@@ -147,53 +147,56 @@ spmm_gemm_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_constant
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
   if (warp == kSgWarpRaw) {
-    // ---- the points of B that a brick reads, a slice at a time ----
-    if (lane == 0) {
-      int rs = 0, used = 0;
-      unsigned rph = 0;
-      bool ok = true;
-      for (int t = first; t < tiles && ok; t += pairs) {
-        int x, y, z;
-        brick_origin(A.grid, brick0 + 2 * t, x, y, z);
-        for (int sl = 0; sl < A.slices; ++sl) {
-          if (used >= A.raws && !(ok = pair_wait(&s.raw_empty[rs], rph ^ 1u, s.dead, A.wait_limit))) break;
-          char *o = raw + rs * raw_bytes;
+    // ---- the points of B that a brick reads, a slice at a time (the whole warp, see elect_one) ----
+    int rs = 0, used = 0;
+    unsigned rph = 0;
+    bool ok = true;
+    for (int t = first; t < tiles && ok; t += pairs) {
+      int x, y, z;
+      brick_origin(A.grid, brick0 + 2 * t, x, y, z);
+      for (int sl = 0; sl < A.slices; ++sl) {
+        if (used >= A.raws && !(ok = __all_sync(kFull, pair_wait(&s.raw_empty[rs], rph ^ 1u, s.dead, A.wait_limit)))) break;
+        char *o = raw + rs * raw_bytes;
+        if (elect_one()) {
           mbar_expect_tx(&s.raw_full[rs], (unsigned)raw_bytes);
           load_points(o, &tm_b, sl * kTcKSlice, x - 1, y - 1, z, &s.raw_full[rs]);
           if (D3) {  // the layers below and above, without their neighbours
             load_points(o + raw_bytes - 2 * sx * sy * 128, &tm_cap, sl * kTcKSlice, x, y, z - 1, &s.raw_full[rs]);
             load_points(o + raw_bytes - sx * sy * 128, &tm_cap, sl * kTcKSlice, x, y, z + sz, &s.raw_full[rs]);
           }
-          if (used < A.raws) ++used;
-          if (++rs == A.raws) { rs = 0; rph ^= 1u; }
         }
+        __syncwarp();
+        if (used < A.raws) ++used;
+        if (++rs == A.raws) { rs = 0; rph ^= 1u; }
       }
-      // (a copy still in flight must not outlive the CTA: only after a wait ran out is one possible)
-      if (s.dead)
-        for (int i = 0; i < used; ++i) mbar_wait(&s.raw_full[i], i < rs ? rph : rph ^ 1u, A.wait_limit);
     }
+    // (a copy still in flight must not outlive the CTA: only after a wait ran out is one possible)
+    if (!ok || s.dead)
+      for (int i = 0; i < used; ++i) mbar_wait(&s.raw_full[i], i < rs ? rph : rph ^ 1u, A.wait_limit);
   } else if (warp == kSgWarpW) {
     // ---- slices of the weight; the stages of this CTA until the last product that reads one is done ----
-    if (lane == 0) {
-      int st = 0, issued = 0;
-      unsigned ph = 0;
-      bool ok = true;
-      for (int t = first; t < tiles && ok; t += pairs)
-        for (int sl = 0; sl < A.slices; ++sl) {
-          if (issued >= A.stages && !(ok = pair_wait(&s.empty[st], ph ^ 1u, s.dead, A.wait_limit))) break;
-          if (!RES) {
-            char *w = smem + st * stage_bytes + kSgStageA;
-            mbar_expect_tx(&s.wfull[st], (unsigned)slice_w);
-            tma_load_2d(w, &tm_whi, sl * kTcKSlice, (int)rank * half, &s.wfull[st]);
-            tma_load_2d(w + half * 128, &tm_wlo, sl * kTcKSlice, (int)rank * half, &s.wfull[st]);
-          }
-          if (issued < A.stages) ++issued;
-          if (++st == A.stages) { st = 0; ph ^= 1u; }
+    int st = 0, issued = 0;
+    unsigned ph = 0;
+    bool ok = true;
+    auto wait = [&](unsigned long long *bar, unsigned parity) {
+      return ok = __all_sync(kFull, pair_wait(bar, parity, s.dead, A.wait_limit));
+    };
+    for (int t = first; t < tiles && ok; t += pairs)
+      for (int sl = 0; sl < A.slices; ++sl) {
+        if (issued >= A.stages && !wait(&s.empty[st], ph ^ 1u)) break;
+        if (!RES && elect_one()) {
+          char *w = smem + st * stage_bytes + kSgStageA;
+          mbar_expect_tx(&s.wfull[st], (unsigned)slice_w);
+          tma_load_2d(w, &tm_whi, sl * kTcKSlice, (int)rank * half, &s.wfull[st]);
+          tma_load_2d(w + half * 128, &tm_wlo, sl * kTcKSlice, (int)rank * half, &s.wfull[st]);
         }
-      for (int i = 0; ok && i < issued; ++i) ok = pair_wait(&s.empty[i], i < st ? ph : ph ^ 1u, s.dead, A.wait_limit);
-      if (!RES && s.dead)
-        for (int i = 0; i < issued; ++i) mbar_wait(&s.wfull[i], i < st ? ph : ph ^ 1u, A.wait_limit);
-    }
+        __syncwarp();
+        if (issued < A.stages) ++issued;
+        if (++st == A.stages) { st = 0; ph ^= 1u; }
+      }
+    for (int i = 0; ok && i < issued; ++i) wait(&s.empty[i], i < st ? ph : ph ^ 1u);
+    if (!RES && (!ok || s.dead))
+      for (int i = 0; i < issued; ++i) mbar_wait(&s.wfull[i], i < st ? ph : ph ^ 1u, A.wait_limit);
   } else if (warp == kSgWarpMma) {
     // ---- products (even CTA): the whole warp, see elect_one ----
     if (rank == 0) {
