@@ -594,14 +594,14 @@ star_march_kernel(const __grid_constant__ CUtensorMap tm, const MarchParams P, i
   extern __shared__ char dyn[];
   __shared__ int ctl[2];
   const unsigned buf = (smem_u32(dyn) + 1023u) & ~1023u, full = buf + kStarStages * kStarBytes, empty = full + 8 * kStarStages;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, pi = lane >> 2, c4 = lane & 3;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, pi = lane >> 2, c4 = lane & 3;
   volatile int *abort = &ctl[1];
   if (tid == 0) {
     for (int s = 0; s < kStarStages; ++s) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, kMarchThreads / 32); }
     ctl[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  unsigned n_use = 0, n_iss = 0;  // planes read, planes asked for (thread 0) so far
+  unsigned n_use = 0, n_iss = 0;  // planes read, planes asked for (the first warp, see elect_lane) so far
   const int plane_words = P.pnx * P.pny;
   const unsigned zero_a = 0x01010101u * (unsigned)P.ncls_a;
   const size_t drow = (size_t)P.nx * P.n_cols, dplane = drow * P.ny;
@@ -617,15 +617,19 @@ star_march_kernel(const __grid_constant__ CUtensorMap tm, const MarchParams P, i
     auto issue = [&](int step) {
       const unsigned st = n_iss % kStarStages;
       ++n_iss;
-      mbar_expect_tx(full + 8 * st, kStarBytes);
-      tma_load_plane(buf + st * kStarBytes, &tm, c0col, x0 / 2 - 1, y0 - 1, zs - 1 + step, full + 8 * st);
+      if (elect_lane()) {
+        mbar_expect_tx(full + 8 * st, kStarBytes);
+        tma_load_plane(buf + st * kStarBytes, &tm, c0col, x0 / 2 - 1, y0 - 1, zs - 1 + step, full + 8 * st);
+      }
+      __syncwarp();
     };
-    int asked = 0;  // (thread 0) planes of this item asked for
+    int asked = 0;  // (the first warp) planes of this item asked for
     bool ok = true;
     // a stage is filled again once every warp has read what was in it
     auto refill = [&](int upto) {
       for (; ok && asked < min(upto, steps); ++asked) {
-        if (n_iss >= (unsigned)kStarStages) ok = wait_or_abort(empty + 8 * (n_iss % kStarStages), (n_iss / kStarStages - 1) & 1u, P.wait_limit, abort);
+        if (n_iss >= (unsigned)kStarStages)
+          ok = __all_sync(0xffffffffu, wait_or_abort(empty + 8 * (n_iss % kStarStages), (n_iss / kStarStages - 1) & 1u, P.wait_limit, abort));
         if (ok) issue(asked);
       }
     };
@@ -645,7 +649,7 @@ star_march_kernel(const __grid_constant__ CUtensorMap tm, const MarchParams P, i
     unsigned word = cls.at(zs - 1, P.nz, plane_words, zero_a), next = cls.at(zs, P.nz, plane_words, zero_a);
     for (int step = 0; step < steps && ok; ++step) {
       const int k = zs - 1 + step;
-      if (tid == 0) refill(step + kStarStages - 1);
+      if (warp == 0) refill(step + kStarStages - 1);
       const unsigned st = n_use % kStarStages;
       if (!ok || !wait_or_abort(full + 8 * st, (n_use / kStarStages) & 1u, P.wait_limit, abort)) { ok = false; break; }
       ++n_use;
