@@ -51,6 +51,27 @@ def test_line_march(built_lib, dims, n_cols):
         ref.close()
 
 
+# grids whose segments are long enough that warps ask L2 for lines ahead: to the grid's last line, a ragged last chunk of columns
+@pytest.mark.parametrize("dims,n_cols", [((611, 280), 100), ((1023, 331), 64), ((300, 701), 128)])
+def test_segments_that_read_ahead(built_lib, dims, n_cols):
+    import torch
+    a = synth.laplacian(dims)
+    n = len(a[0]) - 1
+    rows = np.repeat(np.arange(n), np.diff(a[0]))
+    b = (a[0], a[1], (a[2] * (1.0 + (rows % 2))).astype(np.float32))
+    c = torch.from_numpy(synth.uniform(3, (n, n_cols))).cuda()
+    for B in (None, _csr(b)):
+        out = []
+        for kw in ({}, dict(mode=api.MODE_UNFUSED, tile_slots=-1, lattice_march=-1)):
+            plan = api.Plan("spmm_spmm", _csr(a), B=B, n_cols=n_cols, **kw)
+            d = torch.full((n, n_cols), float("nan"), device="cuda")
+            plan.spmm_spmm(c, d)
+            plan.status()
+            out.append(d)
+            plan.close()
+        assert torch.equal(*out)
+
+
 def test_infinities_stay_where_they_are(built_lib):
     """Rows beyond the grid are zero and not multiplied by it: infinities on the rim reach their neighbours only."""
     import torch

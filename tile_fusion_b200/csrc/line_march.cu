@@ -11,7 +11,7 @@
 // bit those of the CSR executors.  Rows of T that do not exist are set to zero and not multiplied by it, so an infinity
 // in C stays where it belongs.
 // What bounds it is memory: every element of C is read once and every element of D written once.  1023 x 777, 64 columns:
-// 96.5 us (4.6 TB/s of those bytes); the tile pipeline, which writes T and reads it back, took 183.
+// 94.9 us (4.3 TB/s of those bytes; 96.5 before L2 was asked for lines ahead); the tile pipeline, which writes T and reads it back, took 183.
 #include <algorithm>
 
 #include "line_march.h"
@@ -22,6 +22,13 @@ namespace tfk {
 namespace {
 
 constexpr unsigned kAll = 0xffffffffu;
+// Lines between the line that a warp asks L2 for and the one that it completes, and the shortest segment that does so.  Two
+// lines in registers do not cover a read from memory; asking L2 for a line six ahead does, without a register.  Measured (no
+// request; 4, 6, 8, 12 lines): 1400 x 1400, 96 columns 342 us; 308, 308, 313, 352; 1000 x 1000, 100 columns 197; 190, 186, 188,
+// 199; 1023 x 777, 64 columns 100.4; 98.3, 99.1, 102, 106.  Short segments have no line left to ask for: the requests cost
+// 500 x 300, 32 columns (seven lines) 19.5 -> 21.5.  With single columns a line of a warp is sixteen instructions of two
+// points each, and asking for it too costs more than it hides: 900 x 700, 33 columns 117 -> 164, with a lane per point 124.
+constexpr int kLineAhead = 6, kLineAheadSegment = 24;
 constexpr int line_ctas(bool vec) { return vec ? 3 : 2; }  // resident per SM (with single columns a lane holds four times the points)
 
 template <int V>
@@ -128,6 +135,7 @@ __global__ void __launch_bounds__(32 * kLineWarps, line_ctas(V == 4)) line_march
 #pragma unroll
   for (int i = 0; i < W; ++i) { wf[3][i] = A.none_f; wap[i] = A.none_a; wa[3][i] = A.none_a; }
   const int k0 = ys - 2, k1 = ye + 1;  // lines of C that the segment reads
+  const bool ahead = A.seg_len >= kLineAheadSegment;
   load_line(k0, c[0]);
   load_line(k0 + 1, c[1]);
   load_words(wf_at, A.none_f, k0, wf[0]);
@@ -152,6 +160,12 @@ __global__ void __launch_bounds__(32 * kLineWarps, line_ctas(V == 4)) line_march
       unsigned (&wfc)[W] = wf[j];
       unsigned (&wac)[W] = SAME ? wf[(j + 3) & 3] : wa[(j + 3) & 3];  // second operator, line k - 1
       load_line(k + 2 <= k1 ? k + 2 : -1, c[(j + 2) & 3]);
+      if (V == 4 && ahead && k + kLineAhead <= k1 && k + kLineAhead < A.ny) {  // (k >= -2, so the line exists)
+        const float *q = src + (long long)(k + kLineAhead) * (long long)line;
+#pragma unroll
+        for (int i = 0; i < P; ++i)
+          if (in >> i & 1u) asm volatile("prefetch.global.L2 [%0];" ::"l"(q + (size_t)i * A.n_cols));
+      }
       load_words(wf_at, A.none_f, k + 2, wf[(j + 2) & 3]);
       if (!SAME) load_words(wa_at, A.none_a, k + 2, wa[(j + 2) & 3]);
       unsigned any = 0;
