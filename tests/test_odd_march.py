@@ -66,3 +66,39 @@ def test_infinities_stay_where_they_are(built_lib, dims):
     np.testing.assert_array_equal(np.isinf(got), np.isinf(want))
     assert not np.isnan(got).any()
     plan.close()
+
+
+# widths off the multiples of four march from a padded copy: either parity of x, the narrowest taken and the one below it, a last
+# chunk of one column, operands off the 16-byte grid, infinities on the rim
+@pytest.mark.parametrize("dims", [(16, 8, 7), (33, 17, 9), (18, 11, 4)])
+@pytest.mark.parametrize("n_cols", [3, 5, 33, 47])
+def test_widths_off_the_multiples_of_four(built_lib, dims, n_cols):
+    import torch
+    a = synth.laplacian(dims)
+    n = len(a[0]) - 1
+    rows = np.repeat(np.arange(n), np.diff(a[0]))
+    b = (a[0], a[1], (a[2] * (1.0 + (rows % 2)) * np.where(a[1] > rows, 0.5, 1.0)).astype(np.float32))
+    c = torch.from_numpy(synth.uniform(3, (n, n_cols))).cuda()
+    ci = c.clone()
+    ci[[0, dims[0] - 1, dims[0] * dims[1] - 1, n - 1]] = float("inf")
+    for B in (None, _csr(b)):
+        plan = api.Plan("spmm_spmm", _csr(a), B=B, n_cols=n_cols)
+        assert (plan.info()["threads"] == 128) == (n_cols >= 5)
+        ref = api.Plan("spmm_spmm", _csr(a), B=B, n_cols=n_cols, mode=api.MODE_UNFUSED, tile_slots=-1, lattice_march=-1)
+        for x in (c, ci):
+            xu = torch.empty(n * n_cols + 1, device="cuda")[1:].view(n, n_cols).copy_(x)
+            du = torch.full((n * n_cols + 3,), float("nan"), device="cuda")
+            d = du[1:-2].view(n, n_cols)
+            plan.spmm_spmm(xu, d)
+            plan.status()
+            d0 = torch.empty((n, n_cols), device="cuda")
+            ref.spmm_spmm(x, d0)
+            ref.status()
+            assert torch.equal(torch.nan_to_num(d, nan=7.0), torch.nan_to_num(d0, nan=7.0))
+            assert torch.isnan(du[[0, -2, -1]]).all()
+        dh = np.full((n, n_cols), np.nan, np.float32)
+        plan.spmm_spmm_host(c.cpu().numpy(), dh)
+        plan.spmm_spmm(c, d)
+        np.testing.assert_array_equal(dh, d.cpu().numpy())
+        plan.close()
+        ref.close()

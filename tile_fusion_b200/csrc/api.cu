@@ -279,6 +279,8 @@ struct tf_plan {
   // plane-marching executor (both operators are star stencils on one grid)
   struct March {
     bool on = false, same = false;  // same: one operator on both sides (B == A)
+    bool ragged = false;            // a width off the multiples of four: C is padded to rows of ld_t in g_pad (see build_march)
+    bool halves = false;            // planes from the half maps: nx is odd, or ragged
     bool identity_first = false;    // GeMM-SpMM: the first operator is the identity, the operand is the producer's T
     bool halo_lo = false, halo_hi = false;  // a neighbour rank below / above supplies plane -1 / nz of T
     int nx = 0, ny = 0, nz = 0, ncls_f = 0, ncls_a = 0, z_shift = 0, grid = 0, n_items = 0, n_phase1 = 0;
@@ -483,6 +485,9 @@ std::vector<int4> march_items_raw(const std::vector<tf::MarchItem> &items) {
 // Fp == null: the first operator is the identity (GeMM-SpMM: the dense producer has written T, and the marching
 // kernel computes D = A * (I * T); the products with the identity's zeros and its one are exact, so D is what the
 // CSR consumer gives).
+// The narrowest width off the multiples of four that marches: 16 columns are computed whatever the width, so one to three stay with
+// the gather, whose reads of four columns are a quarter of that (5 columns at 100 x 90 x 110: 187 us there, 71 here).
+constexpr int kMarchMinRagged = 5;
 // star: behind the dense product on the one-product march.  Taken only where every row names all of its neighbours: the march
 // multiplies a neighbour that is not named by zero, and an infinity there would not stay where it belongs.
 int build_march(tf_plan &p, const tf_csr *Fp, const tf_csr &A, int halo_rows, int sm_count, const std::vector<int> &boundary_rows,
@@ -511,6 +516,13 @@ int build_march(tf_plan &p, const tf_csr *Fp, const tf_csr &A, int halo_rows, in
   }
   const tf_csr &F = Fp ? *Fp : A;
   if (la.nx != lf.nx || la.ny != lf.ny || la.nz != lf.nz) return TF_OK;
+  // Widths off the multiples of four march from a padded copy of C: the copy is a pass more, but the gather took two with seven row
+  // reads each (and the same copy).  Infinities stay where the gather leaves them: full stencils and half maps only.
+  // Gather and march, us: 100 x 90 x 110, 9 columns 202 and 77, 33 406 and 212, 47 454 and 235, 99 798 and 460; 31 x 40 x 50, 33 columns
+  // 40 and 28; 12 x 16 x 20 19.5 and 17.4.  (48 columns of the first take 142: the copy is 60 of the difference.  Marching to a padded D
+  // that another launch crops: 318 at 47 columns.)
+  const bool ragged = p.n_cols % 4 != 0;
+  if (ragged && (p.n_cols < kMarchMinRagged || halo_rows > 0 || !lf.full || !la.full)) return TF_OK;
   if (halo_rows == 0 && (la.ghost_lo || la.ghost_hi)) return TF_OK;
   // with a neighbour rank below (above), the first operator must reach one plane of C below (above) the rank's
   // own: the boundary planes of T that the rank computes itself need them
@@ -519,6 +531,8 @@ int build_march(tf_plan &p, const tf_csr *Fp, const tf_csr &A, int halo_rows, in
   if (occ <= 0) return TF_OK;  // the kernel does not fit this device: general path
   tf_plan::March &M = p.march;
   M.nx = lf.nx; M.ny = lf.ny; M.nz = lf.nz;
+  M.ragged = ragged;
+  M.halves = ragged || M.nx % 2 != 0;
   M.ncls_f = lf.n_classes; M.ncls_a = la.n_classes;
   M.z_shift = lf.ghost_lo;
   M.planes_c = (long long)lf.nz + lf.ghost_lo + lf.ghost_hi;
@@ -538,7 +552,7 @@ int build_march(tf_plan &p, const tf_csr *Fp, const tf_csr &A, int halo_rows, in
   if (M.halo_hi && M.nz > 1)
     tf::build_march_items(M.nx, M.ny, M.nz - 1, M.nz, p.n_cols, tfk::kMarchW, tfk::kMarchH, tfk::kMarchCols, M.grid, 1, M.host_items);
   M.n_items = (int)M.host_items.size();
-  if (halo_rows == 0 && M.nz >= 8) {
+  if (halo_rows == 0 && M.nz >= 8 && !ragged) {  // (host calls of ragged widths go through the gather's pieces)
     const int n_slabs = std::min(32, M.nz / 4);
     for (int sl = 0; sl < n_slabs; ++sl) {
       const int za = (int)((long long)M.nz * sl / n_slabs), zb = (int)((long long)M.nz * (sl + 1) / n_slabs);
@@ -582,11 +596,12 @@ int run_march(tf_plan &p, const float *C, float *D, int item_begin, int item_end
   tf_plan::March &M = p.march;
   if (item_end <= item_begin) { p.launches = 0; return TF_OK; }
   CUtensorMap tm, tm_odd;
-  const bool odd = M.nx % 2 != 0;
-  int mr = odd ? tfk::march_make_half_map(&tm, C, p.n_cols, M.nx, M.ny, M.planes_c, 0)
-               : tfk::march_make_map(&tm, C, p.n_cols, M.nx, M.ny, M.ny, M.planes_c);
+  const int ld = M.ragged ? p.ld_t : p.n_cols;
+  const float *src = M.ragged ? p.g_pad.p : C;
+  int mr = M.halves ? tfk::march_make_half_map(&tm, src, ld, M.nx, M.ny, M.planes_c, 0)
+                    : tfk::march_make_map(&tm, src, ld, M.nx, M.ny, M.ny, M.planes_c);
   tm_odd = tm;
-  if (odd && mr == 0) mr = tfk::march_make_half_map(&tm_odd, C, p.n_cols, M.nx, M.ny, M.planes_c, 1);
+  if (M.halves && mr == 0) mr = tfk::march_make_half_map(&tm_odd, src, ld, M.nx, M.ny, M.planes_c, 1);
   if (mr != 0) return fail(TF_ERR_CUDA, "cuTensorMapEncodeTiled failed for the dense operand (code " + std::to_string(mr) + ")");
   tfk::MarchParams Q;
   std::memset(&Q, 0, sizeof(Q));
@@ -612,8 +627,9 @@ int run_march(tf_plan &p, const float *C, float *D, int item_begin, int item_end
   // phase 1 of a plan with neighbour ranks keeps the last SMs free; every other launch uses what it finds
   const bool keep_free = !with_halo && p.halo_rows > 0;
   Q.first_idle_sm = keep_free ? M.first_idle_sm : INT_MAX;
-  TF_CUDA(tfk::launch_lattice_march(keep_free ? M.grid : std::min(M.grid, std::max(1, item_end - item_begin)), tm, tm_odd, Q, s));
-  p.launches = 1;
+  if (M.ragged) TF_CUDA(tfk::launch_pad_rows(C, p.first_cols, p.n_cols, ld, p.g_pad.p, s));
+  TF_CUDA(tfk::launch_lattice_march(keep_free ? M.grid : std::min(M.grid, std::max(1, item_end - item_begin)), tm, tm_odd, Q, M.halves, M.ragged, s));
+  p.launches = M.ragged ? 2 : 1;
   return TF_OK;
 }
 
@@ -679,7 +695,7 @@ int make_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &F, const tf_csr 
   p->hp.inter_rows = p->m;
   p->hp.n_prod = (p->first_is_second ? p->g_second : p->g_first).n_units;
   p->hp.n_cons = p->g_second.n_units;
-  if (o.lattice_march >= 0 && p->n_cols % 4 == 0) {
+  if (o.lattice_march >= 0) {
     rc = build_march(*p, &F, A, 0, sm_count, {});
     if (rc != TF_OK) return rc;
   }
@@ -1179,7 +1195,7 @@ tfk::Params base_params(tf_plan &p) {
 
 bool aligned(const void *q, size_t a) { return (reinterpret_cast<uintptr_t>(q) % a) == 0; }
 bool march_usable(const tf_plan &p, const float *C, const float *D) {
-  return p.march.on && !(p.keep_t && p.march.nx % 2) && aligned(C, 16) && aligned(D, 16);
+  return p.march.on && !(p.keep_t && p.march.halves) && (p.march.ragged || (aligned(C, 16) && aligned(D, 16)));
 }
 
 // vector width usable with the caller's pointers (plan-owned buffers are always aligned)

@@ -154,12 +154,27 @@ __global__ void __launch_bounds__(kGatherThreads, kGatherCtas) gather_kernel(con
   put(P.out + own + (size_t)h.x * P.ld_out, P.relu != 0);
 }
 
+// Rows of n_cols floats to rows of ld, the next multiple of four, with zeros behind.  Memory bounds it where no thread divides
+// for every element: a thread steps through (row, column) instead (100 000 rows of 47, two products of a graph behind it: 81 us, 75 now).
 __global__ void pad_rows_kernel(const float *__restrict__ src, long long rows, int n_cols, int ld, float *__restrict__ dst) {
-  const long long total = rows * ld;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / ld;
-    const int c = (int)(i - r * ld);
-    dst[i] = c < n_cols ? __ldg(src + r * n_cols + c) : 0.f;
+  const int q = ld / 4;
+  const long long step = (long long)gridDim.x * blockDim.x, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long dr = step / q;
+  const int dc = (int)(step - dr * q);
+  long long r = first / q;
+  int c = (int)(first - r * q);
+  while (r < rows) {
+    const float *p = src + r * n_cols + 4 * c;
+    const int left = n_cols - 4 * c;
+    float4 v;
+    v.x = __ldg(p);  // (left > 0: ld is less than four columns wider)
+    v.y = left > 1 ? __ldg(p + 1) : 0.f;
+    v.z = left > 2 ? __ldg(p + 2) : 0.f;
+    v.w = left > 3 ? __ldg(p + 3) : 0.f;
+    *reinterpret_cast<float4 *>(dst + r * ld + 4 * c) = v;
+    r += dr;
+    c += dc;
+    if (c >= q) { c -= q; ++r; }
   }
 }
 
@@ -205,9 +220,9 @@ cudaError_t launch_gather(bool vec_in, bool vec_out, const GatherParams &p, cuda
 }
 
 cudaError_t launch_pad_rows(const float *src, long long rows, int n_cols, int ld, float *dst, cudaStream_t s) {
-  const long long total = rows * ld;
+  const long long total = rows * (ld / 4);
   if (total <= 0) return cudaSuccess;
-  pad_rows_kernel<<<(int)std::min<long long>((total + 255) / 256, 148LL * 16), 256, 0, s>>>(src, rows, n_cols, ld, dst);
+  pad_rows_kernel<<<(int)std::min<long long>((total + 255) / 256, 148LL * 8), 256, 0, s>>>(src, rows, n_cols, ld, dst);
   return cudaGetLastError();
 }
 

@@ -74,6 +74,7 @@ int sddmm_group(int kq, int nv);              // lanes that work on a unit
 int sddmm_resident(int kq, int nv);           // threads of the kernel resident per SM
 cudaError_t launch_sddmm_gather(const GatherParams &p, const float *Q, const float *K, int kq, int m, cudaStream_t s);
 // dst[r][0:ld] = src[r][0:n_cols], the rest zero: rows of a width that is no multiple of four made readable as float4.
+// (dst on a 16-byte boundary, ld the next multiple of four)
 cudaError_t launch_pad_rows(const float *src, long long rows, int n_cols, int ld, float *dst, cudaStream_t s);
 
 }  // namespace tfk

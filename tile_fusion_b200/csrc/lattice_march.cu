@@ -268,7 +268,7 @@ static_assert(W == 16 && H == 8 && kMarchThreads == 128 && kMarchCols == 16,
 
 // One work item, seen by one thread: its 2 x 2 patch of the tile at (x, y) (both products) and kRing single
 // rows of the ring of T around the tile at (rx[r], ry[r]) (first product only; `ring` = this warp has any).
-template <bool ODD>
+template <bool ODD, bool RAGGED>
 __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParams &P, const Shared &S, CtaState &cs,
                                          int x0, int y0, int zs, int ze, int c0col, int x, int y, bool ring,
                                          const int (&rx)[kRing], const int (&ry)[kRing], bool pair_x,
@@ -383,7 +383,17 @@ __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParam
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float4 d = fma4(czpD[j], tcur[j], accD[j]);
-        if (live >> j & 1u) *reinterpret_cast<float4 *>(dptr + (j & 1) * (size_t)P.n_cols + (j >> 1) * drow) = d;
+        if (live >> j & 1u) {
+          float *q = dptr + (j & 1) * (size_t)P.n_cols + (j >> 1) * drow;
+          if (RAGGED) {
+            q[0] = d.x;
+            if (col + 1 < P.n_cols) q[1] = d.y;
+            if (col + 2 < P.n_cols) q[2] = d.z;
+            if (col + 3 < P.n_cols) q[3] = d.w;
+          } else {
+            *reinterpret_cast<float4 *>(q) = d;
+          }
+        }
       }
     }
     // T(k): everything but the z+ product
@@ -464,8 +474,8 @@ __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParam
 
 }  // namespace
 
-// ODD: the x extent is odd.
-template <bool ODD>
+// ODD: planes come from the two half maps (any x extent; the only form for an odd one).  RAGGED: rows of D are no multiple of four columns.
+template <bool ODD, bool RAGGED>
 __global__ void __launch_bounds__(kMarchThreads, kMarchCtasPerSm)
 lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_odd, const MarchParams P) {
   const PlaneMaps maps{&tm_c, &tm_odd};
@@ -554,7 +564,7 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
     int rx[kRing], ry[kRing];
 #pragma unroll
     for (int r = 0; r < kRing; ++r) { rx[r] = x0 + rdx[r]; ry[r] = y0 + rdy[r]; }
-    if (!run_item<ODD>(maps, P, S, cs, x0, y0, zs, ze, c0col, x0 + 2 * pi, y0 + 2 * warp, ring, rx, ry, warp < 2, nxt, pre, loader)) { failed = true; break; }
+    if (!run_item<ODD, RAGGED>(maps, P, S, cs, x0, y0, zs, ze, c0col, x0 + 2 * pi, y0 + 2 * warp, ring, rx, ry, warp < 2, nxt, pre, loader)) { failed = true; break; }
   }
   if (failed && tid == 0) atomicExch(&P.st->error, 1);
   // A thread that gave up has raised the CTA's abort flag; the others notice it in their own bounded waits
@@ -742,11 +752,11 @@ int march_make_half_map(CUtensorMap *out, const float *c, int n_cols, int nx, in
 }
 
 // CTAs of the kernel that fit one SM (0 on error).  The first call also raises the kernel's shared-memory limits.
-template <bool ODD>
+template <bool ODD, bool RAGGED>
 static int ctas_per_sm() {
   static int occ = -1;
   if (occ >= 0) return occ;
-  const void *fn = (const void *)lattice_march_kernel<ODD>;
+  const void *fn = (const void *)lattice_march_kernel<ODD, RAGGED>;
   int n = 0;
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMarchSmemBytes) != cudaSuccess ||
       cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
@@ -755,11 +765,12 @@ static int ctas_per_sm() {
   occ = n;
   return occ;
 }
-int march_ctas_per_sm() { return std::min(ctas_per_sm<false>(), ctas_per_sm<true>()); }
+int march_ctas_per_sm() { return std::min({ctas_per_sm<false, false>(), ctas_per_sm<true, false>(), ctas_per_sm<true, true>()}); }
 
-cudaError_t launch_lattice_march(int grid, const CUtensorMap &tm_c, const CUtensorMap &tm_odd, const MarchParams &p, cudaStream_t s) {
+cudaError_t launch_lattice_march(int grid, const CUtensorMap &tm_c, const CUtensorMap &tm_odd, const MarchParams &p, bool halves, bool ragged, cudaStream_t s) {
   if (march_ctas_per_sm() <= 0) return cudaErrorLaunchOutOfResources;
-  (p.nx % 2 ? lattice_march_kernel<true> : lattice_march_kernel<false>)<<<grid, kMarchThreads, kMarchSmemBytes, s>>>(tm_c, tm_odd, p);
+  auto f = ragged ? lattice_march_kernel<true, true> : (halves ? lattice_march_kernel<true, false> : lattice_march_kernel<false, false>);
+  f<<<grid, kMarchThreads, kMarchSmemBytes, s>>>(tm_c, tm_odd, p);
   return cudaGetLastError();
 }
 

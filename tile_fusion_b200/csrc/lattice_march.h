@@ -47,10 +47,12 @@ struct MarchParams {
 int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, int lines, long long planes,
                    int box_lines = kMarchH + 4);
 int march_ctas_per_sm();
-// Where nx is odd: the points with even (odd) x as (n_cols, x / 2, y, plane), box = 16 columns x (W+4)/2 x (H+4) x 1.
+// Half maps: the points with even (odd) x as (n_cols, x / 2, y, plane), box = 16 columns x (W+4)/2 x (H+4) x 1.
 int march_make_half_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, long long planes, int odd_x);
-// Where nx is odd: tm_c and tm_odd are the half maps, else tm_c is march_make_map's.
-cudaError_t launch_lattice_march(int grid, const CUtensorMap &tm_c, const CUtensorMap &tm_odd, const MarchParams &p, cudaStream_t s);
+// halves: tm_c and tm_odd are the half maps (any nx; needed where it is odd), and rows of T that do not exist are zero rather than a
+// product with it; else tm_c is march_make_map's.  ragged (with halves): D's rows of p.n_cols floats are stored value by value, the
+// maps are of rows padded to a multiple of four.
+cudaError_t launch_lattice_march(int grid, const CUtensorMap &tm_c, const CUtensorMap &tm_odd, const MarchParams &p, bool halves, bool ragged, cudaStream_t s);
 
 // One product D = A * T (p.out, p.pcls_a, p.dict_a): tm is a map of T with boxes of kMarchH + 2 lines.
 int star_ctas_per_sm();
