@@ -479,15 +479,16 @@ std::vector<int4> march_items_raw(const std::vector<tf::MarchItem> &items) {
   return raw;
 }
 
+// The narrowest width off the multiples of four that marches plane by plane: 16 columns are computed whatever the width, so one to three stay with
+// the gather, whose reads of four columns are a quarter of that (5 columns at 100 x 90 x 110: 187 us there, 71 here).
+constexpr int kMarchMinRagged = 5;
+
 // Plane-marching executor: taken when both operators of an SpMM-SpMM chain are star stencils on the same
 // grid (lattice.cpp).  The general plan is built as well and serves calls whose operands are not 16-byte
 // aligned.
 // Fp == null: the first operator is the identity (GeMM-SpMM: the dense producer has written T, and the marching
 // kernel computes D = A * (I * T); the products with the identity's zeros and its one are exact, so D is what the
 // CSR consumer gives).
-// The narrowest width off the multiples of four that marches: 16 columns are computed whatever the width, so one to three stay with
-// the gather, whose reads of four columns are a quarter of that (5 columns at 100 x 90 x 110: 187 us there, 71 here).
-constexpr int kMarchMinRagged = 5;
 // star: behind the dense product on the one-product march.  Taken only where every row names all of its neighbours: the march
 // multiplies a neighbour that is not named by zero, and an infinity there would not stay where it belongs.
 int build_march(tf_plan &p, const tf_csr *Fp, const tf_csr &A, int halo_rows, int sm_count, const std::vector<int> &boundary_rows,

@@ -25,6 +25,9 @@
 // the lanes that share an entry in one broadcast, where a 16-byte load from shared memory costs four
 // wavefronts of the pipe that is this kernel's busiest.
 //
+// Where the x extent is odd, or a row of D is no multiple of four columns (C is then a padded copy), the plane comes as two 4-D boxes,
+// its even and its odd points, and rows of T that do not exist are set to zero instead of being multiplied by it.
+//
 // Every wait is bounded: a thread whose wait runs out raises the CTA's abort flag, the CTA leaves the item
 // loop together, waits (bounded) for its copies in flight, sets the error flag and returns.
 #include <cuda.h>
