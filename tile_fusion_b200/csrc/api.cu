@@ -1067,8 +1067,8 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
     p->dyn_smem = std::max(p->dyn_smem, (size_t)tfk::tc_smem_bytes_host(n_cols));
     if (o.rows_per_block == 0) pp.rows_per_block = tfk::kTcRowsHost;
     pp.max_block_nnz = pp.rows_per_block * 32;
-    rc = p->w_hi.alloc((size_t)tfk::row_gemm_pad_k(k_dim) * tfk::row_gemm_pad_n(n_cols));  // either producer's form
-    if (rc == TF_OK) rc = p->w_lo.alloc((size_t)tfk::row_gemm_pad_k(k_dim) * tfk::row_gemm_pad_n(n_cols));
+    rc = p->w_hi.alloc((size_t)k_dim * tfk::row_gemm_pad_n(n_cols));  // either producer's form (k_dim is a multiple of four)
+    if (rc == TF_OK) rc = p->w_lo.alloc((size_t)k_dim * tfk::row_gemm_pad_n(n_cols));
     if (rc == TF_OK) rc = tfk::tc_make_map(&p->tm_whi, p->w_hi.p, n_cols, k_dim, n_cols);
     if (rc == TF_OK) rc = tfk::tc_make_map(&p->tm_wlo, p->w_lo.p, n_cols, k_dim, n_cols);
     if (rc == TF_OK) rc = finish_plan(*p, o, sm_count, false);

@@ -55,43 +55,10 @@ __device__ __forceinline__ void pair_mma(unsigned d, unsigned long long da, unsi
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
 }
-// The same with bf16 operands, sixteen terms at a time.
-__device__ __forceinline__ unsigned pair_idesc_bf16(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(2 * kTcRows >> 4) << 24);
-}
-__device__ __forceinline__ void pair_mma_bf16(unsigned d, unsigned long long da, unsigned long long db, unsigned idesc, unsigned acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
-}
 // Both CTAs' barriers at this offset are arrived on when the products issued so far have been computed.
 __device__ __forceinline__ void pair_commit(unsigned long long *bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
                    smem_u32(bar)), "h"((unsigned short)3) : "memory");
-}
-
-// ---- the mixed form: x = hi + lo, hi*hi from TF32, hi*lo + lo*hi from bf16 ----
-// Rounded to eight bits, the small products lose half a millionth of the result; what the tensor core cuts off of a wide
-// product's one accumulator is more from about 128 terms on, and the mixed form adds to it a third less
-// often (sixteen terms of bf16 at a time, eight of TF32) and takes two thirds of the tensor core's time.
-// Two numbers as bf16, the first in the low half.  (A number that would round to infinity is cut; so is a NaN's, whose lo keeps it.)
-__device__ __forceinline__ float bf16_range(float x) { return fminf(fmaxf(x, -__uint_as_float(0x7f7f0000u)), __uint_as_float(0x7f7f0000u)); }
-__device__ __forceinline__ unsigned bf16_pack(float a, float b) {
-  unsigned d;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(b), "f"(a));
-  return d;
-}
-// Of a row of 32 values, four to a lane (lane c of eight those from 4 c on), the row of 64 bf16 that the small products read: hi of
-// all of them, then lo (the weight has it the other way round).  Lanes c and c ^ 1 are neighbours in a warp.  Returns this lane's
-// sixteen bytes and their place among the row's eight.
-__device__ __forceinline__ uint4 cross_quad(const float4 &x, const float4 &lo, int c, int &place) {
-  const uint2 h = make_uint2(bf16_pack(bf16_range(x.x), bf16_range(x.y)), bf16_pack(bf16_range(x.z), bf16_range(x.w)));
-  const uint2 l = make_uint2(bf16_pack(lo.x, lo.y), bf16_pack(lo.z, lo.w));
-  const bool odd = c & 1;
-  const unsigned a = __shfl_xor_sync(kFull, odd ? h.x : l.x, 1), b = __shfl_xor_sync(kFull, odd ? h.y : l.y, 1);
-  place = (odd ? 4 : 0) + (c >> 1);
-  return odd ? make_uint4(a, b, l.x, l.y) : make_uint4(h.x, h.y, a, b);
 }
 
 // 32 (16) columns of a warp's 32 tensor-memory lanes.  The registers hold them after tcgen05.wait::ld only: tmem_loaded keeps the

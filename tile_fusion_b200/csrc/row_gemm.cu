@@ -49,10 +49,6 @@ constexpr int kRgAhead = 3, kRgAheadSlices = 8, kRgAheadWidth = 128;
 // uniform operands, 1.02e-7 and 1.03e-7 on normal ones, 6.1e-8 and 8.3e-8 on positive ones; 17 terms: 8.6e-8 and 7.6e-8);
 // shapes of fewer that the tensor-core tile does not take are multiplied with those.
 constexpr int kRgPreciseMinK = 32;
-// Terms from which on the mixed form is no less exact than three TF32 products (256 columns, rel., uniform and normal operands: 256 terms 1.32e-6
-// and 1.86e-6, 128 terms 8.0e-7 to 8.4e-7 and 9.6e-7; but 100 terms, 160 columns, normal 8.5e-7 and 8.1e-7; 64 terms 7.1e-7 and 5.2e-7).  2.1 M
-// rows, 256 -> 256: 908 us and 1 014.
-constexpr int kRgMixedMinK = 128;
 constexpr int kRgPrecisePanel = 64;  // columns: four accumulators, twice, in 512 columns of tensor memory
 constexpr int kRgSmemMax = 227 * 1024;
 constexpr int kRgEpiBytes = 8 * 32 * 128;  // 32 x 32 blocks: two per warp, one where eight warps drain
@@ -83,9 +79,9 @@ __device__ __forceinline__ void rg_split(float x, float round_low, float &hi, fl
   lo = (x - __uint_as_float(h & 0xffffe000u)) * round_low;
 }
 
-// PRECISE: see above; n_pad <= 64.  MIXED: see pair_mma.cuh; one accumulator.
+// PRECISE: see above; n_pad <= 64.
 // n_pad: columns of W rounded up to 32 (rows of the split weight beyond n_real are zero).
-template <bool PRECISE, bool MIXED>
+template <bool PRECISE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(rg_threads(PRECISE), 1)
 row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_whi,
                 const __grid_constant__ CUtensorMap tm_wlo, const __grid_constant__ CUtensorMap tm_out, const RowGemmParams P) {
@@ -170,7 +166,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   } else if (warp == kRgEpiWarps + kRgSplitWarps + 1) {
     // ---- products (even CTA): the whole warp, see elect_one ----
     if (rank == 0) {
-      const unsigned idesc = pair_idesc(N), idesc_small = pair_idesc_bf16(N);
+      const unsigned idesc = pair_idesc(N);
       int st = 0, buf = 0, uses = 0;  // uses: accumulators handed out so far
       unsigned ph = 0, acc_ph = 0;
       bool ok = true;
@@ -200,12 +196,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                      idesc, add);
           };
           if (elect_one()) {
-            if (MIXED) {
-#pragma unroll
-              for (int j = 0; j < kTcKSlice / 8; ++j) pair_mma_bf16(d, al + j * kUmmaStep, wl + j * kUmmaStep, idesc_small, fresh && j == 0 ? 0u : 1u);
-#pragma unroll
-              for (int j = 0; j < kTcKSlice / 8; ++j) mma(j, 2, 1u);
-            } else if (accs > 1 || P.small_first) {
+            if (accs > 1 || P.small_first) {
 #pragma unroll
               for (int term = 0; term < 3; ++term)
 #pragma unroll
@@ -238,7 +229,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     // ---- split the raw rows: hi in place, lo beside it ----
     const int w = tid - 32 * kRgEpiWarps;
     constexpr int kStep = 32 * kRgSplitWarps, kQuads = kTcRows * 8 / kStep;  // quads of a thread in a slice, from one to the next
-    const float round_low = MIXED || P.cut_low ? 1.f : kRgRoundLow;
+    const float round_low = P.cut_low ? 1.f : kRgRoundLow;
     int st = 0;
     unsigned ph = 0;
     bool ok = true;
@@ -267,14 +258,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           rg_split(a[i].x, round_low, h.x, l.x); rg_split(a[i].y, round_low, h.y, l.y);
           rg_split(a[i].z, round_low, h.z, l.z); rg_split(a[i].w, round_low, h.w, l.w);
           hi[w + i * kStep] = h;
-          if (MIXED) {
-            const int q = w + i * kStep, r = q >> 3;
-            int place;
-            const uint4 b = cross_quad(a[i], l, (q ^ r) & 7, place);
-            reinterpret_cast<uint4 *>(lo)[r * 8 + (place ^ (r & 7))] = b;
-          } else {
-            lo[w + i * kStep] = l;
-          }
+          lo[w + i * kStep] = l;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read next by the tensor core
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -463,8 +447,7 @@ row_fma_kernel(const float *__restrict__ X, int m, int K, int ld_x, const float 
 }
 
 // hi / lo [n_pad][ldk] (K contiguous, rows from n on and columns from K on zero) from W [K][n], or from W [n][K] when w_transposed.
-// mixed: the place of 32 columns of lo holds their 64 bf16, lo of all of them and then hi.
-__global__ void split_weight_pad_kernel(const float *__restrict__ W, int w_transposed, int K, int ldk, int n, int n_pad, bool ticket, bool mixed,
+__global__ void split_weight_pad_kernel(const float *__restrict__ W, int w_transposed, int K, int ldk, int n, int n_pad, bool ticket,
                                         float *__restrict__ hi, float *__restrict__ lo) {
   const int total = n_pad * ldk;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -473,13 +456,7 @@ __global__ void split_weight_pad_kernel(const float *__restrict__ W, int w_trans
     if (r < n && k < K) w = w_transposed ? __ldg(W + (size_t)r * K + k) : __ldg(W + (size_t)k * n + r);
     const float h = tf32_round(w);
     hi[i] = h;
-    if (mixed) {
-      unsigned short *o = reinterpret_cast<unsigned short *>(lo + (i - (k & 31))) + (k & 31);
-      o[0] = (unsigned short)bf16_pack(w - h, 0.f);
-      o[32] = (unsigned short)bf16_pack(bf16_range(w), 0.f);
-    } else {
-      lo[i] = ticket ? w - h : tf32_round(w - h);
-    }
+    lo[i] = ticket ? w - h : tf32_round(w - h);
   }
 }
 
@@ -487,8 +464,7 @@ __global__ void split_weight_pad_kernel(const float *__restrict__ W, int w_trans
 
 bool row_gemm_supported(int n) { return n >= 1 && n <= kTcMaxN; }
 int row_gemm_pad_n(int n) { return (n + 31) / 32 * 32; }  // cta_group::2 takes multiples of 32
-int row_gemm_pad_k(int k) { return (k + kTcKSlice - 1) / kTcKSlice * kTcKSlice; }
-bool row_gemm_mixed(int K, int n) { return tc_supported(K, n) && row_gemm_pad_n(n) > 128 && K >= kRgMixedMinK; }
+int row_gemm_pad_k(int k) { return (k + 3) / 4 * 4; }
 
 RowGemmForm row_gemm_form(int K, int n) { return tc_supported(K, n) ? kRowTile : (K >= kRgPreciseMinK ? kRowPrecise : kRowFma); }
 
@@ -496,7 +472,7 @@ cudaError_t row_gemm_split(const float *W, int w_transposed, int K, int n, RowGe
   if (row_gemm_form(K, n) == kRowFma) return cudaSuccess;
   const bool ticket = sums == kSumsTicket && row_gemm_form(K, n) == kRowTile;
   const int ldk = row_gemm_pad_k(K), n_pad = row_gemm_pad_n(n);
-  split_weight_pad_kernel<<<std::min((n_pad * ldk + 255) / 256, 148 * 4), 256, 0, s>>>(W, w_transposed, K, ldk, n, n_pad, ticket, sums != kSumsTicket && row_gemm_mixed(K, n), hi, lo);
+  split_weight_pad_kernel<<<std::min((n_pad * ldk + 255) / 256, 148 * 4), 256, 0, s>>>(W, w_transposed, K, ldk, n, n_pad, ticket, hi, lo);
   return cudaGetLastError();
 }
 
@@ -518,7 +494,6 @@ static int launch_panel(const float *X, int m, int K, int ld_x, const float *W, 
   RowGemmParams P;
   P.x = X; P.k = K; P.ld_x = ld_x;
   P.w = W; P.w_k = w_k; P.w_c = w_c;
-  P.mixed = sums != kSumsTicket && !precise && row_gemm_mixed(K, n) ? 1 : 0;
   P.cut_low = sums != kSumsFree ? 1 : 0;
   P.small_first = sums == kSumsSpmmGemm ? 1 : 0;
   P.direct = ld_x % 4 != 0 || (reinterpret_cast<uintptr_t>(X) & 15) != 0;
@@ -537,7 +512,7 @@ static int launch_panel(const float *X, int m, int K, int ld_x, const float *W, 
   if (rc == TF_OK && P.tma_store) rc = tc_make_map(&mo, out, m, n, 32, ld_out);
   if (rc != TF_OK) return rc;
   const size_t smem = (size_t)P.stages * rg_stage_bytes(n_pad) + kRgEpiBytes + 1024;
-  auto f = precise ? row_gemm_kernel<true, false> : (P.mixed ? row_gemm_kernel<false, true> : row_gemm_kernel<false, false>);
+  auto f = precise ? row_gemm_kernel<true> : row_gemm_kernel<false>;
   // (the limit is the kernel's, not the call's: the same for all widths, so that threads with different plans don't lower it
   // for one another)
   cudaError_t e = cudaFuncSetAttribute((const void *)f, cudaFuncAttributeMaxDynamicSharedMemorySize, kRgSmemMax - 1024);

@@ -11,13 +11,12 @@ struct RowGemmParams {
   int *error;
   int m, n_real, n_pad, n_slices, tiles, stages, accs, ld_out, k, ld_x;
   int direct, relu, tma_store, wait_limit, w_k, w_c;
-  int mixed;
   int cut_low, small_first;  // the low halves of X are not rounded; the small products of a slice come first whatever the accumulators
 };
 
 // Whose sums a product's are, bit for bit: nobody's; the ticket executor's tile, where there is one (one accumulator whatever the
 // width, no low half rounded); those of spmm_gemm.cu where that has one accumulator, above 128 columns (the small products of a
-// slice first, the low halves of X not rounded or, where the form is the mixed one, as it has them).
+// slice first, the low halves of X not rounded).
 enum RowGemmSums { kSumsFree, kSumsTicket, kSumsSpmmGemm };
 bool row_gemm_supported(int n);  // n <= 256 columns
 // Which of its forms a product takes (see row_gemm.cu).
@@ -25,9 +24,6 @@ enum RowGemmForm { kRowTile, kRowPrecise, kRowFma };
 RowGemmForm row_gemm_form(int K, int n);
 int row_gemm_pad_n(int n);       // rows of the split weight
 int row_gemm_pad_k(int k);       // floats per row of it
-// Whether the small products of a shape of the tensor-core tile are multiplied in bf16 (see pair_mma.cuh): wide ones of 128 terms and more,
-// for everybody's sums but the ticket executor's.
-bool row_gemm_mixed(int K, int n);
 // hi, lo: row_gemm_pad_n(n) x row_gemm_pad_k(K) floats each.  W is K x n, or n x K when w_transposed.  (kRowFma needs neither:
 // nothing is launched.)
 cudaError_t row_gemm_split(const float *W, int w_transposed, int K, int n, RowGemmSums sums, float *hi, float *lo, cudaStream_t s);

@@ -83,9 +83,8 @@ __device__ __forceinline__ void brick_origin(const tf::BrickGrid &g, int brick, 
   z = layer << g.lz;
 }
 
-// D3: seven points, else five.  RES: the weight lies in shared memory, else its slices come with the stages.  MIXED: see
-// pair_mma.cuh; one accumulator.
-template <bool D3, bool RES, bool MIXED>
+// D3: seven points, else five.  RES: the weight lies in shared memory, else its slices come with the stages.
+template <bool D3, bool RES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSgThreads, 1)
 spmm_gemm_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_cap, const __grid_constant__ CUtensorMap tm_whi,
                  const __grid_constant__ CUtensorMap tm_wlo, const __grid_constant__ SpmmGemmParams A) {
@@ -128,16 +127,8 @@ spmm_gemm_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_constant
       const float4 h = make_float4(tf32_round(x.x), tf32_round(x.y), tf32_round(x.z), tf32_round(x.w));
       char *o = wbuf + (q >> 3) * slice_w + r * 128 + (((q & 7) ^ (r & 7)) << 4);
       *reinterpret_cast<float4 *>(o) = h;
-      if (MIXED) {
-        char *b = wbuf + (q >> 3) * slice_w + half * 128 + r * 128 + (q & 1) * 8;
-        const int c2 = (q & 7) >> 1;  // lo of all columns, then hi
-        *reinterpret_cast<uint2 *>(b + ((c2 ^ (r & 7)) << 4)) = make_uint2(bf16_pack(x.x - h.x, x.y - h.y), bf16_pack(x.z - h.z, x.w - h.w));
-        *reinterpret_cast<uint2 *>(b + (((4 + c2) ^ (r & 7)) << 4)) =
-            make_uint2(bf16_pack(bf16_range(x.x), bf16_range(x.y)), bf16_pack(bf16_range(x.z), bf16_range(x.w)));
-      } else {
-        *reinterpret_cast<float4 *>(o + half * 128) =
-            make_float4(tf32_round(x.x - h.x), tf32_round(x.y - h.y), tf32_round(x.z - h.z), tf32_round(x.w - h.w));
-      }
+      *reinterpret_cast<float4 *>(o + half * 128) =
+          make_float4(tf32_round(x.x - h.x), tf32_round(x.y - h.y), tf32_round(x.z - h.z), tf32_round(x.w - h.w));
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -200,7 +191,7 @@ spmm_gemm_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_constant
   } else if (warp == kSgWarpMma) {
     // ---- products (even CTA): the whole warp, see elect_one ----
     if (rank == 0) {
-      const unsigned idesc = pair_idesc(N), idesc_small = pair_idesc_bf16(N);
+      const unsigned idesc = pair_idesc(N);
       int st = 0, buf = 0, uses = 0;
       unsigned ph = 0, acc_ph = 0;
       bool ok = true;
@@ -231,15 +222,10 @@ spmm_gemm_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_constant
             if (big == wrap) big = d;
           }
           if (elect_one()) {
-            if (MIXED) {
-#pragma unroll
-              for (int j = 0; j < kTcKSlice / 8; ++j) pair_mma_bf16(d, al + j * kUmmaStep, wl + j * kUmmaStep, idesc_small, first_slice && j == 0 ? 0u : 1u);
-            } else {
 #pragma unroll
             for (int j = 0; j < kTcKSlice / 8; ++j) pair_mma(small, al + j * kUmmaStep, wh + j * kUmmaStep, idesc, first_slice && j == 0 ? 0u : 1u);
 #pragma unroll
             for (int j = 0; j < kTcKSlice / 8; ++j) pair_mma(small, ah + j * kUmmaStep, wl + j * kUmmaStep, idesc, 1u);
-            }
 #pragma unroll
             for (int j = 0; j < kTcKSlice / 8; ++j) pair_mma(to[j], ah + j * kUmmaStep, wh + j * kUmmaStep, idesc, fresh[j] ? 0u : 1u);
             pair_commit(&s.empty[st]);
@@ -314,13 +300,7 @@ spmm_gemm_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_constant
           float4 hi, lo;
           split_tf32(a.x, hi.x, lo.x); split_tf32(a.y, hi.y, lo.y); split_tf32(a.z, hi.z, lo.z); split_tf32(a.w, hi.w, lo.w);
           *reinterpret_cast<float4 *>(stage + at[i]) = hi;
-          if (MIXED) {
-            int place;
-            const uint4 b = cross_quad(a, lo, c, place);
-            *reinterpret_cast<uint4 *>(stage + kSgRows * 128 + (r0 + i) * 128 + ((place ^ ((r0 + i) & 7)) << 4)) = b;
-          } else {
-            *reinterpret_cast<float4 *>(stage + at[i] + kSgRows * 128) = lo;
-          }
+          *reinterpret_cast<float4 *>(stage + at[i] + kSgRows * 128) = lo;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read next by the tensor core
         if (!RES && w == 0 && !(ok = __all_sync(kFull, pair_wait(&s.wfull[st], ph, s.dead, A.wait_limit)))) break;
@@ -480,11 +460,8 @@ int spmm_gemm(SpmmGemmParams p, const float *hi, const float *lo, int sm_count, 
   if (rc == TF_OK && !res) rc = tc_make_map(&mh, hi, p.n_pad, ldk, p.n_pad / 2, ldk);
   if (rc == TF_OK && !res) rc = tc_make_map(&ml, lo, p.n_pad, ldk, p.n_pad / 2, ldk);
   if (rc != TF_OK) return rc;
-  typedef void (*Fn)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const SpmmGemmParams);
-  const Fn fs[8] = {spmm_gemm_kernel<false, false, false>, spmm_gemm_kernel<false, false, true>, spmm_gemm_kernel<false, true, false>,
-                    spmm_gemm_kernel<false, true, true>,   spmm_gemm_kernel<true, false, false>, spmm_gemm_kernel<true, false, true>,
-                    spmm_gemm_kernel<true, true, false>,   spmm_gemm_kernel<true, true, true>};
-  const Fn f = fs[4 * deep + 2 * res + row_gemm_mixed(p.k, p.n)];
+  auto f = deep ? (res ? spmm_gemm_kernel<true, true> : spmm_gemm_kernel<true, false>)
+                : (res ? spmm_gemm_kernel<false, true> : spmm_gemm_kernel<false, false>);
   // (the limit is the kernel's, not the call's, see row_gemm.cu)
   cudaError_t e = cudaFuncSetAttribute((const void *)f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSgSmemMax);
   if (e == cudaSuccess) {
