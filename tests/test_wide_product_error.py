@@ -58,3 +58,20 @@ def test_terms(built_lib, route, kind, k, n_cols):
     rel = np.linalg.norm(_run(plan, b, w) - want) / np.linalg.norm(want)
     assert rel < BOUND[kind], rel
     plan.close()
+
+
+def _tf32(x):
+    return ((x.view(np.uint32) + np.uint32(0x1000)) & np.uint32(0xFFFFE000)).view(np.float32)
+
+
+# (up to 128 columns the two passes are the ticket executor's tile, which cuts the low halves off)
+@pytest.mark.parametrize("route,k", [(r, k) for r in ("default", "two_launches") for k in (64, 128, 256)] + [("two_passes", 256)])
+def test_low_halves_are_rounded(built_lib, route, k):
+    """Identity operator and weight: D is hi + lo with lo rounded to eleven bits, which fp32 holds exactly."""
+    dims = (70, 60)
+    n = dims[0] * dims[1]
+    b = synth.uniform(3, (n, k))
+    plan = api.Plan("gemm_spmm", api.CSRMatrix(n, n, *_identity(dims)), k=k, n_cols=k, **ROUTES[route])
+    hi = _tf32(b)
+    np.testing.assert_array_equal(_run(plan, b, np.eye(k, dtype=np.float32)), hi + _tf32(b - hi))
+    plan.close()

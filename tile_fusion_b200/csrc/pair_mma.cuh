@@ -61,6 +61,18 @@ __device__ __forceinline__ void pair_commit(unsigned long long *bar) {
                    smem_u32(bar)), "h"((unsigned short)3) : "memory");
 }
 
+// x = hi + lo for the tensor core, which reads the first eleven bits of either.  hi is rounded to them by the addition (its last bits
+// need not be cleared); a NaN may be lost there, but not in lo.  lo is a power of two or has at most twelve bits: if the last of
+// them is set, lo / 2048 carries into the bit before (it is at least one unit there and less than two), if not, what it adds
+// is cut off again, so that lo is rounded like hi.  (Clearing hi, rounding lo like hi and looking for NaNs first took
+// eight instructions of the half-rate integer pipe, which bounded the splitting, instead of two.)
+constexpr float kRoundLow = 1.f + 1.f / 2048;
+__device__ __forceinline__ void split_pair(float x, float round_low, float &hi, float &lo) {
+  const unsigned h = __float_as_uint(x) + 0x1000u;
+  hi = __uint_as_float(h);
+  lo = (x - __uint_as_float(h & 0xffffe000u)) * round_low;
+}
+
 // 32 (16) columns of a warp's 32 tensor-memory lanes.  The registers hold them after tcgen05.wait::ld only: tmem_loaded keeps the
 // compiler from using them before.
 __device__ __forceinline__ void tmem_load32(float (&v)[32], unsigned taddr) {

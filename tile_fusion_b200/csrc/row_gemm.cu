@@ -67,18 +67,6 @@ constexpr int rg_stages(int n) {
 }
 static_assert(rg_stages(256) >= 2, "a full-width tile needs two stages");
 
-// x = hi + lo for the tensor core, which reads the first eleven bits of either.  hi is rounded to them by the addition (its last bits
-// need not be cleared); a NaN may be lost there, but not in lo.  lo is a power of two or has at most twelve bits: if the last of
-// them is set, lo / 2048 carries into the bit before (it is at least one unit there and less than two), if not, what it adds
-// is cut off again, so that lo is rounded like hi.  (Clearing hi, rounding lo like hi and looking for NaNs first took
-// eight instructions of the half-rate integer pipe, which bounded the splitting, instead of two.)
-constexpr float kRgRoundLow = 1.f + 1.f / 2048;
-__device__ __forceinline__ void rg_split(float x, float round_low, float &hi, float &lo) {
-  const unsigned h = __float_as_uint(x) + 0x1000u;
-  hi = __uint_as_float(h);
-  lo = (x - __uint_as_float(h & 0xffffe000u)) * round_low;
-}
-
 // PRECISE: see above; n_pad <= 64.
 // n_pad: columns of W rounded up to 32 (rows of the split weight beyond n_real are zero).
 template <bool PRECISE>
@@ -229,7 +217,7 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     // ---- split the raw rows: hi in place, lo beside it ----
     const int w = tid - 32 * kRgEpiWarps;
     constexpr int kStep = 32 * kRgSplitWarps, kQuads = kTcRows * 8 / kStep;  // quads of a thread in a slice, from one to the next
-    const float round_low = P.cut_low ? 1.f : kRgRoundLow;
+    const float round_low = P.cut_low ? 1.f : kRoundLow;
     int st = 0;
     unsigned ph = 0;
     bool ok = true;
@@ -255,8 +243,8 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 #pragma unroll
         for (int i = 0; i < kQuads; ++i) {
           float4 h, l;
-          rg_split(a[i].x, round_low, h.x, l.x); rg_split(a[i].y, round_low, h.y, l.y);
-          rg_split(a[i].z, round_low, h.z, l.z); rg_split(a[i].w, round_low, h.w, l.w);
+          split_pair(a[i].x, round_low, h.x, l.x); split_pair(a[i].y, round_low, h.y, l.y);
+          split_pair(a[i].z, round_low, h.z, l.z); split_pair(a[i].w, round_low, h.w, l.w);
           hi[w + i * kStep] = h;
           lo[w + i * kStep] = l;
         }
@@ -494,7 +482,7 @@ static int launch_panel(const float *X, int m, int K, int ld_x, const float *W, 
   RowGemmParams P;
   P.x = X; P.k = K; P.ld_x = ld_x;
   P.w = W; P.w_k = w_k; P.w_c = w_c;
-  P.cut_low = sums != kSumsFree ? 1 : 0;
+  P.cut_low = sums == kSumsTicket ? 1 : 0;
   P.small_first = sums == kSumsSpmmGemm ? 1 : 0;
   P.direct = ld_x % 4 != 0 || (reinterpret_cast<uintptr_t>(X) & 15) != 0;
   int rc = tc_make_map(&mh, hi, n_pad, ldk, n_pad / 2, ldk);

@@ -16,7 +16,7 @@ struct RowGemmParams {
 
 // Whose sums a product's are, bit for bit: nobody's; the ticket executor's tile, where there is one (one accumulator whatever the
 // width, no low half rounded); those of spmm_gemm.cu where that has one accumulator, above 128 columns (the small products of a
-// slice first, the low halves of X not rounded).
+// slice first).
 enum RowGemmSums { kSumsFree, kSumsTicket, kSumsSpmmGemm };
 bool row_gemm_supported(int n);  // n <= 256 columns
 // Which of its forms a product takes (see row_gemm.cu).

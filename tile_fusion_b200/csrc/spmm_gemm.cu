@@ -63,13 +63,6 @@ __device__ __forceinline__ void load_points(void *smem, const CUtensorMap *tm, i
       "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
       ::"r"(smem_u32(smem)), "l"((unsigned long long)tm), "r"(smem_u32(bar)), "r"(col), "r"(x), "r"(y), "r"(z) : "memory");
 }
-// x = hi + lo for the tensor core, which reads the first eleven bits of either: hi is rounded to them by the addition.  x is the
-// result of an FMA, so a NaN has all bits set; hi loses it to the addition, lo keeps it.
-__device__ __forceinline__ void split_tf32(float x, float &hi, float &lo) {
-  const unsigned h = __float_as_uint(x) + 0x1000u;
-  hi = __uint_as_float(h);
-  lo = x - __uint_as_float(h & 0xffffe000u);
-}
 __device__ __forceinline__ float4 lds4(const char *p) { return *reinterpret_cast<const float4 *>(p); }
 __device__ __forceinline__ void fma4(float4 &a, float v, const float4 &x) {
   a.x = fmaf(v, x.x, a.x); a.y = fmaf(v, x.y, a.y); a.z = fmaf(v, x.z, a.z); a.w = fmaf(v, x.w, a.w);
@@ -298,7 +291,8 @@ spmm_gemm_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_constant
           fma4(a, v[i][5], lds4(x + centre + py + i * 128));
           if (D3) fma4(a, v[i][6], lds4(x + above + i * 128));
           float4 hi, lo;
-          split_tf32(a.x, hi.x, lo.x); split_tf32(a.y, hi.y, lo.y); split_tf32(a.z, hi.z, lo.z); split_tf32(a.w, hi.w, lo.w);
+          split_pair(a.x, kRoundLow, hi.x, lo.x); split_pair(a.y, kRoundLow, hi.y, lo.y);
+          split_pair(a.z, kRoundLow, hi.z, lo.z); split_pair(a.w, kRoundLow, hi.w, lo.w);
           *reinterpret_cast<float4 *>(stage + at[i]) = hi;
           *reinterpret_cast<float4 *>(stage + at[i] + kSgRows * 128) = lo;
         }
