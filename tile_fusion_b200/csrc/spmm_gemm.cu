@@ -158,17 +158,17 @@ spmm_gemm_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_constant
     if (!ok || s.dead)
       for (int i = 0; i < used; ++i) mbar_wait(&s.raw_full[i], i < rs ? rph : rph ^ 1u, A.wait_limit);
   } else if (warp == kSgWarpW) {
-    // ---- slices of the weight; the stages of this CTA until the last product that reads one is done ----
+    // ---- slices of the weight (where they come with the stages) ----
     int st = 0, issued = 0;
     unsigned ph = 0;
     bool ok = true;
     auto wait = [&](unsigned long long *bar, unsigned parity) {
       return ok = __all_sync(kFull, pair_wait(bar, parity, s.dead, A.wait_limit));
     };
-    for (int t = first; t < tiles && ok; t += pairs)
+    for (int t = RES ? tiles : first; t < tiles && ok; t += pairs)
       for (int sl = 0; sl < A.slices; ++sl) {
         if (issued >= A.stages && !wait(&s.empty[st], ph ^ 1u)) break;
-        if (!RES && elect_one()) {
+        if (elect_one()) {
           char *w = smem + st * stage_bytes + kSgStageA;
           mbar_expect_tx(&s.wfull[st], (unsigned)slice_w);
           tma_load_2d(w, &tm_whi, sl * kTcKSlice, (int)rank * half, &s.wfull[st]);
@@ -178,8 +178,7 @@ spmm_gemm_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_constant
         if (issued < A.stages) ++issued;
         if (++st == A.stages) { st = 0; ph ^= 1u; }
       }
-    for (int i = 0; ok && i < issued; ++i) wait(&s.empty[i], i < st ? ph : ph ^ 1u);
-    if (!RES && (!ok || s.dead))
+    if (!ok || s.dead)
       for (int i = 0; i < issued; ++i) mbar_wait(&s.wfull[i], i < st ? ph : ph ^ 1u, A.wait_limit);
   } else if (warp == kSgWarpMma) {
     // ---- products (even CTA): the whole warp, see elect_one ----
@@ -308,6 +307,10 @@ spmm_gemm_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_constant
         if (++rs == A.raws) { rs = 0; rph ^= 1u; }
       }
     }
+    // The tensor core's arrivals on the stages of this CTA come from the other one too: the last of them must be in before the CTA
+    // may end.  (For this a warp that waits for every phase as it comes: one that has nothing to do in between can be a phase of the
+    // same parity late, and then waits for one that never comes.)
+    for (int i = 0; w == 0 && ok && i < n; ++i) ok = __all_sync(kFull, pair_wait(&s.empty[i], i < st ? ph : ph ^ 1u, s.dead, A.wait_limit));
   } else {
     // ---- rows of D: warp w drains the rows 32 w .. 32 w + 31 of the CTA's tile ----
     int buf = 0;
