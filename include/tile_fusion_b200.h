@@ -221,7 +221,10 @@ int tf_exec_spmm_spmm(tf_plan *p, const float *C, float *D, void *stream);
 /* forwardForOneLayerFusedParallelSeparatedVectorizedSP
  * (fusion/gcn/GCN_Layer_MKL_Forward_Utils.h:218; weight k x n) and, with w_transposed != 0,
  * the scalar / torch-binding layout weight n x k (ibid. :182; binding-project/src/Functions.cpp:629).
- * relu != 0 applies max(0, .) to D (binding-project/gcn-e2e-training/FusedGCNModule.py:16). */
+ * relu != 0 applies max(0, .) to D (binding-project/gcn-e2e-training/FusedGCNModule.py:16).
+ * D may lie over B (k == n_cols, or in part) where the plan forms the two products one after the other.  Plans that run in one
+ * launch (star stencils, see tf_plan_opts.lattice_march) take a call whose D lies over B or W in two, with T in memory of the
+ * device's default pool for as long as the call runs. */
 int tf_exec_gemm_spmm(tf_plan *p, const float *B, const float *W, int w_transposed, int relu, float *D,
                       void *stream);
 

@@ -1524,23 +1524,42 @@ int run_one_launch(tf_plan &p, const float *B, const float *W, int w_transposed,
   return tfk::spmm_gemm(P, p.w_hi.p, p.w_lo.p, p.sm_count, s);
 }
 
-int run_gather_gemm_spmm(tf_plan &p, const float *B, const float *W, int w_transposed, bool relu, float *D, cudaStream_t s) {
+// The two products in launches of their own, T in between (`t`, rows of p.ld_t floats).
+int run_two_products(tf_plan &p, const float *B, const float *W, int w_transposed, bool relu, float *D, float *t, cudaStream_t s) {
   const int n = p.n_cols, k = p.k_dim;
-  const bool out16 = n % 4 == 0 && aligned(D, 16);
-  if (p.dyn_smem > 0 && !(aligned(B, 16) && aligned(D, 16)))
-    return fail(TF_ERR_ARG, "this plan (gather tiles or tensor-core producer) needs 16-byte aligned dense operands "
-                            "(build the plan with tile_slots < 0 and tensor_cores < 0 otherwise)");
-  if (p.one.on && !p.keep_t) return run_one_launch(p, B, W, w_transposed, relu, D, 0, p.one.par.grid.bricks(), true, s);
   TF_CUDA(tfk::row_gemm_split(W, w_transposed, k, n, p.sums(), p.w_hi.p, p.w_lo.p, s));
   p.launches = tfk::row_gemm_form(k, n) == tfk::kRowFma ? 2 : 3;
   if (p.spmm_first) {
-    TF_TRY(run_gather(p.g_second, B, k, aligned(B, 16), p.inter.p, p.ld_t, true, k, false, s));
-    return tfk::row_gemm(p.inter.p, p.m, k, p.ld_t, W, w_transposed, p.w_hi.p, p.w_lo.p, n, D, n, relu, p.sums(), &p.state.p->error,
+    TF_TRY(run_gather(p.g_second, B, k, aligned(B, 16), t, p.ld_t, true, k, false, s));
+    return tfk::row_gemm(t, p.m, k, p.ld_t, W, w_transposed, p.w_hi.p, p.w_lo.p, n, D, n, relu, p.sums(), &p.state.p->error,
                          p.spin_limit, p.sm_count, s);
   }
-  TF_TRY(tfk::row_gemm(B, p.m, k, k, W, w_transposed, p.w_hi.p, p.w_lo.p, n, p.inter.p, p.ld_t, false, p.sums(),
+  TF_TRY(tfk::row_gemm(B, p.m, k, k, W, w_transposed, p.w_hi.p, p.w_lo.p, n, t, p.ld_t, false, p.sums(),
                        &p.state.p->error, p.spin_limit, p.sm_count, s));
-  return run_gather(p.g_second, p.inter.p, p.ld_t, true, D, n, out16, n, relu, s);
+  return run_gather(p.g_second, t, p.ld_t, true, D, n, n % 4 == 0 && aligned(D, 16), n, relu, s);
+}
+
+bool overlap(const float *a, size_t na, const float *b, size_t nb) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return x < y + nb * sizeof(float) && y < x + na * sizeof(float);
+}
+
+int run_gather_gemm_spmm(tf_plan &p, const float *B, const float *W, int w_transposed, bool relu, float *D, cudaStream_t s) {
+  const size_t rows = (size_t)p.m, n = (size_t)p.n_cols, k = (size_t)p.k_dim;
+  if (p.dyn_smem > 0 && !(aligned(B, 16) && aligned(D, 16)))
+    return fail(TF_ERR_ARG, "this plan (gather tiles or tensor-core producer) needs 16-byte aligned dense operands "
+                            "(build the plan with tile_slots < 0 and tensor_cores < 0 otherwise)");
+  if (!p.one.on || p.keep_t) return run_two_products(p, B, W, w_transposed, relu, D, p.inter.p, s);
+  if (!overlap(D, rows * n, B, rows * k) && !overlap(D, rows * n, W, k * n))
+    return run_one_launch(p, B, W, w_transposed, relu, D, 0, p.one.par.grid.bricks(), true, s);
+  // The one launch reads B and W while it writes D.  Where D lies over either, T is formed first; it comes from the stream's pool
+  // for the call, so that such a call can be captured as any other.
+  float *t = nullptr;
+  TF_CUDA(cudaMallocAsync(&t, rows * p.ld_t * sizeof(float), s));
+  const int rc = run_two_products(p, B, W, w_transposed, relu, D, t, s);
+  const cudaError_t e = cudaFreeAsync(t, s);
+  if (rc == TF_OK) TF_CUDA(e);
+  return rc;
 }
 
 int set_device(const tf_plan &p) {
