@@ -202,7 +202,7 @@ band_lane_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_constant
   for (int s = jb - 1; s <= je + 1; ++s) {
     if (warp == 0 && s + 2 >= issued && s + 2 < end) { load(s + 2); issued = s + 3; }
     for (; ok && landed < min(end, s + 2); ++landed)
-      ok = mbar_wait(&full[landed & 3], (unsigned)((landed - first) >> 2) & 1u, P.wait_limit);
+      ok = __all_sync(kFull, mbar_wait(&full[landed & 3], (unsigned)((landed - first) >> 2) & 1u, P.wait_limit));  // (the warp leaves as one)
     float4 acc[8];
     if (warp < kHalf) {
       if (ok && s >= 0 && s < P.blocks && s <= je) {
