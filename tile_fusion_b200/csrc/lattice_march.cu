@@ -45,6 +45,7 @@ namespace tfk {
 namespace {
 
 constexpr int W = kMarchW, H = kMarchH;
+constexpr unsigned kAll = 0xffffffffu;
 constexpr int PC = W + 4;  // pitch (rows) of the staged C rectangle
 constexpr int PT = W + 2;  // pitch of the T rectangle
 
@@ -55,16 +56,18 @@ __device__ __forceinline__ void mbar_init(unsigned bar, int count) {
 __device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ bool mbar_try(unsigned a, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done) : "r"(a), "r"(parity) : "memory");
+  return done != 0;
+}
 __device__ __forceinline__ bool mbar_wait(unsigned a, unsigned parity, int limit) {
-  for (int i = 0; i < limit; ++i) {
-    unsigned done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(a), "r"(parity) : "memory");
-    if (done) return true;
-  }
+  for (int i = 0; i < limit; ++i)
+    if (mbar_try(a, parity)) return true;
   return false;
 }
 // One plane of C for a tile: coordinates (column, x / 2, x % 2, y, plane).
@@ -219,26 +222,14 @@ __device__ __forceinline__ bool elect_lane() {
 __device__ __forceinline__ void mbar_arrive(unsigned bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Bounded wait that also gives up when another thread of the CTA already has.
-__device__ __forceinline__ bool wait_or_abort(unsigned a, unsigned parity, int limit, volatile int *abort) {
-  {
-    unsigned done;   // the usual case: one try, no counters
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(a), "r"(parity) : "memory");
-    if (done) return true;
-  }
+// Bounded wait of a warp, which also gives up when another thread of the CTA already has.  The warp leaves as one: its lanes meet
+// afterwards, and those that were served would wait there without a limit for the others.  (128^3, 128 columns: 527 us without a vote, 531
+// like this, 1.4 % more with the vote behind a wait of the lanes', 5 % with one vote a step behind the loads.)
+__device__ __forceinline__ bool warp_wait(unsigned a, unsigned parity, int limit, volatile int *abort) {
+  if (__all_sync(kAll, mbar_try(a, parity))) return true;  // the usual case: one try, no counters
   for (int i = 0; i < limit; ++i) {
-    unsigned done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(a), "r"(parity) : "memory");
-    if (done) return true;
-    if ((i & 255) == 255 && *abort) break;
+    if (__all_sync(kAll, mbar_try(a, parity))) return true;
+    if ((i & 255) == 255 && __any_sync(kAll, *abort)) break;
   }
   *abort = 1;
   return false;
@@ -338,7 +329,7 @@ __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParam
                       unsigned &wa_next, unsigned wr, unsigned &wr_next) -> bool {
     const int k = kfirst + step;
     const unsigned stage = cs.n_use % kMarchStages;
-    if (!wait_or_abort(S.full + 8 * stage, (cs.n_use / kMarchStages) & 1u, P.wait_limit, S.abort)) return false;
+    if (!warp_wait(S.full + 8 * stage, (cs.n_use / kMarchStages) & 1u, P.wait_limit, S.abort)) return false;
     const unsigned cb = S.cbuf + stage * kMarchCBytes;
     float4 nb[8];
     const unsigned baseC = cb + boC;
@@ -426,7 +417,7 @@ __device__ __forceinline__ bool run_item(const PlaneMaps &tm_c, const MarchParam
       }
     }
     // every warp has stored its rows of T(k-1) and is done with the plane C(k)
-    if (!wait_or_abort(S.tbar, cs.n_use & 1u, P.wait_limit, S.abort)) return false;
+    if (!warp_wait(S.tbar, cs.n_use & 1u, P.wait_limit, S.abort)) return false;
     // Every warp has therefore finished step k-1, ring rows included (those read their plane after the
     // arrive): the stage of plane k-1 can take plane k-1 + stages.
     // When this item has no such plane left, the stage takes a plane of the CTA's next item (thread 0 knows
@@ -491,7 +482,7 @@ lattice_march_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   S.full = S.tbuf + 2 * kMarchTBytes;
   S.tbar = S.full + 8 * kMarchStages;
   S.abort = &ctl[1];
-  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(kAll, tid >> 5, 0), lane = tid & 31;
   const bool loader = warp == 0;  // the warp that asks for the planes
 
   if (tid == 0) {
@@ -607,7 +598,7 @@ star_march_kernel(const __grid_constant__ CUtensorMap tm, const MarchParams P, i
   extern __shared__ char dyn[];
   __shared__ int ctl[2];
   const unsigned buf = (smem_u32(dyn) + 1023u) & ~1023u, full = buf + kStarStages * kStarBytes, empty = full + 8 * kStarStages;
-  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, pi = lane >> 2, c4 = lane & 3;
+  const int tid = threadIdx.x, warp = __shfl_sync(kAll, tid >> 5, 0), lane = tid & 31, pi = lane >> 2, c4 = lane & 3;
   volatile int *abort = &ctl[1];
   if (tid == 0) {
     for (int s = 0; s < kStarStages; ++s) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, kMarchThreads / 32); }
@@ -642,7 +633,7 @@ star_march_kernel(const __grid_constant__ CUtensorMap tm, const MarchParams P, i
     auto refill = [&](int upto) {
       for (; ok && asked < min(upto, steps); ++asked) {
         if (n_iss >= (unsigned)kStarStages)
-          ok = __all_sync(0xffffffffu, wait_or_abort(empty + 8 * (n_iss % kStarStages), (n_iss / kStarStages - 1) & 1u, P.wait_limit, abort));
+          ok = warp_wait(empty + 8 * (n_iss % kStarStages), (n_iss / kStarStages - 1) & 1u, P.wait_limit, abort);
         if (ok) issue(asked);
       }
     };
@@ -664,7 +655,7 @@ star_march_kernel(const __grid_constant__ CUtensorMap tm, const MarchParams P, i
       const int k = zs - 1 + step;
       if (warp == 0) refill(step + kStarStages - 1);
       const unsigned st = n_use % kStarStages;
-      if (!ok || !wait_or_abort(full + 8 * st, (n_use / kStarStages) & 1u, P.wait_limit, abort)) { ok = false; break; }
+      if (!ok || !warp_wait(full + 8 * st, (n_use / kStarStages) & 1u, P.wait_limit, abort)) { ok = false; break; }
       ++n_use;
       const unsigned base = buf + st * kStarBytes + base0;
       float4 own[4], nb[8];
