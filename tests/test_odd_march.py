@@ -102,3 +102,24 @@ def test_widths_off_the_multiples_of_four(built_lib, dims, n_cols):
         np.testing.assert_array_equal(dh, d.cpu().numpy())
         plan.close()
         ref.close()
+
+
+# cross-sections of which the tiles find little, and widths of which the chunks do: the gather, and the same bits
+@pytest.mark.parametrize("dims,n_cols,marches", [((2, 2, 9000), 33, False), ((2, 2, 9000), 5, False), ((10, 10, 400), 47, False), ((4, 4, 500), 33, False),
+                                                 ((12, 6, 500), 18, False), ((12, 6, 500), 99, True), ((12, 6, 500), 13, True), ((20, 12, 90), 7, True),
+                                                 ((24, 24, 60), 18, True), ((9, 9, 250), 7, False), ((40, 33, 20), 35, True),
+                                                 ((20, 20, 20), 47, False), ((17, 17, 17), 33, False), ((40, 4, 9), 33, True)])
+def test_ragged_widths_on_thin_grids(built_lib, dims, n_cols, marches):
+    import torch
+    a = _csr(synth.laplacian(dims))
+    c = torch.from_numpy(synth.uniform(3, (int(np.prod(dims)), n_cols))).cuda()
+    out = []
+    for kw in ({}, dict(mode=api.MODE_UNFUSED, tile_slots=-1, lattice_march=-1)):
+        plan = api.Plan("spmm_spmm", a, n_cols=n_cols, **kw)
+        if not kw:
+            assert (plan.info()["threads"] == 128) == marches
+        out.append(torch.full_like(c, float("nan")))
+        plan.spmm_spmm(c, out[-1])
+        plan.status()
+        plan.close()
+    assert torch.equal(*out)

@@ -483,6 +483,23 @@ std::vector<int4> march_items_raw(const std::vector<tf::MarchItem> &items) {
 // the gather, whose reads of four columns are a quarter of that (5 columns at 100 x 90 x 110: 187 us there, 71 here).
 constexpr int kMarchMinRagged = 5;
 
+// Whether a width off the multiples of four marches on such a grid.  A tile of 16 x 8 points is marched through whatever the grid
+// has of it, and 16 columns whatever the width: from two chunks of columns on, what exists must be more than half of the points and two
+// fifths of points and columns together; one chunk, whose rows cost the gather a line each for a few columns, is ahead from 45 % of the
+// points on.  March and gather, us: 2 x 2 x 30 000, 33 columns (3 % of the points) 576 and 40; 10 x 10 x 1500 (39 %), 33 86 and 59, 5 40
+// and 36; 20 x 12 x 500 (47 %), 47 64 and 54, 5 32 and 34; 12 x 6 x 2000 (56 %), 18 (32 % with the columns) 49 and 40, 99 (50 %) 102 and
+// 110; 36 x 36 x 100 (68 %), 33 (46 %) 52 and 52; 24 x 24 x 300 (75 %), 18 (42 %) 47 and 46, 47 66 and 75.  Up to 16 384 rows the chain of
+// steps counts for more (20 x 20 x 20 (52 %), 99 25 and 20; 12 x 12 x 50 (56 %), 47 22 and 20; 12 x 16 x 20 (75 %), 33 19 and 20), except
+// on few planes, where launches are all that either takes (33 x 17 x 9 (49 %), 33 19 and 20; 18 x 11 x 4 (39 %) 19 and 20).
+bool ragged_march_pays(int nx, int ny, int nz, int n_cols) {
+  const long long chunks = (n_cols + tfk::kMarchCols - 1) / tfk::kMarchCols, rows = (long long)nx * ny * nz;
+  const long long tiles = (long long)((nx + tfk::kMarchW - 1) / tfk::kMarchW) * ((ny + tfk::kMarchH - 1) / tfk::kMarchH);
+  const double points = (double)nx * ny / ((double)tiles * tfk::kMarchW * tfk::kMarchH);
+  const double columns = (double)n_cols / ((double)chunks * tfk::kMarchCols);
+  if (nz <= 16 && rows * chunks <= 16384) return points > 1. / 3;
+  return chunks == 1 ? points >= 0.45 : points > (rows <= 16384 ? 0.6 : 0.5) && points * columns >= 0.4;
+}
+
 // Plane-marching executor: taken when both operators of an SpMM-SpMM chain are star stencils on the same
 // grid (lattice.cpp).  The general plan is built as well and serves calls whose operands are not 16-byte
 // aligned.
@@ -523,7 +540,7 @@ int build_march(tf_plan &p, const tf_csr *Fp, const tf_csr &A, int halo_rows, in
   // 40 and 28; 12 x 16 x 20 19.5 and 17.4.  (48 columns of the first take 142: the copy is 60 of the difference.  Marching to a padded D
   // that another launch crops: 318 at 47 columns.)
   const bool ragged = p.n_cols % 4 != 0;
-  if (ragged && (p.n_cols < kMarchMinRagged || halo_rows > 0 || !lf.full || !la.full)) return TF_OK;
+  if (ragged && (p.n_cols < kMarchMinRagged || halo_rows > 0 || !lf.full || !la.full || !ragged_march_pays(lf.nx, lf.ny, lf.nz, p.n_cols))) return TF_OK;
   if (halo_rows == 0 && (la.ghost_lo || la.ghost_hi)) return TF_OK;
   // with a neighbour rank below (above), the first operator must reach one plane of C below (above) the rank's
   // own: the boundary planes of T that the rank computes itself need them
