@@ -103,3 +103,20 @@ def test_intermediate(built_lib):
     _lib.check(_lib.lib().tf_spmm_dev(*(q.data_ptr() for q in one[:3]), n, p.value, 64, out.data_ptr(), torch.cuda.current_stream().cuda_stream))
     common.assert_close(out.cpu().numpy(), b.astype(np.float64) @ w.astype(np.float64), "T")
     plan.close()
+
+
+# thin grids, bricks of which much lies outside: an operator whose coefficients differ is left to the gather earlier
+@pytest.mark.parametrize("dims,k,n_cols,uniform,varying", [((5, 60_000), 256, 32, True, False), ((5, 60_000), 64, 64, True, True), ((9, 40_000), 256, 32, True, True),
+                                                           ((5, 4000), 256, 32, True, True), ((5, 2, 30_000), 256, 256, True, False),
+                                                           ((5, 5, 12_000), 80, 64, True, False), ((5, 6, 10_000), 64, 64, True, True),
+                                                           ((5, 5, 12_000), 24, 16, True, True), ((40, 40, 40), 96, 64, True, True)])
+def test_thin_grids(built_lib, dims, k, n_cols, uniform, varying):
+    t = synth.laplacian(dims)
+    n = len(t[0]) - 1
+    b, w = synth.uniform(3, (n, k)), synth.uniform(4, (k, n_cols))
+    for tr, one in ((t, uniform), (_varying(t), varying)):
+        plan = api.Plan("gemm_spmm", api.CSRMatrix(n, n, *tr), k=k, n_cols=n_cols)
+        assert (plan.info()["threads"] == 480) == one
+        rel, _ = common.assert_close(_run(plan, b, w), _scipy(tr, n) @ (b.astype(np.float64) @ w.astype(np.float64)), f"{dims} {k} {n_cols}")
+        assert rel < 2e-6, rel
+        plan.close()

@@ -880,15 +880,31 @@ int leave_intermediate(tf_plan &p, const float *C, cudaStream_t s) {
 // GeMM-SpMM in one launch (spmm_gemm.cu): star stencils with every neighbour stored, shapes of the tensor-core tile.  It adds up
 // rows of B, so B should not be much wider than the result: on flat grids it is ahead up to K = 8 N (700 000 points, 128 -> 16:
 // 126 us and 131, 256 -> 16: 216 and 210), on 3-D grids up to 1.5 N (1 M points, 128 -> 128: 290 and 382, 100 -> 64: 271 and 253,
-// 128 -> 64: 258 and 251, 64 -> 16: 124 and 106).  Small grids keep the executors they had: there is a launch or two to gain
-// (4 913 points in 3-D, 64 -> 64: 9.0 us and 15.3), and callers compare the march with the gather bit for bit on them.
+// 128 -> 64: 258 and 251, 64 -> 16: 124 and 106).  Small grids keep the executors they had, although a launch or two could be gained
+// there too (4 913 points in 3-D, 64 -> 64: 9.0 us and 15.3): the march and the gather behind the dense product give the same bits, which
+// (A B) W does not, and on such grids they are compared.
+// Where coefficients differ from row to row and bricks are cut off by a thin grid, the gather behind the dense product is ahead earlier: it
+// has no brick to fill, and reads the coefficients with the columns.  With e of the bricks' points in the grid (former and one launch, us):
+// flat, 5 x 100 000 (e = 0.63), K = 2 N 64 -> 32 105 and 103, 3 N 126 and 133, 8 N 256 -> 32 235 and 262; 9 x 50 000 (0.75), 8 N 210 and 198.
+// 3-D, 5 x 2 x 30 000, 256 -> 256 (e = 0.31) 308 and 480; 5 x 6 x 10 000 (0.47) 314 and 343; 17 x 5 x 4000 (0.53), 256 -> 256 359 and 341,
+// 320 -> 256 394 and 412; 5 x 6 x 10 000 (0.63), 160 -> 128 175 and 175, 192 -> 128 189 and 200; 9 x 9 x 4000 (0.68), 192 -> 128 208 and 202.
+// What launches cost counts for less on larger grids (5 x 20 000, 4 N 128 -> 32 44 and 40).  At 16 columns the dense product in front
+// computes as many for nothing: 5 x 6 x 10 000, 24 -> 16 56 and 47.
+double one_launch_depth(const tf::StarOp &op, const tf::BrickGrid &g, long long rows, int n_cols) {  // largest K / N
+  const bool flat = op.nz == 1;
+  const double e = (double)rows / ((double)g.bricks() * tf::kStarRows);
+  if (flat) return op.uniform || e > 0.7 ? 8. : std::min(8., 2. + (1 << 18) / (double)rows);
+  return op.uniform || n_cols <= 16 ? 1.5 : std::min(1.5, 4. * e - 1.1 + (1 << 14) / (double)rows);
+}
+
 int build_one_launch(tf_plan &p, const tf_csr &A) {
   if (p.ticket_sums || !tfk::tc_supported(p.k_dim, p.n_cols) || A.m < (1 << 12)) return TF_OK;
   tf::StarOp op;
   tf::analyse_star_operator(A.m, A.n, A.ap, A.ai, A.ax, op);
-  if (!op.nx || (op.nz == 1 ? p.k_dim > 8 * p.n_cols : 2 * p.k_dim > 3 * p.n_cols || A.m < (1 << 15))) return TF_OK;
+  if (!op.nx || (op.nz > 1 && A.m < (1 << 15))) return TF_OK;
   tf_plan::OneLaunch &O = p.one;
   if (!tf::choose_bricks(op, tfk::spmm_gemm_points(p.k_dim, p.n_cols), O.par.grid)) return TF_OK;
+  if (p.k_dim > one_launch_depth(op, O.par.grid, A.m, p.n_cols) * p.n_cols) return TF_OK;
   if (op.uniform) std::copy(op.coef.begin(), op.coef.end(), O.par.uniform);
   else TF_TRY(O.coef.upload(op.coef));
   O.par.coef = O.coef.p;
