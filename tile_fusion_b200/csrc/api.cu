@@ -897,14 +897,21 @@ double one_launch_depth(const tf::StarOp &op, const tf::BrickGrid &g, long long 
   return op.uniform || n_cols <= 16 ? 1.5 : std::min(1.5, 4. * e - 1.1 + (1 << 14) / (double)rows);
 }
 
-int build_one_launch(tf_plan &p, const tf_csr &A) {
-  if (p.ticket_sums || !tfk::tc_supported(p.k_dim, p.n_cols) || A.m < (1 << 12)) return TF_OK;
-  tf::StarOp op;
+bool one_launch_pays(const tf_plan &p, const tf_csr &A, tf::StarOp &op, tf::BrickGrid &grid) {
+  if (p.ticket_sums || !tfk::tc_supported(p.k_dim, p.n_cols) || A.m < (1 << 12)) return false;
   tf::analyse_star_operator(A.m, A.n, A.ap, A.ai, A.ax, op);
-  if (!op.nx || (op.nz > 1 && A.m < (1 << 15))) return TF_OK;
+  return op.nx && (op.nz == 1 || A.m >= (1 << 15)) && tf::choose_bricks(op, tfk::spmm_gemm_points(p.k_dim, p.n_cols), grid) &&
+         p.k_dim <= one_launch_depth(op, grid, A.m, p.n_cols) * p.n_cols;
+}
+
+int build_one_launch(tf_plan &p, const tf_csr &A) {
+  tf::StarOp op;
   tf_plan::OneLaunch &O = p.one;
-  if (!tf::choose_bricks(op, tfk::spmm_gemm_points(p.k_dim, p.n_cols), O.par.grid)) return TF_OK;
-  if (p.k_dim > one_launch_depth(op, O.par.grid, A.m, p.n_cols) * p.n_cols) return TF_OK;
+  if (!one_launch_pays(p, A, op, O.par.grid)) return TF_OK;
+  if (p.mode == TF_MODE_UNFUSED) {  // what runs in one launch otherwise, in two: only the order of the sums
+    p.one_sums = true;
+    return TF_OK;
+  }
   if (op.uniform) std::copy(op.coef.begin(), op.coef.end(), O.par.uniform);
   else TF_TRY(O.coef.upload(op.coef));
   O.par.coef = O.coef.p;
@@ -926,12 +933,7 @@ int build_one_launch(tf_plan &p, const tf_csr &A) {
 // (Rows of B that do not start on 16-byte boundaries would be gathered value by value; then B C comes first.  So it does
 // on grids and bands: with a handful of nonzeros a row there is little to choose, and every consumer gives the same bits.)
 int make_gemm_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &A, const tf_plan_opts &o, bool tiled, int sm_count, tf_plan **out) {
-  if (p->mode == TF_MODE_UNFUSED) {  // what runs in one launch otherwise, in two
-    p->one.on = false;
-    p->spmm_first = p->one_sums = true;
-  } else {
-    p->spmm_first = !tiled && !p->ticket_sums && p->k_dim % 4 == 0 && p->k_dim < p->n_cols;
-  }
+  p->spmm_first = p->one_sums || (!tiled && !p->ticket_sums && p->k_dim % 4 == 0 && p->k_dim < p->n_cols);
   const int width = p->spmm_first ? p->k_dim : p->n_cols;
   p->ld_t = (width + 3) / 4 * 4;
   const size_t wn = (size_t)tfk::row_gemm_pad_n(p->n_cols) * tfk::row_gemm_pad_k(p->k_dim);
@@ -1139,7 +1141,7 @@ int make_chain_plan(int chain, const tf_csr *A, const tf_csr *B, int k_dim, int 
     bool whole = o.mode == TF_MODE_UNFUSED;
     if (!whole) TF_TRY(keeps_whole((size_t)A->m * n_cols * sizeof(float), whole));
     if (whole && ct.tiled && o.lattice_march >= 0) TF_TRY(build_one_launch(*p, *A));
-    if (whole && (o.mode == TF_MODE_STREAM || p->one.on)) return make_gemm_gather_plan(p, *A, o, ct.tiled, sm_count, out);
+    if (whole && (o.mode == TF_MODE_STREAM || p->one_sums)) return make_gemm_gather_plan(p, *A, o, ct.tiled, sm_count, out);
   }
   rc = p->second.upload(*A);
   if (rc == TF_OK && F && F != A) rc = p->first.upload(*F);
