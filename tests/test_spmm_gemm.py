@@ -120,3 +120,14 @@ def test_thin_grids(built_lib, dims, k, n_cols, uniform, varying):
         rel, _ = common.assert_close(_run(plan, b, w), _scipy(tr, n) @ (b.astype(np.float64) @ w.astype(np.float64)), f"{dims} {k} {n_cols}")
         assert rel < 2e-6, rel
         plan.close()
+
+
+def test_rows_of_the_intermediate(built_lib):
+    """A plan that keeps no intermediate says so."""
+    t = synth.laplacian((80, 70))
+    n = len(t[0]) - 1
+    plan = api.Plan("gemm_spmm", api.CSRMatrix(n, n, *t), k=32, n_cols=64)
+    assert plan.info()["intermediate_rows"] == 0
+    _lib.check(_lib.lib().tf_plan_intermediate(plan._h, None, None, None))
+    assert plan.info()["intermediate_rows"] == n
+    plan.close()

@@ -944,7 +944,7 @@ int make_gemm_gather_plan(std::unique_ptr<tf_plan> &p, const tf_csr &A, const tf
   if (rc == TF_OK) rc = zero_state(*p);
   if (rc != TF_OK) return rc;
   make_gather_pieces(*p, 16);
-  p->hp.inter_rows = p->m;
+  p->hp.inter_rows = p->one.on ? 0 : p->m;
   p->hp.n_cons = p->g_second.n_units;
   if (tiled && o.lattice_march >= 0 && p->n_cols % 4 == 0 && !p->one.on && !p->one_sums) {
     rc = build_march(*p, nullptr, A, 0, sm_count, {}, true);
@@ -1880,6 +1880,7 @@ int tf_plan_intermediate(tf_plan *p, float **dev_ptr, long long *rows, int *cols
       p->hp.inter_rows = p->m;
     } else if (p->one.on) {
       TF_TRY(p->inter.alloc((size_t)(p->m + 1) * p->ld_t));
+      p->hp.inter_rows = p->m;
     }
     p->keep_t = true;
   }
