@@ -195,14 +195,16 @@ _torch = None
 
 
 def _stream_ptr():
-    """The current stream of the current device, as torch.cuda.current_stream() gives it (which takes 3 us to say so)."""
+    """The current stream of the current device, as torch.cuda.current_stream() gives it (which takes 3 us to say so, and is asked where
+    torch has no entry that says it at once)."""
     global _torch
     if _torch is None:
         import torch
         _torch = torch
-    if not _torch.cuda.is_initialized():
+    raw = getattr(_torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None or not _torch.cuda.is_initialized():
         return _torch.cuda.current_stream().cuda_stream
-    return _torch._C._cuda_getCurrentRawStream(_torch._C._cuda_getDevice())
+    return raw(_torch.cuda.current_device())
 
 
 class Plan:
