@@ -4,6 +4,12 @@
 #include <cuda_runtime.h>
 
 namespace tfk {
+// cuTensorMapEncodeTiled, looked up in the driver once; null where it has none.
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_fn();
+
 constexpr int kTcRowsHost = 128;  // rows per tensor-core tile (= kTcRows)
 // dynamic shared memory of one K slice for width n: B hi/lo (2 x 16 KB), W hi/lo (2 x n x 128 B), alignment slack
 inline int tc_smem_bytes_host(int n) { return 2 * 128 * 128 + 2 * n * 128 + 1024; }

@@ -38,6 +38,7 @@
 
 #include <algorithm>
 
+#include "gemm_tc_host.h"
 #include "lattice_march.h"
 
 namespace tfk {
@@ -698,21 +699,6 @@ star_march_kernel(const __grid_constant__ CUtensorMap tm, const MarchParams P, i
       __threadfence();
     }
   }
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = [] {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess
-               ? (EncodeTiledFn)p
-               : (EncodeTiledFn) nullptr;
-  }();
-  return fn;
 }
 
 int march_make_map(CUtensorMap *out, const float *c, int n_cols, int nx, int ny, int lines, long long planes, int box_lines) {

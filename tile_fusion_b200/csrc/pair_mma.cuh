@@ -73,7 +73,7 @@ __device__ __forceinline__ void split_pair(float x, float round_low, float &hi, 
   lo = (x - __uint_as_float(h & 0xffffe000u)) * round_low;
 }
 
-// 32 (16) columns of a warp's 32 tensor-memory lanes.  The registers hold them after tcgen05.wait::ld only: tmem_loaded keeps the
+// 32 columns of a warp's 32 tensor-memory lanes.  The registers hold them after tcgen05.wait::ld only: tmem_loaded keeps the
 // compiler from using them before.
 __device__ __forceinline__ void tmem_load32(float (&v)[32], unsigned taddr) {
   asm volatile(
@@ -86,18 +86,9 @@ __device__ __forceinline__ void tmem_load32(float (&v)[32], unsigned taddr) {
         "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
       : "r"(taddr) : "memory");
 }
-__device__ __forceinline__ void tmem_load16(float (&v)[16], unsigned taddr) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
-        "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
-      : "r"(taddr) : "memory");
-}
-template <int C>
-__device__ __forceinline__ void tmem_loaded(float (&v)[C]) {
+__device__ __forceinline__ void tmem_loaded(float (&v)[32]) {
 #pragma unroll
-  for (int i = 0; i < C; ++i) asm volatile("" : "+f"(v[i]));
+  for (int i = 0; i < 32; ++i) asm volatile("" : "+f"(v[i]));
 }
 
 }  // namespace tfk

@@ -407,19 +407,9 @@ bool fit(int K, int n, const tf::BrickGrid &g, int &stages, int &raws, size_t &s
   return stages >= 2 && raws >= 2;
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 // B as (column, x, y, z), boxes of 32 columns x bx x by x bz points.
 int points_map(CUtensorMap *out, const float *b, int K, const tf::BrickGrid &g, int bx, int by, int bz) {
-  static EncodeTiledFn fn = [] {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess
-               ? (EncodeTiledFn)p
-               : (EncodeTiledFn) nullptr;
-  }();
+  EncodeTiledFn fn = encode_fn();
   if (!fn) return tf::fail(TF_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
   const cuuint64_t row = (cuuint64_t)K * 4;
   cuuint64_t gdim[4] = {(cuuint64_t)K, (cuuint64_t)g.nx, (cuuint64_t)g.ny, (cuuint64_t)g.nz};
