@@ -545,6 +545,8 @@ def run_lattice_workload(name, args, ctx, headline):
         kernel = "spmm_gemm_kernel"
     elif chain == "gemm_spmm" and args.mode == "stream" and world == 1:
         kernel = "row_gemm_kernel (dense product) + gather_kernel"
+    elif chain == "gemm_spmm" and world == 1 and threads == 256:  # (unfused: the sums of the one launch in two passes)
+        kernel = "gather_kernel + row_gemm_kernel (dense product)"
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": None, "peak_source": f"of {peak_kind}", "algorithmic_bytes_per_launch": bytes_local,
                 "kernel": kernel + (" (persistent fused executor)" if "+" not in kernel else " (two launches per step)"),

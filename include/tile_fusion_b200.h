@@ -106,7 +106,9 @@ typedef struct {
 typedef enum {
   TF_MODE_STREAM = 0,   /* one persistent launch; the intermediate lives in an L2-sized ring */
   TF_MODE_SCHEDULE = 1, /* follow a reference-format schedule tile by tile (two waves)       */
-  TF_MODE_UNFUSED = 2   /* two full passes, intermediate through HBM (self-check baseline)   */
+  TF_MODE_UNFUSED = 2   /* two full passes, intermediate through HBM (self-check baseline): B W, then A T; but A B first
+                           where a GeMM-SpMM plan of more than 128 columns runs in one launch otherwise (see lattice_march),
+                           so that both modes give the same bits there.  With lattice_march < 0 it is B W always */
 } tf_exec_mode;
 
 typedef struct {
@@ -141,6 +143,10 @@ typedef struct {
                              0 = run the plane-marching kernel, which keeps the intermediate in shared memory,
                              <0 = never (general CSR path).  GeMM-SpMM plans on such an operator use the same
                              kernel as the consumer of the dense product's rows (0) or the balanced gather (<0).
+                             GeMM-SpMM plans with K % 4 == 0 and N % 16 == 0 on a large enough 2-D or 3-D grid, every
+                             neighbour stored, and K not much above N, run in one launch as (A B) W (0); <0 keeps A (B W), in
+                             launches of their own.  (A B is formed first: |B| beyond 3.4e38 over the largest row sum of
+                             |A| overflows there, as |B W| beyond it does otherwise.)
                              The same switch covers the executors that march along the lines of a 2-D five-point operator
                              and down the blocks of a banded one. */
   int exchange;           /* tf_multi_plan only: 0 = halo rows are written by the copy engines straight into the
@@ -197,8 +203,8 @@ int tf_lattice_preview(const tf_csr *A, int halo_rows, int n_cols, int ctas, int
 int tf_plan_tile_info(const tf_plan *p, int info[8]);
 
 /* info[0] items, [1] producer blocks, [2] consumer blocks, [3] ring rows (0 = full-size
- * intermediate), [4] grid CTAs, [5] threads per CTA, [6] kernels launched by the last call,
- * [7] intermediate rows allocated. */
+ * intermediate), [4] grid CTAs, [5] threads per CTA (256 for the balanced gather and the SDDMM, whatever their launches take),
+ * [6] kernels launched by the last call, [7] intermediate rows allocated. */
 int tf_plan_info(const tf_plan *p, long long info[8]);
 /* Number of polls (each followed by a short sleep) after which an in-kernel wait on another
  * block's completion gives up, sets the plan's error status and lets the kernel return.

@@ -1,5 +1,5 @@
-"""The plane-marching kernel on 3-D grids with an odd x extent: the pair behind the last point of a line, and the last line of
-the last plane, are patched up in shared memory.  Bit for bit the CSR products."""
+"""The plane-marching kernel on 3-D grids with an odd x extent and on widths off the multiples of four: the points with even and with odd x come
+through maps of their own, and rows of T that do not exist are zero.  Bit for bit the CSR products."""
 import numpy as np
 import pytest
 

@@ -41,7 +41,7 @@ int analyse_lattice_operator(int m, int ncols, const int *ap, const int *ai, con
   out = LatticeOp();
   const Lattice L = detect_lattice(m, ap, ai);
   if (L.dims != 3 || L.nx < 2 || L.ny < 2) return TF_OK;
-  const bool odd = L.nx % 2 != 0;  // (the executor reads x in pairs and patches up the point behind the last one)
+  const bool odd = L.nx % 2 != 0;  // (the executor then reads the points with even and with odd x apart)
   if (odd && !(allow_odd && halo_rows == 0 && m == ncols)) return TF_OK;
   const long long plane = (long long)L.nx * L.ny;
   if (plane <= L.nx || m % plane != 0) return TF_OK;

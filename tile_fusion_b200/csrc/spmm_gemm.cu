@@ -14,8 +14,8 @@
 // What bounds it on 3-D grids is shared memory (per slice, K = N = 256: 768 cycles of the tensor core's reads, 960 of the
 // sparse product's, 560 of the copies', of 2 400), on flat grids memory and the latency of a round of bricks.
 // Against the dense product and the march or gather of their own launches, us: 65 536 points flat, 64 -> 64: 12.6 and 27;
-// 700 000 flat, 32 -> 256: 156 and 513, 128 -> 128: 165 and 313, 256 -> 64: 233 and 286; 1 M in 3-D, 64 -> 64: 142 and 193,
-// 256 -> 256: 700 and 910; 561 661 in 3-D, 100 -> 64: 157 and 154, 256 -> 16: 265 and 161 (see build_one_launch).
+// 700 000 flat, 32 -> 256: 156 and 513, 128 -> 128: 155 and 303, 256 -> 64: 226 and 280; 1 M in 3-D, 64 -> 64: 142 and 193,
+// 256 -> 256: 646 and 910; 561 661 in 3-D, 100 -> 64: 157 and 154, 256 -> 16: 265 and 161 (see one_launch_depth).
 // (Tried: rows gathered by nonzeros into registers, two CTAs of eight warps in turns of everything: 440 us instead of 233 at
 // 700 000 points, 256 -> 64; rows listed and copied by a warp's cp.async: 619; four warps to a slice with 4 x 2 points to a group: 235, on
 // 3-D grids 178 instead of 160.)
