@@ -143,9 +143,9 @@ typedef struct {
                              0 = run the plane-marching kernel, which keeps the intermediate in shared memory,
                              <0 = never (general CSR path).  GeMM-SpMM plans on such an operator use the same
                              kernel as the consumer of the dense product's rows (0) or the balanced gather (<0).
-                             GeMM-SpMM plans with K % 4 == 0 and N % 16 == 0 on a large enough 2-D or 3-D grid, every
-                             neighbour stored, and K not much above N, run in one launch as (A B) W (0); <0 keeps A (B W), in
-                             launches of their own.  (A B is formed first: |B| beyond 3.4e38 over the largest row sum of
+                             GeMM-SpMM plans with K % 4 == 0 and N % 16 == 0 on a 2-D grid (from 4 096 rows, K up to 8 N) or
+                             a 3-D one (from 32 768 rows, K up to 1.5 N; less on thin grids of differing coefficients), every
+                             neighbour stored, run in one launch as (A B) W (0); <0 keeps A (B W), in launches of their own.  (A B is formed first: |B| beyond 3.4e38 over the largest row sum of
                              |A| overflows there, as |B W| beyond it does otherwise.)
                              The same switch covers the executors that march along the lines of a 2-D five-point operator
                              and down the blocks of a banded one. */
